@@ -14,6 +14,22 @@ from . import _lib
 from ._lib import Q4Error, check, q4_qweight  # noqa: F401
 
 
+_native = None
+
+
+def _n():
+    """The wrappers' native half (csrc/q4_pyops.c): a call takes the tensors and returns the C ABI's status code."""
+    global _native
+    if _native is None:
+        _lib.lib()   # loads the shared library, loudly when it is missing
+        try:
+            from . import _q4ops
+        except ImportError as e:
+            raise RuntimeError("llama_cu_awq_b200/_q4ops.so is missing: build it with `python -m llama_cu_awq_b200.build`; there is no fallback path") from e
+        _native = _q4ops
+    return _native
+
+
 def _stream(stream=None):
     s = stream if stream is not None else torch.cuda.current_stream()
     return C.c_void_p(s.cuda_stream)
@@ -32,6 +48,7 @@ class QWeight:
         assert weight.is_cuda and weight.is_contiguous() and zeros.is_contiguous() and scales.is_contiguous()
         self.weight, self.zeros, self.scales = weight, zeros, scales
         self.c = q4_qweight(weight.data_ptr(), zeros.data_ptr(), scales.data_ptr())
+        self._addr = C.addressof(self.c)
 
     @classmethod
     def from_numpy(cls, d, device="cuda"):
@@ -44,29 +61,33 @@ class QWeight:
 
 
 def rmsnorm(o, x, weight, size, stream=None):
-    check(_lib.lib().q4_rmsnorm(_stream(stream), _p(o), _p(x), _p(weight), size), "rmsnorm")
+    if e := _n().rmsnorm(stream, o, x, weight, size):
+        check(e, "rmsnorm")
 
 
 def matmul(xout, x, w, inpSize, opSize, accum=False, gpu_count=1, loff=-1, pPos=None, alpha=1.0, stream=None):
     """matmul(): quantized form when `w` is a QWeight (llama2_q4.cu:367), fp16 form otherwise (:357)."""
     if isinstance(w, QWeight):
-        check(_lib.lib().q4_matmul_q4(_stream(stream), _p(xout), _p(x), w.ref, inpSize, opSize, int(bool(accum)), gpu_count, loff, _p(pPos)),
-              "matmul")
+        e = _n().matmul_q4(stream, xout, x, w, inpSize, opSize, accum, gpu_count, loff, pPos)
     else:
-        check(_lib.lib().q4_matmul_f16(_stream(stream), _p(xout), _p(x), _p(w), inpSize, opSize, alpha), "matmul")
+        e = _n().matmul_f16(stream, xout, x, w, inpSize, opSize, alpha)
+    if e:
+        check(e, "matmul")
 
 
 def qkv_matvec(q, key_cache, value_cache, x, qw, kw, vw, inpSize, opSize, loff, pPos, kvSize=None, stream=None):
-    check(_lib.lib().q4_qkv_matvec(_stream(stream), _p(q), _p(key_cache), _p(value_cache), _p(x), qw.ref, kw.ref, vw.ref, inpSize, opSize,
-                                   opSize if kvSize is None else kvSize, loff, _p(pPos)), "qkv_matvec")
+    if e := _n().qkv_matvec(stream, q, key_cache, value_cache, x, qw, kw, vw, inpSize, opSize, opSize if kvSize is None else kvSize, loff, pPos):
+        check(e, "qkv_matvec")
 
 
 def ffn_matvec_silu(xout, x, gate_w, up_w, inpSize, opSize, stream=None):
-    check(_lib.lib().q4_ffn_matvec_silu(_stream(stream), _p(xout), _p(x), gate_w.ref, up_w.ref, inpSize, opSize), "ffn_matvec_silu")
+    if e := _n().ffn_matvec_silu(stream, xout, x, gate_w, up_w, inpSize, opSize):
+        check(e, "ffn_matvec_silu")
 
 
 def RoPERotation(q, k, num_heads, num_kv_heads, head_size, pPos, loff, rope_theta, stream=None):
-    check(_lib.lib().q4_rope(_stream(stream), _p(q), _p(k), num_heads, num_kv_heads, head_size, _p(pPos), loff, rope_theta), "RoPERotation")
+    if e := _n().rope(stream, q, k, num_heads, num_kv_heads, head_size, pPos, loff, rope_theta):
+        check(e, "RoPERotation")
 
 
 def attention_scratch(num_heads, head_size, device="cuda"):
@@ -76,24 +97,25 @@ def attention_scratch(num_heads, head_size, device="cuda"):
 
 def MultiHeadAttention(output, q, key_cache, value_cache, att, num_heads, head_size, kv_mul, max_seq_len, pPos, stream=None):
     """`att` is the scratch buffer from attention_scratch() (the reference passes its score buffer there)."""
-    check(_lib.lib().q4_attention(_stream(stream), _p(output), _p(q), _p(key_cache), _p(value_cache), _p(att), num_heads, head_size, kv_mul,
-                                  max_seq_len, _p(pPos)), "MultiHeadAttention")
+    if e := _n().attention(stream, output, q, key_cache, value_cache, att, num_heads, head_size, kv_mul, max_seq_len, pPos):
+        check(e, "MultiHeadAttention")
 
 
 def copy_embedding(x, table, dim, tokens_ptr, pPos, stream=None):
-    check(_lib.lib().q4_embed(_stream(stream), _p(x), _p(table), dim, C.c_void_p(tokens_ptr), _p(pPos)), "copy_embedding")
+    if e := _n().embed(stream, x, table, dim, tokens_ptr, pPos):
+        check(e, "copy_embedding")
 
 
 def sample_greedy(logits, size, tokens_ptr, pos_pinned_ptr, pos_dev, gen_token, stream=None):
     """Greedy branch of sample() (sampler.h:77-84): tokens/pos pointers are pinned host addresses."""
-    check(_lib.lib().q4_argmax(_stream(stream), _p(logits), size, C.c_void_p(tokens_ptr), C.c_void_p(pos_pinned_ptr), _p(pos_dev),
-                               int(bool(gen_token))), "sample")
+    if e := _n().argmax(stream, logits, size, tokens_ptr, pos_pinned_ptr, pos_dev, gen_token):
+        check(e, "sample")
 
 
 def sample_topp(logits, size, temperature, topp, coin, tokens_ptr, pos_pinned_ptr, pos_dev, stream=None):
     """Non-greedy branch of sample() (sampler.h:85-115): logits become probabilities, the token goes to the mailbox."""
-    check(_lib.lib().q4_sample_topp(_stream(stream), _p(logits), size, temperature, topp, coin, C.c_void_p(tokens_ptr),
-                                    C.c_void_p(pos_pinned_ptr), _p(pos_dev)), "sample")
+    if e := _n().sample_topp(stream, logits, size, temperature, topp, coin, tokens_ptr, pos_pinned_ptr, pos_dev):
+        check(e, "sample")
 
 
 def dequant(w, K, N, stream=None):
@@ -126,8 +148,8 @@ class BatchedMatmul:
 
     def __call__(self, y, x, rows, stream=None):
         assert rows <= self.max_rows
-        check(_lib.lib().q4_matmul_q4_batched(_stream(stream), _p(y), _p(x), self.w.ref, _p(self.wi), rows, self.K, self.N, _p(self.ws), self.ws_bytes),
-              "matmul_batched")
+        if e := _n().matmul_q4_batched(stream, y, x, self.w, self.wi, rows, self.K, self.N, self.ws, self.ws_bytes):
+            check(e, "matmul_batched")
 
     def status(self, stream=None):
         return _lib.lib().q4_matmul_q4_batched_status(_stream(stream), _p(self.ws))
@@ -135,15 +157,17 @@ class BatchedMatmul:
 
 def matmul_rows(y, x, w, rows, inpSize, opSize, residual=None, residual_scale=1.0, stream=None):
     """matmul(QWeight) for 1..16 rows (q4_matmul_q4_rows): y[m] = x[m] * deq(w) [+ residual[m] * residual_scale]."""
-    check(_lib.lib().q4_matmul_q4_rows(_stream(stream), _p(y), _p(x), w.ref, rows, inpSize, opSize, _p(residual), residual_scale), "matmul_rows")
+    if e := _n().matmul_rows(stream, y, x, w, rows, inpSize, opSize, residual, residual_scale):
+        check(e, "matmul_rows")
 
 
 def qkv_matmul_rows(q, k, v, x, qw, kw, vw, rows, inpSize, opSize, kvSize, stream=None):
     """qkv_matvec for 1..16 rows (q4_qkv_matmul_rows); K and V rows land in plain [rows][kvSize] buffers."""
-    check(_lib.lib().q4_qkv_matmul_rows(_stream(stream), _p(q), _p(k), _p(v), _p(x), qw.ref, kw.ref, vw.ref, rows, inpSize, opSize, kvSize),
-          "qkv_matmul_rows")
+    if e := _n().qkv_matmul_rows(stream, q, k, v, x, qw, kw, vw, rows, inpSize, opSize, kvSize):
+        check(e, "qkv_matmul_rows")
 
 
 def ffn_silu_rows(h, x, gate_w, up_w, rows, inpSize, opSize, stream=None):
     """ffn_matvec_silu for 1..16 rows (q4_ffn_silu_rows)."""
-    check(_lib.lib().q4_ffn_silu_rows(_stream(stream), _p(h), _p(x), gate_w.ref, up_w.ref, rows, inpSize, opSize), "ffn_silu_rows")
+    if e := _n().ffn_silu_rows(stream, h, x, gate_w, up_w, rows, inpSize, opSize):
+        check(e, "ffn_silu_rows")
