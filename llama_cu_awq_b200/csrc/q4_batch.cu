@@ -473,19 +473,31 @@ __global__ void __launch_bounds__(256) matvec_f16_rows_kernel(__half* y, const _
     }
 }
 
-// The same product on mma.sync m16n8k16 when the shapes allow (n % 32 == 0, d % 16 == 0): a warp takes 16 classifier rows
-// and the whole of n. The k index of an MMA is only a summation label, so thread (g, t) feeds the eight consecutive
-// weights it loaded with one 16-byte load (rows g and g + 8, inputs 32 c + 8 t ..) as A and the same eight inputs of batch
-// row g as B - no shuffles, no shared memory; fp32 accumulation over the whole row as mat_vec_kernel does.
+// The same product on mma.sync m16n8k16 when the shapes allow (n % 32 == 0, d % 16 == 0): a CTA takes 16 classifier rows, its
+// eight warps an eighth of n each, and the warps' partial tiles are added in warp order (bit-reproducible). The k index of
+// an MMA is only a summation label, so thread (g, t) feeds the eight consecutive weights it loaded with one 16-byte load
+// (rows g and g + 8, inputs 32 c + 8 t ..) as A and the same eight inputs of batch row g as B; fp32 accumulation as in
+// mat_vec_kernel. HBM-bound when all SMs stream: with a warp over the whole of n and 128 rows per CTA, a rank's or a small
+// model's few thousand rows left most SMs idle (4000 x 4096, 8 rows: 70 us; one 16-row tile per CTA: 18 us).
+constexpr int kClsWarps = 8;
 template <int NT>
-__global__ void __launch_bounds__(256) classifier_rows_kernel(__half* y, const __half* x, const __half* w, int n, int d, int B, int y_stride) {
-    griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
-    griddep_launch_dependents();
+__global__ void __launch_bounds__(kClsWarps * 32) classifier_rows_kernel(__half* y, const __half* x, const __half* w, int n, int d, int B, int y_stride) {
+    __shared__ float part[kClsWarps][NT][4][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int tile = blockIdx.x * 8 + warp;
-    if (tile * 16 >= d) return;
+    const int chunks = n / 32, c_begin = chunks * warp / kClsWarps, c_end = chunks * (warp + 1) / kClsWarps;
+    const int tile = blockIdx.x;
     const uint4* wa = reinterpret_cast<const uint4*>(w + (size_t)(tile * 16 + g) * n) + t;
     const uint4* wb = reinterpret_cast<const uint4*>(w + (size_t)(tile * 16 + g + 8) * n) + t;
+    constexpr int U = 4;
+    uint4 a[U], b[U];
+    auto fetch = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (c0 + u < c_end) { a[u] = ldg_stream(wa + 4 * (c0 + u)); b[u] = ldg_stream(wb + 4 * (c0 + u)); }
+    };
+    fetch(c_begin);   // the weights do not depend on the previous kernel: the first loads run while it finishes
+    griddep_wait();
+    griddep_launch_dependents();
     const uint4* xr[NT];
     bool ok[NT];
 #pragma unroll
@@ -496,22 +508,19 @@ __global__ void __launch_bounds__(256) classifier_rows_kernel(__half* y, const _
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-    const int chunks = n / 32;
-    constexpr int U = 4;
-    for (int c0 = 0; c0 < chunks; c0 += U) {
-        uint4 a[U], b[U];
+    for (int c0 = c_begin; c0 < c_end; c0 += U) {
+        uint4 ca[U], cb[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) { ca[u] = a[u]; cb[u] = b[u]; }
+        fetch(c0 + U);
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (c0 + u < chunks) { a[u] = ldg_stream(wa + 4 * (c0 + u)); b[u] = ldg_stream(wb + 4 * (c0 + u)); }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (c0 + u < chunks) {
+            if (c0 + u < c_end) {
 #pragma unroll
                 for (int nt = 0; nt < NT; nt++) {
                     uint4 xv = make_uint4(0, 0, 0, 0);
                     if (ok[nt]) xv = xr[nt][4 * (c0 + u)];
-                    const uint32_t A0[4] = {a[u].x, b[u].x, a[u].y, b[u].y}, A1[4] = {a[u].z, b[u].z, a[u].w, b[u].w};
+                    const uint32_t A0[4] = {ca[u].x, cb[u].x, ca[u].y, cb[u].y}, A1[4] = {ca[u].z, cb[u].z, ca[u].w, cb[u].w};
                     mma_f16(acc[nt], A0, xv.x, xv.y);
                     mma_f16(acc[nt], A1, xv.z, xv.w);
                 }
@@ -521,10 +530,16 @@ __global__ void __launch_bounds__(256) classifier_rows_kernel(__half* y, const _
 #pragma unroll
     for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int row = 8 * nt + 2 * t + (e & 1);
-            if (row < B) y[(size_t)row * y_stride + tile * 16 + g + 8 * (e >> 1)] = __float2half(acc[nt][e]);
-        }
+        for (int e = 0; e < 4; e++) part[warp][nt][e][lane] = acc[nt][e];
+    __syncthreads();
+    for (int i = threadIdx.x; i < NT * 128; i += kClsWarps * 32) {
+        const int l = i & 31, e = (i >> 5) & 3, nt = i >> 7;
+        const int row = 8 * nt + 2 * (l & 3) + (e & 1);
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < kClsWarps; k++) v += part[k][nt][e][l];
+        if (row < B) y[(size_t)row * y_stride + tile * 16 + (l >> 2) + 8 * (e >> 1)] = __float2half(v);
+    }
 }
 
 // argmax per row (lowest index among equal maxima, like q4_argmax) and the hand-off of batched decode: the id becomes
@@ -903,8 +918,8 @@ static int batch_step(q4_batch* b, cudaStream_t s) {
     __half* cls_out = m->g == 1 ? b->logits : b->part;   // TP: every rank computes its vocabulary slice of every row; the slices are gathered row by row
     const int cls_stride = m->g == 1 ? c.vocab_size : m->v_n;
     if (c.dim % 32 == 0 && m->v_n % 16 == 0) {
-        if (n <= 8) launch_rows(overlap, classifier_rows_kernel<1>, dim3(q4_div_up(m->v_n / 16, 8)), dim3(256), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
-        else launch_rows(overlap, classifier_rows_kernel<2>, dim3(q4_div_up(m->v_n / 16, 8)), dim3(256), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
+        if (n <= 8) launch_rows(overlap, classifier_rows_kernel<1>, dim3(m->v_n / 16), dim3(kClsWarps * 32), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
+        else launch_rows(overlap, classifier_rows_kernel<2>, dim3(m->v_n / 16), dim3(kClsWarps * 32), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
     } else {
         launch_rows(overlap, matvec_f16_rows_kernel, dim3(148 * 2), dim3(256), smem, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
     }
