@@ -55,6 +55,18 @@ def test_sample_topp_kernel(n, topp):
     assert same >= total // 2   # identical probabilities (and then the identical token) in most cases
 
 
+@pytest.mark.parametrize("n", [1, 127, 128, 1023, 1024, 1025, 43 * 1024 + 1, 1 << 18])   # edges of the 128-column slices, of the rows of 1024, largest
+@pytest.mark.parametrize("topp", [0.7, 1.0])
+def test_sample_topp_slice_edges(n, topp):
+    rng = np.random.default_rng(n)
+    logits = np.round(rng.standard_normal(n) * 4).astype(np.float16)   # few distinct values: long runs of equal probabilities
+    for coin in (0.0, 0.31, 0.9, 0.9999):
+        tok, p = Mailbox().run(logits, 1.0, topp, coin)
+        assert tok == select_float64(p, topp, coin), coin   # the rule applied to the kernel's own probabilities: exact
+    logits[n // 2] = np.nan
+    assert Mailbox().run(logits, 1.0, topp, 0.5)[0] == 0   # every probability is NaN: the first element of the order
+
+
 def test_sample_topp_threshold_never_reached():
     logits = np.zeros(4096, np.float16)
     logits[7] = np.float16(-20.0)
