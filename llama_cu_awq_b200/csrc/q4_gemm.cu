@@ -4,22 +4,29 @@
 // the batch-1 GEMV token by token (llama2_q4.cu:710-735, mat_vec_kernel_int4 gpu_kernels.h:179-248); M rows here are M
 // applications of that GEMV, and that is what the tests compare against.
 //
-// Swap-AB: the weights fill the 128-row M side of the MMA (tile = 128 output features), the batch is the MMA's N side
-// (16, 64 or 256 rows of X per tile), so small batches still use whole instructions: D[128 x MT] += A[128 x 16] * B[MT x 16]^T.
+// Swap-AB: the weights are the MMA's 256-row operand, the batch its N side (a multiple of 32 up to 256 rows of X per tile).
+// A pair of SMs (cluster of two, cta_group::2) works on one tile of 256 features x MT rows: each CTA dequantises its own 128
+// features and fetches half of the X tile, so X crosses the L2-to-SM path once per 256 features. The dequantised weights
+// never touch shared memory: the converters store them straight into tensor memory, from where the MMA reads them as
+// its A operand. Both follow from what bounded the kernel before (one CTA per tile, A staged in shared memory, 845
+// TFLOP/s at 2000 rows): 72 B per clock and SM of L2 reads for a 64 B port, and 200 B per clock of shared-memory traffic
+// (MMA operands, conversion stores, TMA writes) for 128 B. Now: 40 and 80.
 //
-// One CTA per SM, persistent over work units (feature tile, batch tile, K split), four roles:
-//   warp 0      weight producer: TMA (cp.async.bulk.tensor.2d, no multicast, this GPU's memory only) of packed weight chunks
-//               (128 features x 256 inputs = 128 B per row, 128-byte swizzle) into a staging ring
-//   warp 14     X producer: TMA of X tiles (MT x 64, 128-byte swizzle) straight into the (deep) B operand ring
-//   warps 2-9   converters: a warp takes every eighth 64-input block, reads its nibbles from the staging ring (conflict free
-//               thanks to the swizzle), dequantises them to fp16 in registers (LOP3 magic-number unpack, one exact
-//               subtract, one rounding multiply) and stores them into its own A operand stage in the K-major
-//               128-byte-swizzled layout the MMA descriptors describe
-//   warp 1      MMA: one elected thread issues tcgen05.mma.cta_group::1.kind::f16 (4 per 64-input stage) into a TMEM
-//               accumulator and tcgen05.commit's the stage back to the producer / converters
-//   warps 10-13 epilogue: tcgen05.ld the accumulator (lane = feature, column = batch row), convert, store
-// K is split over work units when there are fewer feature tiles than SMs; the partial sums go through an fp32 workspace
-// and the unit that arrives last adds them in split order (deterministic) and writes Y.
+// Persistent pairs; a pair takes an equal, contiguous share of all (tile, 256-input chunk) steps, so no wave is ever partly
+// empty (96 tiles of a 512-row QKV projection over 74 pairs would take two waves, 65 % busy). A tile cut by a share boundary
+// is summed through fp32 partial tiles in the workspace, always in K order, by whichever CTA arrives last.
+// Roles (512 threads; registers are moved from the first warpgroup to the epilogue):
+//   warp 0      TMA of packed weight chunks (128 features x 256 inputs = 128 B per row, 128-byte swizzle) into a staging ring
+//   warp 1      TMA of X slabs (MT / 2 rows x 64 inputs, 128-byte swizzle); both CTAs' copies report to the leader's barrier
+//   warp 2      leader CTA: one thread issues tcgen05.mma.cta_group::2.kind::f16 and commits the stages back to both CTAs
+//   warps 4-11  converters, two warpgroups on alternate 128-input blocks (= quantisation groups): a thread owns a feature
+//               row, reads 64 B of nibbles (conflict free thanks to the swizzle), dequantises in registers (LOP3 magic-number
+//               unpack, one exact subtract, one rounding multiply) and writes 64 tensor-memory columns (tcgen05.st)
+//   warps 12-15 epilogue: drain the accumulator into registers, release it, then scale / add / store while the next
+//               tile's MMAs run
+// Tensor memory: columns 0 .. MT - 1 accumulator, behind it as many A stages of 64 columns as fit (four at 256 rows, seven at
+// 64). A stage and the X slabs of the same 128 inputs form one ring entry: one wait and one commit per eight MMAs, because at
+// small MT the issuing warp's waits and commits are what bounds the kernel.
 //
 // Every wait is bounded by the global timer; on expiry the kernel records Q4_ERR_TIMEOUT in the workspace's status word,
 // lets all later waits fall through, waits (bounded) for its own copies in flight, frees its tensor memory and returns.
@@ -28,51 +35,39 @@
 
 #include <mutex>
 
-#include "q4_common.cuh"
+#include "q4_model.h"
 
 namespace {
 
-constexpr int kBN = 128;        // output features per tile = rows of the MMA
-constexpr int kBK = 64;         // inputs per pipeline stage (one 128-byte swizzle row of fp16)
+constexpr int kBN = 128;        // output features per CTA
+constexpr int kPairN = 256;     // per tile (two CTAs)
 constexpr int kChunkK = 256;    // inputs per packed-weight copy: 32 words = 128 B per feature row
-constexpr int kKbPerChunk = kChunkK / kBK;
-constexpr int kConvWarps = 8, kEpiWarps = 4;
-constexpr int kFirstConvWarp = 2, kFirstEpiWarp = kFirstConvWarp + kConvWarps;   // epilogue warps 10..13: warp % 4 covers the four TMEM lane quarters
-constexpr int kXWarp = kFirstEpiWarp + kEpiWarps;                // 14: X-tile producer
-constexpr int kGemmThreads = (kXWarp + 1) * 32;                  // 480
-constexpr int kAStageBytes = kBN * kBK * 2;                      // 16 KB
+constexpr int kBlockK = 128;    // inputs per A stage: one quantisation group
+constexpr int kSlabK = 64;      // inputs per X copy: one 128-byte swizzle row of fp16
+constexpr int kMaxMT = 256;
+constexpr int kMaxStages = 7, kAStageCols = kBlockK / 2, kTmemCols = 512;
+constexpr int kConvWarp0 = 4, kConvWarps = 8, kEpiWarp0 = 12, kEpiWarps = 4;
+constexpr int kGemmThreads = 512;
 constexpr int kPStageBytes = kBN * (kChunkK / 8) * 4;            // 16 KB
+constexpr int kRingBytes = 208 * 1024;                           // shared memory of the two rings
+constexpr int kOutRows = 32;                                     // rows of Y per staged store
+constexpr int kOutBytes = kOutRows * kBN * 2;                    // 8 KB, two buffers
+constexpr int kMaxP = 12;
 constexpr unsigned long long kGemmWaitNs = 300ULL * 1000 * 1000;   // limit of every device-side wait
-constexpr int kMaxStages = 16;
-
-template <int MT> struct GemmCfg {
-    // Converter warps = A operand stages (each warp owns one 16 KB stage). What is left of the 227 KB goes to the two rings
-    // that hide memory latency: X tiles (MT x 128 B each, from L2, about a microsecond) and packed-weight chunks (16 KB
-    // each, from HBM, about two microseconds); the converters hold up to kConverters blocks more in registers. The staging
-    // ring has an even length, so that a slot always serves the same four converter warps.
-    //              A stages     X ring          weight staging
-    //   MT = 16    8 (128 KB)   16 (32 KB)      4 (64 KB)
-    //   MT = 64    4 (64 KB)     8 (64 KB)      6 (96 KB)
-    //   MT = 256   4 (64 KB)     4 (128 KB)     2 (32 KB)    (bound by the tensor pipe, not by the conversion)
-    static constexpr int kConverters = MT <= 16 ? 8 : 4;
-    static constexpr int kBStages = MT >= 256 ? 4 : MT >= 64 ? 8 : 16;
-    static constexpr int kPStages = MT >= 256 ? 2 : MT >= 64 ? 6 : 4;
-    static constexpr int kBStageBytes = MT * kBK * 2;
-    static constexpr int kTmemCols = MT < 32 ? 32 : MT;                    // power of two >= 32
-    static constexpr size_t kSmemBytes = (size_t)kConverters * kAStageBytes + (size_t)kBStages * kBStageBytes + (size_t)kPStages * kPStageBytes + 1024;
-};
+enum GemmEpi { EPI_PLAIN = 0, EPI_RESIDUAL = 1, EPI_SILU = 2 };
 
 struct GemmParams {
     const uint32_t* zeros;
     const __half* scales;
-    __half* y;
-    const __half* residual;   // optional [M][N]: y = product + residual * residual_scale, rounded once (may alias y)
+    const __half* residual;   // EPI_RESIDUAL: [M][N], y = product + residual * residual_scale, rounded once (may alias y)
     float residual_scale;
-    float* partials;     // [feature tile][batch tile][split][MT][128] fp32, used when splits > 1
-    int* counters;       // [feature tile][batch tile]
+    float* partials;     // [pair][2 slots][2 CTAs][MT / 4][128][4] fp32
+    int* counters;       // [tile][2 CTAs]
     int* status;         // [0] error code, [1] where
     int M, K, N, G, PZ;
-    int n_tiles, m_tiles, splits, n_chunks, total_units;
+    int MT, m_tiles, n_chunks;
+    long long total_chunks;   // tiles * n_chunks
+    int stages, np, slab_bytes;   // operand stages (A in tensor memory, X in shared memory), weight copies in flight, bytes of an X slab
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -81,14 +76,31 @@ __device__ __forceinline__ unsigned long long gtimer() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// cluster address of the leader's copy of a barrier
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_addr(p)));
+    return r;
+}
 __device__ __forceinline__ void mb_init(uint64_t* b, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count)); }
 __device__ __forceinline__ void mb_expect_tx(uint64_t* b, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void mb_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory"); }
+__device__ __forceinline__ void mb_arrive_cluster(uint32_t addr) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory"); }
 __device__ __forceinline__ bool mb_try(uint64_t* b, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0,1,0,p; }" : "=r"(ok) : "r"(smem_addr(b)), "r"(parity) : "memory");
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0,1,0,p; }"
+                 : "=r"(ok) : "r"(smem_addr(b)), "r"(parity) : "memory");
     return ok != 0;
 }
 // Bounded wait: false when the limit is hit (the error is recorded) or an error is already on record.
@@ -106,34 +118,56 @@ __device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, int* statu
     if (atomicCAS(status, 0, Q4_ERR_TIMEOUT) == 0) status[1] = where;
     return false;
 }
+// the same for a whole warp; the result is warp-uniform
+__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, int* status, int where) { return __all_sync(0xffffffffu, mb_wait(b, parity, status, where)); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0,1,0,p; }" : "=r"(e));
+    return e != 0;
+}
+// after an error: gives a copy in flight up to 50 ms to land
+__device__ __forceinline__ void mb_drain(uint64_t* b, uint32_t parity) {
+    const unsigned long long t0 = gtimer();
+    while (!mb_try(b, parity) && gtimer() - t0 < 50ULL * 1000 * 1000) {}
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_addr(dst)),
                  "l"(map), "r"(smem_addr(bar)), "r"(x), "r"(y)
                  : "memory");
 }
+// into this CTA's shared memory, reporting to a barrier of either CTA of the pair (no multicast)
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_addr(dst)),
+                 "l"(map), "r"(bar), "r"(x), "r"(y)
+                 : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+// arrives on this barrier in both CTAs of the pair when the MMAs issued so far have completed
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)), "h"((uint16_t)3) : "memory");
 }
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// D[256 x N] (+)= A[256 x 16] (tensor memory, each CTA its 128 rows) * B[N x 16]^T (shared memory, each CTA half of the rows)
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-                   "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr));
+#define Q4_R8(v, i) "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]), "r"(v[i + 4]), "r"(v[i + 5]), "r"(v[i + 6]), "r"(v[i + 7])
+#define Q4_W8(v, i) "=r"(v[i]), "=r"(v[i + 1]), "=r"(v[i + 2]), "=r"(v[i + 3]), "=r"(v[i + 4]), "=r"(v[i + 5]), "=r"(v[i + 6]), "=r"(v[i + 7])
+#define Q4_RW8(v, i) "+r"(v[i]), "+r"(v[i + 1]), "+r"(v[i + 2]), "+r"(v[i + 3]), "+r"(v[i + 4]), "+r"(v[i + 5]), "+r"(v[i + 6]), "+r"(v[i + 7])
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+                 ::"r"(taddr), Q4_R8(v, 0), Q4_R8(v, 8), Q4_R8(v, 16), Q4_R8(v, 24) : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 : Q4_W8(v, 0), Q4_W8(v, 8), Q4_W8(v, 16), Q4_W8(v, 24) : "r"(taddr));
     // the registers are listed as operands of the wait, so that no use of them can be scheduled ahead of it
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]),
-                   "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
-                 :
-                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : Q4_RW8(v, 0), Q4_RW8(v, 8), Q4_RW8(v, 16), Q4_RW8(v, 24) : : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major operand tile [rows][64 halfs] stored with the 128-byte swizzle: rows of
@@ -144,327 +178,472 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ULL << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ULL << 46) | (2ULL << 61);
 }
 // Instruction descriptor, kind::f16: D fp32 (bits 4-5 = 1), A and B fp16 (0), both K-major (0), N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t umma_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBN >> 4) << 24); }
+__device__ __forceinline__ uint32_t umma_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kPairN >> 4) << 24); }
 
 // One packed word (8 nibbles) -> 8 fp16 weights in input order. INTERLEAVED: the word's nibbles hold inputs 0,2,4,6,1,3,5,7
 // (prepared by q4_gemm_interleave_weights), so the two mask patterns yield the pairs (0,1) (2,3) (4,5) (6,7) directly; the file
-// layout yields (0,4) (1,5) (2,6) (3,7) and needs four byte permutes. (q - z) is exact in fp16 (|q - z| <= 15), the
-// multiplication by the fp16 scale rounds once.
+// layout yields (0,4) (1,5) (2,6) (3,7) and needs four byte permutes. (q - z) is exact in fp16 (|q - z| <= 15; (w & 0x00F0) | 0x5400
+// is the half 64 + q), the multiplication by the fp16 scale rounds once.
 template <bool INTERLEAVED>
-__device__ __forceinline__ uint4 dequant8(uint32_t w, uint32_t zlo, uint32_t zhi, __half2 s2) {
-    const __half2 sixteenth = u2h2(0x2C002C00u);
-    const __half2 a = __hmul2(__hsub2(u2h2(lop3_and_or(w, 0x000F000Fu, 0x64006400u)), u2h2(zlo)), s2);
-    const __half2 b = __hmul2(__hfma2(u2h2(lop3_and_or(w, 0x00F000F0u, 0x64006400u)), sixteenth, u2h2(zhi)), s2);
+__device__ __forceinline__ void dequant8(uint32_t w, __half2 zlo, __half2 zhi, __half2 s2, uint32_t* o) {
+    const __half2 a = __hmul2(__hsub2(u2h2(lop3_and_or(w, 0x000F000Fu, 0x64006400u)), zlo), s2);
+    const __half2 b = __hmul2(__hsub2(u2h2(lop3_and_or(w, 0x00F000F0u, 0x54005400u)), zhi), s2);
     w >>= 8;
-    const __half2 c = __hmul2(__hsub2(u2h2(lop3_and_or(w, 0x000F000Fu, 0x64006400u)), u2h2(zlo)), s2);
-    const __half2 d = __hmul2(__hfma2(u2h2(lop3_and_or(w, 0x00F000F0u, 0x64006400u)), sixteenth, u2h2(zhi)), s2);
-    if (INTERLEAVED) return make_uint4(h22u(a), h22u(b), h22u(c), h22u(d));
-    // a = (0,4) b = (1,5) c = (2,6) d = (3,7)
-    return make_uint4(prmt(h22u(a), h22u(b), 0x5410), prmt(h22u(c), h22u(d), 0x5410), prmt(h22u(a), h22u(b), 0x7632), prmt(h22u(c), h22u(d), 0x7632));
+    const __half2 c = __hmul2(__hsub2(u2h2(lop3_and_or(w, 0x000F000Fu, 0x64006400u)), zlo), s2);
+    const __half2 d = __hmul2(__hsub2(u2h2(lop3_and_or(w, 0x00F000F0u, 0x54005400u)), zhi), s2);
+    if (INTERLEAVED) {
+        o[0] = h22u(a); o[1] = h22u(b); o[2] = h22u(c); o[3] = h22u(d);
+    } else {   // a = (0,4) b = (1,5) c = (2,6) d = (3,7)
+        o[0] = prmt(h22u(a), h22u(b), 0x5410); o[1] = prmt(h22u(c), h22u(d), 0x5410);
+        o[2] = prmt(h22u(a), h22u(b), 0x7632); o[3] = prmt(h22u(c), h22u(d), 0x7632);
+    }
 }
 
-struct UnitInfo { int tile, mt, split, c0, c1; };
-__device__ __forceinline__ UnitInfo unit_info(const GemmParams& p, int u) {
-    UnitInfo i;
-    i.split = u % p.splits;
-    const int t = u / p.splits;
-    i.mt = t % p.m_tiles;
-    i.tile = t / p.m_tiles;
-    i.c0 = (int)((long long)p.n_chunks * i.split / p.splits);
-    i.c1 = (int)((long long)p.n_chunks * (i.split + 1) / p.splits);
-    return i;
-}
+// A pair's share of the work, segment by segment: consecutive chunks of one tile.
+struct Segments {
+    long long c, end;
+    int n_chunks;
+    int tile, c0, c1;
+    __device__ __forceinline__ Segments(const GemmParams& p, int pair, int pairs) {
+        c = p.total_chunks * pair / pairs;
+        end = p.total_chunks * (pair + 1) / pairs;
+        n_chunks = p.n_chunks;
+    }
+    __device__ __forceinline__ bool next() {
+        if (c >= end) return false;
+        tile = (int)(c / n_chunks);
+        c0 = (int)(c - (long long)tile * n_chunks);
+        const long long left = end - c;
+        c1 = left < n_chunks - c0 ? c0 + (int)left : n_chunks;
+        c += c1 - c0;
+        return true;
+    }
+};
+// the pair whose share holds global chunk c
+__device__ __forceinline__ int pair_of(long long c, long long total, int pairs) { return (int)(((c + 1) * pairs - 1) / total); }
 
-// Every chunk is processed as four 64-input blocks, also the last chunk of a K that is not a multiple of 256: TMA fills
-// what lies outside the tensors with zeros on both operands, so the extra blocks add nothing. That keeps the pipeline
-// regular: block q of a CTA (counted over all its units) is converted by converter warp q % NC into operand stage
-// q % NC, which that warp alone ever fills - every barrier is then waited on by one party, phase after phase without
-// gaps (a parity wait cannot tell phase k from phase k + 2).
-template <int MT, bool INTERLEAVED>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-    using Cfg = GemmCfg<MT>;
-    constexpr int NC = Cfg::kConverters, NP = Cfg::kPStages, NB = Cfg::kBStages;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* sA = smem;
-    uint8_t* sB = sA + (size_t)NC * kAStageBytes;
-    uint8_t* sP = sB + (size_t)NB * Cfg::kBStageBytes;
-    __shared__ uint64_t full_p[kMaxStages], empty_p[kMaxStages], full_a[kMaxStages], empty_a[kMaxStages], full_b[kMaxStages], empty_b[kMaxStages], tmem_full,
-        tmem_empty;
-    __shared__ uint32_t s_tmem_base;
-    __shared__ int s_last;
+// silu(g) * u with the hardware's exponential and reciprocal (relative error near 1e-6, the result is rounded to fp16): four warps
+// evaluate 128 of them per thread and tile, and with expf and an IEEE division that took longer than the tile's MMAs.
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        for (int s = 0; s < kMaxStages; s++) {
-            mb_init(&full_p[s], 1); mb_init(&empty_p[s], kKbPerChunk);   // a chunk's four blocks go to four converter warps
-            mb_init(&full_a[s], 1); mb_init(&empty_a[s], 1); mb_init(&full_b[s], 1); mb_init(&empty_b[s], 1);
+// ---- epilogue pieces: 32 accumulator columns (= batch rows c0 .. c0 + 31 of the tile) of one feature, as 16 packed words ----
+template <int EPI>
+__device__ __forceinline__ void epi_pack(const float (&v)[32], const uint32_t* res, float rscale, uint32_t* out) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        float a = v[2 * j], b = v[2 * j + 1];
+        if (EPI == EPI_RESIDUAL) {
+            const float2 f = __half22float2(u2h2(res[j]));
+            a += f.x * rscale;
+            b += f.y * rscale;
         }
+        out[j] = h22u(__floats2half2_rn(a, b));
+    }
+}
+// The 32 rows of the chunk into the staging buffer [row][this CTA's outputs of a row] (two bytes per lane, 64 B per warp store).
+// EPI_SILU: features 2j and 2j + 1 are gate j and up j (rounded to fp16 like every GEMM result, silu and product in fp32:
+// gpu_kernels.h:278-281). Neighbouring lanes swap halves of a word so that the even lane holds the pair of the even row and the
+// odd lane that of the odd one.
+template <int EPI>
+__device__ __forceinline__ void epi_stage(const uint32_t* out, uint8_t* buf, int r) {
+    if (EPI == EPI_SILU) {
+        const bool odd = r & 1;
+        unsigned short* p = reinterpret_cast<unsigned short*>(buf) + (odd ? kBN / 2 : 0) + (r >> 1);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, out[j], 1);
+            const __half2 mine = u2h2(out[j]), theirs = u2h2(got);
+            const float gate = odd ? __high2float(theirs) : __low2float(mine), up = odd ? __high2float(mine) : __low2float(theirs);
+            p[j * kBN] = __half_as_ushort(__float2half(silu_mul(gate, up)));
+        }
+    } else {
+        unsigned short* p = reinterpret_cast<unsigned short*>(buf) + r;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            p[(2 * j) * kBN] = (unsigned short)(out[j] & 0xFFFFu);
+            p[(2 * j + 1) * kBN] = (unsigned short)(out[j] >> 16);
+        }
+    }
+}
+__device__ __forceinline__ void epi_load_residual(uint32_t* res, const __half* x, int c0, int rows, size_t ld) {
+    const unsigned short* p = reinterpret_cast<const unsigned short*>(x) + (size_t)c0 * ld;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        uint32_t a = 0, b = 0;
+        if (c0 + 2 * j < rows) a = *p;
+        p += ld;
+        if (c0 + 2 * j + 1 < rows) b = *p;
+        p += ld;
+        res[j] = a | (b << 16);
+    }
+}
+
+template <bool INTERLEAVED, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
+               const GemmParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sB = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sP = sB + (size_t)p.stages * 2 * p.slab_bytes;
+    __shared__ uint64_t full_p[kMaxP], empty_p[kMaxP], full[kMaxStages], empty[kMaxStages], tmem_full, tmem_empty, drained;
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_flag;
+
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    if (tid == 0) {
+        for (int s = 0; s < kMaxP; s++) { mb_init(&full_p[s], 1); mb_init(&empty_p[s], kConvWarps); }
+        for (int s = 0; s < kMaxStages; s++) { mb_init(&full[s], 9); mb_init(&empty[s], 1); }   // (four converter warps of each CTA, X copies)
         mb_init(&tmem_full, 1);
-        mb_init(&tmem_empty, kEpiWarps);
+        mb_init(&tmem_empty, 2 * kEpiWarps);
+        mb_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {   // tensor memory for the accumulator: the whole warp allocates, the address lands in shared memory
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem_base)), "r"(Cfg::kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (warp == 2) {   // all of the tensor memory, in both CTAs (one CTA per SM: nobody else holds any)
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem_base)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers and tensor memory are ready before either is touched from the other side
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t*)&s_tmem_base;
     // everything above overlaps the tail of the previous kernel on the stream (programmatic dependent launch); from here
     // on this kernel reads what that kernel wrote
     griddep_wait();
     griddep_launch_dependents();
+    Segments seg(p, pair, pairs);
 
-    if (warp == 0) {
-        // ===================== weight producer =====================
-        // keeps the packed-weight staging ring full: it waits only for free staging slots, so it runs ahead of the math and
-        // across unit boundaries
-        if (lane == 0) {
-            unsigned pit = 0;
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == 0 && lane == 0) {
+            // ===================== packed weights =====================
+            int ps = 0;
+            uint32_t ph = 1;
+            unsigned issued = 0;
             bool ok = true;
-            for (int u = blockIdx.x; u < p.total_units && ok; u += gridDim.x) {
-                const UnitInfo ui = unit_info(p, u);
-                for (int c = ui.c0; c < ui.c1; c++, pit++) {
-                    const int ps = pit % NP;
-                    if (!mb_wait(&empty_p[ps], ((pit / NP) & 1) ^ 1, p.status, 0x100)) { ok = false; break; }
+            while (ok && seg.next()) {
+                const int row = (seg.tile / p.m_tiles) * kPairN + rank * kBN;
+                for (int c = seg.c0; c < seg.c1; c++) {
+                    if (!mb_wait(&empty_p[ps], ph, p.status, 0x100)) { ok = false; break; }
                     mb_expect_tx(&full_p[ps], kPStageBytes);
-                    tma_load_2d(sP + (size_t)ps * kPStageBytes, &map_w, c * (kChunkK / 8), ui.tile * kBN, &full_p[ps]);
+                    tma_load_2d(sP + (size_t)ps * kPStageBytes, &map_w, c * (kChunkK / 8), row, &full_p[ps]);
+                    issued++;
+                    if (++ps == p.np) { ps = 0; ph ^= 1; }
                 }
             }
-            if (!ok) {   // after an error the newest copy of every ring position may still be in flight: give each up to 50 ms
-                for (unsigned i = pit > (unsigned)NP ? pit - NP : 0; i < pit; i++) {
-                    const unsigned long long t0 = gtimer();
-                    while (!mb_try(&full_p[i % NP], (i / NP) & 1) && gtimer() - t0 < 50ULL * 1000 * 1000) {}
-                }
-            }
-        }
-    } else if (warp == kXWarp) {
-        // ===================== X producer =====================
-        // loads the X tile of every 64-input block as soon as the MMA has released that slot of the (deep) B ring
-        if (lane == 0) {
-            unsigned q = 0;
+            if (!ok)   // the newest copy of every ring position may still be in flight
+                for (unsigned i = issued > (unsigned)p.np ? issued - p.np : 0; i < issued; i++) mb_drain(&full_p[i % p.np], (i / p.np) & 1);
+        } else if (warp == 1 && lane == 0) {
+            // ===================== X slabs =====================
+            int s = 0;
+            uint32_t ph = 1;
             bool ok = true;
-            for (int u = blockIdx.x; u < p.total_units && ok; u += gridDim.x) {
-                const UnitInfo ui = unit_info(p, u);
-                for (int kb = ui.c0 * kKbPerChunk; kb < ui.c1 * kKbPerChunk; kb++, q++) {
-                    const int s = q % NB;
-                    if (!mb_wait(&empty_b[s], ((q / NB) & 1) ^ 1, p.status, 0x200)) { ok = false; break; }
-                    mb_expect_tx(&full_b[s], Cfg::kBStageBytes);
-                    tma_load_2d(sB + (size_t)s * Cfg::kBStageBytes, &map_x, kb * kBK, ui.mt * MT, &full_b[s]);
+            const int half_rows = p.MT / 2;
+            while (ok && seg.next()) {
+                const int row = (seg.tile % p.m_tiles) * p.MT + rank * half_rows;
+                for (int b = seg.c0 * 2; b < seg.c1 * 2; b++) {   // 128-input blocks
+                    if (!mb_wait(&empty[s], ph, p.status, 0x200)) { ok = false; break; }
+                    if (rank == 0) mb_expect_tx(&full[s], 4 * p.slab_bytes);   // (the peer's bytes may be counted before: same phase)
+                    uint8_t* dst = sB + (size_t)s * 2 * p.slab_bytes;
+                    const uint32_t bar = leader_addr(&full[s]);
+                    tma_load_2d_pair(dst, &map_x, b * kBlockK, row, bar);
+                    tma_load_2d_pair(dst + p.slab_bytes, &map_x, b * kBlockK + kSlabK, row, bar);
+                    if (++s == p.stages) { s = 0; ph ^= 1; }
                 }
             }
-            if (!ok) {
-                for (unsigned i = q > (unsigned)NB ? q - NB : 0; i < q; i++) {
-                    const unsigned long long t0 = gtimer();
-                    while (!mb_try(&full_b[i % NB], (i / NB) & 1) && gtimer() - t0 < 50ULL * 1000 * 1000) {}
-                }
+            if (!ok) {   // an error: this CTA's copies report to the leader, whose barriers may never complete; both CTAs leave together
+                const unsigned long long t0 = gtimer();
+                while (gtimer() - t0 < 1000000ULL) {}   // a millisecond: far beyond a copy's flight time
             }
-        }
-    } else if (warp == 1) {
-        // ===================== MMA issuer =====================
-        // one thread does it all: the instructions are asynchronous, and at small batch tiles their issue rate is what
-        // bounds the kernel, so nothing else shares this warp's issue slots
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc(MT);
-            const uint64_t adesc0 = umma_desc(smem_addr(sA)), bdesc0 = umma_desc(smem_addr(sB));
-            unsigned q = 0, uit = 0;
+        } else if (warp == 2 && rank == 0) {
+            // ===================== MMA issuer =====================
+            // The whole warp walks the loop with warp-uniform values (descriptors and addresses then live in uniform registers) and
+            // one elected lane issues.
+            const uint32_t idesc = umma_idesc(p.MT);
+            const uint64_t bdesc0 = umma_desc(smem_addr(sB));
+            const bool issuer = elect_one();
+            int st = 0;
+            uint32_t ph = 0, pe = 1;
             bool ok = true;
-            for (int u = blockIdx.x; u < p.total_units && ok; u += gridDim.x, uit++) {
-                const UnitInfo ui = unit_info(p, u);
-                if (!mb_wait(&tmem_empty, (uit & 1) ^ 1, p.status, 0x300)) { ok = false; break; }   // the epilogue has drained the accumulator
-                const int nkb = (ui.c1 - ui.c0) * kKbPerChunk;
-                for (int i = 0; i < nkb; i++, q++) {
-                    const int s = q % NC, sb = q % NB;
-                    if (!mb_wait(&full_a[s], (q / NC) & 1, p.status, 0x400) || !mb_wait(&full_b[sb], (q / NB) & 1, p.status, 0x500)) { ok = false; break; }
+            while (ok && seg.next()) {
+                if (!warp_wait(&tmem_empty, pe, p.status, 0x300)) { ok = false; break; }   // both epilogues have drained the accumulator
+                pe ^= 1;
+                uint32_t accumulate = 0;
+                const int blocks = (seg.c1 - seg.c0) * (kChunkK / kBlockK);
+                for (int b = 0; b < blocks; b++) {
+                    if (!warp_wait(&full[st], ph, p.status, 0x400)) { ok = false; break; }
                     tc_fence_after();
-                    const uint64_t ad = adesc0 + (uint64_t)((s * kAStageBytes) >> 4), bd = bdesc0 + (uint64_t)((sb * Cfg::kBStageBytes) >> 4);
+                    if (issuer) {
+                        const uint32_t at = tmem_base + p.MT + st * kAStageCols;
+                        const uint64_t bd = bdesc0 + (uint64_t)((st * 2 * p.slab_bytes) >> 4);
 #pragma unroll
-                    for (int k16 = 0; k16 < kBK / 16; k16++) tc_mma_f16(tmem_base, ad + 2 * k16, bd + 2 * k16, idesc, (i == 0 && k16 == 0) ? 0u : 1u);
-                    tc_commit(&empty_a[s]);    // both arrive when these MMAs have read their operands
-                    tc_commit(&empty_b[sb]);
+                        for (int k16 = 0; k16 < kBlockK / 16; k16++)
+                            tc_mma_f16_pair(tmem_base, at + k16 * 8, bd + (k16 >= 4 ? p.slab_bytes >> 4 : 0) + 2 * (k16 & 3), idesc, k16 == 0 ? accumulate : 1u);
+                        tc_commit_pair(&empty[st]);   // arrives when these MMAs have read their operands
+                        if (b == blocks - 1) tc_commit_pair(&tmem_full);
+                    }
+                    __syncwarp();
+                    accumulate = 1;
+                    if (++st == p.stages) { st = 0; ph ^= 1; }
                 }
-                tc_commit(&tmem_full);
             }
+            if (!ok && issuer) {   // MMAs in flight read shared memory and report to both CTAs: let them finish
+                tc_commit_pair(&drained);
+                mb_drain(&drained, 0);
+            }
+            __syncwarp();
         }
-    } else if (warp < kFirstEpiWarp) {
+    } else if (warp < kEpiWarp0) {
         // ===================== converters =====================
-        // Warp w converts blocks q = w, w + NC, ...: a whole 128-feature x 64-input operand stage per block, four feature
-        // rows per lane, so that the fixed cost of a hand-over (barrier round trips, store drain) is paid once per 8192
-        // weights and NC blocks are in flight at once.
-        const int cw = warp - kFirstConvWarp;
-        if (cw < NC) {
-            const int sw = lane & 7;   // rows lane + 32 i share lane & 7, hence the swizzle term
-            bool ok = true;
-            unsigned q = 0;            // first block of the current unit
-            // zero points and scales of this warp's next block, requested one block of its own ahead
-            uint32_t z_next[4] = {0, 0, 0, 0};
-            __half s_next[4];
-            auto fetch_meta = [&](int tile, int kb) {
-                const int g = kb >> 1;
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+        const int wg = (warp - kConvWarp0) >> 2;              // this warpgroup takes block wg of every chunk
+        const int r = (warp & 3) * 32 + lane;                 // feature row of this CTA's half = tensor-memory lane
+        const uint32_t a_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + p.MT;
+        const int sw = r & 7;
+        int ps = 0;
+        uint32_t pp = 0, pe = 1;
+        int sa = wg;   // its blocks go to every second stage of the ring
+        bool ok = true;
+        while (ok && seg.next()) {
+            const int n = (seg.tile / p.m_tiles) * kPairN + rank * kBN + r;
+            const uint32_t* zrow = p.zeros + (size_t)n * p.PZ;
+            const __half* srow = p.scales + (size_t)n * p.G;
+            // Zero points and scales: one zeros word covers four chunks, and their four scales of this warpgroup's blocks are
+            // requested with it, one span of four chunks ahead (a load consumed in the block it is issued for would stall
+            // the warp for a memory latency per block). Beyond the matrix both are 0, and so are the weights.
+            uint32_t z_next = 0, z_cur = 0;
+            __half s_next[4], s_cur[4];
+            auto fetch_meta = [&](int span) {
+                const int g0 = span * 8;
+                z_next = 0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) s_next[i] = __float2half(0.f);
+                if (n < p.N && g0 < p.G) {
+                    z_next = __ldg(zrow + span);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (g0 + 2 * i + wg < p.G) s_next[i] = __ldg(srow + g0 + 2 * i + wg);
+                }
+            };
+            const int span_end = (seg.c1 - 1) >> 2;
+            fetch_meta(seg.c0 >> 2);
+            for (int span = seg.c0 >> 2; span <= span_end && ok; span++) {
+                z_cur = z_next;
+#pragma unroll
+                for (int i = 0; i < 4; i++) s_cur[i] = s_next[i];
+                if (span < span_end) fetch_meta(span + 1);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const int n = tile * kBN + lane + 32 * i;
-                    z_next[i] = 0;
-                    s_next[i] = __float2half(0.f);
-                    if (n < p.N && g < p.G) {
-                        z_next[i] = (__ldg(p.zeros + (size_t)n * p.PZ + (g >> 3)) >> (4 * (g & 7))) & 0xFu;
-                        s_next[i] = __ldg(p.scales + (size_t)n * p.G + g);
-                    }
+                const int c = span * 4 + i;
+                if (c < seg.c0 || c >= seg.c1) continue;
+                const uint32_t z = (z_cur >> (8 * i + 4 * wg)) & 0xFu;
+                const __half2 s2 = __half2half2(s_cur[i]);
+                const __half2 zlo = u2h2((0x6400u | z) * 0x00010001u), zhi = u2h2((0x5400u | (z << 4)) * 0x00010001u);
+                if (!mb_wait(&full_p[ps], pp, p.status, 0x600)) { ok = false; break; }
+                const uint8_t* src = sP + (size_t)ps * kPStageBytes + r * 128;
+                uint4 pk[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) pk[j] = *reinterpret_cast<const uint4*>(src + (((wg * 4 + j) ^ sw) << 4));
+                uint32_t o[32];
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    dequant8<INTERLEAVED>(pk[j].x, zlo, zhi, s2, o + 16 * j);
+                    dequant8<INTERLEAVED>(pk[j].y, zlo, zhi, s2, o + 16 * j + 4);
+                    dequant8<INTERLEAVED>(pk[j].z, zlo, zhi, s2, o + 16 * j + 8);
+                    dequant8<INTERLEAVED>(pk[j].w, zlo, zhi, s2, o + 16 * j + 12);
                 }
-            };
-            bool have_meta = false;
-            for (int u = blockIdx.x; u < p.total_units && ok; u += gridDim.x) {
-                const UnitInfo ui = unit_info(p, u);
-                const unsigned nkb = (unsigned)(ui.c1 - ui.c0) * kKbPerChunk;
-                // this warp's first block of the unit
-                unsigned i = (cw + NC - (q % NC)) % NC;
-                if (!have_meta && i < nkb) fetch_meta(ui.tile, ui.c0 * kKbPerChunk + i);
-                for (; i < nkb && ok; i += NC) {
-                    const unsigned qi = q + i;                      // this block's number: stage qi % NC == cw
-                    const int kb = ui.c0 * kKbPerChunk + (int)i;    // 64-input block inside K
-                    const unsigned pit = qi / kKbPerChunk;          // chunk number (chunks are four blocks, always)
-                    const int kbl = qi % kKbPerChunk, ps = pit % NP;
-                    uint32_t zz[4];
-                    __half ss[4];
+                if (!mb_wait(&empty[sa], pe, p.status, 0x700)) { ok = false; break; }
+                tc_fence_after();
+                tc_st32(a_lane + sa * kAStageCols, o);
 #pragma unroll
-                    for (int r4 = 0; r4 < 4; r4++) { zz[r4] = z_next[r4]; ss[r4] = s_next[r4]; }
-                    have_meta = false;
-                    if (i + NC < nkb) { fetch_meta(ui.tile, kb + NC); have_meta = true; }
-                    if (!mb_wait(&full_p[ps], (pit / NP) & 1, p.status, 0x600)) { ok = false; break; }
-                    uint4 pk[8];   // rows lane + 32 r4, the block's two 16-byte pieces of each row
-#pragma unroll
-                    for (int r4 = 0; r4 < 4; r4++)
-#pragma unroll
-                        for (int h = 0; h < 2; h++)
-                            pk[r4 * 2 + h] = *reinterpret_cast<const uint4*>(sP + (size_t)ps * kPStageBytes + (lane + 32 * r4) * 128 + (((kbl * 2 + h) ^ sw) << 4));
-                    __syncwarp();
-                    if (lane == 0) mb_arrive(&empty_p[ps]);   // the nibbles are in registers: one of the chunk's four releases
-                    if (!mb_wait(&empty_a[cw], ((qi / NC) & 1) ^ 1, p.status, 0x700)) { ok = false; break; }
-                    uint8_t* stage = sA + (size_t)cw * kAStageBytes;
-#pragma unroll
-                    for (int r4 = 0; r4 < 4; r4++) {
-                        const int r = lane + 32 * r4;
-                        uint32_t zlo, zhi;
-                        zero_consts(zz[r4], zlo, zhi);
-                        const __half2 s2 = __half2half2(ss[r4]);
-                        uint8_t* arow = stage + (r >> 3) * 1024 + sw * 128;
-                        const uint32_t words[8] = {pk[r4 * 2].x, pk[r4 * 2].y, pk[r4 * 2].z, pk[r4 * 2].w, pk[r4 * 2 + 1].x, pk[r4 * 2 + 1].y, pk[r4 * 2 + 1].z, pk[r4 * 2 + 1].w};
-#pragma unroll
-                        for (int j = 0; j < 8; j++) *reinterpret_cast<uint4*>(arow + ((j ^ sw) << 4)) = dequant8<INTERLEAVED>(words[j], zlo, zhi, s2);
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores before the MMA's async-proxy reads
-                    __syncwarp();
-                    if (lane == 0) mb_arrive(&full_a[cw]);
+                for (int j = 0; j < 2; j++) {
+                    dequant8<INTERLEAVED>(pk[2 + j].x, zlo, zhi, s2, o + 16 * j);
+                    dequant8<INTERLEAVED>(pk[2 + j].y, zlo, zhi, s2, o + 16 * j + 4);
+                    dequant8<INTERLEAVED>(pk[2 + j].z, zlo, zhi, s2, o + 16 * j + 8);
+                    dequant8<INTERLEAVED>(pk[2 + j].w, zlo, zhi, s2, o + 16 * j + 12);
                 }
-                q += nkb;
+                tc_st32(a_lane + sa * kAStageCols + 32, o);
+                tc_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                // The staging slot is given back only here, behind the tensor-memory stores that consumed its words: an arrive placed
+                // right behind the loads was moved ahead of some of them by the compiler, and the copy engine overwrote rows that
+                // had not been read (a few wrong feature rows in one launch out of hundreds).
+                if (lane == 0) {
+                    mb_arrive_cluster(leader_addr(&full[sa]));
+                    mb_arrive(&empty_p[ps]);
+                }
+                if (++ps == p.np) { ps = 0; pp ^= 1; }
+                sa += 2;
+                if (sa >= p.stages) { sa -= p.stages; pe ^= 1; }
+                }
             }
         }
-    } else if (warp < kFirstEpiWarp + kEpiWarps) {
+    } else {
         // ===================== epilogue =====================
-        const int qtr = warp & 3;              // the TMEM lane quarter this warp may read
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+        const int qtr = warp & 3;              // the tensor-memory lane quarter this warp may read
         const int r = qtr * 32 + lane;
-        const int etid = (warp - kFirstEpiWarp) * 32 + lane;
-        unsigned uit = 0;
-        bool ok = true;
-        for (int u = blockIdx.x; u < p.total_units && ok; u += gridDim.x, uit++) {
-            const UnitInfo ui = unit_info(p, u);
-            const int n = ui.tile * kBN + r;
-            // The residual may be y itself, so a residual load cannot be moved across a store of y by the compiler: the
-            // loads of a 16-row chunk are issued together and one chunk ahead of the stores, the first chunk's while the MMAs
-            // of the unit still run.
-            float res_next[16];
-            auto load_res = [&](int c0, float (&res)[16]) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int m = ui.mt * MT + c0 + j;
-                    res[j] = (n < p.N && m < p.M) ? __half2float(p.residual[(size_t)m * p.N + n]) : 0.f;
-                }
-            };
-            const bool add_res = p.residual != nullptr && p.splits == 1;
-            if (add_res) load_res(0, res_next);
-            if (!mb_wait(&tmem_full, uit & 1, p.status, 0x800)) { ok = false; break; }
-            tc_fence_after();
-            float* part = p.partials + (((size_t)(ui.tile * p.m_tiles + ui.mt) * p.splits + ui.split) * MT) * kBN;
-#pragma unroll 1
-            for (int c0 = 0; c0 < MT; c0 += 16) {
-                uint32_t v[16];
-                float res[16];
-                if (add_res) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++) res[j] = res_next[j];
-                    if (c0 + 16 < MT) load_res(c0 + 16, res_next);
-                }
-                tc_ld16(tmem_base + ((uint32_t)(qtr * 32) << 16) + (uint32_t)c0, v);
-                if (p.splits == 1) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        const int m = ui.mt * MT + c0 + j;
-                        if (n < p.N && m < p.M) {
-                            float val = __uint_as_float(v[j]);
-                            if (add_res) val += res[j] * p.residual_scale;
-                            p.y[(size_t)m * p.N + n] = __float2half(val);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; j++) part[(size_t)(c0 + j) * kBN + r] = __uint_as_float(v[j]);
-                }
-            }
+        const int etid = (warp - kEpiWarp0) * 32 + lane;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(qtr * 32) << 16);
+        const uint32_t empty_addr = leader_addr(&tmem_empty);
+        const size_t ld = p.N;
+        const int MT = p.MT;
+        auto release = [&]() {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive(&tmem_empty);
-            if (p.splits > 1) {
-                // the unit that arrives last at the tile's counter adds the partial sums in split order and writes Y
-                __threadfence();
-                asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
-                if (etid == 0) {
-                    const int old = atomicAdd(p.counters + ui.tile * p.m_tiles + ui.mt, 1);
-                    s_last = old == p.splits - 1;
-                    if (s_last) p.counters[ui.tile * p.m_tiles + ui.mt] = 0;   // ready for the next launch
+            if (lane == 0) mb_arrive_cluster(empty_addr);
+        };
+        auto partial_of = [&](int pr, bool head) { return reinterpret_cast<float4*>(p.partials) + ((size_t)((pr * 2 + (head ? 1 : 0)) * 2 + rank) * (MT / 4)) * kBN + r; };
+        // Y leaves through shared memory: 32 rows are staged and written by one tensor copy (rows and columns beyond Y are
+        // clipped there) while the next 32 are staged. Storing from the registers (a lane is a feature, so two bytes per lane and
+        // row) took 34000 to 40000 clocks per 256-row tile, more than its 32 chunks of MMAs.
+        uint8_t* sY = sB + kRingBytes;
+        int buf = 0;
+        auto put = [&](const uint32_t* out, int nt, int row0, int rows_left) {   // all epilogue threads; rows_left > 0
+            if (etid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the copy that read this buffer last is done
+            asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+            epi_stage<EPI>(out, sY + buf * kOutBytes, r);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+            if (etid == 0) {
+                const int col = (nt * kPairN + rank * kBN) / (EPI == EPI_SILU ? 2 : 1);
+                if (rows_left > 0 && nt * kPairN + rank * kBN < p.N)
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&map_y), "r"(smem_addr(sY + buf * kOutBytes)), "r"(col), "r"(row0)
+                                 : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            buf ^= 1;
+        };
+        uint32_t pf = 0;
+        while (seg.next()) {
+            const int nt = seg.tile / p.m_tiles, mt = seg.tile - nt * p.m_tiles;
+            const int n = nt * kPairN + rank * kBN + r;
+            const int rows = min(MT, p.M - mt * MT), my_rows = n < p.N ? rows : 0;
+            const __half* res = EPI == EPI_RESIDUAL ? p.residual + (size_t)mt * MT * ld + n : nullptr;
+            const bool whole = seg.c0 == 0 && seg.c1 == p.n_chunks;
+            if (whole) {
+                // drain everything into registers (packed halfs), give the accumulator back, then store: the stores run
+                // under the next tile's MMAs. The residual (which may be y itself) is in registers before the wait.
+                constexpr int W = 16;
+                uint32_t out[W * 8];
+                if (EPI == EPI_RESIDUAL) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (32 * i < MT) epi_load_residual(out + W * i, res, 32 * i, my_rows, ld);
                 }
-                asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
-                if (s_last) {
-                    __threadfence();
-                    const float* base = p.partials + ((size_t)(ui.tile * p.m_tiles + ui.mt) * p.splits) * MT * kBN + r;
-                    const int rows = min(MT, p.M - ui.mt * MT);
-                    // eight batch rows at a time, all their loads in flight together (the partial sums come from L2); the
-                    // splits are added in split order, so the result does not depend on which unit arrived last
-                    for (int c0 = 0; c0 < rows; c0 += 8) {
-                        float acc[8];
+                if (!mb_wait(&tmem_full, pf, p.status, 0x800)) break;
+                pf ^= 1;
+                tc_fence_after();
 #pragma unroll
-                        for (int j = 0; j < 8; j++) acc[j] = 0.f;
-                        float res[8];
+                for (int i = 0; i < 8; i++) {
+                    if (32 * i < MT) {
+                        uint32_t v[32];
+                        float f[32];
+                        tc_ld32(t_lane + 32 * i, v);
 #pragma unroll
-                        for (int j = 0; j < 8; j++)   // all eight before any store of y (the residual may be y)
-                            res[j] = (p.residual && c0 + j < rows && n < p.N) ? __half2float(p.residual[(size_t)(ui.mt * MT + c0 + j) * p.N + n]) : 0.f;
-                        for (int s = 0; s < p.splits; s++) {
-                            float v[8];
-#pragma unroll
-                            for (int j = 0; j < 8; j++) v[j] = c0 + j < rows ? __ldcg(base + ((size_t)s * MT + c0 + j) * kBN) : 0.f;
-#pragma unroll
-                            for (int j = 0; j < 8; j++) acc[j] += v[j];
-                        }
-#pragma unroll
-                        for (int j = 0; j < 8; j++)
-                            if (c0 + j < rows && n < p.N) {
-                                const size_t at = (size_t)(ui.mt * MT + c0 + j) * p.N + n;
-                                if (p.residual) acc[j] += res[j] * p.residual_scale;
-                                p.y[at] = __float2half(acc[j]);
-                            }
+                        for (int j = 0; j < 32; j++) f[j] = __uint_as_float(v[j]);
+                        epi_pack<EPI>(f, out + W * i, p.residual_scale, out + W * i);
                     }
                 }
-                asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");   // s_last is rewritten by the next unit
+                release();
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (32 * i < MT) put(out + W * i, nt, mt * MT + 32 * i, rows - 32 * i);
+                continue;
             }
+            // ---- a tile shared with other pairs: partial sums in K order, finished by the CTA that arrives last ----
+            const long long t0 = (long long)seg.tile * p.n_chunks;
+            const int first = pair_of(t0, p.total_chunks, pairs), last = pair_of(t0 + p.n_chunks - 1, p.total_chunks, pairs);
+            int* counter = p.counters + seg.tile * 2 + rank;
+            if (!mb_wait(&tmem_full, pf, p.status, 0x800)) break;
+            pf ^= 1;
+            tc_fence_after();
+            if (etid == 0) {
+                int seen;
+                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+                s_flag = seen == last - first;
+            }
+            asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+            bool finish = s_flag != 0, own_in_tmem = finish;
+            if (!finish) {
+                float4* mine = partial_of(pair, pair == first);
+#pragma unroll 1
+                for (int c0 = 0; c0 < MT; c0 += 32) {
+                    uint32_t v[32];
+                    tc_ld32(t_lane + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        __stcg(mine + (size_t)(c0 / 4 + j) * kBN, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
+                }
+                release();
+                __threadfence();
+                asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");   // (all have read s_flag and written their partials)
+                if (etid == 0) s_flag = atomicAdd(counter, 1) == last - first;
+                asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+                finish = s_flag != 0;
+            }
+            if (finish) {
+                __threadfence();
+                // the first two stored partials of the next 32 columns are requested before the current ones are staged: a
+                // round trip to L2 per 32 columns and partial, one after the other, took 30 us for a 256-row tile in four parts
+                const int m0 = own_in_tmem && pair == first ? first + 1 : first;
+                const int m1 = own_in_tmem && pair == m0 + 1 ? m0 + 2 : m0 + 1;
+                float4 n0[8], n1[8];
+                auto fetch = [&](float4 (&v)[8], int pr, int c0) {
+                    const float4* part = partial_of(pr, pr == first) + (size_t)(c0 / 4) * kBN;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] = __ldcg(part + (size_t)j * kBN);
+                };
+                fetch(n0, m0, 0);
+                if (m1 <= last) fetch(n1, m1, 0);
+#pragma unroll 1
+                for (int c0 = 0; c0 < MT; c0 += 32) {
+                    float acc[32];
+                    uint32_t rs[16], out[16];
+                    if (EPI == EPI_RESIDUAL) epi_load_residual(rs, res, c0, my_rows, ld);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) acc[j] = 0.f;
+                    auto add = [&](const float4 (&v)[8]) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) { acc[4 * j] += v[j].x; acc[4 * j + 1] += v[j].y; acc[4 * j + 2] += v[j].z; acc[4 * j + 3] += v[j].w; }
+                    };
+                    for (int pr = first; pr <= last; pr++) {
+                        if (pr == m0) add(n0);
+                        else if (pr == m1) add(n1);
+                        else if (pr == pair && own_in_tmem) {
+                            uint32_t v[32];
+                            tc_ld32(t_lane + c0, v);
+#pragma unroll
+                            for (int j = 0; j < 32; j++) acc[j] += __uint_as_float(v[j]);
+                        } else {
+                            float4 v[8];
+                            fetch(v, pr, c0);
+                            add(v);
+                        }
+                    }
+                    if (c0 + 32 < MT) {
+                        fetch(n0, m0, c0 + 32);
+                        if (m1 <= last) fetch(n1, m1, c0 + 32);
+                    }
+                    epi_pack<EPI>(acc, rs, p.residual_scale, out);
+                    put(out, nt, mt * MT + c0, rows - c0);
+                }
+                if (own_in_tmem) release();
+                if (etid == 0) *counter = 0;   // ready for the next launch
+            }
+            asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");   // s_flag is rewritten by the next segment
         }
+        if (etid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // Y is written before this CTA leaves
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) {
+    cluster_sync_all();   // no CTA leaves while the other may still report to its barriers
+    if (warp == 2) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
 }
 
@@ -499,7 +678,7 @@ int get_encode(EncodeTiledFn* out) {
 }
 
 int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes, uint32_t box_inner,
-                uint32_t box_outer) {
+                uint32_t box_outer, bool swizzle = true) {
     EncodeTiledFn enc;
     if (int e = get_encode(&enc)) return e;
     const cuuint64_t dims[2] = {inner, outer};
@@ -507,36 +686,63 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const 
     const cuuint32_t box[2] = {box_inner, box_outer};
     const cuuint32_t estr[2] = {1, 1};
     (void)elem_bytes;
-    const CUresult r = enc(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    const CUresult r = enc(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { fprintf(stderr, "q4 gemm: cuTensorMapEncodeTiled failed (%d)\n", (int)r); return Q4_ERR_CUDA; }
     return Q4_OK;
 }
 
-struct GemmPlan { int mt, m_tiles, n_tiles, splits, n_chunks, units; size_t partial_floats; };
+// Workspace layout, the same for every shape, so that calls of different shapes can share one workspace (the tile counters
+// must read zero at the start of every call): status words | tile counters | fp32 partial sums.
+constexpr size_t kWsHeader = 256;
+constexpr int kWsMaxTiles = 8192;
+constexpr size_t kWsPartials = kWsHeader + sizeof(int) * kWsMaxTiles;
 
-// Batch tile (the MMA's N), and how far K is split so that the work units fill the SMs evenly.
+constexpr double kConvClocks = 1250.0;
+
+struct GemmPlan { int MT, m_tiles, n_tiles, n_chunks, pairs, stages, np, slab; long long total; };
+
+// Batch tile and number of pairs, by an estimate of the slowest pair's clocks over all of them (what each line costs was
+// read off clock stamps inside the kernel):
+//   chunk    a 256-input chunk: 8.6 per batch row on the tensor pipe (MT / 2 per K = 16 step), or the conversion of its 128 x 256
+//            weights by the eight converter warps, whichever is longer
+//   tile     draining the accumulator; the last tile's output is not hidden by anything: 400 per 32 rows
+//   split    a tile cut by a share boundary: one partial tile written, and by the last CTA one read per other contributor
+// Large matrices end up with 256-row tiles on all pairs; small ones with smaller tiles (the conversion is repeated, but no K split
+// is needed) or with fewer pairs whose shares are whole halves or thirds of a tile.
+// Rings: operand stages as tensor memory allows, the shared memory that their X slabs leave for packed weights (at few rows
+// the kernel is a weight stream: ten 16 KB copies in flight per SM cover HBM's latency).
 GemmPlan make_plan(int M, int K, int N, int sms) {
-    GemmPlan g;
-    g.mt = M <= 16 ? 16 : M <= 64 ? 64 : 256;
-    g.m_tiles = q4_div_up(M, g.mt);
-    g.n_tiles = q4_div_up(N, kBN);
+    GemmPlan g = {};
+    g.n_tiles = q4_div_up(N, kPairN);
     g.n_chunks = q4_div_up(K, kChunkK);
-    const int base = g.n_tiles * g.m_tiles;
-    int best = 1;
-    double best_cost = 1e30;
-    for (int s = 1; s <= 16 && s <= g.n_chunks; s++) {
-        if (s > 1 && g.n_chunks / s < 2) break;   // at least two chunks (512 inputs) per unit
-        const int units = base * s;
-        // time of the slowest SM in chunk steps: its units' chunks, plus per unit a fixed cost (pipeline fill, epilogue)
-        // and, when K is split, the partial-sum round trip, which grows with the batch tile
-        const double per_unit = (double)q4_div_up(g.n_chunks, s) + 1.0 + (s > 1 ? 0.5 + g.mt / 64.0 : 0.0);
-        const double cost = q4_div_up(units, sms) * per_unit;
-        if (cost < best_cost * 0.97) { best_cost = cost; best = s; }
+    const int max_pairs = sms / 2 > 0 ? sms / 2 : 1;
+    double best = 1e300;
+    int last_mt = 0;
+    for (int m_tiles = q4_div_up(M, kMaxMT); m_tiles <= q4_div_up(M, kMaxMT) * 8; m_tiles++) {
+        const int mt = q4_div_up(q4_div_up(M, m_tiles), 32) * 32;
+        if (mt == last_mt || (long long)g.n_tiles * q4_div_up(M, mt) * 2 > kWsMaxTiles) continue;
+        last_mt = mt;
+        const int mtl = q4_div_up(M, mt);
+        const long long total = (long long)g.n_tiles * mtl * g.n_chunks;
+        const double t_chunk = 8.6 * mt > kConvClocks ? 8.6 * mt : kConvClocks;
+        for (int P = (int)(total < max_pairs ? total : max_pairs); P >= 1; P--) {
+            const long long share = (total + P - 1) / P;
+            if (share * t_chunk >= best) break;   // fewer pairs only take longer from here on
+            const bool even = total % P == 0;
+            double cost = share * t_chunk + 1000.0 * q4_div_up((int)share, g.n_chunks) + 12.5 * mt;
+            if (!(even && share % g.n_chunks == 0)) {
+                const bool aligned = even && g.n_chunks % share == 0;
+                const double readers = share >= g.n_chunks ? 1.0 : (double)(g.n_chunks + share - 1) / share - (aligned ? 1.0 : 0.0);
+                cost += 1000.0 + 6.0 * mt + readers * (1000.0 + 8.0 * mt);
+            }
+            if (cost < best * 0.99) { best = cost; g.pairs = P; g.MT = mt; g.m_tiles = mtl; g.total = total; }
+        }
     }
-    g.splits = best;
-    g.units = base * best;
-    g.partial_floats = best > 1 ? (size_t)g.units * g.mt * kBN : 0;
+    if (g.pairs == 0) return g;
+    g.slab = g.MT / 2 * kSlabK * 2;
+    g.stages = (kTmemCols - g.MT) / kAStageCols < kMaxStages ? (kTmemCols - g.MT) / kAStageCols : kMaxStages;
+    g.np = (kRingBytes - g.stages * 2 * g.slab) / kPStageBytes < kMaxP ? (kRingBytes - g.stages * 2 * g.slab) / kPStageBytes : kMaxP;
     return g;
 }
 
@@ -547,29 +753,24 @@ int sm_count(int* out) {
     return Q4_OK;
 }
 
-// Workspace layout, the same for every shape, so that calls of different shapes can share one workspace (the tile counters
-// must read zero at the start of every call): status words | tile counters | fp32 partial sums.
-constexpr size_t kWsHeader = 256;
-constexpr int kWsMaxTiles = 8192;
-constexpr size_t kWsPartials = kWsHeader + sizeof(int) * kWsMaxTiles;
-
-template <int MT, bool IL>
-int launch_gemm(cudaStream_t s, int grid, const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p) {
-    const size_t smem = GemmCfg<MT>::kSmemBytes;
-    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_gemm_kernel<MT, IL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    Q4Launch L(dim3(grid), dim3(kGemmThreads), smem, s);   // programmatic dependent launch: the prologue overlaps the previous kernel's tail
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemm_kernel<MT, IL>, mw, mx, p));
+template <bool IL, int EPI>
+int launch_gemm(cudaStream_t s, int pairs, const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& my, const GemmParams& p) {
+    const size_t smem = kRingBytes + 2 * kOutBytes + 1024;
+    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_gemm_kernel<IL, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    Q4Launch L(dim3(2 * pairs), dim3(kGemmThreads), smem, s);   // programmatic dependent launch: the prologue overlaps the previous kernel's tail
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemm_kernel<IL, EPI>, mw, mx, my, p));
     return Q4_OK;
 }
 
 }  // namespace
 
+// Grows with M only (the largest batch tile of up to M rows), so that a workspace for M rows serves every smaller call.
 extern "C" size_t q4_matmul_q4_batched_workspace_bytes(int M, int K, int N) {
     if (M <= 0 || K <= 0 || N <= 0) return 0;
     int sms = 148;
     sm_count(&sms);
-    const GemmPlan g = make_plan(M, K, N, sms);
-    return kWsPartials + g.partial_floats * sizeof(float);
+    const int mt = M >= kMaxMT ? kMaxMT : q4_div_up(M, 32) * 32;
+    return kWsPartials + (size_t)(sms / 2 > 0 ? sms / 2 : 1) * 4 * kBN * mt * sizeof(float);
 }
 
 extern "C" int q4_gemm_interleave_weights(void* stream, uint32_t* dst, const uint32_t* weight, int K, int N) {
@@ -587,9 +788,15 @@ extern "C" int q4_matmul_q4_batched(void* stream, uint16_t* y, const uint16_t* x
 
 extern "C" int q4_matmul_q4_batched_residual(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M,
                                              int K, int N, const uint16_t* residual, float residual_scale, void* workspace, size_t workspace_bytes) {
+    return q4_gemm_launch(stream, y, x, w, weight_interleaved, M, K, N, residual, residual_scale, false, workspace, workspace_bytes);
+}
+
+int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M, int K, int N,
+                   const uint16_t* residual, float residual_scale, bool silu, void* workspace, size_t workspace_bytes) {
     if (!y || !x || !w || !workspace || M <= 0 || K <= 0 || N <= 0) return Q4_ERR_INVALID;
     if ((K % 128) || (N % 8)) return Q4_ERR_UNSUPPORTED_SIZE;
-    if (((uintptr_t)x & 15) || ((uintptr_t)w->weight & 15) || ((uintptr_t)weight_interleaved & 15) || ((uintptr_t)workspace & 15)) return Q4_ERR_INVALID;
+    if (silu && (N % 16)) return Q4_ERR_UNSUPPORTED_SIZE;
+    if (((uintptr_t)x & 15) || ((uintptr_t)y & 15) || ((uintptr_t)w->weight & 15) || ((uintptr_t)weight_interleaved & 15) || ((uintptr_t)workspace & 15)) return Q4_ERR_INVALID;
     if (workspace_bytes < q4_matmul_q4_batched_workspace_bytes(M, K, N)) return Q4_ERR_LIMIT;
     cudaStream_t s = (cudaStream_t)stream;
     int sms = 0;
@@ -598,28 +805,29 @@ extern "C" int q4_matmul_q4_batched_residual(void* stream, uint16_t* y, const ui
     GemmParams p;
     p.zeros = w->zeros;
     p.scales = (const __half*)w->scales;
-    p.y = (__half*)y;
     p.residual = (const __half*)residual;
     p.residual_scale = residual_scale;
     p.status = (int*)workspace;
     p.counters = (int*)((char*)workspace + kWsHeader);
     p.partials = (float*)((char*)workspace + kWsPartials);
-    if (g.n_tiles * g.m_tiles > kWsMaxTiles) return Q4_ERR_UNSUPPORTED_SIZE;
+    if (g.pairs == 0) return Q4_ERR_UNSUPPORTED_SIZE;   // more tiles than counters
     p.M = M; p.K = K; p.N = N;
     p.G = q4_groups(K);
     p.PZ = q4_pz(K);
-    p.n_tiles = g.n_tiles; p.m_tiles = g.m_tiles; p.splits = g.splits; p.n_chunks = g.n_chunks; p.total_units = g.units;
+    p.MT = g.MT; p.m_tiles = g.m_tiles; p.n_chunks = g.n_chunks; p.total_chunks = g.total;
+    p.stages = g.stages; p.np = g.np; p.slab_bytes = g.slab;
     // (status word and tile counters start at zero: the caller zeroes the workspace once, the kernel leaves the counters at
     // zero; after a recorded time-out the caller zeroes it again)
-    CUtensorMap mw, mx;
+    CUtensorMap mw, mx, my;
     const uint32_t* wsrc = weight_interleaved ? weight_interleaved : w->weight;
     if (int e = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, wsrc, (uint64_t)q4_pw(K), (uint64_t)N, (uint64_t)q4_pw(K) * 4, kChunkK / 8, kBN)) return e;
-    if (int e = make_map_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kBK, (uint32_t)g.mt)) return e;
-    const int grid = g.units < sms ? g.units : sms;
+    if (int e = make_map_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kSlabK, (uint32_t)(g.MT / 2))) return e;
+    const int n_out = silu ? N / 2 : N;
+    if (int e = make_map_2d(&my, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, y, (uint64_t)n_out, (uint64_t)M, (uint64_t)n_out * 2, silu ? kBN / 2 : kBN, kOutRows, false)) return e;
     const bool il = weight_interleaved != nullptr;
-    if (g.mt == 16) return il ? launch_gemm<16, true>(s, grid, mw, mx, p) : launch_gemm<16, false>(s, grid, mw, mx, p);
-    if (g.mt == 64) return il ? launch_gemm<64, true>(s, grid, mw, mx, p) : launch_gemm<64, false>(s, grid, mw, mx, p);
-    return il ? launch_gemm<256, true>(s, grid, mw, mx, p) : launch_gemm<256, false>(s, grid, mw, mx, p);
+    if (silu) return il ? launch_gemm<true, EPI_SILU>(s, g.pairs, mw, mx, my, p) : Q4_ERR_INVALID;
+    if (residual) return il ? launch_gemm<true, EPI_RESIDUAL>(s, g.pairs, mw, mx, my, p) : launch_gemm<false, EPI_RESIDUAL>(s, g.pairs, mw, mx, my, p);
+    return il ? launch_gemm<true, EPI_PLAIN>(s, g.pairs, mw, mx, my, p) : launch_gemm<false, EPI_PLAIN>(s, g.pairs, mw, mx, my, p);
 }
 
 extern "C" int q4_matmul_q4_batched_status(void* stream, const void* workspace) {

@@ -59,9 +59,15 @@ void q4_fused_free(q4_model* m);
 int q4_fused_status(q4_model* m);
 void q4_rows_free(q4_model* m);   // q4_batch.cu
 int q4_rows_status(q4_model* m);
+int q4_prefill_cache(q4_model* m, cudaStream_t s, int n_tokens);   // q4_model_prefill without the last row's logits: positions and K/V rows only
 void q4_fused_set_wait_limit(q4_model* m, unsigned long long ns);   // device-side wait limit of the fused kernel (0 = default)
 
 // q4_synth.cu: counter-based synthetic tensors generated on the device, shard by shard (see q4_model_create_synthetic)
 int q4_synth_qweight(uint32_t* w, uint32_t* z, uint16_t* s, int K_full, int K, int k_begin, int N, int n_begin, unsigned long long seed, int tid);
 int q4_synth_normal(uint16_t* dst, long long count, long long idx0, unsigned long long seed, int tid);
 int q4_synth_const(uint16_t* dst, int n, uint16_t value);
+
+// q4_gemm.cu: q4_matmul_q4_batched_residual, and with silu = true (interleaved weights only) the fused gate / up form: rows 2j and
+// 2j + 1 of the weights are gate j and up j, y is [M][N / 2] = silu(gate) * up.
+int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M, int K, int N,
+                   const uint16_t* residual, float residual_scale, bool silu, void* workspace, size_t workspace_bytes);

@@ -37,6 +37,19 @@ def test_small_shapes_against_the_oracle_rows(M, K, N, interleave):
     assert_close(y, x.astype(np.float64) @ w.T, f"{M}x{K}x{N} vs f64", max_rel=4e-3)
 
 
+@pytest.mark.parametrize("M,K,N", [(31, 256, 256), (32, 384, 248), (33, 512, 264), (65, 4096, 72), (97, 640, 4096), (160, 2048, 520), (223, 1024, 1000), (256, 1152, 16),
+                                    (257, 896, 776), (385, 5120, 256), (700, 256, 2056)])
+def test_batch_tiles_and_shares(M, K, N):
+    """Batch tiles of every size (32 .. 256 rows, one to several), feature tiles that are not full on either CTA of a pair,
+    shares that cut tiles into two and more parts; against an fp64 product of the bit-exact weights."""
+    q, x, y, mm, xd = _case(M, K, N, seed=M + K + N, interleave=True)
+    w = O.dequant(q, K, N).astype(np.float64)
+    assert_close(y, x.astype(np.float64) @ w.T, f"{M}x{K}x{N} vs f64", max_rel=4e-3)
+    y2 = torch.empty_like(torch.from_numpy(y)).cuda()
+    mm(y2, xd, M)
+    assert mm.status() == 0 and (y2.cpu().numpy().view(np.uint16) == y.view(np.uint16)).all()
+
+
 @pytest.mark.parametrize("M", [16, 64, 512])
 @pytest.mark.parametrize("K,N", [(4096, 12288), (4096, 22016), (11008, 4096), (4096, 4096)])
 def test_7b_projection_shapes(M, K, N):
@@ -70,6 +83,19 @@ def test_back_to_back_launches_are_bit_reproducible():
         for o in outs:
             assert torch.equal(o, first)
     assert mm.status() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(40, 1024, 520), (300, 4096, 256), (512, 11008, 512)])
+def test_residual_epilogue(M, K, N):
+    """y = product + y * scale in place (q4_matmul_q4_batched_residual), whole tiles and tiles in several parts."""
+    from llama_cu_awq_b200 import _lib
+    q, x, y, mm, xd = _case(M, K, N, seed=M, interleave=True)
+    r = np.random.default_rng(1).standard_normal((M, N)).astype(np.float16)
+    yd = torch.from_numpy(r).cuda()
+    e = _lib.lib().q4_matmul_q4_batched_residual(ops._stream(), ops._p(yd), ops._p(xd), mm.w.ref, ops._p(mm.wi), M, K, N, ops._p(yd), 0.5, ops._p(mm.ws), mm.ws_bytes)
+    assert e == 0 and mm.status() == 0
+    w = O.dequant(q, K, N).astype(np.float64)
+    assert_close(yd.cpu().numpy(), x.astype(np.float64) @ w.T + 0.5 * r, f"{M}x{K}x{N} + residual", max_rel=4e-3)
 
 
 def test_rejects_unsupported_arguments():
