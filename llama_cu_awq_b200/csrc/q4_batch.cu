@@ -21,11 +21,7 @@ constexpr int kRowThreads = 256;
 
 // Every kernel of this file starts with griddepcontrol.wait + launch_dependents, so it may be launched with programmatic
 // stream serialisation: its successor (often a weight-streaming kernel whose first loads do not depend on it) then begins
-// its prologue while this one runs, and waits for this one's completion before it touches anything produced here. The
-// batched-decode step (a handful of rows, latency-bound small kernels) is launched that way. A prompt's rows are not:
-// with hundreds of rows the overlap buys nothing measurable, and with the rotation and attention kernels launched that way
-// two runs of the same 512-token prompt did not always give the same bits on this GPU and driver (about one run in ten
-// differed in the last bits of a few logits; cause not found), so those launches keep plain stream order.
+// its prologue while this one runs, and waits for this one's completion before it touches anything produced here.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_rows(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     Q4Launch L(grid, block, smem, s, overlap);
@@ -69,23 +65,48 @@ __device__ __forceinline__ uint4 scale8(const uint4& v, const uint4& w, float r)
     }
     return o;
 }
-__global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, const __half* x, const __half* w, int size) {
+// x = half(y + x): the residual of matmul(QWeight)'s accum form (gpu_kernels.h:237-238) on a GEMM result that was written without it
+__device__ __forceinline__ uint4 add8(const uint4& x, const uint4& y) {
+    const __half2* xh = reinterpret_cast<const __half2*>(&x);
+    const __half2* yh = reinterpret_cast<const __half2*>(&y);
+    uint4 o;
+    __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float2 a = __half22float2(xh[j]), b = __half22float2(yh[j]);
+        oh[j] = __floats2half2_rn(b.x + a.x, b.y + a.y);
+    }
+    return o;
+}
+// ADD: the row is x + y first, and goes back to x (a prompt's projections on one GPU: the GEMM's own residual epilogue reads two
+// bytes per lane and row, 20 us per 512 x 4096 tile row, where this pass has the row in registers anyway).
+template <bool ADD>
+__global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __half* x, const __half* y, const __half* w, int size) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
     __shared__ float red[kRowThreads / 32];
-    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * size);
+    uint4* xr = reinterpret_cast<uint4*>(x + (size_t)blockIdx.x * size);
+    const uint4* yr = reinterpret_cast<const uint4*>(y + (size_t)blockIdx.x * size);
     uint4* orow = reinterpret_cast<uint4*>(o + (size_t)blockIdx.x * size);
     const uint4* wv = reinterpret_cast<const uint4*>(w);
     const int nvec = size / 8;
     constexpr int kKeep = 4;
     uint4 v[kKeep];
     float ss = 0.f;
+    auto row = [&](int i) {
+        uint4 r = xr[i];
+        if (ADD) {
+            r = add8(r, yr[i]);
+            xr[i] = r;
+        }
+        return r;
+    };
 #pragma unroll
     for (int c = 0; c < kKeep; c++) {
         const int i = threadIdx.x + c * kRowThreads;
-        if (i < nvec) { v[c] = xr[i]; ss += sumsq8(v[c]); }
+        if (i < nvec) { v[c] = row(i); ss += sumsq8(v[c]); }
     }
-    for (int i = threadIdx.x + kKeep * kRowThreads; i < nvec; i += kRowThreads) ss += sumsq8(xr[i]);
+    for (int i = threadIdx.x + kKeep * kRowThreads; i < nvec; i += kRowThreads) ss += sumsq8(row(i));
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
@@ -105,38 +126,49 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, co
 
 // RoPERotation_kernel (gpu_kernels.h:340-363) per row, and the row's K and V into the cache: query heads are rotated in place,
 // the key heads are rotated on their way into cache row `pos` of the row's sequence, the value heads are copied there.
-// A block takes kRopeHeads heads (query heads first, then key/value heads) of one row: the head_size / 2 rotation angles
-// depend on the position only and are computed once per block, in the reference's arithmetic (powf, cosf, sinf in fp32).
-// head_size <= 256. grid (rows, ceil((heads + kv_heads) / kRopeHeads)), block 256.
-constexpr int kRopeHeads = 4;
+// head_size 128. A thread takes eight rotation pairs of one head (16 bytes of each half of the head); the angles come from a
+// table [position][pair] built once with the reference's arithmetic (evaluating powf, cosf and sinf per block of four heads,
+// two bytes per access, took 21.6 us for 512 rows of 32 + 32 heads). grid (rows, parts), block 256.
 __global__ void __launch_bounds__(256) rope_store_rows_kernel(__half* q, const __half* k, const __half* v, int ldq, int ldkv, __half* kc, __half* vc, int n_heads,
-                                                              int n_kv_heads, int head_size, const int* row_seq, const int* row_pos, long long seq_stride, long long loff,
-                                                              float theta) {
+                                                              int n_kv_heads, const float2* table, const int* row_seq, const int* row_pos, long long seq_stride,
+                                                              long long loff) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
-    __shared__ float2 table[128];
+    constexpr int HS = 128, kPer = 8;   // threads per head
     const int m = blockIdx.x;
     const int pos = row_pos[m];
-    const int half_hs = head_size / 2;
-    for (int i = threadIdx.x; i < half_hs; i += blockDim.x) table[i] = rope_cos_sin(pos, i, head_size, theta);
-    __syncthreads();
-    __half* qr = q + (size_t)m * ldq;      // ldq, ldkv: halfs between rows of q and of k / v (they may be slices of one wider buffer)
-    const size_t src0 = (size_t)m * ldkv;
-    const size_t dst0 = (size_t)row_seq[m] * seq_stride + loff + (size_t)pos * n_kv_heads * head_size;
-    const int h_first = blockIdx.y * kRopeHeads, h_end = min(h_first + kRopeHeads, n_heads + n_kv_heads);
-    for (int e = threadIdx.x; e < (h_end - h_first) * half_hs; e += blockDim.x) {
-        const int hh = h_first + e / half_hs, i = e % half_hs;
-        if (hh < n_heads) {
-            __half* p = qr + (size_t)hh * head_size;
-            rope_rotate(p + i, p + i + half_hs, p + i, p + i + half_hs, table[i]);
-        } else {
-            const int h = hh - n_heads;
-            const size_t src = src0 + (size_t)h * head_size, dst = dst0 + (size_t)h * head_size;
-            rope_rotate(k + src + i, k + src + i + half_hs, kc + dst + i, kc + dst + i + half_hs, table[i]);
-            vc[dst + i] = v[src + i];
-            vc[dst + i + half_hs] = v[src + i + half_hs];
+    const size_t dst0 = (size_t)row_seq[m] * seq_stride + loff + (size_t)pos * n_kv_heads * HS;
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < (n_heads + 2 * n_kv_heads) * kPer; e += gridDim.y * blockDim.x) {
+        const int hh = e / kPer, i = (e % kPer) * 8;
+        if (hh >= n_heads + n_kv_heads) {
+            const int h = hh - n_heads - n_kv_heads;
+            const uint4* src = reinterpret_cast<const uint4*>(v + (size_t)m * ldkv + (size_t)h * HS + 2 * i);
+            uint4* dst = reinterpret_cast<uint4*>(vc + dst0 + (size_t)h * HS + 2 * i);
+            dst[0] = src[0];
+            dst[1] = src[1];
+            continue;
         }
+        const bool is_q = hh < n_heads;
+        const __half* src = is_q ? q + (size_t)m * ldq + (size_t)hh * HS : k + (size_t)m * ldkv + (size_t)(hh - n_heads) * HS;
+        __half* dst = is_q ? q + (size_t)m * ldq + (size_t)hh * HS : kc + dst0 + (size_t)(hh - n_heads) * HS;
+        uint4 lo = *reinterpret_cast<const uint4*>(src + i), hi = *reinterpret_cast<const uint4*>(src + i + HS / 2);
+        const float4* tp = reinterpret_cast<const float4*>(table + (size_t)pos * (HS / 2) + i);
+        __half* l = reinterpret_cast<__half*>(&lo);
+        __half* g = reinterpret_cast<__half*>(&hi);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float4 cs = __ldg(tp + j);
+            rope_rotate(l + 2 * j, g + 2 * j, l + 2 * j, g + 2 * j, make_float2(cs.x, cs.y));
+            rope_rotate(l + 2 * j + 1, g + 2 * j + 1, l + 2 * j + 1, g + 2 * j + 1, make_float2(cs.z, cs.w));
+        }
+        *reinterpret_cast<uint4*>(dst + i) = lo;
+        *reinterpret_cast<uint4*>(dst + i + HS / 2) = hi;
     }
+}
+__global__ void rope_rows_table_kernel(float2* table, int positions, int head_size, float theta) {
+    const int half_hs = head_size / 2;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < positions * half_hs; i += gridDim.x * blockDim.x)
+        table[i] = rope_cos_sin(i / half_hs, i % half_hs, head_size, theta);
 }
 
 // MultiHeadAttention (llama2_q4.cu:410-427) for one (row, head): the query attends to cached positions 0 .. pos of its own
@@ -368,49 +400,11 @@ __global__ void __launch_bounds__(128) attention_prefill_kernel(__half* out, con
     }
 }
 
-// ffn_matvec_silu's epilogue (gpu_kernels.h:278-281) on the result of the fused gate|up GEMM: row m of gu holds the hid gate
-// values and then the hid up values; h[m][j] = silu(gate) * up in fp32, fp16 out. hid % 8 == 0.
-__global__ void silu_mul_rows_kernel(__half* h, const __half* gu, int hid, int rows) {
-    griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
-    griddep_launch_dependents();
-    const int per_row = hid / 8;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)rows * per_row; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t m = i / per_row, j = i - m * per_row;
-        const uint4 gv = reinterpret_cast<const uint4*>(gu + m * 2 * hid)[j], uv = reinterpret_cast<const uint4*>(gu + m * 2 * hid + hid)[j];
-        const __half2* gh = reinterpret_cast<const __half2*>(&gv);
-        const __half2* uh = reinterpret_cast<const __half2*>(&uv);
-        uint4 o;
-        __half2* oh = reinterpret_cast<__half2*>(&o);
-#pragma unroll
-        for (int jj = 0; jj < 4; jj++) {
-            const float2 g = __half22float2(gh[jj]), u = __half22float2(uh[jj]);
-            float a = g.x, b = g.y;
-            a *= 1.0f / (1.0f + expf(-a));
-            b *= 1.0f / (1.0f + expf(-b));
-            oh[jj] = __floats2half2_rn(a * u.x, b * u.y);
-        }
-        reinterpret_cast<uint4*>(h + m * hid)[j] = o;
-    }
-}
-
-// x = y + x * scale: the residual of matmul(QWeight)'s accum form (gpu_kernels.h:237-238) applied to a GEMM result that
-// was written without it (the GEMM's own residual epilogue reads x element by element behind the tile's fp32 sums, which
-// costs more than this pass over two small matrices). fp32 inside, rounded once. n % 8 == 0.
-__global__ void add_residual_rows_kernel(__half* x, const __half* y, float scale, size_t n) {
-    griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
-    griddep_launch_dependents();
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n / 8; i += (size_t)gridDim.x * blockDim.x) {
-        const uint4 xv = reinterpret_cast<const uint4*>(x)[i], yv = reinterpret_cast<const uint4*>(y)[i];
-        const __half2* xh = reinterpret_cast<const __half2*>(&xv);
-        const __half2* yh = reinterpret_cast<const __half2*>(&yv);
-        uint4 o;
-        __half2* oh = reinterpret_cast<__half2*>(&o);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 a = __half22float2(xh[j]), b = __half22float2(yh[j]);
-            oh[j] = __floats2half2_rn(b.x + a.x * scale, b.y + a.y * scale);
-        }
-        reinterpret_cast<uint4*>(x)[i] = o;
+// Rows of `len` 16-bit words to every step-th row of dst (set-up only: q|k|v behind one another, gate and up in turn).
+__global__ void place_rows_kernel(uint16_t* dst, const uint16_t* src, int len, size_t step, size_t total) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t row = i / len;
+        dst[row * step * len + (i - row * len)] = src[i];
     }
 }
 
@@ -591,12 +585,14 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const __half* logits,
 struct q4_rows {
     int cap = 0;   // rows the buffers hold
     __half *X = nullptr, *XB = nullptr, *Q = nullptr, *K = nullptr, *V = nullptr, *ATT = nullptr, *G = nullptr;
-    __half *QKV = nullptr, *GU = nullptr;   // GEMM path: [rows][q_n + 2 kv_n] and [rows][2 hid], written by one GEMM each
+    __half *QKV = nullptr, *Y = nullptr;   // GEMM path: [rows][q_n + 2 kv_n], written by one GEMM; [rows][dim], a projection's result
     int *row_seq = nullptr, *row_pos = nullptr;
+    float2* rope = nullptr;   // [seq_len][head_size / 2] (cos, sin)
     void* ws = nullptr;
     size_t ws_bytes = 0;
-    // GEMM path, per layer four matrices: q|k|v and gate|up stacked along the output axis (one launch each), o, down.
-    // Interleaved copy of the packed words, and for the stacked ones a copy of zeros and scales in the same order.
+    // GEMM path, per layer four matrices: q|k|v stacked along the output axis, gate and up row by row in turn (row 2j = gate j,
+    // 2j + 1 = up j: the GEMM's epilogue finds both in neighbouring lanes and writes silu(gate) * up), o, down; one launch each.
+    // Interleaved copy of the packed words, and for the joined ones a copy of zeros and scales in the same order.
     struct GemmMat { uint32_t* wi; q4_qweight w; int K, N; };
     std::vector<GemmMat> gm;     // [layer * 4 + {0 qkv, 1 o, 2 gate|up, 3 down}]
     std::vector<void*> allocs;
@@ -654,21 +650,34 @@ static int rows_prepare(q4_model* m, int rows) {
                     RTRY(rows_alloc(r, (void**)&zeros, (size_t)N * q4_pz(K) * 4));
                     RTRY(rows_alloc(r, (void**)&scales, (size_t)N * q4_groups(K) * 2));
                 }
+                // part j's rows go to rows row0, row0 + step, ... of the joined matrix
+                const size_t step = i == 2 ? 2 : 1;
                 size_t row0 = 0;
+                auto place = [&](void* dst, const void* src, size_t row_bytes, int rows) {   // row_bytes is a multiple of 2
+                    place_rows_kernel<<<148 * 8, 256>>>((uint16_t*)dst + row0 * (row_bytes / 2), (const uint16_t*)src, (int)(row_bytes / 2), step, (size_t)rows * (row_bytes / 2));
+                };
                 for (int j = 0; j < parts; j++) {
                     const DevQW* q = groups[i][j];
-                    RTRY(q4_gemm_interleave_weights(nullptr, gmat.wi + row0 * q4_pw(K), q->w.weight, K, q->N));
+                    place(gmat.wi, q->w.weight, (size_t)q4_pw(K) * 4, q->N);
                     if (parts > 1) {
-                        Q4_CUDA_TRY(cudaMemcpy(zeros + row0 * q4_pz(K), q->w.zeros, (size_t)q->N * q4_pz(K) * 4, cudaMemcpyDeviceToDevice));
-                        Q4_CUDA_TRY(cudaMemcpy(scales + row0 * q4_groups(K), q->w.scales, (size_t)q->N * q4_groups(K) * 2, cudaMemcpyDeviceToDevice));
+                        place(zeros, q->w.zeros, (size_t)q4_pz(K) * 4, q->N);
+                        place(scales, q->w.scales, (size_t)q4_groups(K) * 2, q->N);
                     }
-                    row0 += q->N;
+                    row0 += i == 2 ? 1 : q->N;
                 }
+                Q4_CUDA_TRY(cudaGetLastError());
+                RTRY(q4_gemm_interleave_weights(nullptr, gmat.wi, gmat.wi, K, N));   // (word by word: in place)
                 gmat.w.weight = gmat.wi;   // (the GEMM reads the interleaved words; this field only has to be non-null)
                 gmat.w.zeros = parts > 1 ? zeros : groups[i][0]->w.zeros;
                 gmat.w.scales = parts > 1 ? scales : groups[i][0]->w.scales;
             }
         }
+        Q4_CUDA_TRY(cudaDeviceSynchronize());
+    }
+    if (!r->rope) {
+        RTRY(rows_alloc(r, (void**)&r->rope, sizeof(float2) * (size_t)c.seq_len * (m->head_size / 2)));
+        rope_rows_table_kernel<<<148 * 2, 256>>>(r->rope, c.seq_len, m->head_size, c.rope_theta);
+        Q4_CUDA_TRY(cudaGetLastError());
         Q4_CUDA_TRY(cudaDeviceSynchronize());
     }
     if (rows > r->cap) {
@@ -683,7 +692,7 @@ static int rows_prepare(q4_model* m, int rows) {
         RTRY(rows_alloc(r, (void**)&r->G, 2 * cap * hk));
         if (cap > kSkinnyRows) {
             RTRY(rows_alloc(r, (void**)&r->QKV, 2 * (size_t)cap * (m->q_n + 2 * m->kv_n)));
-            RTRY(rows_alloc(r, (void**)&r->GU, 2 * cap * 2 * hk));
+            RTRY(rows_alloc(r, (void**)&r->Y, 2 * cap * dim));
         }
         RTRY(rows_alloc(r, (void**)&r->row_seq, sizeof(int) * cap));
         RTRY(rows_alloc(r, (void**)&r->row_pos, sizeof(int) * cap));
@@ -714,38 +723,67 @@ static int rows_all_reduce(q4_model* m, cudaStream_t s, __half* buf, size_t coun
     return Q4_OK;
 }
 
+// What the caller needs behind the last layer: every row (batched decode), the last row (a prompt: only its logits are asked for)
+// or nothing but the K/V rows (a prompt whose last position follows through another path).
+enum RowsWanted { WANT_ALL, WANT_LAST, WANT_CACHE };
+
 // All layers for `n` rows whose embeddings are in r->X; K/V rows go to (kc, vc) with `seq_stride` halfs between sequences.
 // pos0 >= 0: the rows are positions pos0 .. pos0 + n - 1 of one sequence (prompt); -1: one row per sequence (batched decode).
-static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* vc, long long seq_stride, int pos0) {
+// In the last layer the rows that nobody asks for end at their K/V row: no later layer reads them.
+static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* vc, long long seq_stride, int pos0, RowsWanted want) {
     q4_rows* r = m->rows;
     const q4_config& c = m->cfg;
-    const int g = m->g, dim = c.dim, hs = m->head_size;
+    const int g = m->g, dim = c.dim;
     const int heads = c.n_heads / g, kv_heads = c.n_kv_heads / g;
     int e;
 #define OP(expr) do { e = (expr); if (e != Q4_OK) return e; } while (0)
-    auto gemm = [&](__half* y, const __half* x, int l, int mat) {   // mat: 0 q|k|v, 1 o, 2 gate|up, 3 down
+    // mat: 0 q|k|v, 1 o, 2 gate / up with silu(gate) * up, 3 down; residual: y = product + y / g
+    auto gemm = [&](__half* y, const __half* x, int l, int mat, bool residual) {
         const q4_rows::GemmMat& gmat = r->gm[(size_t)l * 4 + mat];
-        return q4_matmul_q4_batched(s, (uint16_t*)y, (const uint16_t*)x, &gmat.w, gmat.wi, n, gmat.K, gmat.N, r->ws, r->ws_bytes);
+        return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &gmat.w, gmat.wi, n, gmat.K, gmat.N, residual ? (const uint16_t*)y : nullptr, 1.0f / g, mat == 2, r->ws,
+                              r->ws_bytes);
     };
     // q, k, v of the rows: three buffers (few-rows kernels) or three slices of the fused GEMM's output
     const int nqkv = m->q_n + 2 * m->kv_n;
     const bool skinny = n <= kSkinnyRows;
-    const bool overlap = pos0 < 0;   // batched decode: programmatic dependent launches (see launch_rows)
+    const bool overlap = true;
+    // A prompt's rows on one GPU: the o and down projections leave their result in XB / ATT and the next RMSNorm adds it to x
+    // (with more ranks the partial sums have to be exchanged as x first: the GEMM adds the residual itself).
+    const bool fused_add = !skinny && g == 1;
+    auto norm = [&](const __half* w, const __half* y) {
+        if (y) launch_rows(overlap, rmsnorm_rows_kernel<true>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, y, w, dim);
+        else launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, w, dim);
+    };
     for (int l = 0; l < c.n_layers; l++) {
         const DevLayer& L = m->layers[l];
         const long long loff = (long long)l * c.seq_len * m->kv_n;
-        launch_rows(overlap, rmsnorm_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)L.rms_att, dim);
+        norm((const __half*)L.rms_att, fused_add && l > 0 ? r->Y : nullptr);
         if (skinny) {
             OP(q4_qkv_matmul_rows(s, (uint16_t*)r->Q, (uint16_t*)r->K, (uint16_t*)r->V, (const uint16_t*)r->XB, &L.q.w, &L.k.w, &L.v.w, n, dim, m->q_n, m->kv_n));
         } else {
-            OP(gemm(r->QKV, r->XB, l, 0));
+            OP(gemm(r->QKV, r->XB, l, 0, false));
         }
         __half* qp = skinny ? r->Q : r->QKV;
         const __half* kp = skinny ? r->K : r->QKV + m->q_n;
         const __half* vp = skinny ? r->V : r->QKV + m->q_n + m->kv_n;
         const int ldq = skinny ? m->q_n : nqkv, ldkv = skinny ? m->kv_n : nqkv;
-        launch_rows(overlap, rope_store_rows_kernel, dim3(n, q4_div_up(heads + kv_heads, kRopeHeads)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads, hs,
-                    r->row_seq, r->row_pos, seq_stride, loff, c.rope_theta);
+        launch_rows(overlap, rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
+                    r->rope, r->row_seq, r->row_pos, seq_stride, loff);
+        if (l == c.n_layers - 1 && want != WANT_ALL) {
+            if (want == WANT_CACHE) break;
+            // one row: the split attention of the batch-1 path and the few-rows kernels
+            const size_t last = (size_t)(n - 1);
+            uint16_t* x = (uint16_t*)(r->X + last * dim);
+            OP(q4_attention(s, (uint16_t*)r->ATT, (const uint16_t*)qp + last * ldq, (const uint16_t*)(kc + loff), (const uint16_t*)(vc + loff), m->attn_scratch, heads, m->head_size,
+                            m->kv_mul, c.seq_len, r->row_pos + last));
+            OP(q4_matmul_q4_rows(s, x, (const uint16_t*)r->ATT, &L.o.w, 1, m->o_kc, dim, x, 1.0f / g));
+            OP(rows_all_reduce(m, s, (__half*)x, dim, true));
+            launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);
+            OP(q4_ffn_silu_rows(s, (uint16_t*)r->G, (const uint16_t*)r->XB, &L.gate.w, &L.up.w, 1, dim, m->h_kc));
+            OP(q4_matmul_q4_rows(s, x, (const uint16_t*)r->G, &L.down.w, 1, m->h_kc, dim, x, 1.0f / g));
+            OP(rows_all_reduce(m, s, (__half*)x, dim, true));
+            break;
+        }
         if (pos0 >= 0 && !skinny)
             launch_rows(overlap, attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), 0, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
                         m->kv_mul, n, pos0, m->kv_n);
@@ -754,21 +792,16 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
                         r->row_pos, seq_stride, loff, m->kv_n);
         // x = o_proj(att) + x / g, summed over the ranks (gpu_kernels.h:237-238, llama2_q4.cu:472-476)
         if (skinny) OP(q4_matmul_q4_rows(s, (uint16_t*)r->X, (const uint16_t*)r->ATT, &L.o.w, n, m->o_kc, dim, (const uint16_t*)r->X, 1.0f / g));
-        else {   // the normalised rows in XB are spent: the projection lands there, then x = projection + x / g
-            OP(gemm(r->XB, r->ATT, l, 1));
-            launch_rows(overlap, add_residual_rows_kernel, dim3(148 * 4), dim3(256), 0, s, r->X, (const __half*)r->XB, 1.0f / g, (size_t)n * dim);
-        }
+        else OP(gemm(fused_add ? r->Y : r->X, r->ATT, l, 1, !fused_add));
         OP(rows_all_reduce(m, s, r->X, (size_t)n * dim, pos0 >= 0));
-        launch_rows(overlap, rmsnorm_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)L.rms_ffn, dim);
+        norm((const __half*)L.rms_ffn, fused_add ? r->Y : nullptr);
         if (skinny) {
             // gate and up stay in fp32 until silu(gate) * up, as in ffn_matvec_silu_kernel (gpu_kernels.h:278-281)
             OP(q4_ffn_silu_rows(s, (uint16_t*)r->G, (const uint16_t*)r->XB, &L.gate.w, &L.up.w, n, dim, m->h_kc));
             OP(q4_matmul_q4_rows(s, (uint16_t*)r->X, (const uint16_t*)r->G, &L.down.w, n, m->h_kc, dim, (const uint16_t*)r->X, 1.0f / g));
         } else {
-            OP(gemm(r->GU, r->XB, l, 2));
-            launch_rows(overlap, silu_mul_rows_kernel, dim3(148 * 4), dim3(256), 0, s, r->G, (const __half*)r->GU, m->h_kc, n);
-            OP(gemm(r->XB, r->G, l, 3));
-            launch_rows(overlap, add_residual_rows_kernel, dim3(148 * 4), dim3(256), 0, s, r->X, (const __half*)r->XB, 1.0f / g, (size_t)n * dim);
+            OP(gemm(r->G, r->XB, l, 2, false));
+            OP(gemm(fused_add ? r->Y : r->X, r->G, l, 3, !fused_add));
         }
         OP(rows_all_reduce(m, s, r->X, (size_t)n * dim, pos0 >= 0));
     }
@@ -780,33 +813,34 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
 // ------------------------------------------------------------------------------------------------------------
 // prefill
 // ------------------------------------------------------------------------------------------------------------
-extern "C" int q4_model_prefill(q4_model* m, void* stream, int n_tokens, int gen_token) {
-    if (!m || n_tokens < 1) return Q4_ERR_INVALID;
+static int prefill(q4_model* m, cudaStream_t s, int n, int gen_token, bool logits) {
+    if (!m || n < 1) return Q4_ERR_INVALID;
     const q4_config& c = m->cfg;
     const int pos0 = m->host_pos;
-    if (pos0 + n_tokens > c.seq_len || pos0 + n_tokens >= Q4_MAX_SEQ_LEN) return Q4_ERR_LIMIT;
-    if (int e = rows_prepare(m, n_tokens)) return e;
+    if (pos0 + n > c.seq_len || pos0 + n >= Q4_MAX_SEQ_LEN) return Q4_ERR_LIMIT;
+    if (int e = rows_prepare(m, n)) return e;
     q4_rows* r = m->rows;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int n = n_tokens;
-    const bool overlap = false;
+    const bool overlap = true;
     launch_rows(overlap, iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, 0, pos0, 0);
     launch_rows(overlap, embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size);
-    if (int e = rows_layers(m, s, n, (__half*)m->kc, (__half*)m->vc, 0, pos0)) return e;
-    // the last row goes on through the batch-1 tail (llama2_q4.cu:528-537, sampler.h:77-84): final norm, classifier,
-    // [all-gather], hand-off; the position words are moved to that row first, the hand-off then steps them past it
-    Q4_CUDA_TRY(cudaMemcpyAsync(m->x, r->X + (size_t)(n - 1) * c.dim, 2 * (size_t)c.dim, cudaMemcpyDeviceToDevice, s));
-    launch_rows(overlap, set_pos_kernel, dim3(1), dim3(1), 0, s, m->pos, &m->shared->pos, pos0 + n - 1);
-    int e;
-    if ((e = q4_rmsnorm(s, m->x, m->x, m->rms_final, c.dim)) != Q4_OK) return e;
-    if ((e = q4_matmul_f16(s, m->logits + (size_t)m->rank * m->v_n, m->x, m->wcls, c.dim, m->v_n, 1.0f)) != Q4_OK) return e;
-    if (m->g > 1 && (e = q4_all_gather(m->comm, s, m->logits + (size_t)m->rank * m->v_n, m->logits, m->v_n)) != Q4_OK) return e;
-    if ((e = q4_argmax(s, m->logits, c.vocab_size, (int*)m->shared->tokens, &m->shared->pos, m->pos, gen_token != 0)) != Q4_OK) return e;
+    if (int e = rows_layers(m, s, n, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) return e;
     // sample() draws one coin per position, used or not (sampler.h:79): keep the generator where n token steps leave it
     for (int i = 0; i < n; i++) (void)q4_random_f32(&m->rng_state);
     m->host_pos = pos0 + n;
-    return Q4_OK;
+    launch_rows(overlap, set_pos_kernel, dim3(1), dim3(1), 0, s, m->pos, &m->shared->pos, logits ? pos0 + n - 1 : pos0 + n);
+    if (!logits) return Q4_OK;
+    // the last row goes on through the batch-1 tail (llama2_q4.cu:528-537, sampler.h:77-84): final norm, classifier,
+    // [all-gather], hand-off; the position words were moved to that row, the hand-off steps them past it
+    int e;
+    if ((e = q4_rmsnorm(s, m->x, (const uint16_t*)(r->X + (size_t)(n - 1) * c.dim), m->rms_final, c.dim)) != Q4_OK) return e;
+    if ((e = q4_matmul_f16(s, m->logits + (size_t)m->rank * m->v_n, m->x, m->wcls, c.dim, m->v_n, 1.0f)) != Q4_OK) return e;
+    if (m->g > 1 && (e = q4_all_gather(m->comm, s, m->logits + (size_t)m->rank * m->v_n, m->logits, m->v_n)) != Q4_OK) return e;
+    return q4_argmax(s, m->logits, c.vocab_size, (int*)m->shared->tokens, &m->shared->pos, m->pos, gen_token != 0);
 }
+
+extern "C" int q4_model_prefill(q4_model* m, void* stream, int n_tokens, int gen_token) { return prefill(m, (cudaStream_t)stream, n_tokens, gen_token, true); }
+// The prompt positions into the cache and nothing else: what follows takes its own logits (q4_generate).
+int q4_prefill_cache(q4_model* m, cudaStream_t s, int n_tokens) { return prefill(m, s, n_tokens, 0, false); }
 
 // ------------------------------------------------------------------------------------------------------------
 // batched decode: several sequences, one position each per step
@@ -912,8 +946,8 @@ static int batch_step(q4_batch* b, cudaStream_t s) {
     launch_rows(overlap, iota_rows_kernel, dim3(1), dim3(32), 0, s, r->row_seq, nullptr, n, 0, 0, 1);
     Q4_CUDA_TRY(cudaMemcpyAsync(r->row_pos, b->pos, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     launch_rows(overlap, embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, b->tokens, b->max_len + 1, r->row_seq, r->row_pos, c.vocab_size);
-    if (int e = rows_layers(m, s, n, b->kc, b->vc, b->seq_stride, -1)) return e;
-    launch_rows(overlap, rmsnorm_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)m->rms_final, c.dim);
+    if (int e = rows_layers(m, s, n, b->kc, b->vc, b->seq_stride, -1, WANT_ALL)) return e;
+    launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)nullptr, (const __half*)m->rms_final, c.dim);
     const size_t smem = 2 * (size_t)n * c.dim;
     __half* cls_out = m->g == 1 ? b->logits : b->part;   // TP: every rank computes its vocabulary slice of every row; the slices are gathered row by row
     const int cls_stride = m->g == 1 ? c.vocab_size : m->v_n;

@@ -558,7 +558,7 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
     if (one_pass && n_prompt > 1 && steps > n_prompt - 1) {
         // all prompt positions but the last in one pass; the last one goes through the token path, which also draws the
         // first generated id (greedy or sampled). A model the many-row kernels do not serve falls back to the loop.
-        e = q4_model_prefill(m, s, n_prompt - 1, 0);
+        e = q4_prefill_cache(m, s, n_prompt - 1);
         if (e == Q4_OK) pos = n_prompt - 1;
         else if (e != Q4_ERR_UNSUPPORTED_SIZE) { cudaStreamDestroy(s); return e; }
     }
