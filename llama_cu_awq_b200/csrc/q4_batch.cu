@@ -256,12 +256,20 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* 
 
 // ---- causal attention of a prompt (rows = consecutive positions of one sequence) on the tensor cores ----
 // The (row, head) kernel above re-reads the whole K/V history once per row; for a prompt that is rows^2 / 2 cache rows per
-// head. Here a CTA takes 64 consecutive rows of one head (a warp: 16 of them) and walks the keys in chunks of 64 staged in
-// shared memory, so a cache row is read once per 64 query rows. S = Q K^T and O += P V run as mma.sync m16n8k16 (fp16 in,
-// fp32 out); the scores are scaled and rounded to fp16 exactly where MultiHeadAttention stores them (gpu_kernels.h:171-175),
-// the softmax is the online form in fp32, P is rounded to fp16 for the second product (the reference's att buffer is fp16
-// too). head_size 128. Keys beyond the last row's position are zero-filled in shared memory and masked.
+// head. Here a CTA takes 64 consecutive rows of one head (a warp: 16 of them) and walks the keys in chunks of 64, so a cache
+// row is read once per 64 query rows. S = Q K^T and O += P V run as mma.sync m16n8k16 (fp16 in, fp32 out); the scores are
+// scaled and rounded to fp16 exactly where MultiHeadAttention stores them (gpu_kernels.h:171-175), the softmax is the online
+// form in fp32, P is rounded to fp16 for the second product (the reference's att buffer is fp16 too) and its row sums come
+// from the same product with a column of ones. head_size 128. Keys beyond the last row's position are zero-filled and masked.
+//
+// The tensor pipe is the bound (1024 clocks per 64 x 64 block and SM); everything else has to fit under it. Chunks are copied
+// with cp.async one ahead of the math; both operands come through ldmatrix (K as it lies, V transposed); only the chunks a
+// warp's diagonal crosses are masked; the running output is scaled only when a maximum moved; the CTAs with the most keys
+// start first; three CTAs of four warps per SM cover each other's softmax. 2000 rows of 32 heads: 231 -> 143 us, 512 rows:
+// 42 -> 22 us (before: single-buffered chunks, 4-byte fragment loads of K, every chunk masked).
 constexpr int kAtRows = 64, kAtKeys = 64, kAtLd = 136;   // 136 halfs = 272 B between rows: conflict-free fragment loads
+constexpr int kAtChunk = kAtKeys * kAtLd;                // halfs of a chunk of K or V
+constexpr size_t kAtSmem = 2 * 2 * (size_t)kAtChunk * sizeof(__half);   // two buffers of K and V
 
 __device__ __forceinline__ void mma_f16(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -273,23 +281,43 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// 16 bytes to shared memory, zeros where !valid (src is readable either way)
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
 
 // grid (heads, ceil(n / 64)), block 128. kc / vc point at this layer's cache rows of the sequence (position 0).
-__global__ void __launch_bounds__(128) attention_prefill_kernel(__half* out, const __half* q, int ldq, const __half* kc, const __half* vc, int n_heads, int kv_mul,
-                                                                int n, int pos0, int kv_n) {
+__global__ void __launch_bounds__(128, 3) attention_prefill_kernel(__half* out, const __half* q, int ldq, const __half* kc, const __half* vc, int n_heads, int kv_mul,
+                                                                   int n, int pos0, int kv_n) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
     constexpr int HS = 128;
-    __shared__ __align__(16) __half sK[kAtKeys][kAtLd];
-    __shared__ __align__(16) __half sV[kAtKeys][kAtLd];
-    const int h = blockIdx.x, m0 = blockIdx.y * kAtRows;
+    extern __shared__ __align__(16) __half at_smem[];   // [2 buffers][K, V][kAtKeys][kAtLd]
+    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(at_smem);
+    const int h = blockIdx.x, m0 = (int)(gridDim.y - 1 - blockIdx.y) * kAtRows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int row_a = m0 + warp * 16 + g, row_b = row_a + 8;          // this thread's two query rows
     const int last_pos = pos0 + n - 1;                                // newest cache row that is valid
     const int pos_a = min(pos0 + row_a, last_pos), pos_b = min(pos0 + row_b, last_pos);
+    const int warp_first = min(pos0 + m0 + warp * 16, last_pos);      // newest key that every row of this warp attends to
     const int warp_last = min(pos0 + m0 + warp * 16 + 15, last_pos);  // newest key any row of this warp attends to
     const int cta_last = min(pos0 + m0 + kAtRows - 1, last_pos);
     const size_t head_off = (size_t)(h / kv_mul) * HS;
+
+    const int piece = (threadIdx.x & 15) * 8, row0 = threadIdx.x >> 4;   // this thread copies rows row0, row0 + 8, ... of a chunk
+    auto load_chunk = [&](int t0, int buf) {
+        const uint32_t dst = smem + (uint32_t)(2 * buf * kAtChunk + row0 * kAtLd + piece) * 2;
+#pragma unroll
+        for (int i = 0; i < kAtKeys / 8; i++) {
+            const int key = t0 + row0 + 8 * i;
+            const bool valid = key <= cta_last;
+            const size_t off = (size_t)(valid ? key : 0) * kv_n + head_off + piece;
+            cp_async16_or_zero(dst + i * 8 * kAtLd * 2, kc + off, valid);
+            cp_async16_or_zero(dst + (kAtChunk + i * 8 * kAtLd) * 2, vc + off, valid);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_chunk(0, 0);
 
     // Q fragments: 8 k-steps of 16 dims; rows past the prompt read as zero
     uint32_t qa[8][4];
@@ -305,94 +333,99 @@ __global__ void __launch_bounds__(128) attention_prefill_kernel(__half* out, con
         }
     }
     const float alpha = (float)(1.0 / sqrt((double)HS));
-    float o[16][4];
+    float o[16][4], l[4] = {0.f, 0.f, 0.f, 0.f};   // l: row sums of P (rows a: elements 0, 1; rows b: 2, 3)
 #pragma unroll
     for (int d = 0; d < 16; d++) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
-    float mx_a = -CUDART_INF_F, mx_b = -CUDART_INF_F, l_a = 0.f, l_b = 0.f;
+    float mx_a = -CUDART_INF_F, mx_b = -CUDART_INF_F;
 
-    for (int t0 = 0; t0 <= cta_last; t0 += kAtKeys) {
-        __syncthreads();   // the previous chunk is consumed
-        for (int i = threadIdx.x; i < kAtKeys * (HS / 8); i += 128) {
-            const int r = i >> 4, c = (i & 15) * 8, key = t0 + r;
-            uint4 kv = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
-            if (key <= cta_last) {
-                kv = *reinterpret_cast<const uint4*>(kc + (size_t)key * kv_n + head_off + c);
-                vv = *reinterpret_cast<const uint4*>(vc + (size_t)key * kv_n + head_off + c);
+    for (int t0 = 0, buf = 0; t0 <= cta_last; t0 += kAtKeys, buf ^= 1) {
+        if (t0 + kAtKeys <= cta_last) {
+            load_chunk(t0 + kAtKeys, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();           // the chunk has landed for every thread
+        if (t0 <= warp_last) {     // (warp-uniform; else nothing of this chunk is visible to the warp's rows)
+            const uint32_t sk = smem + (uint32_t)(2 * buf * kAtChunk) * 2, sv = sk + kAtChunk * 2;
+            // S = Q K^T for 16 rows x 64 keys, scaled and rounded to fp16 as the reference stores the scores
+            __half2 sc[8][2];
+#pragma unroll
+            for (int jj = 0; jj < 8; jj += 4) {
+                float c[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+#pragma unroll
+                for (int s = 0; s < 8; s += 2) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        uint32_t b0, b1, b2, b3;
+                        const uint32_t addr = sk + (uint32_t)((8 * (jj + j) + (lane & 7)) * kAtLd + 16 * s + 8 * (lane >> 3)) * 2;
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr) : "memory");
+                        mma_f16(c[j], qa[s], b0, b1);
+                        mma_f16(c[j], qa[s + 1], b2, b3);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    sc[jj + j][0] = __floats2half2_rn(c[j][0] * alpha, c[j][1] * alpha);
+                    sc[jj + j][1] = __floats2half2_rn(c[j][2] * alpha, c[j][3] * alpha);
+                }
             }
-            *reinterpret_cast<uint4*>(&sK[r][c]) = kv;
-            *reinterpret_cast<uint4*>(&sV[r][c]) = vv;
-        }
-        __syncthreads();
-        if (t0 > warp_last) continue;   // warp-uniform: nothing of this chunk is visible to the warp's rows
-
-        // S = Q K^T for 16 rows x 64 keys
-        float sc[8][4];
+            if (t0 + kAtKeys - 1 > warp_first) {   // the diagonal, or the end of the keys
+                const __half ninf = __ushort_as_half((unsigned short)0xFC00u);
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
+                for (int j = 0; j < 8; j++) {
+                    const int key = t0 + 8 * j + 2 * t;
+                    sc[j][0] = __halves2half2(key <= pos_a ? __low2half(sc[j][0]) : ninf, key + 1 <= pos_a ? __high2half(sc[j][0]) : ninf);
+                    sc[j][1] = __halves2half2(key <= pos_b ? __low2half(sc[j][1]) : ninf, key + 1 <= pos_b ? __high2half(sc[j][1]) : ninf);
+                }
+            }
+            __half2 cm_a = sc[0][0], cm_b = sc[0][1];
 #pragma unroll
-            for (int s = 0; s < 8; s++) {
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&sK[8 * j + g][16 * s + 2 * t]);
-                const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&sK[8 * j + g][16 * s + 2 * t + 8]);
-                mma_f16(sc[j], qa[s], b0, b1);
+            for (int j = 1; j < 8; j++) {
+                cm_a = __hmax2(cm_a, sc[j][0]);
+                cm_b = __hmax2(cm_b, sc[j][1]);
+            }
+            float ca = fmaxf(__low2float(cm_a), __high2float(cm_a)), cb = fmaxf(__low2float(cm_b), __high2float(cm_b));
+            ca = fmaxf(ca, __shfl_xor_sync(0xffffffffu, ca, 1));
+            ca = fmaxf(ca, __shfl_xor_sync(0xffffffffu, ca, 2));
+            cb = fmaxf(cb, __shfl_xor_sync(0xffffffffu, cb, 1));
+            cb = fmaxf(cb, __shfl_xor_sync(0xffffffffu, cb, 2));
+            // key 0 is visible to every row, so after the first chunk the running maxima are finite
+            const float nm_a = fmaxf(mx_a, ca), nm_b = fmaxf(mx_b, cb);
+            if (__any_sync(0xffffffffu, nm_a != mx_a || nm_b != mx_b)) {
+                const float corr_a = __expf(mx_a - nm_a), corr_b = __expf(mx_b - nm_b);
+#pragma unroll
+                for (int d = 0; d < 16; d++) { o[d][0] *= corr_a; o[d][1] *= corr_a; o[d][2] *= corr_b; o[d][3] *= corr_b; }
+                l[0] *= corr_a; l[1] *= corr_a; l[2] *= corr_b; l[3] *= corr_b;
+                mx_a = nm_a; mx_b = nm_b;
+            }
+            // P = exp(S - max), rounded to fp16, as A fragments (k-step jj covers keys 16 jj .. 16 jj + 15); O += P V with the V
+            // fragments through ldmatrix.trans (V is [key][dim]; the product wants keys along k)
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+                uint32_t pa[4];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const float2 fa = __half22float2(sc[2 * jj + u][0]), fb = __half22float2(sc[2 * jj + u][1]);
+                    pa[2 * u] = pack_h2(__expf(fa.x - nm_a), __expf(fa.y - nm_a));
+                    pa[2 * u + 1] = pack_h2(__expf(fb.x - nm_b), __expf(fb.y - nm_b));
+                }
+                mma_f16(l, pa, 0x3C003C00u, 0x3C003C00u);
+#pragma unroll
+                for (int d = 0; d < 16; d += 2) {
+                    uint32_t v0, v1, v2, v3;
+                    const uint32_t addr = sv + (uint32_t)((16 * jj + (lane & 15)) * kAtLd + 8 * d + 8 * (lane >> 4)) * 2;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3) : "r"(addr) : "memory");
+                    mma_f16(o[d], pa, v0, v1);
+                    mma_f16(o[d + 1], pa, v2, v3);
+                }
             }
         }
-        // scale, round to fp16 as the reference stores the scores, mask, chunk maxima
-        float cm_a = -CUDART_INF_F, cm_b = -CUDART_INF_F;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int key = t0 + 8 * j + 2 * t + (e & 1);
-                const int pos = (e < 2) ? pos_a : pos_b;
-                float v = __half2float(__float2half(sc[j][e] * alpha));
-                v = key <= pos ? v : -CUDART_INF_F;
-                sc[j][e] = v;
-                if (e < 2) cm_a = fmaxf(cm_a, v); else cm_b = fmaxf(cm_b, v);
-            }
-        }
-        cm_a = fmaxf(cm_a, __shfl_xor_sync(0xffffffffu, cm_a, 1));
-        cm_a = fmaxf(cm_a, __shfl_xor_sync(0xffffffffu, cm_a, 2));
-        cm_b = fmaxf(cm_b, __shfl_xor_sync(0xffffffffu, cm_b, 1));
-        cm_b = fmaxf(cm_b, __shfl_xor_sync(0xffffffffu, cm_b, 2));
-        // key 0 is visible to every row, so after the first chunk the running maxima are finite
-        const float nm_a = fmaxf(mx_a, cm_a), nm_b = fmaxf(mx_b, cm_b);
-        const float corr_a = __expf(mx_a - nm_a), corr_b = __expf(mx_b - nm_b);
-        mx_a = nm_a; mx_b = nm_b;
-        float sum_a = 0.f, sum_b = 0.f;
-        uint32_t pa[4][4];   // P as A fragments: k-step jj covers keys 16 jj .. 16 jj + 15
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const __half2 p01 = __floats2half2_rn(__expf(sc[j][0] - nm_a), __expf(sc[j][1] - nm_a));
-            const __half2 p23 = __floats2half2_rn(__expf(sc[j][2] - nm_b), __expf(sc[j][3] - nm_b));
-            sum_a += __low2float(p01) + __high2float(p01);
-            sum_b += __low2float(p23) + __high2float(p23);
-            pa[j >> 1][(j & 1) * 2 + 0] = *reinterpret_cast<const uint32_t*>(&p01);
-            pa[j >> 1][(j & 1) * 2 + 1] = *reinterpret_cast<const uint32_t*>(&p23);
-        }
-        l_a = l_a * corr_a + sum_a;
-        l_b = l_b * corr_b + sum_b;
-#pragma unroll
-        for (int d = 0; d < 16; d++) { o[d][0] *= corr_a; o[d][1] *= corr_a; o[d][2] *= corr_b; o[d][3] *= corr_b; }
-        // O += P V: V fragments through ldmatrix.trans (V is [key][dim]; the product wants keys along k)
-#pragma unroll
-        for (int jj = 0; jj < 4; jj++) {
-#pragma unroll
-            for (int d = 0; d < 16; d += 2) {
-                uint32_t v0, v1, v2, v3;
-                const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&sV[16 * jj + (lane & 15)][8 * d + 8 * (lane >> 4)]);
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3) : "r"(addr));
-                mma_f16(o[d], pa[jj], v0, v1);
-                mma_f16(o[d + 1], pa[jj], v2, v3);
-            }
-        }
+        __syncthreads();   // the chunk is consumed: its buffer is filled again in the next round
     }
-    // the quad's partial row sums, then O / l
-    l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
-    l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
-    l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
-    l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-    const float inv_a = l_a > 0.f ? 1.0f / l_a : 0.f, inv_b = l_b > 0.f ? 1.0f / l_b : 0.f;
+    const float inv_a = l[0] > 0.f ? 1.0f / l[0] : 0.f, inv_b = l[2] > 0.f ? 1.0f / l[2] : 0.f;
 #pragma unroll
     for (int d = 0; d < 16; d++) {
         if (row_a < n) *reinterpret_cast<uint32_t*>(out + ((size_t)row_a * n_heads + h) * HS + 8 * d + 2 * t) = pack_h2(o[d][0] * inv_a, o[d][1] * inv_a);
@@ -753,6 +786,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
     // A prompt's rows on one GPU: the o and down projections leave their result in XB / ATT and the next RMSNorm adds it to x
     // (with more ranks the partial sums have to be exchanged as x first: the GEMM adds the residual itself).
     const bool fused_add = !skinny && g == 1;
+    if (pos0 >= 0 && !skinny) Q4_CUDA_TRY(cudaFuncSetAttribute(attention_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAtSmem));
     auto norm = [&](const __half* w, const __half* y) {
         if (y) launch_rows(overlap, rmsnorm_rows_kernel<true>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, y, w, dim);
         else launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, w, dim);
@@ -788,7 +822,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
             break;
         }
         if (pos0 >= 0 && !skinny)
-            launch_rows(overlap, attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), 0, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
+            launch_rows(overlap, attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), kAtSmem, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
                         m->kv_mul, n, pos0, m->kv_n);
         else
             launch_rows(overlap, attention_rows_kernel, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,

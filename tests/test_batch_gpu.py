@@ -90,6 +90,32 @@ def test_prefill_hand_off_and_pieces(mid_path):
     t.close()
 
 
+@pytest.fixture(scope="module")
+def long_path(tmp_path_factory):
+    p = tmp_path_factory.mktemp("models") / "mid_long.bin"
+    synth.write_model_file(str(p), "mid-long", seed=6)
+    return str(p)
+
+
+@pytest.mark.parametrize("history,n", [(0, 64), (0, 65), (1, 63), (63, 17), (64, 64), (30, 129)])
+def test_prefill_attention_at_chunk_edges(long_path, history, n):
+    """The prompt attention works on 64 query rows and 64 keys at a time: prompts that end on, before and behind such an edge,
+    and whose diagonal crosses a chunk elsewhere because of a history, against the token-by-token run."""
+    vocab = synth.CONFIGS["mid-long"][5]
+    tokens = np.random.default_rng(history + n).integers(3, vocab, size=history + n, dtype=np.int32)
+    ref = token_by_token(long_path, tokens, 1, {history + n - 1})
+    t = Transformer(long_path)
+    t.reset(tokens, 0)
+    for pos in range(history):
+        t.forward(gen_token=False, path=1)
+    t.prefill(n, gen_token=False)
+    t.synchronize()
+    got = t.logits()
+    assert t.status() == 0 and t.shared().pos == history + n
+    t.close()
+    assert_close(got, ref[history + n - 1], f"{n} tokens behind {history}", max_rel=2 * MAX_REL)   # both sides are within MAX_REL of the oracle
+
+
 def test_generate_with_the_prompt_in_one_pass(mid_path):
     """q4_generate with Q4_PATH_PROMPT_ONE_PASS: same ids as prefill of the prompt but its last position followed by the
     token loop done by hand, the same count of timed tokens as the plain loop, and a sampled run draws the coins the token
