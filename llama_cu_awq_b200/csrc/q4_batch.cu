@@ -171,37 +171,61 @@ __global__ void rope_rows_table_kernel(float2* table, int positions, int head_si
         table[i] = rope_cos_sin(i / half_hs, i % half_hs, head_size, theta);
 }
 
-// MultiHeadAttention (llama2_q4.cu:410-427) for one (row, head): the query attends to cached positions 0 .. pos of its own
-// sequence (its own K/V row was stored by the RoPE kernel before). Scores are rounded to fp16 as the reference stores them
-// (gpu_kernels.h:171-175); the softmax runs online in fp32 over the keys a warp visits, the warps are merged at the end.
-// A warp takes four keys per round (keys 4 (warp + 8 i) .. + 3) and issues their eight K/V loads together, so a round costs
-// one memory latency, not eight. head_size 128: a lane holds four dims. grid (heads, rows), block 256.
+// MultiHeadAttention (llama2_q4.cu:410-427) for one (row, head): the query attends to positions 0 .. pos of its own sequence.
+// Scores are rounded to fp16 as the reference stores them (gpu_kernels.h:171-175); the softmax runs online in fp32 over the keys
+// a warp visits, the warps are merged at the end. A warp takes four keys per round (keys 4 (warp + 8 i) .. + 3) and issues
+// their eight K/V loads together, so a round costs one memory latency, not eight. head_size 128: a lane holds four dims.
+// grid (heads, rows), block 256.
+// FUSED (batched decode: no two rows of a launch share a sequence): q, k and v come as the projections left them. Every warp
+// rotates its query (rope_store_rows_kernel's table and rounding), the warp whose turn position pos is rotates the new key
+// and takes it and the new value from registers, and the first query head of a key/value head files both in the cache: one
+// launch less per layer (batch-8 step of four 7B layers: 247 -> 231 us). Otherwise the row's K and V are in the cache already and q is rotated.
 constexpr int kAttWarps = 8, kAttKeys = 4;
-__global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* out, const __half* q, int ldq, const __half* kc, const __half* vc, int n_heads, int kv_mul,
-                                                                       const int* row_seq, const int* row_pos, long long seq_stride, long long loff, int kv_n) {
+template <bool FUSED>
+__global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* out, const __half* q, int ldq, __half* kc, __half* vc, int n_heads, int kv_mul,
+                                                                       const int* row_seq, const int* row_pos, long long seq_stride, long long loff, int kv_n,
+                                                                       const __half* knew, const __half* vnew, const float2* table) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
     constexpr int HS = 128;
     const int h = blockIdx.x, m = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int T = row_pos[m] + 1;
-    const __half* kb = kc + (size_t)row_seq[m] * seq_stride + loff + (size_t)(h / kv_mul) * HS + lane * 4;
-    const __half* vb = vc + (size_t)row_seq[m] * seq_stride + loff + (size_t)(h / kv_mul) * HS + lane * 4;
+    const int pos = row_pos[m];
+    const int T = FUSED ? pos : pos + 1;   // positions read from the cache
+    const size_t head_at = (size_t)row_seq[m] * seq_stride + loff + (size_t)(h / kv_mul) * HS + lane * 4;
+    const __half* kb = kc + head_at;
+    const __half* vb = vc + head_at;
+    float4 cs01 = {}, cs23 = {};   // (cos, sin) of this lane's four pairs
+    if (FUSED) {
+        const float4* tp = reinterpret_cast<const float4*>(table + (size_t)pos * (HS / 2) + (lane & 15) * 4);
+        cs01 = __ldg(tp);
+        cs23 = __ldg(tp + 1);
+    }
+    // four elements of a head whose other halves of the pairs lie 16 lanes away, rotated and rounded to fp16
+    auto rotate = [&](uint2 v) {
+        uint2 o;
+        o.x = __shfl_xor_sync(0xffffffffu, v.x, 16);
+        o.y = __shfl_xor_sync(0xffffffffu, v.y, 16);
+        const uint2 l = lane < 16 ? v : o, g = lane < 16 ? o : v;
+        __half lo[4], hi[4];
+        *reinterpret_cast<uint2*>(lo) = l;
+        *reinterpret_cast<uint2*>(hi) = g;
+        rope_rotate(lo, hi, lo, hi, make_float2(cs01.x, cs01.y));
+        rope_rotate(lo + 1, hi + 1, lo + 1, hi + 1, make_float2(cs01.z, cs01.w));
+        rope_rotate(lo + 2, hi + 2, lo + 2, hi + 2, make_float2(cs23.x, cs23.y));
+        rope_rotate(lo + 3, hi + 3, lo + 3, hi + 3, make_float2(cs23.z, cs23.w));
+        return lane < 16 ? *reinterpret_cast<uint2*>(lo) : *reinterpret_cast<uint2*>(hi);
+    };
     float qf[4];
     {
-        const uint2 qv = *reinterpret_cast<const uint2*>(q + (size_t)m * ldq + (size_t)h * HS + lane * 4);
+        uint2 qv = *reinterpret_cast<const uint2*>(q + (size_t)m * ldq + (size_t)h * HS + lane * 4);
+        if (FUSED) qv = rotate(qv);
         const __half2* qh = reinterpret_cast<const __half2*>(&qv);
         qf[0] = __low2float(qh[0]); qf[1] = __high2float(qh[0]); qf[2] = __low2float(qh[1]); qf[3] = __high2float(qh[1]);
     }
     const float alpha = (float)(1.0 / sqrt((double)HS));
     float mx = -CUDART_INF_F, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int t0 = warp * kAttKeys; t0 < T; t0 += kAttWarps * kAttKeys) {
-        uint2 kv[kAttKeys], vv[kAttKeys];
-#pragma unroll
-        for (int u = 0; u < kAttKeys; u++) {
-            const int t = min(t0 + u, T - 1);   // a round's tail re-reads the last key; its weight is forced to zero below
-            kv[u] = *reinterpret_cast<const uint2*>(kb + (size_t)t * kv_n);
-            vv[u] = *reinterpret_cast<const uint2*>(vb + (size_t)t * kv_n);
-        }
+    // keys kv[u], values vv[u]; those with u >= live do not count (the first always does)
+    auto round4 = [&](const uint2 (&kv)[kAttKeys], const uint2 (&vv)[kAttKeys], int live) {
         float sc[kAttKeys];
 #pragma unroll
         for (int u = 0; u < kAttKeys; u++) {
@@ -215,10 +239,10 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* 
         float mn = mx;
 #pragma unroll
         for (int u = 0; u < kAttKeys; u++) {
-            sc[u] = t0 + u < T ? __half2float(__float2half(sc[u] * alpha)) : -CUDART_INF_F;
+            sc[u] = u < live ? __half2float(__float2half(sc[u] * alpha)) : -CUDART_INF_F;
             mn = fmaxf(mn, sc[u]);
         }
-        const float corr = expf(mx - mn);   // key t0 itself is always valid, so mn is finite
+        const float corr = expf(mx - mn);   // the round's first key is always valid, so mn is finite
         l *= corr;
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[j] *= corr;
@@ -233,6 +257,28 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* 
             acc[3] += pr * __high2float(vh[1]);
         }
         mx = mn;
+    };
+    for (int t0 = warp * kAttKeys; t0 <= pos; t0 += kAttWarps * kAttKeys) {
+        uint2 kv[kAttKeys], vv[kAttKeys];
+        const bool with_new = FUSED && t0 + kAttKeys > pos;   // position pos is one of this round's keys
+#pragma unroll
+        for (int u = 0; u < kAttKeys; u++) {
+            const int t = max(min(t0 + u, T - 1), 0);   // a round's tail reads some earlier row instead (row 0 where there is none)
+            kv[u] = *reinterpret_cast<const uint2*>(kb + (size_t)t * kv_n);
+            vv[u] = *reinterpret_cast<const uint2*>(vb + (size_t)t * kv_n);
+        }
+        if (with_new) {
+            const size_t at = (size_t)m * kv_n + (size_t)(h / kv_mul) * HS + lane * 4;
+            const uint2 k = rotate(*reinterpret_cast<const uint2*>(knew + at)), v = *reinterpret_cast<const uint2*>(vnew + at);
+#pragma unroll
+            for (int u = 0; u < kAttKeys; u++)
+                if (t0 + u >= pos) { kv[u] = k; vv[u] = v; }   // (those behind it do not count, but must not bring in a NaN)
+            if (h % kv_mul == 0) {
+                *reinterpret_cast<uint2*>(kc + head_at + (size_t)pos * kv_n) = k;
+                *reinterpret_cast<uint2*>(vc + head_at + (size_t)pos * kv_n) = v;
+            }
+        }
+        round4(kv, vv, pos + 1 - t0);
     }
     __shared__ float s_m[kAttWarps], s_l[kAttWarps], s_acc[kAttWarps][HS];
     if (lane == 0) { s_m[warp] = mx; s_l[warp] = l; }
@@ -804,8 +850,9 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
         const __half* kp = skinny ? r->K : r->QKV + m->q_n;
         const __half* vp = skinny ? r->V : r->QKV + m->q_n + m->kv_n;
         const int ldq = skinny ? m->q_n : nqkv, ldkv = skinny ? m->kv_n : nqkv;
-        launch_rows(overlap, rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
-                    r->rope, r->row_seq, r->row_pos, seq_stride, loff);
+        if (pos0 >= 0)   // (batched decode: the attention kernel rotates and files)
+            launch_rows(overlap, rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
+                        r->rope, r->row_seq, r->row_pos, seq_stride, loff);
         if (l == c.n_layers - 1 && want != WANT_ALL) {
             if (want == WANT_CACHE) break;
             // one row: the split attention of the batch-1 path and the few-rows kernels
@@ -824,9 +871,12 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
         if (pos0 >= 0 && !skinny)
             launch_rows(overlap, attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), kAtSmem, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
                         m->kv_mul, n, pos0, m->kv_n);
+        else if (pos0 >= 0)
+            launch_rows(overlap, attention_rows_kernel<false>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
+                        r->row_pos, seq_stride, loff, m->kv_n, (const __half*)nullptr, (const __half*)nullptr, (const float2*)nullptr);
         else
-            launch_rows(overlap, attention_rows_kernel, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
-                        r->row_pos, seq_stride, loff, m->kv_n);
+            launch_rows(overlap, attention_rows_kernel<true>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
+                        r->row_pos, seq_stride, loff, m->kv_n, kp, vp, r->rope);
         // x = o_proj(att) + x / g, summed over the ranks (gpu_kernels.h:237-238, llama2_q4.cu:472-476)
         if (skinny) OP(q4_matmul_q4_rows(s, (uint16_t*)r->X, (const uint16_t*)r->ATT, &L.o.w, n, m->o_kc, dim, (const uint16_t*)r->X, 1.0f / g));
         else OP(gemm(fused_add ? r->Y : r->X, r->ATT, l, 1, !fused_add));
