@@ -153,13 +153,15 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const __half* __restrict__
 }
 
 // fp16 GEMV (classifier): out[d] = alpha * sum_n w[d][n] * x[n]. gpu_kernels.h:117-147.
-// One warp per 2 output rows; each lane streams 16-byte pieces, 4 per row in flight.
+// WK warps per 2 output rows, each taking every WK-th stretch of 128 16-byte pieces of the rows; their sums are added in warp
+// order. Each lane streams 16-byte pieces, 4 per row in flight.
 constexpr int kF16Rows = 2;
+template <int WK>
 __global__ void __launch_bounds__(256) matvec_f16_kernel(__half* out, const __half* x, const __half* __restrict__ w, int n, int d,
                                                          float alpha) {
     const int lane = threadIdx.x & 31;
-    const int warp_global = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int row0 = warp_global * kF16Rows;
+    const int warp = threadIdx.x >> 5;
+    const int row0 = (blockIdx.x * (8 / WK) + warp / WK) * kF16Rows;
     const bool active = row0 < d;
     const int nvec = n >> 3;  // uint4 per row
     constexpr int U = 4;
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(256) matvec_f16_kernel(__half* out, const __ha
     const uint4* wr[kF16Rows];
 #pragma unroll
     for (int r = 0; r < kF16Rows; r++) wr[r] = reinterpret_cast<const uint4*>(w + (size_t)min(row0 + r, d - 1) * n);
-    int c = lane;
+    int c = lane + (warp % WK) * U * 32;
     if (active) {
 #pragma unroll
         for (int r = 0; r < kF16Rows; r++)
@@ -177,16 +179,16 @@ __global__ void __launch_bounds__(256) matvec_f16_kernel(__half* out, const __ha
     }
     griddep_wait();
     griddep_launch_dependents();
-    if (!active) return;
+    if (WK == 1 && !active) return;
     float acc[kF16Rows] = {0.f, 0.f};
     const uint4* xv = reinterpret_cast<const uint4*>(x);
-    while (c < nvec) {
+    while (active && c < nvec) {
         uint4 cur[kF16Rows][U];
 #pragma unroll
         for (int r = 0; r < kF16Rows; r++)
 #pragma unroll
             for (int u = 0; u < U; u++) cur[r][u] = wv[r][u];
-        const int cn = c + U * 32;
+        const int cn = c + WK * U * 32;
 #pragma unroll
         for (int r = 0; r < kF16Rows; r++)
 #pragma unroll
@@ -210,6 +212,21 @@ __global__ void __launch_bounds__(256) matvec_f16_kernel(__half* out, const __ha
             }
         }
         c = cn;
+    }
+    __shared__ float part[8][kF16Rows];
+    if (WK > 1) {
+#pragma unroll
+        for (int r = 0; r < kF16Rows; r++) {
+            const float s = warp_sum(acc[r]);
+            if (lane == 0) part[warp][r] = s;
+        }
+        __syncthreads();
+        if (warp % WK || lane >= kF16Rows || row0 + lane >= d) return;
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < WK; k++) s += part[warp + k][lane];
+        out[row0 + lane] = __float2half(s * alpha);
+        return;
     }
 #pragma unroll
     for (int r = 0; r < kF16Rows; r++) {
@@ -273,9 +290,16 @@ extern "C" int q4_argmax(void* stream, const uint16_t* logits, int size, int* to
 extern "C" int q4_matmul_f16(void* stream, uint16_t* xout, const uint16_t* x, const uint16_t* w, int n, int d, float alpha) {
     if ((n & 7) || (d & 7) || n <= 0 || d <= 0) return Q4_ERR_UNSUPPORTED_SIZE;
     if (!xout || !x || !w) return Q4_ERR_INVALID;
-    const int rows_per_block = 8 * kF16Rows;
-    Q4Launch L(dim3(q4_div_up(d, rows_per_block)), dim3(256), 0, (cudaStream_t)stream);
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, matvec_f16_kernel, (__half*)xout, (const __half*)x, (const __half*)w, n, d, alpha));
+    // As many warps per row pair as keep the grid within two CTAs per SM: one warp over the whole of a row is a chain of loads that
+    // a few CTAs cannot cover (8192 x 384: 12.1 us with one, 2.6 with eight; 4096 x 1000: 6.6, 2.7 with four; 4096 x 2000: 7.4, 4.7
+    // with two), and beyond that the split only costs (4096 x 4000: 8.3 us with one, 9.3 with two; 4096 x 32000: 45.2, 46.2).
+    constexpr int kMaxCtas = 2 * 148;
+    auto launch = [&](auto kernel, int wk) {
+        Q4Launch L(dim3(q4_div_up(d, 8 / wk * kF16Rows)), dim3(256), 0, (cudaStream_t)stream);
+        return cudaLaunchKernelEx(&L.cfg, kernel, (__half*)xout, (const __half*)x, (const __half*)w, n, d, alpha);
+    };
+    auto fits = [&](int wk) { return q4_div_up(d, 8 / wk * kF16Rows) <= kMaxCtas; };
+    Q4_CUDA_TRY(fits(8) ? launch(matvec_f16_kernel<8>, 8) : fits(4) ? launch(matvec_f16_kernel<4>, 4) : fits(2) ? launch(matvec_f16_kernel<2>, 2) : launch(matvec_f16_kernel<1>, 1));
     return Q4_OK;
 }
 

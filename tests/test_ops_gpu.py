@@ -84,6 +84,23 @@ def test_classifier_matvec_f16(n, d):
     assert_close(y.cpu().numpy(), O.matvec_f16(x, W, n, d, order=1), "classifier", max_rel=2e-3)
 
 
+@pytest.mark.parametrize("d", [8, 592, 600, 1184, 1192, 2368, 2376])
+@pytest.mark.parametrize("n", [8, 1032, 4096])
+def test_classifier_matvec_f16_split_edges(n, d):
+    """The sizes on both sides of every split of a row over warps, rows shorter than the split and rows with a remainder. Against
+    64 bits: one rounding to fp16 (2^-11 of the value, 2^-25 where it is a denormal) and fp32 roundings of a chain of n / 32 fused
+    multiply-adds in a lane (rounded up to a 16-byte piece), five additions of lanes and at most eight of warps."""
+    rng = np.random.default_rng(n * d)
+    W = (rng.standard_normal((d, n)) * 0.02).astype(np.float16)
+    x = rng.standard_normal(n).astype(np.float16)
+    y = torch.full((d,), float("nan"), dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), dev(W), n, d)
+    ref = W.astype(np.float64) @ x.astype(np.float64)
+    terms = np.abs(W).astype(np.float64) @ np.abs(x).astype(np.float64)
+    bound = np.abs(ref) * 2.0**-11 + 2.0**-25 + 1.01 * (n / 32 + 8 + 5 + 8) * 2.0**-24 * terms
+    assert (np.abs(y.cpu().numpy().astype(np.float64) - ref) <= bound).all()
+
+
 def _pinned_mailbox():
     t = torch.zeros(4 + 64, dtype=torch.int32).pin_memory()
     return t  # [0] = pos, [4:] = tokens (layout is private to this test)
