@@ -222,9 +222,17 @@ struct Segments {
 // the pair whose share holds global chunk c
 __device__ __forceinline__ int pair_of(long long c, long long total, int pairs) { return (int)(((c + 1) * pairs - 1) / total); }
 
-// silu(g) * u with the hardware's exponential and reciprocal (relative error near 1e-6, the result is rounded to fp16): four warps
-// evaluate 128 of them per thread and tile, and with expf and an IEEE division that took longer than the tile's MMAs.
-__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
+// silu(g) * u in the arithmetic of ffn_matvec_silu_kernel (gpu_kernels.h:278-281): g *= 1 / (1 + expf(-g)), times u, in fp32. The
+// reciprocal is the hardware's with one Newton step: compared over all 65536 fp16 gates, g / (1 + e) has the bits of the IEEE division
+// but for the 22 gates between -88.75 and -87.3, whose reciprocal is a denormal and whose result is zero in fp16 either way. The
+// division's own branch kept the compiler from interleaving evaluations (512 x 4096 x 22016: 12 us longer).
+__device__ __forceinline__ float silu_mul(float g, float u) {
+    const float d = 1.0f + expf(-g);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = d < 0x1p126f ? fmaf(r, fmaf(-d, r, 1.0f), r) : r;
+    return g * r * u;
+}
 
 // ---- epilogue pieces: 32 accumulator columns (= batch rows c0 .. c0 + 31 of the tile) of one feature, as 16 packed words ----
 template <int EPI>
@@ -240,29 +248,30 @@ __device__ __forceinline__ void epi_pack(const float (&v)[32], const uint32_t* r
         out[j] = h22u(__floats2half2_rn(a, b));
     }
 }
-// The 32 rows of the chunk into the staging buffer [row][this CTA's outputs of a row] (two bytes per lane, 64 B per warp store).
-// EPI_SILU: features 2j and 2j + 1 are gate j and up j (rounded to fp16 like every GEMM result, silu and product in fp32:
-// gpu_kernels.h:278-281). Neighbouring lanes swap halves of a word so that the even lane holds the pair of the even row and the
-// odd lane that of the odd one.
-template <int EPI>
+// The 32 rows of the chunk into a staging buffer [row][128 features] (two bytes per lane, 64 B per warp store).
 __device__ __forceinline__ void epi_stage(const uint32_t* out, uint8_t* buf, int r) {
-    if (EPI == EPI_SILU) {
-        const bool odd = r & 1;
-        unsigned short* p = reinterpret_cast<unsigned short*>(buf) + (odd ? kBN / 2 : 0) + (r >> 1);
+    unsigned short* p = reinterpret_cast<unsigned short*>(buf) + r;
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, out[j], 1);
-            const __half2 mine = u2h2(out[j]), theirs = u2h2(got);
-            const float gate = odd ? __high2float(theirs) : __low2float(mine), up = odd ? __high2float(mine) : __low2float(theirs);
-            p[j * kBN] = __half_as_ushort(__float2half(silu_mul(gate, up)));
-        }
-    } else {
-        unsigned short* p = reinterpret_cast<unsigned short*>(buf) + r;
+    for (int j = 0; j < 16; j++) {
+        p[(2 * j) * kBN] = (unsigned short)(out[j] & 0xFFFFu);
+        p[(2 * j + 1) * kBN] = (unsigned short)(out[j] >> 16);
+    }
+}
+// EPI_SILU: features 2j and 2j + 1 are gate j and up j (rounded to fp16 like every GEMM result), one word of the staged rows; silu
+// and product in fp32 go to the store buffer [row][64]. Rolled over the staged words: evaluated on the registers before they are
+// staged, fully unrolled, the same arithmetic cost 27 us more for 512 x 4096 x 22016 (64 evaluations per thread and tile in each of
+// nine places of the code).
+__device__ __forceinline__ void epi_silu(const uint8_t* staged, uint8_t* buf, int etid) {
+    const __half2* src = reinterpret_cast<const __half2*>(staged);
+    __half* dst = reinterpret_cast<__half*>(buf);
+    constexpr int U = 8;   // in flight per thread
+#pragma unroll 1
+    for (int i = etid; i < kOutRows * kBN / 2; i += U * kEpiWarps * 32) {
+        float2 gu[U];
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            p[(2 * j) * kBN] = (unsigned short)(out[j] & 0xFFFFu);
-            p[(2 * j + 1) * kBN] = (unsigned short)(out[j] >> 16);
-        }
+        for (int k = 0; k < U; k++) gu[k] = __half22float2(src[i + k * kEpiWarps * 32]);
+#pragma unroll
+        for (int k = 0; k < U; k++) dst[i + k * kEpiWarps * 32] = __float2half(silu_mul(gu[k].x, gu[k].y));
     }
 }
 __device__ __forceinline__ void epi_load_residual(uint32_t* res, const __half* x, int c0, int rows, size_t ld) {
@@ -499,18 +508,25 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // Y leaves through shared memory: 32 rows are staged and written by one tensor copy (rows and columns beyond Y are
         // clipped there) while the next 32 are staged. Storing from the registers (a lane is a feature, so two bytes per lane and
         // row) took 34000 to 40000 clocks per 256-row tile, more than its 32 chunks of MMAs.
-        uint8_t* sY = sB + kRingBytes;
+        uint8_t* sY = sB + kRingBytes;   // two store buffers; EPI_SILU: the staged gates and ups, and two store buffers of half the size
         int buf = 0;
         auto put = [&](const uint32_t* out, int nt, int row0, int rows_left) {   // all epilogue threads; rows_left > 0
+            uint8_t* store = EPI == EPI_SILU ? sY + kOutBytes + buf * (kOutBytes / 2) : sY + buf * kOutBytes;
             if (etid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the copy that read this buffer last is done
             asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
-            epi_stage<EPI>(out, sY + buf * kOutBytes, r);
+            if (EPI == EPI_SILU) {
+                epi_stage(out, sY, r);
+                asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+                epi_silu(sY, store, etid);
+            } else {
+                epi_stage(out, store, r);
+            }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
             if (etid == 0) {
                 const int col = (nt * kPairN + rank * kBN) / (EPI == EPI_SILU ? 2 : 1);
                 if (rows_left > 0 && nt * kPairN + rank * kBN < p.N)
-                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&map_y), "r"(smem_addr(sY + buf * kOutBytes)), "r"(col), "r"(row0)
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&map_y), "r"(smem_addr(store)), "r"(col), "r"(row0)
                                  : "memory");
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
@@ -872,3 +888,12 @@ extern "C" int q4_time_matmul_q4_batched(void* stream, uint16_t* y, const uint16
     *us_per_launch = 1e3 * ms / ((double)reps * nmat);
     return Q4_OK;
 }
+
+#ifdef Q4_TEST_BUILD
+// The gate / up form by itself (the product reaches it through prompts only). `weight` is in file layout, rows 2j and 2j + 1 gate j and
+// up j; `interleaved` as from q4_gemm_interleave_weights; y is [M][N / 2].
+extern "C" int q4_test_gemm_silu(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* interleaved, int M, int K, int N,
+                                 void* workspace, size_t workspace_bytes) {
+    return q4_gemm_launch(stream, y, x, w, interleaved, M, K, N, nullptr, 0.f, true, workspace, workspace_bytes);
+}
+#endif  // Q4_TEST_BUILD

@@ -98,6 +98,38 @@ def test_residual_epilogue(M, K, N):
     assert_close(yd.cpu().numpy(), x.astype(np.float64) @ w.T + 0.5 * r, f"{M}x{K}x{N} + residual", max_rel=4e-3)
 
 
+@pytest.mark.parametrize("M", [40, 512])
+def test_gate_up_epilogue_values(M):
+    """silu(gate) * up as the GEMM's epilogue forms it, for gates and ups that the test chooses (one weight of a row is not zero): the
+    result is the rounding of a value within the fp32 evaluation's error of the 64-bit one. That error: expf 2 ulp (2^-22), then
+    one rounding each (2^-24) of 1 + e, of the division and of the two products."""
+    from llama_cu_awq_b200 import _lib
+    L = _lib.test_lib()
+    K, hid = 128, 2048
+    rng = np.random.default_rng(M)
+    w = np.zeros((2 * hid, 16), np.uint32)
+    w[0::2, 0], w[1::2, 0] = 1, 1 << 4   # gate = scale * x[0], up = x[1] (zero points 0)
+    scales = np.ones((2 * hid, 1), np.float16)
+    scales[0::2, 0] = rng.uniform(0.5, 1.0, hid).astype(np.float16)
+    q = ops.QWeight.from_numpy({"weight": w, "zeros": np.zeros((2 * hid, 1), np.uint32), "scales": scales})
+    x = np.zeros((M, K), np.float16)
+    x[:, 0] = rng.uniform(-20.0, -8.0, M)              # where the exponential decides the bits
+    x[: M // 4, 0] = rng.uniform(-8.0, 100.0, M // 4)
+    x[:4, 0] = [0.0, -0.0, -100.0, 100.0]
+    x[:, 1] = np.where(x[:, 0] < -8, 6e4, 90.0) * rng.uniform(0.5, 1.0, M) * rng.choice([-1, 1], M)
+    mm = ops.BatchedMatmul(q, K, 2 * hid, M)
+    y = torch.full((M, hid), float("nan"), dtype=torch.float16, device="cuda")
+    xd = torch.from_numpy(x).cuda()
+    assert L.q4_test_gemm_silu(ops._stream(), ops._p(y), ops._p(xd), q.ref, ops._p(mm.wi), M, K, 2 * hid, ops._p(mm.ws), mm.ws_bytes) == 0 and mm.status() == 0
+    gate = (x[:, :1].astype(np.float32) * scales[0::2, 0].astype(np.float32)).astype(np.float16).astype(np.float64)
+    ref = gate / (1.0 + np.exp(-gate)) * x[:, 1:2].astype(np.float64)
+    d = 2.0**-22 + 4 * 2.0**-24
+    a, b = (ref * (1 - d)).astype(np.float16), (ref * (1 + d)).astype(np.float16)
+    got = y.cpu().numpy()
+    wrong = (got < np.minimum(a, b)) | (got > np.maximum(a, b)) | ~np.isfinite(got)
+    assert not wrong.any(), f"{wrong.sum()} of {wrong.size}"
+
+
 def test_rejects_unsupported_arguments():
     from llama_cu_awq_b200 import _lib
     rng = np.random.default_rng(0)
