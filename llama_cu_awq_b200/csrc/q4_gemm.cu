@@ -29,7 +29,9 @@
 // small MT the issuing warp's waits and commits are what bounds the kernel.
 //
 // Every wait is bounded by the global timer; on expiry the kernel records Q4_ERR_TIMEOUT in the workspace's status word,
-// lets all later waits fall through, waits (bounded) for its own copies in flight, frees its tensor memory and returns.
+// lets all later waits fall through (those of launches queued behind it too), waits (bounded) for its own copies in flight, frees
+// its tensor memory and returns. Threads that meet at a barrier or run a warp-wide instruction behind a wait take its outcome
+// together: a warp in the converters and the MMA issuer, all four warps in the epilogue. A role that gives up says so in s_gave_up.
 #include <cuda.h>
 #include <stdio.h>
 
@@ -259,8 +261,7 @@ __device__ __forceinline__ void epi_stage(const uint32_t* out, uint8_t* buf, int
 }
 // EPI_SILU: features 2j and 2j + 1 are gate j and up j (rounded to fp16 like every GEMM result), one word of the staged rows; silu
 // and product in fp32 go to the store buffer [row][64]. Rolled over the staged words: evaluated on the registers before they are
-// staged, fully unrolled, the same arithmetic cost 27 us more for 512 x 4096 x 22016 (64 evaluations per thread and tile in each of
-// nine places of the code).
+// staged, fully unrolled, the same arithmetic cost 27 us more for 512 x 4096 x 22016 (16 evaluations in each of nine places of the code).
 __device__ __forceinline__ void epi_silu(const uint8_t* staged, uint8_t* buf, int etid) {
     const __half2* src = reinterpret_cast<const __half2*>(staged);
     __half* dst = reinterpret_cast<__half*>(buf);
@@ -296,7 +297,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     uint8_t* sP = sB + (size_t)p.stages * 2 * p.slab_bytes;
     __shared__ uint64_t full_p[kMaxP], empty_p[kMaxP], full[kMaxStages], empty[kMaxStages], tmem_full, tmem_empty, drained;
     __shared__ uint32_t s_tmem_base;
-    __shared__ int s_flag;
+    __shared__ int s_flag, s_gave_up;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -306,6 +307,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         mb_init(&tmem_full, 1);
         mb_init(&tmem_empty, 2 * kEpiWarps);
         mb_init(&drained, 1);
+        s_gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {   // all of the tensor memory, in both CTAs (one CTA per SM: nobody else holds any)
@@ -341,6 +343,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     if (++ps == p.np) { ps = 0; ph ^= 1; }
                 }
             }
+            if (!ok) s_gave_up = 1;
             if (!ok)   // the newest copy of every ring position may still be in flight
                 for (unsigned i = issued > (unsigned)p.np ? issued - p.np : 0; i < issued; i++) mb_drain(&full_p[i % p.np], (i / p.np) & 1);
         } else if (warp == 1 && lane == 0) {
@@ -361,10 +364,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     if (++s == p.stages) { s = 0; ph ^= 1; }
                 }
             }
-            if (!ok) {   // an error: this CTA's copies report to the leader, whose barriers may never complete; both CTAs leave together
-                const unsigned long long t0 = gtimer();
-                while (gtimer() - t0 < 1000000ULL) {}   // a millisecond: far beyond a copy's flight time
-            }
+            if (!ok) s_gave_up = 1;   // (its copies report to the leader, whose barriers may never complete: waited out below)
         } else if (warp == 2 && rank == 0) {
             // ===================== MMA issuer =====================
             // The whole warp walks the loop with warp-uniform values (descriptors and addresses then live in uniform registers) and
@@ -398,6 +398,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
             if (!ok && issuer) {   // MMAs in flight read shared memory and report to both CTAs: let them finish
+                s_gave_up = 1;
                 tc_commit_pair(&drained);
                 mb_drain(&drained, 0);
             }
@@ -449,7 +450,12 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 const uint32_t z = (z_cur >> (8 * i + 4 * wg)) & 0xFu;
                 const __half2 s2 = __half2half2(s_cur[i]);
                 const __half2 zlo = u2h2((0x6400u | z) * 0x00010001u), zhi = u2h2((0x5400u | (z << 4)) * 0x00010001u);
-                if (!mb_wait(&full_p[ps], pp, p.status, 0x600)) { ok = false; break; }
+                // Both the words and the stage, one vote for the two: usually neither has to be waited for (a vote at each costs
+                // 2.5 % at 64 rows, where this loop sets the pace).
+                if (!__all_sync(0xffffffffu, mb_try(&full_p[ps], pp) & mb_try(&empty[sa], pe))) {
+                    ok = warp_wait(&full_p[ps], pp, p.status, 0x600) && warp_wait(&empty[sa], pe, p.status, 0x700);
+                    if (!ok) break;
+                }
                 const uint8_t* src = sP + (size_t)ps * kPStageBytes + r * 128;
                 uint4 pk[4];
 #pragma unroll
@@ -462,7 +468,6 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     dequant8<INTERLEAVED>(pk[j].z, zlo, zhi, s2, o + 16 * j + 8);
                     dequant8<INTERLEAVED>(pk[j].w, zlo, zhi, s2, o + 16 * j + 12);
                 }
-                if (!mb_wait(&empty[sa], pe, p.status, 0x700)) { ok = false; break; }
                 tc_fence_after();
                 tc_st32(a_lane + sa * kAStageCols, o);
 #pragma unroll
@@ -489,6 +494,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
         }
+        if (!ok) s_gave_up = 1;
     } else {
         // ===================== epilogue =====================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
@@ -503,6 +509,14 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mb_arrive_cluster(empty_addr);
+        };
+        // the accumulator is complete; the four warps meet at named barriers from here on, so they go on or give up together
+        auto tile_ready = [&](uint32_t parity) {
+            const uint32_t mine = warp_wait(&tmem_full, parity, p.status, 0x800);
+            uint32_t all;
+            asm volatile("{ .reg .pred p, q; setp.ne.u32 q, %1, 0; bar.red.and.pred p, 2, %2, q; selp.u32 %0, 1, 0, p; }" : "=r"(all) : "r"(mine), "n"(kEpiWarps * 32) : "memory");
+            if (!all) s_gave_up = 1;
+            return all != 0;
         };
         auto partial_of = [&](int pr, bool head) { return reinterpret_cast<float4*>(p.partials) + ((size_t)((pr * 2 + (head ? 1 : 0)) * 2 + rank) * (MT / 4)) * kBN + r; };
         // Y leaves through shared memory: 32 rows are staged and written by one tensor copy (rows and columns beyond Y are
@@ -549,7 +563,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     for (int i = 0; i < 8; i++)
                         if (32 * i < MT) epi_load_residual(out + W * i, res, 32 * i, my_rows, ld);
                 }
-                if (!mb_wait(&tmem_full, pf, p.status, 0x800)) break;
+                if (!tile_ready(pf)) break;
                 pf ^= 1;
                 tc_fence_after();
 #pragma unroll
@@ -573,7 +587,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const long long t0 = (long long)seg.tile * p.n_chunks;
             const int first = pair_of(t0, p.total_chunks, pairs), last = pair_of(t0 + p.n_chunks - 1, p.total_chunks, pairs);
             int* counter = p.counters + seg.tile * 2 + rank;
-            if (!mb_wait(&tmem_full, pf, p.status, 0x800)) break;
+            if (!tile_ready(pf)) break;
             pf ^= 1;
             tc_fence_after();
             if (etid == 0) {
@@ -656,6 +670,13 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (s_gave_up) {
+        // Copies or MMAs may be in flight in this CTA only when its epilogue has not seen all of its tiles, and then it gave up as
+        // well: a millisecond is far beyond a copy's flight time or a tile's MMAs.
+        const unsigned long long t0 = gtimer();
+        while (gtimer() - t0 < 1000000ULL) {}
+        __syncwarp();
+    }
     cluster_sync_all();   // no CTA leaves while the other may still report to its barriers
     if (warp == 2) {
         tc_fence_after();

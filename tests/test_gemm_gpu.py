@@ -98,6 +98,22 @@ def test_residual_epilogue(M, K, N):
     assert_close(yd.cpu().numpy(), x.astype(np.float64) @ w.T + 0.5 * r, f"{M}x{K}x{N} + residual", max_rel=4e-3)
 
 
+@pytest.mark.parametrize("M,K,N", [(16, 128, 128), (64, 4096, 4096), (300, 11008, 520), (512, 1024, 22016)])
+def test_calls_behind_a_recorded_time_out_end(M, K, N):
+    """A status word that already holds a time-out (what calls queued behind one that ran out of time meet): every role gives up at
+    its first unfinished wait, the calls end and report the status; with the workspace zeroed the next call is right again."""
+    from llama_cu_awq_b200 import _lib
+    q, x, y, mm, xd = _case(M, K, N, seed=M + N, interleave=True)
+    y2 = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    mm.ws.view(torch.int32)[0] = _lib.Q4_ERR_TIMEOUT
+    for _ in range(4):
+        mm(y2, xd, M)
+    assert mm.status() == _lib.Q4_ERR_TIMEOUT
+    mm.ws.zero_()
+    mm(y2, xd, M)
+    assert mm.status() == 0 and (y2.cpu().numpy().view(np.uint16) == y.view(np.uint16)).all()
+
+
 @pytest.mark.parametrize("M", [40, 512])
 def test_gate_up_epilogue_values(M):
     """silu(gate) * up as the GEMM's epilogue forms it, for gates and ups that the test chooses (one weight of a row is not zero): the
