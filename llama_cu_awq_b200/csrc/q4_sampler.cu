@@ -31,6 +31,7 @@ constexpr int kCtas = 8;                 // one cluster
 constexpr int kCols = kT / kCtas;        // virtual threads per CTA: CTA r owns elements i with i % 1024 in [128 r, 128 r + 128)
 constexpr int kRowsAtOnce = kT / kCols;  // rows (i / 1024) a CTA works on at a time
 constexpr int kMaxRows = (1 << 18) / kT;
+constexpr size_t kRowBytes = (sizeof(float) + sizeof(unsigned short)) * kCols;   // of dynamic shared memory per row
 
 __device__ __forceinline__ unsigned prob_units(unsigned short h) {   // fp16 in [0, 1] -> multiples of 2^-24
     const unsigned e = (h >> 10) & 31u, mnt = h & 1023u;
@@ -290,9 +291,10 @@ extern "C" float q4_random_f32(unsigned long long* state) { return (q4_random_u3
 extern "C" int q4_sample_topp(void* stream, uint16_t* logits, int n, float temperature, float topp, float coin, int* tokens_pinned,
                               volatile int* pos_pinned, int* pos_dev) {
     if (!logits || !tokens_pinned || !pos_pinned || !pos_dev || n <= 0 || n > (1 << 18) || !(temperature > 0.f)) return Q4_ERR_INVALID;
-    const size_t smem = (sizeof(float) + sizeof(unsigned short)) * (size_t)q4_div_up(n, kT) * kCols;
-    if (smem > 32 * 1024)   // (the static arrays take 13 KB of the 48 KB that need no opt-in)
-        Q4_CUDA_TRY(cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = kRowBytes * q4_div_up(n, kT);
+    // The static arrays take 13 KB of the 48 KB that need no opt-in. The limit belongs to the function on the device and not to this
+    // call: it is always set to the largest size, so that calls of other threads between here and the launch cannot lower it.
+    if (smem > 32 * 1024) Q4_CUDA_TRY(cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRowBytes * kMaxRows)));
     Q4Launch L(dim3(kCtas), dim3(kT), smem, (cudaStream_t)stream);
     Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, sample_topp_kernel, (__half*)logits, n, temperature, topp, coin, tokens_pinned, pos_pinned, pos_dev));
     return Q4_OK;

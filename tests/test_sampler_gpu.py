@@ -67,6 +67,33 @@ def test_sample_topp_slice_edges(n, topp):
     assert Mailbox().run(logits, 1.0, topp, 0.5)[0] == 0   # every probability is NaN: the first element of the order
 
 
+def test_two_threads_sample_different_vocabularies():
+    """The kernel's shared memory grows with the vocabulary and its limit is a property of the function on the device: calls of
+    another thread must not lower it between a call's opt-in and its launch."""
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(3)
+    calls = 1500
+
+    def sampled(n, logits, runs):
+        base = torch.from_numpy(logits.view(np.int16)).cuda()
+        host = torch.zeros(8 + runs, dtype=torch.int32).pin_memory()
+        pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            copies = [base.clone() for _ in range(4)]
+            for i in range(runs):
+                copies[i % 4].copy_(base)
+                ops.sample_topp(copies[i % 4], n, 1.0, 0.9, (i % 97) / 97.0, host.data_ptr() + 4, host.data_ptr(), pos)
+        s.synchronize()
+        return host[2 : 2 + runs].tolist()
+
+    cases = [(n, (rng.standard_normal(n) * 3).astype(np.float16)) for n in (50000, 200000)]
+    alone = [sampled(n, logits, 97) for n, logits in cases]
+    with ThreadPoolExecutor(2) as ex:
+        for one, many in zip(alone, ex.map(lambda c: sampled(*c, calls), cases)):
+            assert many == [one[i % 97] for i in range(calls)]
+
+
 def test_sample_topp_threshold_never_reached():
     logits = np.zeros(4096, np.float16)
     logits[7] = np.float16(-20.0)
