@@ -957,8 +957,9 @@ extern "C" int q4_batch_create(q4_batch** out, q4_model* m, int n_seq) {
     if (!out || !m || n_seq < 1 || n_seq > 16) return Q4_ERR_INVALID;
     if (int e = rows_prepare(m, n_seq)) return e;
     const q4_config& c = m->cfg;
-    if (2 * (size_t)n_seq * c.dim > 200 * 1024 && !(c.dim % 32 == 0 && m->v_n % 16 == 0)) return Q4_ERR_UNSUPPORTED_SIZE;   // the plain classifier keeps the rows in shared memory
-    Q4_CUDA_TRY(cudaFuncSetAttribute(matvec_f16_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(2 * (size_t)n_seq * c.dim, 200 * 1024)));
+    constexpr int kMaxSmem = 200 * 1024;   // the plain classifier keeps the rows in shared memory (one limit for all batches: it belongs to the function)
+    if (2 * (size_t)n_seq * c.dim > kMaxSmem && !(c.dim % 32 == 0 && m->v_n % 16 == 0)) return Q4_ERR_UNSUPPORTED_SIZE;
+    Q4_CUDA_TRY(cudaFuncSetAttribute(matvec_f16_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     q4_batch* b = new q4_batch();
     b->m = m;
     b->n_seq = n_seq;

@@ -253,3 +253,25 @@ def test_batched_decode_matches_single_sequence_decode(mid_path, n_seq):
                 t.synchronize()
                 assert_close(per_step[pos][s], t.logits(), f"sequence {s} of {n_seq}, pos {pos}", max_rel=2 * MAX_REL)
     t.close()
+
+
+def test_a_smaller_batch_does_not_lower_the_plain_classifiers_limit():
+    """A vocabulary of no whole 16s goes through the classifier that keeps the rows in shared memory (64 KB for 16 rows of 2048):
+    a batch of one sequence, created after it, must leave the limit of the wide one's launch alone."""
+    cfg = (2048, 512, 1, 16, 16, 40, 32, 10000.0)
+    t = Transformer(None, synthetic=(cfg, 3))
+    wide, narrow = Batch(t, 16), Batch(t, 1)
+    prompts = np.random.default_rng(0).integers(3, cfg[5], size=(16, 3), dtype=np.int32)
+    wide.reset(prompts)
+    for _ in range(3):
+        wide.forward()
+    got = wide.logits()
+    for s in (0, 7, 15):
+        t.reset(prompts[s], 0)
+        for _ in range(3):
+            t.forward(gen_token=False, path=1)
+        t.synchronize()
+        assert_close(got[s], t.logits(), f"sequence {s}", max_rel=2 * MAX_REL)
+    wide.close()
+    narrow.close()
+    t.close()
