@@ -678,7 +678,15 @@ struct q4_rows {
     std::vector<void*> allocs;
 };
 
+#ifdef Q4_TEST_BUILD
+static int g_fail_alloc = -1;   // host-side fault injection: the allocation after this many more fails, once
+extern "C" void q4_test_fail_rows_alloc(int n) { g_fail_alloc = n; }
+#endif
+
 static int rows_alloc(q4_rows* r, void** p, size_t bytes) {
+#ifdef Q4_TEST_BUILD
+    if (g_fail_alloc >= 0 && g_fail_alloc-- == 0) return Q4_ERR_CUDA;
+#endif
     Q4_CUDA_TRY(cudaMalloc(p, bytes));
     r->allocs.push_back(*p);
     return Q4_OK;
@@ -703,11 +711,7 @@ int q4_rows_status(q4_model* m) {
 // More than this many rows go through the tcgen05 GEMM, fewer through the mma.sync kernels that stream the packed weights.
 constexpr int kSkinnyRows = 16;
 
-// Buffers for up to `rows` rows (grown on demand) and, once and only when the GEMM will be used, the interleaved weight copies.
-static int rows_prepare(q4_model* m, int rows) {
-    if (m->column || m->head_size != 128 || (m->cfg.dim % 128) || (m->o_kc % 128) || (m->h_kc % 128)) return Q4_ERR_UNSUPPORTED_SIZE;
-    if (!m->rows) m->rows = new q4_rows();
-    q4_rows* r = m->rows;
+static int rows_grow(q4_model* m, q4_rows* r, int rows) {
     const q4_config& c = m->cfg;
     int e;
 #define RTRY(expr) do { e = (expr); if (e != Q4_OK) return e; } while (0)
@@ -789,6 +793,23 @@ static int rows_prepare(q4_model* m, int rows) {
     }
 #undef RTRY
     return Q4_OK;
+}
+
+// Buffers for up to `rows` rows (grown on demand) and, once and only when the GEMM will be used, the interleaved weight copies.
+// Complete or nothing: when an allocation or a copy fails part-way, what this call made is released and the next call starts over.
+static int rows_prepare(q4_model* m, int rows) {
+    if (m->column || m->head_size != 128 || (m->cfg.dim % 128) || (m->o_kc % 128) || (m->h_kc % 128)) return Q4_ERR_UNSUPPORTED_SIZE;
+    if (!m->rows) m->rows = new q4_rows();
+    q4_rows* r = m->rows;
+    if (rows <= r->cap && r->rope && (rows <= kSkinnyRows || !r->gm.empty())) return Q4_OK;
+    const q4_rows before = *r;   // (buffers that were outgrown stay allocated: a captured batch step may hold their addresses)
+    const int e = rows_grow(m, r, rows);
+    if (e != Q4_OK) {
+        for (size_t i = before.allocs.size(); i < r->allocs.size(); i++) cudaFree(r->allocs[i]);
+        *r = before;
+        cudaGetLastError();   // (reported; a later call's launch check must not find it)
+    }
+    return e;
 }
 
 // Sum of the ranks' partial [count] vectors: NCCL when it is attached, the communicator's choice says so (large messages)

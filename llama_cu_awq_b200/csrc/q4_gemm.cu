@@ -830,7 +830,8 @@ extern "C" int q4_matmul_q4_batched_residual(void* stream, uint16_t* y, const ui
 
 int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M, int K, int N,
                    const uint16_t* residual, float residual_scale, bool silu, void* workspace, size_t workspace_bytes) {
-    if (!y || !x || !w || !workspace || M <= 0 || K <= 0 || N <= 0) return Q4_ERR_INVALID;
+    if (!y || !x || !w || !w->zeros || !w->scales || !workspace || M <= 0 || K <= 0 || N <= 0) return Q4_ERR_INVALID;
+    if (!w->weight && !weight_interleaved) return Q4_ERR_INVALID;
     if ((K % 128) || (N % 8)) return Q4_ERR_UNSUPPORTED_SIZE;
     if (silu && (N % 16)) return Q4_ERR_UNSUPPORTED_SIZE;
     if (((uintptr_t)x & 15) || ((uintptr_t)y & 15) || ((uintptr_t)w->weight & 15) || ((uintptr_t)weight_interleaved & 15) || ((uintptr_t)workspace & 15)) return Q4_ERR_INVALID;

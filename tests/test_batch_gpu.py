@@ -275,3 +275,38 @@ def test_a_smaller_batch_does_not_lower_the_plain_classifiers_limit():
     wide.close()
     narrow.close()
     t.close()
+
+
+def test_failed_set_up_of_the_rows_publishes_nothing(mid_path):
+    """An allocation that fails anywhere in the set-up of a prompt's rows (weight copies, rotation table, row buffers) fails that call
+    only: the next one starts over and gives the bits of a model whose set-up went through; so with buffers that have to grow."""
+    L = _lib.test_lib()
+    vocab, layers = synth.CONFIGS["mid-gqa"][5], synth.CONFIGS["mid-gqa"][2]
+    tokens = np.random.default_rng(8).integers(3, vocab, size=110, dtype=np.int32)
+
+    def prefilled(t, n):
+        t.reset(tokens[:n], 0)
+        t.prefill(n, gen_token=False)
+        t.synchronize()
+        assert t.status() == 0
+        return t.logits().view(np.uint16)
+
+    t = Transformer(mid_path, lib=L)
+    want = {n: prefilled(t, n) for n in (40, 110)}
+    t.close()
+    try:
+        for fail_at in (0, 1, 2, 3, layers * 8 - 1, layers * 8, layers * 8 + 1, layers * 8 + 12):   # a layer: four words, two zeros and scales
+            t = Transformer(mid_path, lib=L)
+            t.reset(tokens[:40], 0)
+            L.q4_test_fail_rows_alloc(fail_at)
+            with pytest.raises(_lib.Q4Error):
+                t.prefill(40, gen_token=False)
+            assert (prefilled(t, 40) == want[40]).all()
+            t.reset(tokens, 0)
+            L.q4_test_fail_rows_alloc(3)   # the larger row buffers
+            with pytest.raises(_lib.Q4Error):
+                t.prefill(110, gen_token=False)
+            assert (prefilled(t, 40) == want[40]).all() and (prefilled(t, 110) == want[110]).all()
+            t.close()
+    finally:
+        L.q4_test_fail_rows_alloc(-1)

@@ -162,3 +162,8 @@ def test_rejects_unsupported_arguments():
     x = torch.zeros((4, 128), dtype=torch.float16, device="cuda")
     assert L.q4_matmul_q4_batched(s, ops._p(y), ops._p(x), W.ref, None, 4, 128, 8, ops._p(ws), 16) == _lib.Q4_ERR_LIMIT   # workspace too small
     assert L.q4_matmul_q4_batched(s, ops._p(y), ops._p(x), W.ref, None, 0, 128, 8, ops._p(ws), 4096) == _lib.Q4_ERR_INVALID
+    nb = L.q4_matmul_q4_batched_workspace_bytes(4, 128, 8)
+    big = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    c = W.c
+    for part in ((None, c.zeros, c.scales), (c.weight, None, c.scales), (c.weight, c.zeros, None)):   # a matrix without one of its parts
+        assert L.q4_matmul_q4_batched(s, ops._p(y), ops._p(x), _lib.q4_qweight(*part), None, 4, 128, 8, ops._p(big), nb) == _lib.Q4_ERR_INVALID
