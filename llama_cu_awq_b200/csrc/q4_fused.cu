@@ -2048,7 +2048,9 @@ static int fused_build(q4_model* m, q4_fused* f) {
     p.meta_off = n_entries * kEntryBytes + p.xq_bytes;
     p.part_off = p.meta_off + meta_bytes;
     f->smem_bytes = (size_t)p.part_off + sizeof(float) * p.part_floats;
-    Q4_CUDA_TRY(cudaFuncSetAttribute(fused_token_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f->smem_bytes));
+    // (the limit belongs to the function, not to this model: always the largest any model may need, so that a smaller one prepared
+    // later does not lower it)
+    Q4_CUDA_TRY(cudaFuncSetAttribute(fused_token_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     int per_sm = 0;
     Q4_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_token_kernel, kThreads, f->smem_bytes));
     if (per_sm < 1) {

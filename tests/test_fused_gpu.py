@@ -247,3 +247,22 @@ def test_model_api_rejects_out_of_range_ids_and_positions(tmp_path):
     # the cache is full: one more call would write row seq_len
     assert L.q4_model_forward(t.h, C.c_void_p(t.stream.cuda_stream), 0, 1) == _lib.Q4_ERR_LIMIT
     t.close()
+
+
+@pytest.mark.parametrize("order", [(0, 1), (1, 0)])
+def test_two_models_keep_their_shared_memory_limits(order):
+    """The fused kernel's shared memory depends on the model's sizes, its limit belongs to the function: a model that is prepared
+    later and needs less must not lower it for the first one."""
+    cfgs = [(512, 1536, 1, 4, 4, 512, 64, 10000.0), (4096, 11008, 1, 32, 32, 2048, 64, 10000.0)]
+    tokens = np.arange(5, 13, dtype=np.int32)
+    models = [Transformer(None, synthetic=(cfgs[i], i)) for i in order]
+    for t in models:
+        assert t.best_path() == 2
+    for t in models:
+        t.reset(tokens, 0)
+        for _ in tokens:
+            t.forward(gen_token=False, path=2)
+        t.synchronize()
+        assert t.status() == 0 and np.isfinite(t.logits()).all()
+    for t in models:
+        t.close()
