@@ -10,26 +10,43 @@
 
 #include "../../include/q4b200.h"
 
-static PyObject *s_data_ptr, *s_cuda_stream, *s_addr;
+static PyObject *s_data_ptr, *s_cuda_stream, *s_c;
 static PyObject *f_raw_stream, *f_device; /* torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice */
 
-/* An argument walk: every getter returns 0 / NULL and leaves a Python error set when the argument is not what it should be. */
-static void* ptr_of(PyObject* o) {
-    if (o == Py_None) return NULL;
-    PyObject* n = PyLong_CheckExact(o) ? Py_NewRef(o) : PyObject_CallMethodNoArgs(o, s_data_ptr);
+/* An argument walk: every getter returns 0 / NULL and leaves a Python error set when the argument is not what it should be, and
+ * does nothing at all behind an argument that failed (no Python code may run with an error set). */
+static void* ptr_of(PyObject* o) { /* a tensor, or None */
+    if (PyErr_Occurred() || o == Py_None) return NULL;
+    PyObject* n = PyObject_CallMethodNoArgs(o, s_data_ptr);
     if (!n) return NULL;
     void* p = PyLong_AsVoidPtr(n);
     Py_DECREF(n);
     return p;
 }
-static const q4_qweight* weight_of(PyObject* o) { /* QWeight._addr: address of its q4_qweight */
-    PyObject* n = PyObject_GetAttr(o, s_addr);
-    if (!n) return NULL;
-    void* p = PyLong_AsVoidPtr(n);
-    Py_DECREF(n);
+static void* addr_of(PyObject* o) { /* an address (pinned host memory), or None */
+    if (PyErr_Occurred() || o == Py_None) return NULL;
+    if (!PyLong_Check(o)) {
+        PyErr_Format(PyExc_TypeError, "an address is an int, not %.100s", Py_TYPE(o)->tp_name);
+        return NULL;
+    }
+    return PyLong_AsVoidPtr(o);
+}
+static const q4_qweight* weight_of(PyObject* o) { /* QWeight.c, a ctypes q4_qweight; the QWeight keeps it */
+    if (PyErr_Occurred()) return NULL;
+    PyObject* c = PyObject_GetAttr(o, s_c);
+    if (!c) return NULL;
+    Py_buffer v;
+    void* p = NULL;
+    if (PyObject_GetBuffer(c, &v, PyBUF_SIMPLE) == 0) {
+        if (v.len == (Py_ssize_t)sizeof(q4_qweight)) p = v.buf;
+        else PyErr_SetString(PyExc_TypeError, "not a q4_qweight");
+        PyBuffer_Release(&v);
+    }
+    Py_DECREF(c);
     return (const q4_qweight*)p;
 }
 static int int_of(PyObject* o) {
+    if (PyErr_Occurred()) return 0;
     const long v = PyLong_AsLong(o);
     if (v > 2147483647L || v < -2147483647L - 1) {
         PyErr_SetString(PyExc_OverflowError, "size does not fit 32 bits");
@@ -37,9 +54,11 @@ static int int_of(PyObject* o) {
     }
     return (int)v;
 }
-static float float_of(PyObject* o) { return (float)PyFloat_AsDouble(o); }
+static int flag_of(PyObject* o) { return PyErr_Occurred() ? 0 : PyObject_IsTrue(o); }
+static float float_of(PyObject* o) { return PyErr_Occurred() ? 0.f : (float)PyFloat_AsDouble(o); }
 /* None: torch's current stream of the current device */
 static void* stream_of(PyObject* o) {
+    if (PyErr_Occurred()) return NULL;
     if (o != Py_None) {
         PyObject* n = PyObject_GetAttr(o, s_cuda_stream);
         if (!n) return NULL;
@@ -75,9 +94,11 @@ static void* stream_of(PyObject* o) {
     return PyLong_FromLong(status);    \
     }
 #define P(i) ptr_of(a[i])
+#define A(i) addr_of(a[i])
 #define W(i) weight_of(a[i])
 #define I(i) int_of(a[i])
 #define F(i) float_of(a[i])
+#define B(i) flag_of(a[i])
 #define S(i) stream_of(a[i])
 
 FN(rmsnorm, 5)
@@ -87,7 +108,7 @@ FN(rmsnorm, 5)
 FN(matmul_q4, 10)
     void *s = S(0), *o = P(1), *x = P(2);
     const q4_qweight* w = W(3);
-    const int k = I(4), m = I(5), accum = PyObject_IsTrue(a[6]), g = I(7), loff = I(8);
+    const int k = I(4), m = I(5), accum = B(6), g = I(7), loff = I(8);
     void* pos = P(9);
     CALL(q4_matmul_q4(s, o, x, w, k, m, accum, g, loff, pos))
 FN(matmul_f16, 7)
@@ -121,19 +142,19 @@ FN(attention, 11)
 FN(embed, 6)
     void *s = S(0), *x = P(1), *table = P(2);
     const int dim = I(3);
-    void *tok = P(4), *pos = P(5);
+    void *tok = A(4), *pos = P(5);
     CALL(q4_embed(s, x, table, dim, tok, pos))
 FN(argmax, 7)
     void *s = S(0), *l = P(1);
     const int size = I(2);
-    void *tok = P(3), *ppos = P(4), *dpos = P(5);
-    const int write = PyObject_IsTrue(a[6]);
+    void *tok = A(3), *ppos = A(4), *dpos = P(5);
+    const int write = B(6);
     CALL(q4_argmax(s, l, size, tok, ppos, dpos, write))
 FN(sample_topp, 9)
     void *s = S(0), *l = P(1);
     const int size = I(2);
     const float t = F(3), topp = F(4), coin = F(5);
-    void *tok = P(6), *ppos = P(7), *dpos = P(8);
+    void *tok = A(6), *ppos = A(7), *dpos = P(8);
     CALL(q4_sample_topp(s, l, size, t, topp, coin, tok, ppos, dpos))
 FN(matmul_q4_batched, 10)
     void *s = S(0), *y = P(1), *x = P(2);
@@ -141,7 +162,7 @@ FN(matmul_q4_batched, 10)
     void* wi = P(4);
     const int m = I(5), k = I(6), n2 = I(7);
     void* ws = P(8);
-    const size_t bytes = PyLong_AsSize_t(a[9]);
+    const size_t bytes = PyErr_Occurred() ? 0 : PyLong_AsSize_t(a[9]);
     CALL(q4_matmul_q4_batched(s, y, x, w, wi, m, k, n2, ws, bytes))
 FN(matmul_rows, 9)
     void *s = S(0), *y = P(1), *x = P(2);
@@ -169,12 +190,12 @@ static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_q4ops", "The op wra
 PyMODINIT_FUNC PyInit__q4ops(void) {
     s_data_ptr = PyUnicode_InternFromString("data_ptr");
     s_cuda_stream = PyUnicode_InternFromString("cuda_stream");
-    s_addr = PyUnicode_InternFromString("_addr");
+    s_c = PyUnicode_InternFromString("c");
     PyObject* c = PyImport_ImportModule("torch._C");
     if (!c) return NULL;
     f_raw_stream = PyObject_GetAttrString(c, "_cuda_getCurrentRawStream");
     f_device = PyObject_GetAttrString(c, "_cuda_getDevice");
     Py_DECREF(c);
-    if (!s_data_ptr || !s_cuda_stream || !s_addr || !f_raw_stream || !f_device) return NULL;
+    if (!s_data_ptr || !s_cuda_stream || !s_c || !f_raw_stream || !f_device) return NULL;
     return PyModule_Create(&module);
 }

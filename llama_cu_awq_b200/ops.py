@@ -48,7 +48,6 @@ class QWeight:
         assert weight.is_cuda and weight.is_contiguous() and zeros.is_contiguous() and scales.is_contiguous()
         self.weight, self.zeros, self.scales = weight, zeros, scales
         self.c = q4_qweight(weight.data_ptr(), zeros.data_ptr(), scales.data_ptr())
-        self._addr = C.addressof(self.c)
 
     @classmethod
     def from_numpy(cls, d, device="cuda"):
