@@ -3,6 +3,7 @@
     python -m llama_cu_awq_b200.build [--force]
 """
 import os
+import shutil
 import subprocess
 import sys
 import sysconfig
@@ -13,7 +14,8 @@ LIB = os.path.join(HERE, "libq4b200.so")
 CLI = os.path.join(HERE, "llama2_q4")
 TEST_LIB = os.path.join(HERE, "libq4b200_test.so")
 PACKER = os.path.join(HERE, "weight_packer")   # offline tool, host code only
-PYOPS = os.path.join(HERE, "_q4ops.so")        # the op wrappers of ops.py as a CPython module over libq4b200.so
+# the op wrappers of ops.py as a CPython module over libq4b200.so, built for (and named after) the interpreter that runs this file
+PYOPS = os.path.join(HERE, "_q4ops" + sysconfig.get_config_var("EXT_SUFFIX"))
 TEST_BUILD_SOURCES = ["q4_comm.cu", "q4_fused.cu", "q4_gemm.cu", "q4_batch.cu"]   # the sources that look at Q4_TEST_BUILD
 LIB_SOURCES = ["q4_gemv.cu", "q4_ops.cu", "q4_attn.cu", "q4_comm.cu", "q4_model.cu", "q4_fused.cu", "q4_sampler.cu", "q4_synth.cu", "q4_tokenizer.cu", "q4_gemm.cu", "q4_skinny.cu", "q4_batch.cu"]
 CLI_SOURCES = ["llama2_q4_main.cpp"]
@@ -70,13 +72,18 @@ def build(force=False, verbose=False, test=True):
     if all(os.path.exists(s) for s in cli_srcs) and (force or _newer(CLI, deps + [LIB])):
         cmd = [nvcc] + NVCC_FLAGS + ["-o", CLI] + cli_srcs + [LIB, "-Xlinker", "-rpath=$ORIGIN", "-lpthread"]
         subprocess.run(cmd, check=True)
-    pyops_src = os.path.join(CSRC, "q4_pyops.c")
-    if force or _newer(PYOPS, [pyops_src, deps[0]]):
-        cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", PYOPS, pyops_src]
-        subprocess.run(cmd + ["-L", HERE, "-l:libq4b200.so", "-Wl,-rpath,$ORIGIN"], check=True)
     packer_src = os.path.join(CSRC, "weight_packer.cpp")
     if os.path.exists(packer_src) and (force or _newer(PACKER, [packer_src])):
         subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-o", PACKER, packer_src], check=True)
+    # last, and no condition of the rest: only the Python wrappers need it, and they say so when it is missing
+    pyops_src, include = os.path.join(CSRC, "q4_pyops.c"), sysconfig.get_paths()["include"]
+    if force or _newer(PYOPS, [pyops_src, deps[0]]):
+        cc = os.environ.get("CC", "gcc")
+        if not os.path.exists(os.path.join(include, "Python.h")) or not shutil.which(cc.split()[0]):
+            print(f"{os.path.basename(PYOPS)} not built (the op wrappers of ops.py need it): no Python.h in {include}, or no {cc}", file=sys.stderr)
+        else:
+            cmd = cc.split() + ["-O2", "-shared", "-fPIC", "-I", include, "-o", PYOPS, pyops_src]
+            subprocess.run(cmd + ["-L", HERE, "-l:libq4b200.so", "-Wl,-rpath,$ORIGIN"], check=True)
     return LIB
 
 

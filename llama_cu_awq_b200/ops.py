@@ -25,7 +25,7 @@ def _n():
         try:
             from . import _q4ops
         except ImportError as e:
-            raise RuntimeError("llama_cu_awq_b200/_q4ops.so is missing: build it with `python -m llama_cu_awq_b200.build`; there is no fallback path") from e
+            raise RuntimeError("llama_cu_awq_b200/_q4ops is missing for this interpreter: build it with `python -m llama_cu_awq_b200.build`; there is no fallback path") from e
         _native = _q4ops
     return _native
 

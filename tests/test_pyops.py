@@ -48,3 +48,13 @@ def test_matrix_is_read_from_the_weight_at_each_call():
     w.c = b"x"
     with pytest.raises(TypeError):
         call()
+
+
+def test_library_is_built_without_the_python_headers(tmp_path, monkeypatch, capsys):
+    """Without Python.h (or a C compiler) the C library and the programs are still built, and the module's absence is announced."""
+    from llama_cu_awq_b200 import build as b
+    assert b.PYOPS.endswith(b.sysconfig.get_config_var("EXT_SUFFIX")) and ops._n().__file__ == b.PYOPS
+    monkeypatch.setattr(b, "PYOPS", str(tmp_path / "_q4ops.so"))
+    monkeypatch.setattr(b.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    assert b.build() == b.LIB
+    assert "not built" in capsys.readouterr().err
