@@ -126,7 +126,7 @@ int q4_attention_static(void* stream, uint16_t* output, const uint16_t* q, const
  * row m being what q4_matmul_q4 computes for x = X[m] (accum = 0). The reference has no such path: it pushes a prompt
  * through the batch-1 kernel token by token (llama2_q4.cu:710-735); this is the dense contraction on the tensor cores
  * (tcgen05.mma with TMEM accumulators, operands staged by TMA). inpSize must be a multiple of 128, opSize of 8; x, y
- * row-major fp16, 16-byte aligned. `weight_interleaved` is either NULL (the packed words of `w` are used as they lie in
+ * row-major fp16, x 16-byte aligned (a y that is not is written element by element). `weight_interleaved` is either NULL (the packed words of `w` are used as they lie in
  * the file) or a copy of w->weight made by q4_gemm_interleave_weights, which saves the kernel four byte permutes per
  * packed word. `workspace` (device memory, 16-byte aligned, q4_matmul_q4_batched_workspace_bytes(M, inpSize, opSize) bytes,
  * caller-owned, not shared between calls that overlap on the GPU) holds a status word, tile counters and the fp32

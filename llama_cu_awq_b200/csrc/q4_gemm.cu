@@ -63,6 +63,7 @@ struct GemmParams {
     const __half* scales;
     const __half* residual;   // EPI_RESIDUAL: [M][N], y = product + residual * residual_scale, rounded once (may alias y)
     float residual_scale;
+    __half* y;           // PLAIN_Y
     float* partials;     // [pair][2 slots][2 CTAs][MT / 4][128][4] fp32
     int* counters;       // [tile][2 CTAs]
     int* status;         // [0] error code, [1] where
@@ -288,7 +289,9 @@ __device__ __forceinline__ void epi_load_residual(uint32_t* res, const __half* x
     }
 }
 
-template <bool INTERLEAVED, int EPI>
+// PLAIN_Y: y does not start on 16 bytes, which a tensor copy cannot write (a template argument: as a branch it took 0.3 us of the
+// 25 of 64 x 4096 x 22016).
+template <bool INTERLEAVED, int EPI, bool PLAIN_Y>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                const GemmParams p) {
@@ -537,7 +540,13 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
-            if (etid == 0) {
+            if (PLAIN_Y) {   // (the next chunk is staged in the other buffer, behind a barrier that follows these reads)
+                const int col = nt * kPairN + rank * kBN, cols = min(kBN, p.N - col);
+                const __half* src = reinterpret_cast<const __half*>(store);
+#pragma unroll 1
+                for (int i = etid; i < kOutRows * kBN; i += kEpiWarps * 32)
+                    if (i / kBN < rows_left && i % kBN < cols) p.y[(size_t)(row0 + i / kBN) * p.N + col + i % kBN] = src[i];
+            } else if (etid == 0) {
                 const int col = (nt * kPairN + rank * kBN) / (EPI == EPI_SILU ? 2 : 1);
                 if (rows_left > 0 && nt * kPairN + rank * kBN < p.N)
                     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&map_y), "r"(smem_addr(store)), "r"(col), "r"(row0)
@@ -790,12 +799,12 @@ int sm_count(int* out) {
     return Q4_OK;
 }
 
-template <bool IL, int EPI>
+template <bool IL, int EPI, bool PLAIN_Y = false>
 int launch_gemm(cudaStream_t s, int pairs, const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& my, const GemmParams& p) {
     const size_t smem = kRingBytes + 2 * kOutBytes + 1024;
-    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_gemm_kernel<IL, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_gemm_kernel<IL, EPI, PLAIN_Y>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     Q4Launch L(dim3(2 * pairs), dim3(kGemmThreads), smem, s);   // programmatic dependent launch: the prologue overlaps the previous kernel's tail
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemm_kernel<IL, EPI>, mw, mx, my, p));
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemm_kernel<IL, EPI, PLAIN_Y>, mw, mx, my, p));
     return Q4_OK;
 }
 
@@ -834,7 +843,7 @@ int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweigh
     if (!w->weight && !weight_interleaved) return Q4_ERR_INVALID;
     if ((K % 128) || (N % 8)) return Q4_ERR_UNSUPPORTED_SIZE;
     if (silu && (N % 16)) return Q4_ERR_UNSUPPORTED_SIZE;
-    if (((uintptr_t)x & 15) || ((uintptr_t)y & 15) || ((uintptr_t)w->weight & 15) || ((uintptr_t)weight_interleaved & 15) || ((uintptr_t)workspace & 15)) return Q4_ERR_INVALID;
+    if (((uintptr_t)x & 15) || ((uintptr_t)y & 1) || ((uintptr_t)w->weight & 15) || ((uintptr_t)weight_interleaved & 15) || ((uintptr_t)workspace & 15)) return Q4_ERR_INVALID;
     if (workspace_bytes < q4_matmul_q4_batched_workspace_bytes(M, K, N)) return Q4_ERR_LIMIT;
     cudaStream_t s = (cudaStream_t)stream;
     int sms = 0;
@@ -861,8 +870,14 @@ int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweigh
     if (int e = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, wsrc, (uint64_t)q4_pw(K), (uint64_t)N, (uint64_t)q4_pw(K) * 4, kChunkK / 8, kBN)) return e;
     if (int e = make_map_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kSlabK, (uint32_t)(g.MT / 2))) return e;
     const int n_out = silu ? N / 2 : N;
-    if (int e = make_map_2d(&my, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, y, (uint64_t)n_out, (uint64_t)M, (uint64_t)n_out * 2, silu ? kBN / 2 : kBN, kOutRows, false)) return e;
+    p.y = (__half*)y;
     const bool il = weight_interleaved != nullptr;
+    if ((uintptr_t)y & 15) {
+        if (silu) return Q4_ERR_INVALID;   // (row buffers of this library only)
+        if (residual) return il ? launch_gemm<true, EPI_RESIDUAL, true>(s, g.pairs, mw, mx, mx, p) : launch_gemm<false, EPI_RESIDUAL, true>(s, g.pairs, mw, mx, mx, p);
+        return il ? launch_gemm<true, EPI_PLAIN, true>(s, g.pairs, mw, mx, mx, p) : launch_gemm<false, EPI_PLAIN, true>(s, g.pairs, mw, mx, mx, p);
+    }
+    if (int e = make_map_2d(&my, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, y, (uint64_t)n_out, (uint64_t)M, (uint64_t)n_out * 2, silu ? kBN / 2 : kBN, kOutRows, false)) return e;
     if (silu) return il ? launch_gemm<true, EPI_SILU>(s, g.pairs, mw, mx, my, p) : Q4_ERR_INVALID;
     if (residual) return il ? launch_gemm<true, EPI_RESIDUAL>(s, g.pairs, mw, mx, my, p) : launch_gemm<false, EPI_RESIDUAL>(s, g.pairs, mw, mx, my, p);
     return il ? launch_gemm<true, EPI_PLAIN>(s, g.pairs, mw, mx, my, p) : launch_gemm<false, EPI_PLAIN>(s, g.pairs, mw, mx, my, p);

@@ -98,6 +98,25 @@ def test_residual_epilogue(M, K, N):
     assert_close(yd.cpu().numpy(), x.astype(np.float64) @ w.T + 0.5 * r, f"{M}x{K}x{N} + residual", max_rel=4e-3)
 
 
+@pytest.mark.parametrize("offset", [1, 4])
+@pytest.mark.parametrize("M,K,N", [(1, 128, 8), (33, 512, 264), (300, 4096, 520)])
+def test_y_of_any_alignment(M, K, N, offset):
+    """A result (and a residual in it) that does not start on 16 bytes: the bits of the aligned call, and nothing written around it."""
+    from llama_cu_awq_b200 import _lib
+    q, x, y, mm, xd = _case(M, K, N, seed=M + K, interleave=True)
+    buf = torch.full((M * N + 16,), 7.0, dtype=torch.float16, device="cuda")
+    view = buf[offset : offset + M * N].view(M, N)
+    mm(view, xd, M)
+    assert mm.status() == 0 and (view.cpu().numpy().view(np.uint16) == y.view(np.uint16)).all()
+    assert (buf[:offset] == 7).all() and (buf[offset + M * N :] == 7).all()
+    outs = []
+    for out in (torch.ones((M, N), dtype=torch.float16, device="cuda"), view.fill_(1)):
+        assert _lib.lib().q4_matmul_q4_batched_residual(ops._stream(), ops._p(out), ops._p(xd), mm.w.ref, ops._p(mm.wi), M, K, N, ops._p(out), 0.5, ops._p(mm.ws),
+                                                        mm.ws_bytes) == 0
+        outs.append(out.cpu().numpy().view(np.uint16))
+    assert mm.status() == 0 and (outs[0] == outs[1]).all()
+
+
 @pytest.mark.parametrize("M,K,N", [(16, 128, 128), (64, 4096, 4096), (300, 11008, 520), (512, 1024, 22016)])
 def test_calls_behind_a_recorded_time_out_end(M, K, N):
     """A status word that already holds a time-out (what calls queued behind one that ran out of time meet): every role gives up at
