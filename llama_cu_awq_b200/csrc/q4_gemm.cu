@@ -741,7 +741,7 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const 
 // Workspace layout, the same for every shape, so that calls of different shapes can share one workspace (the tile counters
 // must read zero at the start of every call): status words | tile counters | fp32 partial sums.
 constexpr size_t kWsHeader = 256;
-constexpr int kWsMaxTiles = 8192;
+constexpr int kWsMaxTiles = 16384;   // (two counters per tile of 256 features: 8192 tiles of 256 x 256 outputs)
 constexpr size_t kWsPartials = kWsHeader + sizeof(int) * kWsMaxTiles;
 
 constexpr double kConvClocks = 1250.0;

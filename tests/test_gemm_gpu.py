@@ -50,6 +50,19 @@ def test_batch_tiles_and_shares(M, K, N):
     assert mm.status() == 0 and (y2.cpu().numpy().view(np.uint16) == y.view(np.uint16)).all()
 
 
+def test_more_rows_than_a_million():
+    """A narrow matrix and so many rows that the tile counters are nearly used up (8192 tiles of 256 rows are accepted)."""
+    M, K, N = 1_060_000, 128, 8
+    q = synth.synth_qweight(np.random.default_rng(0), K, N)
+    mm = ops.BatchedMatmul(ops.QWeight.from_numpy(q), K, N, M)
+    x = torch.randn((M, K), device="cuda", generator=torch.Generator("cuda").manual_seed(1)).half()
+    y = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    mm(y, x, M)
+    assert mm.status() == 0
+    w = torch.from_numpy(O.dequant(q, K, N)).cuda()
+    assert_close(y.cpu().numpy(), (x.double() @ w.double().T).cpu().numpy(), "a million rows vs f64", max_rel=4e-3)
+
+
 @pytest.mark.parametrize("M", [16, 64, 512])
 @pytest.mark.parametrize("K,N", [(4096, 12288), (4096, 22016), (11008, 4096), (4096, 4096)])
 def test_7b_projection_shapes(M, K, N):
