@@ -681,6 +681,8 @@ struct q4_rows {
 #ifdef Q4_TEST_BUILD
 static int g_fail_alloc = -1;   // host-side fault injection: the allocation after this many more fails, once
 extern "C" void q4_test_fail_rows_alloc(int n) { g_fail_alloc = n; }
+static bool g_fail_set_pos = false;   // the next launch of a prompt's position words fails, once
+extern "C" void q4_test_fail_set_pos() { g_fail_set_pos = true; }
 #endif
 
 static int rows_alloc(q4_rows* r, void** p, size_t bytes) {
@@ -921,29 +923,40 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
 // ------------------------------------------------------------------------------------------------------------
 // prefill
 // ------------------------------------------------------------------------------------------------------------
+// Both position words to `pos`, in stream order.
+static int move_pos(q4_model* m, cudaStream_t s, int pos) {
+#ifdef Q4_TEST_BUILD
+    if (g_fail_set_pos) { g_fail_set_pos = false; return Q4_ERR_CUDA; }
+#endif
+    Q4_CUDA_TRY(launch_rows(true, set_pos_kernel, dim3(1), dim3(1), 0, s, m->pos, &m->shared->pos, pos));
+    return Q4_OK;
+}
+
 static int prefill(q4_model* m, cudaStream_t s, int n, int gen_token, bool logits) {
     if (!m || n < 1) return Q4_ERR_INVALID;
     const q4_config& c = m->cfg;
     const int pos0 = m->host_pos;
     if (pos0 + n > c.seq_len || pos0 + n >= Q4_MAX_SEQ_LEN) return Q4_ERR_LIMIT;
-    if (int e = rows_prepare(m, n)) return e;
+    int e;
+    if ((e = rows_prepare(m, n)) != Q4_OK) return e;
     q4_rows* r = m->rows;
     const bool overlap = true;
     launch_rows(overlap, iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, 0, pos0, 0);
     launch_rows(overlap, embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size);
-    if (int e = rows_layers(m, s, n, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) return e;
+    if ((e = rows_layers(m, s, n, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) != Q4_OK) return e;
+    if ((e = move_pos(m, s, logits ? pos0 + n - 1 : pos0 + n)) != Q4_OK) return e;
+    if (logits) {
+        // the last row goes on through the batch-1 tail (llama2_q4.cu:528-537, sampler.h:77-84): final norm, classifier,
+        // [all-gather], hand-off; the position words were moved to that row, the hand-off steps them past it
+        if ((e = q4_rmsnorm(s, m->x, (const uint16_t*)(r->X + (size_t)(n - 1) * c.dim), m->rms_final, c.dim)) != Q4_OK) return e;
+        if ((e = q4_matmul_f16(s, m->logits + (size_t)m->rank * m->v_n, m->x, m->wcls, c.dim, m->v_n, 1.0f)) != Q4_OK) return e;
+        if (m->g > 1 && (e = q4_all_gather(m->comm, s, m->logits + (size_t)m->rank * m->v_n, m->logits, m->v_n)) != Q4_OK) return e;
+        if ((e = q4_argmax(s, m->logits, c.vocab_size, (int*)m->shared->tokens, &m->shared->pos, m->pos, gen_token != 0)) != Q4_OK) return e;
+    }
     // sample() draws one coin per position, used or not (sampler.h:79): keep the generator where n token steps leave it
     for (int i = 0; i < n; i++) (void)q4_random_f32(&m->rng_state);
     m->host_pos = pos0 + n;
-    launch_rows(overlap, set_pos_kernel, dim3(1), dim3(1), 0, s, m->pos, &m->shared->pos, logits ? pos0 + n - 1 : pos0 + n);
-    if (!logits) return Q4_OK;
-    // the last row goes on through the batch-1 tail (llama2_q4.cu:528-537, sampler.h:77-84): final norm, classifier,
-    // [all-gather], hand-off; the position words were moved to that row, the hand-off steps them past it
-    int e;
-    if ((e = q4_rmsnorm(s, m->x, (const uint16_t*)(r->X + (size_t)(n - 1) * c.dim), m->rms_final, c.dim)) != Q4_OK) return e;
-    if ((e = q4_matmul_f16(s, m->logits + (size_t)m->rank * m->v_n, m->x, m->wcls, c.dim, m->v_n, 1.0f)) != Q4_OK) return e;
-    if (m->g > 1 && (e = q4_all_gather(m->comm, s, m->logits + (size_t)m->rank * m->v_n, m->logits, m->v_n)) != Q4_OK) return e;
-    return q4_argmax(s, m->logits, c.vocab_size, (int*)m->shared->tokens, &m->shared->pos, m->pos, gen_token != 0);
+    return Q4_OK;
 }
 
 extern "C" int q4_model_prefill(q4_model* m, void* stream, int n_tokens, int gen_token) { return prefill(m, (cudaStream_t)stream, n_tokens, gen_token, true); }

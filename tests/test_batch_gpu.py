@@ -310,3 +310,28 @@ def test_failed_set_up_of_the_rows_publishes_nothing(mid_path):
             t.close()
     finally:
         L.q4_test_fail_rows_alloc(-1)
+
+
+def test_failed_launch_behind_a_prompts_layers_is_reported(mid_path):
+    """The launch that moves the position words fails (injected): the call says so with and without logits, the model's own position
+    has not moved, and the same prompt goes through afterwards."""
+    L = _lib.test_lib()
+    vocab = synth.CONFIGS["mid-gqa"][5]
+    tokens = np.random.default_rng(9).integers(3, vocab, size=20, dtype=np.int32)
+    t = Transformer(mid_path, lib=L)
+    t.reset(tokens, 0)
+    L.q4_test_fail_set_pos()
+    with pytest.raises(_lib.Q4Error):
+        t.prefill(20, gen_token=False)
+    t.prefill(20, gen_token=False)
+    t.synchronize()
+    assert t.shared().pos == 20
+    got = t.logits().view(np.uint16)
+    L.q4_test_fail_set_pos()
+    with pytest.raises(_lib.Q4Error):
+        t.generate(tokens, 24, path=2, prompt_one_pass=True)
+    t.reset(tokens, 0)
+    t.prefill(20, gen_token=False)
+    t.synchronize()
+    assert (t.logits().view(np.uint16) == got).all()
+    t.close()
