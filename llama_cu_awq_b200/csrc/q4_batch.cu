@@ -258,25 +258,33 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* 
         }
         mx = mn;
     };
-    for (int t0 = warp * kAttKeys; t0 <= pos; t0 += kAttWarps * kAttKeys) {
-        uint2 kv[kAttKeys], vv[kAttKeys];
-        const bool with_new = FUSED && t0 + kAttKeys > pos;   // position pos is one of this round's keys
+    auto load4 = [&](uint2 (&kv)[kAttKeys], uint2 (&vv)[kAttKeys], int t0) {
 #pragma unroll
         for (int u = 0; u < kAttKeys; u++) {
             const int t = max(min(t0 + u, T - 1), 0);   // a round's tail reads some earlier row instead (row 0 where there is none)
             kv[u] = *reinterpret_cast<const uint2*>(kb + (size_t)t * kv_n);
             vv[u] = *reinterpret_cast<const uint2*>(vb + (size_t)t * kv_n);
         }
-        if (with_new) {
-            const size_t at = (size_t)m * kv_n + (size_t)(h / kv_mul) * HS + lane * 4;
-            const uint2 k = rotate(*reinterpret_cast<const uint2*>(knew + at)), v = *reinterpret_cast<const uint2*>(vnew + at);
+    };
+    int t0 = warp * kAttKeys;
+    for (; FUSED ? t0 + kAttKeys <= pos : t0 <= pos; t0 += kAttWarps * kAttKeys) {
+        uint2 kv[kAttKeys], vv[kAttKeys];
+        load4(kv, vv, t0);
+        round4(kv, vv, pos + 1 - t0);
+    }
+    // The round that holds position pos is a warp's last, behind a loop that knows nothing of it (64 registers instead of 79: 16
+    // sequences at position 1900, step of two 7B layers, 415 -> 335 us).
+    if (FUSED && t0 <= pos) {
+        uint2 kv[kAttKeys], vv[kAttKeys];
+        load4(kv, vv, t0);
+        const size_t at = (size_t)m * kv_n + (size_t)(h / kv_mul) * HS + lane * 4;
+        const uint2 k = rotate(*reinterpret_cast<const uint2*>(knew + at)), v = *reinterpret_cast<const uint2*>(vnew + at);
 #pragma unroll
-            for (int u = 0; u < kAttKeys; u++)
-                if (t0 + u >= pos) { kv[u] = k; vv[u] = v; }   // (those behind it do not count, but must not bring in a NaN)
-            if (h % kv_mul == 0) {
-                *reinterpret_cast<uint2*>(kc + head_at + (size_t)pos * kv_n) = k;
-                *reinterpret_cast<uint2*>(vc + head_at + (size_t)pos * kv_n) = v;
-            }
+        for (int u = 0; u < kAttKeys; u++)
+            if (t0 + u >= pos) { kv[u] = k; vv[u] = v; }   // (those behind it do not count, but must not bring in a NaN)
+        if (h % kv_mul == 0) {
+            *reinterpret_cast<uint2*>(kc + head_at + (size_t)pos * kv_n) = k;
+            *reinterpret_cast<uint2*>(vc + head_at + (size_t)pos * kv_n) = v;
         }
         round4(kv, vv, pos + 1 - t0);
     }
