@@ -873,7 +873,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
         const long long loff = (long long)l * c.seq_len * m->kv_n;
         norm((const __half*)L.rms_att, fused_add && l > 0 ? r->Y : nullptr);
         if (skinny) {
-            OP(q4_qkv_matmul_rows(s, (uint16_t*)r->Q, (uint16_t*)r->K, (uint16_t*)r->V, (const uint16_t*)r->XB, &L.q.w, &L.k.w, &L.v.w, n, dim, m->q_n, m->kv_n));
+            OP(q4_qkv_rows_launch(s, (uint16_t*)r->Q, (uint16_t*)r->K, (uint16_t*)r->V, (const uint16_t*)r->XB, &L.q.w, &L.k.w, &L.v.w, n, dim, m->q_n, m->kv_n, pos0 < 0));
         } else {
             OP(gemm(r->QKV, r->XB, l, 0, false));
         }

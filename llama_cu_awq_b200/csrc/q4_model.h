@@ -67,6 +67,10 @@ int q4_synth_qweight(uint32_t* w, uint32_t* z, uint16_t* s, int K_full, int K, i
 int q4_synth_normal(uint16_t* dst, long long count, long long idx0, unsigned long long seed, int tid);
 int q4_synth_const(uint16_t* dst, int n, uint16_t value);
 
+// q4_skinny.cu: q4_qkv_matmul_rows; late: its dependents are signalled at its end
+int q4_qkv_rows_launch(void* stream, uint16_t* q, uint16_t* k, uint16_t* v, const uint16_t* x, const q4_qweight* qw, const q4_qweight* kw, const q4_qweight* vw,
+                       int M, int inpSize, int opSize, int kvSize, bool late);
+
 // q4_gemm.cu: q4_matmul_q4_batched_residual, and with silu = true (interleaved weights only) the fused gate / up form: rows 2j and
 // 2j + 1 of the weights are gate j and up j, y is [M][N / 2] = silu(gate) * up.
 int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M, int K, int N,

@@ -19,7 +19,7 @@
 // Epilogues: plain, residual (y = product + residual * scale: matmul(QWeight)'s accum form, gpu_kernels.h:237-238),
 // and SiLU (ffn_matvec_silu_kernel, gpu_kernels.h:251-283: the CTA holds 16 gate and the same 16 up features and writes
 // silu(gate) * up without rounding gate or up to fp16 first).
-#include "q4_common.cuh"
+#include "q4_model.h"
 
 namespace {
 
@@ -40,6 +40,7 @@ struct SkParams {
     int total_tiles;
     const __half* residual;   // [M][ldy of m[0]] or null
     float rscale;
+    bool late;                // dependents are signalled at the end (q4_qkv_rows_launch)
 };
 
 __device__ __forceinline__ void mma_f16(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -157,10 +158,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
 #pragma unroll
     for (int d = 0; d < D; d++) prefetch(st[d]);
     griddep_wait();
-    // q|k|v: its successor in batched decode is the attention, whose few CTAs would be dealt out as this kernel's CTAs (one per SM,
-    // most of its registers) leave: three or four to each of the first SMs, where they walk their keys while the other SMs idle.
-    // Signalled at the end they spread (one sequence at position 1900, step of two 7B layers: 275 us against 173).
-    if (p.nmat != 3) griddep_launch_dependents();
+    if (!p.late) griddep_launch_dependents();
 
     // x: the batch rows' 32 inputs of this thread's quarter of a group, fetched one step ahead
     const __half* xrow[NT];
@@ -302,7 +300,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
             }
         }
     }
-    if (p.nmat == 3) griddep_launch_dependents();
+    if (p.late) griddep_launch_dependents();
 }
 
 constexpr int kSms = 148;   // B200: one persistent CTA per SM (a smaller part would only leave CTAs queued behind the first wave)
@@ -371,7 +369,17 @@ extern "C" int q4_matmul_q4_rows(void* stream, uint16_t* y, const uint16_t* x, c
 
 extern "C" int q4_qkv_matmul_rows(void* stream, uint16_t* q, uint16_t* k, uint16_t* v, const uint16_t* x, const q4_qweight* qw,
                                   const q4_qweight* kw, const q4_qweight* vw, int M, int inpSize, int opSize, int kvSize) {
+    return q4_qkv_rows_launch(stream, q, k, v, x, qw, kw, vw, M, inpSize, opSize, kvSize, false);
+}
+
+// late: the successor is the attention of batched decode, whose few CTAs would be dealt out as this kernel's CTAs (one per SM, most
+// of its registers) leave: three or four to each of the first SMs, where they walk their keys while the other SMs idle. Signalled
+// at the end they spread (one sequence at position 1900, step of two 7B layers: 275 us against 173). Not for a successor that
+// streams weights, which loses its head start (the 7B product back to back, 8 rows: 10.6 us, 11.7 signalled at the end).
+int q4_qkv_rows_launch(void* stream, uint16_t* q, uint16_t* k, uint16_t* v, const uint16_t* x, const q4_qweight* qw, const q4_qweight* kw, const q4_qweight* vw,
+                       int M, int inpSize, int opSize, int kvSize, bool late) {
     SkParams p = {};
+    p.late = late;
     if (int e = fill(p, x, M, inpSize)) return e;
     if (!q || !k || !v || !qw || !kw || !vw) return Q4_ERR_INVALID;
     if (opSize <= 0 || kvSize <= 0 || (opSize % 32) || (kvSize % 32)) return Q4_ERR_UNSUPPORTED_SIZE;   // a CTA's two tiles lie in one matrix
