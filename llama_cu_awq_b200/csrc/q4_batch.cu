@@ -19,12 +19,12 @@ namespace {
 
 constexpr int kRowThreads = 256;
 
-// Every kernel of this file starts with griddepcontrol.wait + launch_dependents, so it may be launched with programmatic
+// Every kernel of this file starts with griddepcontrol.wait + launch_dependents and is launched with programmatic
 // stream serialisation: its successor (often a weight-streaming kernel whose first loads do not depend on it) then begins
 // its prologue while this one runs, and waits for this one's completion before it touches anything produced here.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_rows(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-    Q4Launch L(grid, block, smem, s, overlap);
+cudaError_t launch_rows(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    Q4Launch L(grid, block, smem, s);
     return cudaLaunchKernelEx(&L.cfg, kernel, KArgs(args)...);
 }
 
@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* 
 // form in fp32, P is rounded to fp16 for the second product (the reference's att buffer is fp16 too) and its row sums come
 // from the same product with a column of ones. head_size 128. Keys beyond the last row's position are zero-filled and masked.
 //
-// The tensor pipe is the bound (1024 clocks per 64 x 64 block and SM); everything else has to fit under it. Chunks are copied
+// It runs at 0.43 of the rate mma.sync reaches here (1024 clocks per 64 x 64 block and SM at that rate; 2000 rows); the rest is the
+// softmax between the two products and, below a thousand rows, CTAs of unequal length that do not fill the SMs. Chunks are copied
 // with cp.async one ahead of the math; both operands come through ldmatrix (K as it lies, V transposed); only the chunks a
 // warp's diagonal crosses are masked; the running output is scaled only when a maximum moved; the CTAs with the most keys
 // start first; three CTAs of four warps per SM cover each other's softmax. 2000 rows of 32 heads: 231 -> 143 us, 512 rows:
@@ -786,10 +787,8 @@ static int rows_grow(q4_model* m, q4_rows* r, int rows) {
         RTRY(rows_alloc(r, (void**)&r->V, 2 * (size_t)cap * m->kv_n));
         RTRY(rows_alloc(r, (void**)&r->ATT, 2 * (size_t)cap * m->q_n));
         RTRY(rows_alloc(r, (void**)&r->G, 2 * cap * hk));
-        if (cap > kSkinnyRows) {
-            RTRY(rows_alloc(r, (void**)&r->QKV, 2 * (size_t)cap * (m->q_n + 2 * m->kv_n)));
-            RTRY(rows_alloc(r, (void**)&r->Y, 2 * cap * dim));
-        }
+        RTRY(rows_alloc(r, (void**)&r->QKV, 2 * (size_t)cap * (m->q_n + 2 * m->kv_n)));
+        RTRY(rows_alloc(r, (void**)&r->Y, 2 * cap * dim));
         RTRY(rows_alloc(r, (void**)&r->row_seq, sizeof(int) * cap));
         RTRY(rows_alloc(r, (void**)&r->row_pos, sizeof(int) * cap));
         size_t ws = 0;
@@ -859,14 +858,16 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
     // q, k, v of the rows: three buffers (few-rows kernels) or three slices of the fused GEMM's output
     const int nqkv = m->q_n + 2 * m->kv_n;
     const bool skinny = n <= kSkinnyRows;
-    const bool overlap = true;
-    // A prompt's rows on one GPU: the o and down projections leave their result in XB / ATT and the next RMSNorm adds it to x
+    // (the attention of batched decode takes k and v as the few-rows kernels leave them, and behind the GEMMs the last layer's down
+    // projection would still have to be added)
+    if (!skinny && (pos0 < 0 || want == WANT_ALL)) return Q4_ERR_INVALID;
+    // A prompt's rows on one GPU: the o and down projections leave their result in Y and the next RMSNorm adds it to x
     // (with more ranks the partial sums have to be exchanged as x first: the GEMM adds the residual itself).
     const bool fused_add = !skinny && g == 1;
     if (pos0 >= 0 && !skinny) Q4_CUDA_TRY(cudaFuncSetAttribute(attention_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAtSmem));
     auto norm = [&](const __half* w, const __half* y) {
-        if (y) launch_rows(overlap, rmsnorm_rows_kernel<true>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, y, w, dim);
-        else launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, w, dim);
+        if (y) launch_rows(rmsnorm_rows_kernel<true>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, y, w, dim);
+        else launch_rows(rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, w, dim);
     };
     for (int l = 0; l < c.n_layers; l++) {
         const DevLayer& L = m->layers[l];
@@ -882,7 +883,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
         const __half* vp = skinny ? r->V : r->QKV + m->q_n + m->kv_n;
         const int ldq = skinny ? m->q_n : nqkv, ldkv = skinny ? m->kv_n : nqkv;
         if (pos0 >= 0)   // (batched decode: the attention kernel rotates and files)
-            launch_rows(overlap, rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
+            launch_rows(rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
                         r->rope, r->row_seq, r->row_pos, seq_stride, loff);
         if (l == c.n_layers - 1 && want != WANT_ALL) {
             if (want == WANT_CACHE) break;
@@ -893,20 +894,20 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
                             m->kv_mul, c.seq_len, r->row_pos + last));
             OP(q4_matmul_q4_rows(s, x, (const uint16_t*)r->ATT, &L.o.w, 1, m->o_kc, dim, x, 1.0f / g));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
-            launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);
+            launch_rows(rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);
             OP(q4_ffn_silu_rows(s, (uint16_t*)r->G, (const uint16_t*)r->XB, &L.gate.w, &L.up.w, 1, dim, m->h_kc));
             OP(q4_matmul_q4_rows(s, x, (const uint16_t*)r->G, &L.down.w, 1, m->h_kc, dim, x, 1.0f / g));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
             break;
         }
         if (pos0 >= 0 && !skinny)
-            launch_rows(overlap, attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), kAtSmem, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
+            launch_rows(attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), kAtSmem, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
                         m->kv_mul, n, pos0, m->kv_n);
         else if (pos0 >= 0)
-            launch_rows(overlap, attention_rows_kernel<false>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
+            launch_rows(attention_rows_kernel<false>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
                         r->row_pos, seq_stride, loff, m->kv_n, (const __half*)nullptr, (const __half*)nullptr, (const float2*)nullptr);
         else
-            launch_rows(overlap, attention_rows_kernel<true>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
+            launch_rows(attention_rows_kernel<true>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
                         r->row_pos, seq_stride, loff, m->kv_n, kp, vp, r->rope);
         // x = o_proj(att) + x / g, summed over the ranks (gpu_kernels.h:237-238, llama2_q4.cu:472-476)
         if (skinny) OP(q4_matmul_q4_rows(s, (uint16_t*)r->X, (const uint16_t*)r->ATT, &L.o.w, n, m->o_kc, dim, (const uint16_t*)r->X, 1.0f / g));
@@ -936,7 +937,7 @@ static int move_pos(q4_model* m, cudaStream_t s, int pos) {
 #ifdef Q4_TEST_BUILD
     if (g_fail_set_pos) { g_fail_set_pos = false; return Q4_ERR_CUDA; }
 #endif
-    Q4_CUDA_TRY(launch_rows(true, set_pos_kernel, dim3(1), dim3(1), 0, s, m->pos, &m->shared->pos, pos));
+    Q4_CUDA_TRY(launch_rows(set_pos_kernel, dim3(1), dim3(1), 0, s, m->pos, &m->shared->pos, pos));
     return Q4_OK;
 }
 
@@ -948,9 +949,8 @@ static int prefill(q4_model* m, cudaStream_t s, int n, int gen_token, bool logit
     int e;
     if ((e = rows_prepare(m, n)) != Q4_OK) return e;
     q4_rows* r = m->rows;
-    const bool overlap = true;
-    launch_rows(overlap, iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, 0, pos0, 0);
-    launch_rows(overlap, embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size);
+    launch_rows(iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, 0, pos0, 0);
+    launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size);
     if ((e = rows_layers(m, s, n, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) != Q4_OK) return e;
     if ((e = move_pos(m, s, logits ? pos0 + n - 1 : pos0 + n)) != Q4_OK) return e;
     if (logits) {
@@ -1072,26 +1072,25 @@ static int batch_step(q4_batch* b, cudaStream_t s) {
     q4_rows* r = m->rows;
     const q4_config& c = m->cfg;
     const int n = b->n_seq;
-    const bool overlap = true;
-    launch_rows(overlap, iota_rows_kernel, dim3(1), dim3(32), 0, s, r->row_seq, nullptr, n, 0, 0, 1);
+    launch_rows(iota_rows_kernel, dim3(1), dim3(32), 0, s, r->row_seq, nullptr, n, 0, 0, 1);
     Q4_CUDA_TRY(cudaMemcpyAsync(r->row_pos, b->pos, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
-    launch_rows(overlap, embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, b->tokens, b->max_len + 1, r->row_seq, r->row_pos, c.vocab_size);
+    launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, b->tokens, b->max_len + 1, r->row_seq, r->row_pos, c.vocab_size);
     if (int e = rows_layers(m, s, n, b->kc, b->vc, b->seq_stride, -1, WANT_ALL)) return e;
-    launch_rows(overlap, rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)nullptr, (const __half*)m->rms_final, c.dim);
+    launch_rows(rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)nullptr, (const __half*)m->rms_final, c.dim);
     const size_t smem = 2 * (size_t)n * c.dim;
     __half* cls_out = m->g == 1 ? b->logits : b->part;   // TP: every rank computes its vocabulary slice of every row; the slices are gathered row by row
     const int cls_stride = m->g == 1 ? c.vocab_size : m->v_n;
     if (c.dim % 32 == 0 && m->v_n % 16 == 0) {
-        if (n <= 8) launch_rows(overlap, classifier_rows_kernel<1>, dim3(m->v_n / 16), dim3(kClsWarps * 32), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
-        else launch_rows(overlap, classifier_rows_kernel<2>, dim3(m->v_n / 16), dim3(kClsWarps * 32), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
+        if (n <= 8) launch_rows(classifier_rows_kernel<1>, dim3(m->v_n / 16), dim3(kClsWarps * 32), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
+        else launch_rows(classifier_rows_kernel<2>, dim3(m->v_n / 16), dim3(kClsWarps * 32), 0, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
     } else {
-        launch_rows(overlap, matvec_f16_rows_kernel, dim3(148 * 2), dim3(256), smem, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
+        launch_rows(matvec_f16_rows_kernel, dim3(148 * 2), dim3(256), smem, s, cls_out, b->xf, (const __half*)m->wcls, c.dim, m->v_n, n, cls_stride);
     }
     if (m->g > 1) {
         for (int i = 0; i < n; i++)
             if (int e = q4_all_gather(m->comm, s, (const uint16_t*)(b->part + (size_t)i * m->v_n), (uint16_t*)(b->logits + (size_t)i * c.vocab_size), m->v_n)) return e;
     }
-    launch_rows(overlap, argmax_rows_kernel, dim3(n), dim3(1024), 0, s, b->logits, c.vocab_size, b->tokens, b->max_len + 1, b->pos, b->n_prompt);
+    launch_rows(argmax_rows_kernel, dim3(n), dim3(1024), 0, s, b->logits, c.vocab_size, b->tokens, b->max_len + 1, b->pos, b->n_prompt);
     Q4_CUDA_TRY(cudaGetLastError());
     return Q4_OK;
 }

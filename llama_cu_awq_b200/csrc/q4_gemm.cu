@@ -322,8 +322,8 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     cluster_sync_all();   // both CTAs' barriers and tensor memory are ready before either is touched from the other side
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t*)&s_tmem_base;
-    // everything above overlaps the tail of the previous kernel on the stream (programmatic dependent launch); from here
-    // on this kernel reads what that kernel wrote
+    // everything above overlaps the tail of the previous kernel on the stream (programmatic dependent launch) where both fit an SM,
+    // that is, not behind another of these, whose shared memory fills it; from here on this kernel reads what that kernel wrote
     griddep_wait();
     griddep_launch_dependents();
     Segments seg(p, pair, pairs);
@@ -484,9 +484,9 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 tc_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                // The staging slot is given back only here, behind the tensor-memory stores that consumed its words: an arrive placed
-                // right behind the loads was moved ahead of some of them by the compiler, and the copy engine overwrote rows that
-                // had not been read (a few wrong feature rows in one launch out of hundreds).
+                // The staging slot is given back only here, behind the tensor-memory stores that consumed its words: with the arrive
+                // right behind the loads a few feature rows were wrong in one launch out of hundreds (the slot's next copy had
+                // landed before all of its reads were done).
                 if (lane == 0) {
                     mb_arrive_cluster(leader_addr(&full[sa]));
                     mb_arrive(&empty_p[ps]);
@@ -748,8 +748,9 @@ constexpr double kConvClocks = 1250.0;
 
 struct GemmPlan { int MT, m_tiles, n_tiles, n_chunks, pairs, stages, np, slab; long long total; };
 
-// Batch tile and number of pairs, by an estimate of the slowest pair's clocks over all of them (what each line costs was
-// read off clock stamps inside the kernel):
+// Batch tile and number of pairs, by an estimate of the slowest pair's clocks over all of them. What each line costs was read off
+// clock stamps inside the kernel; launch, first copies and last drain, much the same for every plan, are in no line, so the
+// estimate ranks plans and is not a time (4096 x 22016: 15.0 us of the 25 measured at 64 rows, 49 of 75 at 512):
 //   chunk    a 256-input chunk: 8.6 per batch row on the tensor pipe (MT / 2 per K = 16 step), or the conversion of its 128 x 256
 //            weights by the eight converter warps, whichever is longer
 //   tile     draining the accumulator; the last tile's output is not hidden by anything: 400 per 32 rows

@@ -7,7 +7,7 @@
 //   otherwise   : order = index order, threshold = coin
 //   token = first element in that order whose inclusive prefix sum of p reaches the threshold; the last one if none does.
 // The reference accumulates the prefix sum in fp16 in whatever order the device-wide scan takes. Here the sum is EXACT:
-// every fp16 probability is an integer multiple of 2^-24, so prefix sums are 64-bit integers and the result does not
+// every fp16 probability is an integer multiple of 2^-24, so prefix sums are integers (below 2^25) and the result does not
 // depend on any summation order. The sorted order is never materialised: two histogram passes over the fp16 bit pattern
 // (high byte, then low byte) find the probability value at which the prefix crosses the threshold, and a count over the
 // ties in index order finds the element.
