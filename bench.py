@@ -443,7 +443,9 @@ def prefill_and_batch(t, cfg, fwd_path, value, rank, world, dist, torch, barrier
         rel_f, cos_f = None, None
     n_layers, dim, hidden = cfg[2], cfg[0], cfg[1]
     kv_dim = dim * cfg[4] // cfg[3]
-    flops = 2.0 * n_pre * n_layers * (2 * dim * dim + 2 * dim * kv_dim + 3 * dim * hidden) / world
+    # the W4 products that run: in the last layer only q|k|v sees every row, the others the last row alone
+    qkv, rest = dim * dim + 2 * dim * kv_dim, dim * dim + 3 * dim * hidden
+    flops = 2.0 * (n_pre * (n_layers * qkv + (n_layers - 1) * rest) + rest) / world
     out["prefill_512"] = {"ms": ms_pre, "tok_s": n_pre / ms_pre * 1e3, "ms_token_by_token": ms_tok, "speedup_vs_token_by_token": ms_tok / ms_pre,
                           "w4_gemm_tflops_per_gpu": flops / (ms_pre * 1e-3) / 1e12, "frac_of_bf16_sustained": flops / (ms_pre * 1e-3) / 1e12 / pk.get("bf16_tflops_sustained", pk["bf16_tflops"]),
                           # position 511 of a 32-layer random-weight model: every path (this one, the fused token kernel) lies this far from
