@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_rows_kernel(__half* 
         load4(kv, vv, t0);
         round4(kv, vv, pos + 1 - t0);
     }
-    // The round that holds position pos is a warp's last, behind a loop that knows nothing of it (64 registers instead of 79: 16
+    // The round that holds position pos is a warp's last, behind a loop that knows nothing of it (64 registers instead of 71: 16
     // sequences at position 1900, step of two 7B layers, 415 -> 335 us).
     if (FUSED && t0 <= pos) {
         uint2 kv[kAttKeys], vv[kAttKeys];
