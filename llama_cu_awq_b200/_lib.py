@@ -136,14 +136,13 @@ SIGNATURES = {
 TEST_SIGNATURES = {
     "q4_test_set_fused_debug": (None, [_I]),
     "q4_test_set_split_len": (None, [_I]),
-    "q4_test_set_ring_entries": (None, [_I]),
+    "q4_test_set_ring_depth": (None, [_I]),
     "q4_test_fail_fused_alloc": (None, [_I]),
     "q4_test_comm_set_peer": (_I, [_P, _I, _P]),
     "q4_test_fused_gemv": (_I, [_P, _P, _P, _QW, _I, _I]),
     "q4_test_fail_rows_alloc": (None, [_I]),
     "q4_test_fail_set_pos": (None, []),
     "q4_test_gemm_silu": (_I, [_P, _P, _P, _QW, _P, _I, _I, _I, _P, C.c_size_t]),
-    "q4_test_model_slot_trace": (_I, [_P, _P]),
 }
 
 _lib = None

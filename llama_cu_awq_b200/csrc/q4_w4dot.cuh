@@ -1,0 +1,128 @@
+// The W4 dot product of one activation row on the integer tensor pipe, shared by the fused decode kernel (q4_fused.cu) and the
+// per-op GEMV (q4_gemv.cu).
+//
+// Activations are re-expressed per group of 128 as 16-bit block fixed point X = rint(x / sx), sx = max|x| / 32512. A packed
+// byte b = 16*qo + ql (odd and even input) is multiplied as it lies and once more with its low nibble:
+//     sum b*Xo + sum ql*(16*Xe - Xo) = 16 * sum q*X,
+// one AND per packed word. Both multipliers are split into signed bytes (weights 65536, 256, 1), which are columns of
+// mma.sync.m16n8k32 (u8 x s8, int32): exact integer arithmetic. Rows 0-7 of the product are 8 output columns over group A of a
+// pair of groups, rows 8-15 the same columns over group B; columns 0-3 are group A's bytes, 4-7 group B's, and the two crosswise
+// quarters are not used. Per (column, group): y += scale * sx * sum (q - zero) * X, fp32. The step of x is max|x| / 65024 per
+// element, below fp16's own rounding of the largest elements; nibbles, zero points and scales are used exactly.
+// Per 16 columns x 128 inputs: 8 half-rate ANDs per lane and 4 products at 8 clocks, where DP4A took 48 half-rate operations and
+// half2 FMA 72.
+#pragma once
+#include <math_constants.h>
+
+#include "q4_common.cuh"
+
+constexpr int kPairScratch = 1024;   // bytes of shared memory per warp: one pair's digits on their way into operand order
+
+__device__ __forceinline__ void mma_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_u8s8_first(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {   // c = a b
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// One pair's activations (2 groups = 256 inputs) in operand order, in registers.
+struct PairX {
+    uint4 raw, lo;      // digits that meet the packed bytes as they lie, and the low nibbles
+    float sx;           // scale of X, divided by 16
+    int s16;            // 16 * sum of X over the lane's group (lanes that hold the high digits), else 0
+};
+
+// Quantises one pair (lane l holds elements 8l..8l+7 as fp16). X comes out of an FMA with a magic constant (the integer sits in the
+// low mantissa bits) that also adds 0x8080: the bytes of X + 0x8080, each with its top bit flipped, are X's signed digits, and
+// likewise those of 16*Xe - Xo + 0x808080. The digits are gathered by four with byte permutes and go through the warp's scratch
+// into the product's column operand. Lane 4n + t of it is column n and holds four of the group's 16 words: t, 4 + t, 8 + t,
+// 12 + t, or with FILE_ORDER 4t..4t + 3, as 16-byte loads of the file layout have them.
+// A NaN makes its group's scale NaN, an infinity makes it infinite (the group's finite elements count as nothing beside it).
+template <bool FILE_ORDER>
+__device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int lane, PairX& px) {
+    constexpr float kMagic = 12582912.0f + 32896.0f;   // 1.5 * 2^23 + 0x8080
+    constexpr uint32_t kBits = 0x4B408080u;
+    const __half2* h = reinterpret_cast<const __half2*>(&hv);
+    const __half2 m2 = __hmax2_nan(__hmax2_nan(__habs2(h[0]), __habs2(h[1])), __hmax2_nan(__habs2(h[2]), __habs2(h[3])));
+    float amax = max_nan(__low2float(m2), __high2float(m2));
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // 16 lanes = 1 group
+    float inv = amax > 0.f ? 32512.0f / amax : 0.f;
+    float2 f[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) f[j] = __half22float2(h[j]);
+    if (amax == CUDART_INF_F) {
+        inv = 32512.0f;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            f[j].x = isinf(f[j].x) ? copysignf(1.f, f[j].x) : 0.f;
+            f[j].y = isinf(f[j].y) ? copysignf(1.f, f[j].y) : 0.f;
+        }
+    }
+    uint32_t e[4], o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        e[j] = __float_as_uint(fmaf(f[j].x, inv, kMagic));
+        o[j] = __float_as_uint(fmaf(f[j].y, inv, kMagic));
+    }
+    int sum = (int)(((e[0] + o[0]) + (e[1] + o[1])) + ((e[2] + o[2]) + (e[3] + o[3])) - 8u * kBits);
+#pragma unroll
+    for (int s = 1; s < 16; s <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+    const uint32_t o01 = prmt(o[0], o[1], 0x5140), o23 = prmt(o[2], o[3], 0x5140);
+    const uint32_t r0 = prmt(o01, o23, 0x5410) ^ 0x80808080u, r1 = prmt(o01, o23, 0x7632) ^ 0x80808080u;
+    uint32_t z[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) z[j] = 16u * e[j] - o[j] + (0x808080u - 15u * kBits);
+    const uint32_t z01 = prmt(z[0], z[1], 0x5140), z23 = prmt(z[2], z[3], 0x5140);
+    const uint32_t l0 = prmt(z01, z23, 0x5410) ^ 0x80808080u, l1 = prmt(z01, z23, 0x7632) ^ 0x80808080u;
+    const uint32_t l2 = prmt(prmt(z[0], z[1], 0x0062), prmt(z[2], z[3], 0x0062), 0x5410) ^ 0x80808080u;
+    // word j = lane & 15 of group lane >> 4 -> [column 4 * group + digit][t][position in t's four words]
+    const int j = lane & 15, at = FILE_ORDER ? j : (j & 3) * 4 + (j >> 2);
+    uint32_t* d = reinterpret_cast<uint32_t*>(scr) + (lane >> 4) * 64 + at;
+    __syncwarp();       // the previous pair's digits have been read
+    d[0] = 0;       d[16] = r1;       d[32] = r0;       d[48] = 0;
+    d[128] = l2;    d[128 + 16] = l1; d[128 + 32] = l0; d[128 + 48] = 0;
+    __syncwarp();
+    px.raw = *reinterpret_cast<const uint4*>(scr + lane * 16);
+    px.lo = *reinterpret_cast<const uint4*>(scr + 512 + lane * 16);
+    px.sx = __shfl_sync(0xffffffffu, amax, (lane & 2) * 8) * (1.0f / (32512.0f * 16.0f));
+    const int sg = __shfl_sync(0xffffffffu, sum, (lane & 2) * 8);
+    px.s16 = (lane & 1) ? 0 : 16 * sg;
+}
+
+// One pair's product with 8 columns. Lane 4c + t: wa = words h = 0, 1 and wb = words h = 2, 3 of its four packed words of column c,
+// each as (group A, h), (group B, h), (group A, h + 1), (group B, h + 1): the product's row operand as it lies in registers.
+__device__ __forceinline__ void pair_mma(int (&c)[4], const uint4& wa, const uint4& wb, const PairX& px) {
+    constexpr uint32_t kLow = 0x0F0F0F0Fu;
+    mma_u8s8_first(c, wa.x, wa.y, wa.z, wa.w, px.raw.x, px.raw.y);
+    mma_u8s8(c, wa.x & kLow, wa.y & kLow, wa.z & kLow, wa.w & kLow, px.lo.x, px.lo.y);
+    mma_u8s8(c, wb.x, wb.y, wb.z, wb.w, px.raw.z, px.raw.w);
+    mma_u8s8(c, wb.x & kLow, wb.y & kLow, wb.z & kLow, wb.w & kLow, px.lo.z, px.lo.w);
+}
+// This lane's share of column lane >> 2, to be added over the quad. meta: fp16 scale | zero point << 16 of the column in group
+// (lane >> 1) & 1. Lanes t = 0, 1 hold rows 0-7, columns 0, 1 (weights 65536, 256) and 2, 3 (1, unused) of group A, t = 2, 3 rows 8-15
+// of group B.
+__device__ __forceinline__ float pair_share(const int (&c)[4], uint32_t meta, const PairX& px, int lane) {
+    const bool upper = lane & 2;
+    const int w0 = (lane & 1) ? 1 : 65536, w1 = (lane & 1) ? 0 : 256;
+    const int v = (upper ? c[2] : c[0]) * w0 + (upper ? c[3] : c[1]) * w1 - (int)(meta >> 16) * px.s16;
+    return (float)v * (__half2float(__ushort_as_half((unsigned short)(meta & 0xFFFFu))) * px.sx);
+}
+__device__ __forceinline__ float quad_sum(float y) {
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    return y + __shfl_xor_sync(0xffffffffu, y, 2);
+}
+// Both sums over the quad: y0's in its even lanes, y1's in its odd ones
+__device__ __forceinline__ float quad_sum2(float y0, float y1, int lane) {
+    const bool odd = lane & 1;
+    const float other = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 1);
+    const float y = (odd ? y1 : y0) + other;
+    return y + __shfl_xor_sync(0xffffffffu, y, 2);
+}
