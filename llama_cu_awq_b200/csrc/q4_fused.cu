@@ -851,7 +851,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                 }
                 __syncwarp();
                 if (first) TRACE(pi, 5);
-                quant_pair<false>(hv, scr, lane, px);
+                quant_pair(hv, scr, lane, px);
                 if (first) TRACE(pi, 1);
             }
             // ---- its n items, two at a time; a tile's later pairs add to the first one's ----
@@ -1495,7 +1495,7 @@ __global__ void __launch_bounds__(kThreads) test_gemv_kernel(const uint8_t* stre
         for (int j = 0; j < 8; j++)
             if (it * 256 + lane * 8 + j < kind.K) h[j] = x[it * 256 + lane * 8 + j];
         PairX px;
-        quant_pair<false>(hv, scr[w], lane, px);
+        quant_pair(hv, scr[w], lane, px);
         const int c = it - s.i0;
         const uint4* src = reinterpret_cast<const uint4*>(stream + ((size_t)(c >> 1) * grid * kW + (size_t)cta * kW + w) * kChunkBytes + (c & 1) * kItemBytes);
         for (int i = lane; i < kItemBytes / 16; i += 32) reinterpret_cast<uint4*>(items[w])[i] = src[i];

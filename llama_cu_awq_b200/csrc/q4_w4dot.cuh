@@ -42,10 +42,8 @@ struct PairX {
 // Quantises one pair (lane l holds elements 8l..8l+7 as fp16). X comes out of an FMA with a magic constant (the integer sits in the
 // low mantissa bits) that also adds 0x8080: the bytes of X + 0x8080, each with its top bit flipped, are X's signed digits, and
 // likewise those of 16*Xe - Xo + 0x808080. The digits are gathered by four with byte permutes and go through the warp's scratch
-// into the product's column operand. Lane 4n + t of it is column n and holds four of the group's 16 words: t, 4 + t, 8 + t,
-// 12 + t, or with FILE_ORDER 4t..4t + 3, as 16-byte loads of the file layout have them.
+// into the product's column operand. Lane 4n + t of it is column n and holds four of the group's 16 words: t, 4 + t, 8 + t, 12 + t.
 // A NaN makes its group's scale NaN, an infinity makes it infinite (the group's finite elements count as nothing beside it).
-template <bool FILE_ORDER>
 __device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int lane, PairX& px) {
     constexpr float kMagic = 12582912.0f + 32896.0f;   // 1.5 * 2^23 + 0x8080
     constexpr uint32_t kBits = 0x4B408080u;
@@ -84,7 +82,7 @@ __device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int la
     const uint32_t l0 = prmt(z01, z23, 0x5410) ^ 0x80808080u, l1 = prmt(z01, z23, 0x7632) ^ 0x80808080u;
     const uint32_t l2 = prmt(prmt(z[0], z[1], 0x0062), prmt(z[2], z[3], 0x0062), 0x5410) ^ 0x80808080u;
     // word j = lane & 15 of group lane >> 4 -> [column 4 * group + digit][t][position in t's four words]
-    const int j = lane & 15, at = FILE_ORDER ? j : (j & 3) * 4 + (j >> 2);
+    const int j = lane & 15, at = (j & 3) * 4 + (j >> 2);
     uint32_t* d = reinterpret_cast<uint32_t*>(scr) + (lane >> 4) * 64 + at;
     __syncwarp();       // the previous pair's digits have been read
     d[0] = 0;       d[16] = r1;       d[32] = r0;       d[48] = 0;
@@ -93,6 +91,7 @@ __device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int la
     px.raw = *reinterpret_cast<const uint4*>(scr + lane * 16);
     px.lo = *reinterpret_cast<const uint4*>(scr + 512 + lane * 16);
     px.sx = __shfl_sync(0xffffffffu, amax, (lane & 2) * 8) * (1.0f / (32512.0f * 16.0f));
+    if (px.sx == CUDART_INF_F && (lane & 1)) px.sx = 0.f;   // (the low digits are zero then, and must not turn the sum into 0 * inf)
     const int sg = __shfl_sync(0xffffffffu, sum, (lane & 2) * 8);
     px.s16 = (lane & 1) ? 0 : 16 * sg;
 }

@@ -155,3 +155,30 @@ def test_unsupported_sizes_return_status():
     with pytest.raises(ops.Q4Error) as e:
         ops.matmul(y, dev(x), dev(x), 12, 8)
     assert e.value.status == _lib.Q4_ERR_UNSUPPORTED_SIZE
+
+
+@pytest.mark.parametrize("K,N", [(256, 8 * 297), (520, 1184 * 8 + 8), (1024, 40008), (8192, 4744 * 8), (28672, 24), (4352, 2376)])
+def test_matvec_splits(K, N):
+    """Tiles and pairs per stage as the launch chooses them: several tiles of short rows in a stage, a last group of tiles that is not
+    full, more tiles than one pass holds, many chunks, a last chunk with one pair. Bound: the rounding of the result to fp16 (2^-11 of
+    each value, relative to the largest at most 4.9e-4) and the fixed-point step of x (2^-16 of a group's largest, averaged over K)."""
+    q, x, _ = mk(K, N, seed=K + N)
+    W = ops.QWeight.from_numpy(q)
+    y = torch.full((N,), float("nan"), dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), W, K, N)
+    assert_close(y.cpu().numpy(), O.matvec_f32(x, q, K, N), f"matvec {K}x{N}", max_rel=1e-3)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_matvec_non_finite_inputs(value):
+    """A NaN in x makes every output NaN, an infinity makes it infinite with the weight's sign, or NaN where the weight is zero."""
+    K, N = 512, 64
+    q, x, _ = mk(K, N, seed=3)
+    x[300] = value
+    W = ops.QWeight.from_numpy(q)
+    y = torch.empty(N, dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), W, K, N)
+    w = O.dequant(q, K, N)[:, 300]
+    with np.errstate(invalid="ignore"):
+        want = w * np.float32(value)
+    assert np.array_equal(y.float().cpu().numpy(), want, equal_nan=True)
