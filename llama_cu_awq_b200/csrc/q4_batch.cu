@@ -887,16 +887,17 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
                         r->rope, r->row_seq, r->row_pos, seq_stride, loff);
         if (l == c.n_layers - 1 && want != WANT_ALL) {
             if (want == WANT_CACHE) break;
-            // one row: the split attention of the batch-1 path and the few-rows kernels
+            // one row: the split attention and the products of the batch-1 path (70B: o, gate / up and down 147 us with the few-rows kernels, 94 so,
+            // and half their error)
             const size_t last = (size_t)(n - 1);
             uint16_t* x = (uint16_t*)(r->X + last * dim);
             OP(q4_attention(s, (uint16_t*)r->ATT, (const uint16_t*)qp + last * ldq, (const uint16_t*)(kc + loff), (const uint16_t*)(vc + loff), m->attn_scratch, heads, m->head_size,
                             m->kv_mul, c.seq_len, r->row_pos + last));
-            OP(q4_matmul_q4_rows(s, x, (const uint16_t*)r->ATT, &L.o.w, 1, m->o_kc, dim, x, 1.0f / g));
+            OP(q4_matmul_q4(s, x, (const uint16_t*)r->ATT, &L.o.w, m->o_kc, dim, 1, g, -1, nullptr));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
             launch_rows(rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);
-            OP(q4_ffn_silu_rows(s, (uint16_t*)r->G, (const uint16_t*)r->XB, &L.gate.w, &L.up.w, 1, dim, m->h_kc));
-            OP(q4_matmul_q4_rows(s, x, (const uint16_t*)r->G, &L.down.w, 1, m->h_kc, dim, x, 1.0f / g));
+            OP(q4_ffn_matvec_silu(s, (uint16_t*)r->G, (const uint16_t*)r->XB, &L.gate.w, &L.up.w, dim, m->h_kc));
+            OP(q4_matmul_q4(s, x, (const uint16_t*)r->G, &L.down.w, m->h_kc, dim, 1, g, -1, nullptr));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
             break;
         }
