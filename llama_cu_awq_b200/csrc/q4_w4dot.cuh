@@ -26,12 +26,6 @@ __device__ __forceinline__ void mma_u8s8_first(int (&c)[4], uint32_t a0, uint32_
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
-__device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
 // One pair's activations (2 groups = 256 inputs) in operand order, in registers.
 struct PairX {
     uint4 raw, lo;      // digits that meet the packed bytes as they lie, and the low nibbles
@@ -48,10 +42,12 @@ __device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int la
     constexpr float kMagic = 12582912.0f + 32896.0f;   // 1.5 * 2^23 + 0x8080
     constexpr uint32_t kBits = 0x4B408080u;
     const __half2* h = reinterpret_cast<const __half2*>(&hv);
-    const __half2 m2 = __hmax2_nan(__hmax2_nan(__habs2(h[0]), __habs2(h[1])), __hmax2_nan(__habs2(h[2]), __habs2(h[3])));
-    float amax = max_nan(__low2float(m2), __high2float(m2));
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // 16 lanes = 1 group
+    const bool high = lane & 16;                    // 16 lanes = 1 group
+    // |x| as integers: fp16 bits without the sign are in the order of the values, NaN above infinity
+    const uint32_t m4 = __vmaxu2(__vmaxu2(hv.x & 0x7FFF7FFFu, hv.y & 0x7FFF7FFFu), __vmaxu2(hv.z & 0x7FFF7FFFu, hv.w & 0x7FFF7FFFu));
+    const uint32_t mine = max(m4 & 0xFFFFu, m4 >> 16);
+    const uint32_t ma = __reduce_max_sync(0xffffffffu, high ? 0u : mine), mb = __reduce_max_sync(0xffffffffu, high ? mine : 0u);
+    const float amax = __half2float(__ushort_as_half((unsigned short)(high ? mb : ma)));
     float inv = amax > 0.f ? 32512.0f / amax : 0.f;
     float2 f[4];
 #pragma unroll
@@ -70,9 +66,8 @@ __device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int la
         e[j] = __float_as_uint(fmaf(f[j].x, inv, kMagic));
         o[j] = __float_as_uint(fmaf(f[j].y, inv, kMagic));
     }
-    int sum = (int)(((e[0] + o[0]) + (e[1] + o[1])) + ((e[2] + o[2]) + (e[3] + o[3])) - 8u * kBits);
-#pragma unroll
-    for (int s = 1; s < 16; s <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+    const int part = (int)(((e[0] + o[0]) + (e[1] + o[1])) + ((e[2] + o[2]) + (e[3] + o[3])) - 8u * kBits);
+    const int sum_a = __reduce_add_sync(0xffffffffu, high ? 0 : part), sum_b = __reduce_add_sync(0xffffffffu, high ? part : 0);
     const uint32_t o01 = prmt(o[0], o[1], 0x5140), o23 = prmt(o[2], o[3], 0x5140);
     const uint32_t r0 = prmt(o01, o23, 0x5410) ^ 0x80808080u, r1 = prmt(o01, o23, 0x7632) ^ 0x80808080u;
     uint32_t z[4];
@@ -90,10 +85,9 @@ __device__ __forceinline__ void quant_pair(const uint4& hv, uint8_t* scr, int la
     __syncwarp();
     px.raw = *reinterpret_cast<const uint4*>(scr + lane * 16);
     px.lo = *reinterpret_cast<const uint4*>(scr + 512 + lane * 16);
-    px.sx = __shfl_sync(0xffffffffu, amax, (lane & 2) * 8) * (1.0f / (32512.0f * 16.0f));
+    px.sx = __half2float(__ushort_as_half((unsigned short)((lane & 2) ? mb : ma))) * (1.0f / (32512.0f * 16.0f));
     if (px.sx == CUDART_INF_F && (lane & 1)) px.sx = 0.f;   // (the low digits are zero then, and must not turn the sum into 0 * inf)
-    const int sg = __shfl_sync(0xffffffffu, sum, (lane & 2) * 8);
-    px.s16 = (lane & 1) ? 0 : 16 * sg;
+    px.s16 = (lane & 1) ? 0 : 16 * ((lane & 2) ? sum_b : sum_a);
 }
 
 // One pair's product with 8 columns. Lane 4c + t: wa = words h = 0, 1 and wb = words h = 2, 3 of its four packed words of column c,
