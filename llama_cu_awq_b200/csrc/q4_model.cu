@@ -563,7 +563,9 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
         else if (e != Q4_ERR_UNSUPPORTED_SIZE) { cudaStreamDestroy(s); return e; }
     }
     while (pos < steps) {
-        cudaStreamSynchronize(s);  // previous token done; its id is in the mailbox
+        // A generated id is in the mailbox when its token is done; a prompt's ids are there already, and its positions are queued without
+        // a wait (48 positions of four 7B layers: 7.55 ms with one each).
+        if (pos >= n_prompt) cudaStreamSynchronize(s);
         e = q4_model_forward(m, s, pos >= n_prompt - 1, path);
         if (e != Q4_OK) break;
         if (pos > 0) {
