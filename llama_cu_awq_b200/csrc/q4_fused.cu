@@ -405,7 +405,8 @@ __device__ __forceinline__ const uint8_t* ring_wait(Ring& r, const FParams& p) {
     }
     return r.base + r.slot * kChunkBytes;
 }
-// The warp has read the chunk (the caller's shuffles of values made from it are behind it).
+// The warp has read the chunk: a shuffle or vote of values made from all that each lane read of it is behind the caller (a barrier alone
+// does not wait for loads in flight).
 __device__ __forceinline__ void ring_release(Ring& r, const FParams& p, const uint8_t* const* streams) {
     __syncwarp();
     if (r.dead) return;
@@ -976,6 +977,8 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                         for (int j = 0; j < 8; j++) a[j] = fma_mixed(wh[j], xh[j], a[j]);
                     }
                 }
+                // The vote needs every lane's a[0], and that every one of its loads of the chunk; no product leaves this NaN's bits.
+                if (!__all_sync(0xffffffffu, __float_as_uint(a[0]) != 0x7F800001u)) break;
                 ring_release(ring, p, streams);
             }
             const float sum = warp_sum(((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])));

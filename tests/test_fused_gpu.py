@@ -266,3 +266,25 @@ def test_two_models_keep_their_shared_memory_limits(order):
         assert t.status() == 0 and np.isfinite(t.logits()).all()
     for t in models:
         t.close()
+
+
+@pytest.mark.parametrize("cfg", [(256, 512, 2, 2, 2, 512, 64, 10000.0),            # fewer items than warps
+                                 (1024, 2816, 2, 8, 2, 2048, 64, 10000.0),         # odd numbers of items per warp, a last pair with one group
+                                 (4096, 11008, 1, 32, 32, 32000, 64, 10000.0)])    # a long classifier: most of a token's chunks
+def test_ring_depth_does_not_change_a_bit(cfg):
+    """A warp's ring with its smallest depths, where a slot is refilled as soon as it has been read, against the depth the model gets."""
+    L = _lib.test_lib()
+    tokens = np.random.default_rng(11).integers(3, cfg[5], size=24, dtype=np.int32)
+    out = []
+    try:
+        for depth in (0, 2, 3):
+            L.q4_test_set_ring_depth(depth)
+            t = Transformer(None, lib=L, synthetic=(cfg, 5))
+            assert t.best_path() == 2
+            out += [_run(t, tokens, queued=True) for _ in range(3)]
+            t.close()
+    finally:
+        L.q4_test_set_ring_depth(0)
+    assert np.isfinite(out[0].astype(np.float32)).all()
+    for o in out[1:]:
+        assert (o.view(np.uint16) == out[0].view(np.uint16)).all()
