@@ -7,8 +7,9 @@
 // one AND per packed word. Both multipliers are split into signed bytes (weights 65536, 256, 1), which are columns of
 // mma.sync.m16n8k32 (u8 x s8, int32): exact integer arithmetic. Rows 0-7 of the product are 8 output columns over group A of a
 // pair of groups, rows 8-15 the same columns over group B; columns 0-3 are group A's bytes, 4-7 group B's, and the two crosswise
-// quarters are not used. Per (column, group): y += scale * sx * sum (q - zero) * X, fp32. The step of x is max|x| / 65024 per
-// element, below fp16's own rounding of the largest elements; nibbles, zero points and scales are used exactly.
+// quarters are not used. Per (column, group): y += scale * sx * sum (q - zero) * X, fp32. An element is off by max|x| / 65024 at most,
+// below fp16's own rounding of the largest elements; nibbles, zero points and scales are used exactly. The fused kernel multiplies so
+// what it has computed itself; a caller's x goes through the exact form below (PairExact).
 // Per 16 columns x 128 inputs: 8 half-rate ANDs per lane and 4 products at 8 clocks, where DP4A took 48 half-rate operations and
 // half2 FMA 72.
 #pragma once
@@ -108,6 +109,124 @@ __device__ __forceinline__ float pair_share(const int (&c)[4], uint32_t meta, co
     const int v = (upper ? c[2] : c[0]) * w0 + (upper ? c[3] : c[1]) * w1 - (int)(meta >> 16) * px.s16;
     return (float)v * (__half2float(__ushort_as_half((unsigned short)(meta & 0xFFFFu))) * px.sx);
 }
+// ---- the same product with x as it is (the per-op GEMV, whose x is the caller's) ----
+// X = x / sx with a power of two for sx, so that the group's largest element has 26 bits: every element down to 2^-15 of it is held
+// exactly, all four columns of a group carry digits (weights 2^24, 65536, 256, 1), and the zero point is taken off column by column, so
+// that an element whose weight is zero leaves nothing behind. Smaller elements are rounded to 2^-27 of the largest (2^-15 of what that
+// one's own fp16 rounding is; an output of SiLU has many such), unless fewer than kManyHeld elements are held exactly: then, and in a
+// group with a NaN or an infinity, the elements that X does not hold are left out of it and multiplied in fp32 (small_dot).
+constexpr int kManyHeld = 32;
+constexpr int kExactScratch = 1152;  // bytes of shared memory per warp
+struct PairExact {
+    uint4 raw, lo;
+    float sx;           // scale of the lane's columns of digits, divided by 16
+    int zero;           // what one step of the zero point adds to them
+};
+
+// Returns true (to the whole warp) when some elements are left to small_dot: those of group A (B) whose magnitude is below the fp16 bits
+// in the lower (upper) half of the scratch's first word.
+__device__ __forceinline__ bool quant_pair_exact(const uint4& hv, uint8_t* scr, int lane, PairExact& px) {
+    const __half2* h = reinterpret_cast<const __half2*>(&hv);
+    const bool high = lane & 16;
+    const uint32_t mag[4] = {hv.x & 0x7FFF7FFFu, hv.y & 0x7FFF7FFFu, hv.z & 0x7FFF7FFFu, hv.w & 0x7FFF7FFFu};
+    const uint32_t m4 = __vmaxu2(__vmaxu2(mag[0], mag[1]), __vmaxu2(mag[2], mag[3]));
+    const uint32_t mine = max(m4 & 0xFFFFu, m4 >> 16);
+    const uint32_t ma = __reduce_max_sync(0xffffffffu, high ? 0u : mine), mb = __reduce_max_sync(0xffffffffu, high ? mine : 0u);
+    // 2^(40 - E) for the largest element's exponent field E (fp16): X = x * that, up to 2^26
+    const float mul = __uint_as_float((167u - ((high ? mb : ma) >> 10)) << 23);
+    float2 f[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) f[j] = __half22float2(h[j]);
+    uint32_t small = 0;
+    if (max(ma, mb) >= (17u << 10)) {   // 4 and more: below, every fp16 has all its bits in X
+        // the fp16 bits below which an element has bits that X does not hold; everything in a group with a NaN or an infinity
+        auto below = [](uint32_t m) { return m >= 0x7C00u ? 0x8000u : m >= (17u << 10) ? ((m >> 10) - 15u) << 10 : 0u; };
+        uint32_t lim = below(high ? mb : ma);
+        int held = 0;       // elements that are not zero and have all their bits in X
+#pragma unroll
+        for (int j = 0; j < 4; j++) held += ((mag[j] & 0xFFFFu) >= max(lim, 1u)) + ((mag[j] >> 16) >= max(lim, 1u));
+        const int na = __reduce_add_sync(0xffffffffu, high ? 0 : held), nb = __reduce_add_sync(0xffffffffu, high ? held : 0);
+        const uint32_t la = ma < 0x7C00u && na >= kManyHeld ? 0u : below(ma), lb = mb < 0x7C00u && nb >= kManyHeld ? 0u : below(mb);
+        small = la | (lb << 16);
+        lim = high ? lb : la;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if ((mag[j] & 0xFFFFu) < lim) f[j].x = 0.f;
+            if ((mag[j] >> 16) < lim) f[j].y = 0.f;
+        }
+    }
+    // The bytes of X + 0x80808080, each with its top bit flipped, are X's signed digits, and likewise those of 16 Xe - Xo + 0x80808080.
+    // (Conversions have a pipe of their own; splitting X by magic constants instead costs twice as many issue slots.)
+    uint32_t o[4], z[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        o[j] = (uint32_t)__float2int_rn(f[j].y * mul) + 0x80808080u;
+        z[j] = 16u * (uint32_t)__float2int_rn(f[j].x * mul) + (0x01010100u - o[j]);
+    }
+    // word j = lane & 15 of group lane >> 4 -> [column 4 * group + digit][j], the groups 16 banks apart
+    uint32_t* d = reinterpret_cast<uint32_t*>(scr) + (lane >> 4) * 80 + (lane & 15);
+    __syncwarp();       // the previous pair's digits have been read
+    auto file = [](uint32_t* to, const uint32_t (&w)[4]) {
+        const uint32_t l01 = prmt(w[0], w[1], 0x5140), l23 = prmt(w[2], w[3], 0x5140), h01 = prmt(w[0], w[1], 0x7362), h23 = prmt(w[2], w[3], 0x7362);
+        to[0] = prmt(h01, h23, 0x7632) ^ 0x80808080u;
+        to[16] = prmt(h01, h23, 0x5410) ^ 0x80808080u;
+        to[32] = prmt(l01, l23, 0x7632) ^ 0x80808080u;
+        to[48] = prmt(l01, l23, 0x5410) ^ 0x80808080u;
+    };
+    file(d, o);
+    file(d + 144, z);
+    __syncwarp();
+    const uint8_t* mine4 = scr + lane * 16 + (lane >> 4) * 64;
+    px.raw = *reinterpret_cast<const uint4*>(mine4);
+    px.lo = *reinterpret_cast<const uint4*>(mine4 + 576);
+    // sx / 16 = 2^(E - 44), and for the upper two digits' columns 65536 times that
+    px.sx = __uint_as_float((((lane & 2) ? mb : ma) >> 10) + ((lane & 1) ? 83u : 99u) << 23);
+    px.zero = 0;        // (zero_step)
+    if (small) {
+        __syncwarp();
+        if (lane == 0) *reinterpret_cast<uint32_t*>(scr) = small;
+        __syncwarp();
+    }
+    return small != 0;
+}
+// The product with weights of one everywhere (17 as a byte, 1 as a low nibble): what one step of the zero point adds to each column. Apart
+// from quant_pair_exact, so that a warp with two pairs does not wait for the first one's digits before it starts on the second's.
+__device__ __forceinline__ void zero_step(PairExact& px) {
+    int a[4], b[4];
+    mma_u8s8_first(a, 0x11111111u, 0x11111111u, 0x11111111u, 0x11111111u, px.raw.x, px.raw.y);
+    mma_u8s8_first(b, 0x11111111u, 0x11111111u, 0x11111111u, 0x11111111u, px.raw.z, px.raw.w);
+    mma_u8s8(a, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, px.lo.x, px.lo.y);
+    mma_u8s8(b, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, px.lo.z, px.lo.w);
+    px.zero = 256 * (a[0] + b[0]) + a[1] + b[1];
+}
+// pair_mma of lane 4c + t with words 4t..4t + 3 of column c in groups A and B, as two chains: a chain's next product waits for the one before
+__device__ __forceinline__ void pair_mma_exact(int (&c)[4], const uint4& a, const uint4& b, const PairExact& px) {
+    constexpr uint32_t kLow = 0x0F0F0F0Fu;
+    int d[4];
+    mma_u8s8_first(c, a.x, b.x, a.y, b.y, px.raw.x, px.raw.y);
+    mma_u8s8_first(d, a.z, b.z, a.w, b.w, px.raw.z, px.raw.w);
+    mma_u8s8(c, a.x & kLow, b.x & kLow, a.y & kLow, b.y & kLow, px.lo.x, px.lo.y);
+    mma_u8s8(d, a.z & kLow, b.z & kLow, a.w & kLow, b.w & kLow, px.lo.z, px.lo.w);
+#pragma unroll
+    for (int i = 0; i < 4; i++) c[i] += d[i];
+}
+// As pair_share: lanes t = 0, 2 hold the upper two digits' columns of their group, t = 1, 3 the lower two.
+__device__ __forceinline__ float pair_share(const int (&c)[4], uint32_t meta, const PairExact& px, int lane) {
+    const bool upper = lane & 2;
+    const uint32_t v = (uint32_t)(upper ? c[2] : c[0]) * 256u + (uint32_t)(upper ? c[3] : c[1]) - (meta >> 16) * (uint32_t)px.zero;
+    return (float)(int)v * (__half2float(__ushort_as_half((unsigned short)(meta & 0xFFFFu))) * px.sx);
+}
+// sum + the products of a packed word's nibbles, less the zero point, with those of its 8 inputs whose magnitude is below lim (fp16 bits)
+__device__ __forceinline__ float small_dot(uint32_t w, const uint4& xv, uint32_t lim, int zero, float sum) {
+    const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const uint32_t bits = (j & 1) ? xw[j >> 1] >> 16 : xw[j >> 1] & 0xFFFFu;
+        if ((bits & 0x7FFFu) < lim) sum = fmaf((float)((int)((w >> (4 * j)) & 0xFu) - zero), __half2float(__ushort_as_half((unsigned short)bits)), sum);
+    }
+    return sum;
+}
+
 __device__ __forceinline__ float quad_sum(float y) {
     y += __shfl_xor_sync(0xffffffffu, y, 1);
     return y + __shfl_xor_sync(0xffffffffu, y, 2);

@@ -58,9 +58,8 @@ def test_config0_single_layer():
     assert r < 3e-3 and c > 0.99999
 
 
-@pytest.mark.parametrize("g", [1, 2, 8])
-def test_matvec_accum_residual(g):
-    K, N = 1024, 256
+@pytest.mark.parametrize("g,K,N", [(1, 1024, 256), (2, 1024, 256), (8, 1024, 256), (2, 11008, 4096)])
+def test_matvec_accum_residual(g, K, N):
     q, x, rng = mk(K, N, seed=g)
     W = ops.QWeight.from_numpy(q)
     y0 = (rng.standard_normal(N) * 5).astype(np.float16)
@@ -157,10 +156,12 @@ def test_unsupported_sizes_return_status():
     assert e.value.status == _lib.Q4_ERR_UNSUPPORTED_SIZE
 
 
-@pytest.mark.parametrize("K,N", [(256, 8 * 297), (520, 1184 * 8 + 8), (1024, 40008), (8192, 4744 * 8), (28672, 24), (4352, 2376)])
+@pytest.mark.parametrize("K,N", [(256, 8 * 297), (520, 1184 * 8 + 8), (1024, 40008), (8192, 4744 * 8), (28672, 24), (4352, 2376),
+                                 (4352, 10400), (520, 90000), (4096, 11008), (4096, 3 * 148 * 8)])
 def test_matvec_splits(K, N):
-    """Tiles and pairs per stage as the launch chooses them: several tiles of short rows in a stage, a last group of tiles that is not
-    full, more tiles than one pass holds, many chunks, a last chunk with one pair. Bound: the rounding of the result to fp16 (2^-11 of
+    """Both forms of the kernel as the launch chooses them. Direct: fewer items than warps, pairs beyond a multiple of 16, more tiles than
+    one pass holds. Ring: several tiles of short rows in a stage, a last group of tiles that is not full, more tiles than one pass holds,
+    many chunks, a last chunk with one pair. Bound: the rounding of the result to fp16 (2^-11 of
     each value, relative to the largest at most 4.9e-4) and the fixed-point step of x (2^-16 of a group's largest, averaged over K)."""
     q, x, _ = mk(K, N, seed=K + N)
     W = ops.QWeight.from_numpy(q)
@@ -169,16 +170,115 @@ def test_matvec_splits(K, N):
     assert_close(y.cpu().numpy(), O.matvec_f32(x, q, K, N), f"matvec {K}x{N}", max_rel=1e-3)
 
 
+def no_weight_on(q, K, ks):
+    """Gives every column the weight zero (nibble = zero point) on the inputs ks."""
+    for k in ks:
+        g, shift = k // 128, np.uint32(4 * (k % 8))
+        z = (q["zeros"][:, g // 8] >> np.uint32(4 * (g % 8))) & np.uint32(15)
+        w = q["weight"][:, k // 8]
+        q["weight"][:, k // 8] = (w & ~(np.uint32(15) << shift)) | (z << shift)
+    return q
+
+
+def check_against_64_bits(got, q, x, K, N, what):
+    """fp16 result of fp32 sums: half a unit of the result's last place (2^-11 of it, 2^-25 at least), 2^-23 per addition of a sum of K / 128
+    group sums, whose sizes are bounded by the sums of the magnitudes, and half a step of the group's fixed point, 2^(e - 26) with e the
+    exponent of its largest input, for each input below 2^(e - 15) where 32 or more are not."""
+    x = x.astype(np.float64)
+    step = np.zeros(K)
+    for g in range(0, K, 128):
+        a = np.abs(x[g:g + 128])
+        e = np.floor(np.log2(a.max()))
+        if (a >= 2.0 ** (e - 15)).sum() >= 32:
+            step[g:g + 128] = np.where((a > 0) & (a < 2.0 ** (e - 15)) & (e >= 2), 2.0 ** (e - 26), 0)
+    w = O.dequant(q, K, N).astype(np.float64)
+    ref = w @ x
+    bound = 2.0**-11 * np.abs(ref) + 2.0**-25 + 2.0**-23 * (2 * K / 128 + 8) * np.abs(w * x).sum(axis=1) + np.abs(w) @ step
+    worst = np.max(np.abs(got.astype(np.float64) - ref) / bound)
+    assert worst <= 1.0, f"{what}: {worst:.2f} of the bound"
+
+
+@pytest.mark.parametrize("large", [(3,), (64,), (1, 2, 3, 4, 5, 6, 7, 8, 9)])     # in each group: odd, even, many
+@pytest.mark.parametrize("ratio", [100.0, 5000.0, 3e4, 1e6])
+@pytest.mark.parametrize("K,N", [(520, 64), (4096, 64), (11008, 32), (4360, 10400)])
+def test_matvec_small_inputs_beside_large_ones(K, N, ratio, large):
+    """Columns that give no weight to a group's large inputs: the small ones' products must come out as if they were alone."""
+    q, x, rng = mk(K, N, seed=K + int(ratio))
+    ks = [k for k in range(K) if k % 128 in large]
+    x = (x.astype(np.float32) * (16000.0 / ratio)).astype(np.float16)
+    x[ks] = (16000.0 * rng.choice([-1, 1], len(ks))).astype(np.float16)
+    q["scales"] = (q["scales"].astype(np.float32) * min(1.0, ratio / 16000.0)).astype(np.float16)
+    no_weight_on(q, K, ks)
+    y = torch.empty(N, dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), ops.QWeight.from_numpy(q), K, N)
+    check_against_64_bits(y.cpu().numpy(), q, x, K, N, f"{K}x{N}, 1 : {ratio:g}")
+
+
+def test_products_of_several_matrices_with_small_inputs_beside_large_ones():
+    """q|k|v and gate/up with several tiles per stage and several chunks, the accumulating form with several chunks."""
+    for K, N, Nkv in [(384, 2368, 2368), (5000, 1024, 256)]:
+        rng = np.random.default_rng(K)
+        x = (rng.standard_normal(K) * 0.01).astype(np.float16)
+        ks = list(range(5, K, 128))
+        x[ks] = 2000.0
+        qs = [no_weight_on(synth.synth_qweight(rng, K, n), K, ks) for n in (N, Nkv, Nkv)]
+        qo, kc, vc = (torch.zeros(n, dtype=torch.float16, device="cuda") for n in (N, Nkv, Nkv))
+        pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+        Ws = [ops.QWeight.from_numpy(q) for q in qs]
+        ops.qkv_matvec(qo, kc, vc, dev(x), *Ws, K, N, 0, pos, kvSize=Nkv)
+        for got, q, n in zip((qo, kc, vc), qs, (N, Nkv, Nkv)):
+            check_against_64_bits(got.cpu().numpy(), q, x, K, n, f"q|k|v {K}x{n}")
+        ops.matmul(qo, dev(x), Ws[0], K, N, accum=True)     # twice the product: half of one rounding and one of the sum
+        got = qo.cpu().numpy().astype(np.float64) / 2
+        ref = O.dequant(qs[0], K, N).astype(np.float64) @ x.astype(np.float64)
+        assert np.abs(got - ref).max() <= 1.5 * 2.0**-11 * 1.01 * np.abs(ref).max()
+        h = torch.empty(Nkv, dtype=torch.float16, device="cuda")
+        ops.ffn_matvec_silu(h, dev(x), Ws[1], Ws[2], K, Nkv)
+        gate, up = (O.dequant(q, K, Nkv).astype(np.float64) @ x.astype(np.float64) for q in qs[1:])
+        want = gate / (1 + np.exp(-gate)) * up
+        # fp16 rounding of the result; expf and the reciprocal are good to a few units of 2^-23
+        assert np.abs(h.cpu().numpy() - want).max() <= 2.0**-11 * 1.02 * np.abs(want).max() + 1e-6
+
+
+@pytest.mark.parametrize("held", [16, 31, 32, 80])
+def test_matvec_small_inputs_beside_many_held_ones(held):
+    """`held` inputs of a group within 2^-15 of its largest, the others far below: rounded from 32 held ones on, exact below that."""
+    K, N = 1024, 64
+    q, _, rng = mk(K, N, seed=held)
+    x = (rng.standard_normal(K) * 1e-4).astype(np.float16)
+    big = np.concatenate([g * 128 + rng.permutation(128)[:held] for g in range(K // 128)])
+    x[big] = (rng.choice([-1, 1], big.size) * rng.uniform(4, 32, big.size)).astype(np.float16)
+    if held < 32:
+        no_weight_on(q, K, big)
+    y = torch.empty(N, dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), ops.QWeight.from_numpy(q), K, N)
+    check_against_64_bits(y.cpu().numpy(), q, x, K, N, f"{held} held")
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
 def test_matvec_non_finite_inputs(value):
     """A NaN in x makes every output NaN, an infinity makes it infinite with the weight's sign, or NaN where the weight is zero."""
     K, N = 512, 64
     q, x, _ = mk(K, N, seed=3)
     x[300] = value
+    x[37] = value                       # an odd position of another group
     W = ops.QWeight.from_numpy(q)
     y = torch.empty(N, dtype=torch.float16, device="cuda")
     ops.matmul(y, dev(x), W, K, N)
     w = O.dequant(q, K, N)[:, 300]
     with np.errstate(invalid="ignore"):
-        want = w * np.float32(value)
+        want = w * np.float32(value) + O.dequant(q, K, N)[:, 37] * np.float32(value)
     assert np.array_equal(y.float().cpu().numpy(), want, equal_nan=True)
+
+
+def test_matvec_opposite_infinities():
+    """Infinities of both signs in one group, and of one sign in two groups: what IEEE sums of the products give."""
+    K, N = 512, 128
+    q, x, _ = mk(K, N, seed=8)
+    x[[130, 201]] = np.inf, -np.inf
+    x[[3, 400]] = np.inf
+    y = torch.empty(N, dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), ops.QWeight.from_numpy(q), K, N)
+    with np.errstate(invalid="ignore"):
+        want = (O.dequant(q, K, N)[:, [130, 201, 3, 400]] * x[[130, 201, 3, 400]].astype(np.float32)).sum(axis=1)
+    assert np.array_equal(y.float().cpu().numpy(), want, equal_nan=True) and np.isnan(want).any() and np.isinf(want).any()
