@@ -48,7 +48,11 @@ typedef struct {
 /* One quantized matrix, K inputs x N outputs, K-contiguous per output. common.h:26-30.
  *   weight u32[N][4*ceil(K/32)]  nibble i of word j holds q(n, 8j+i)
  *   zeros  u32[N][ceil(ceil(K/128)/8)]
- *   scales f16[N][ceil(K/128)] */
+ *   scales f16[N][ceil(K/128)]
+ * A call may read the packed words before the kernel in front of it on the stream has ended (programmatic dependent
+ * launch); the few-rows forms read scales and zero points as early. A host that changes a matrix in place
+ * by a kernel puts an event or a copy between that kernel and the call. The batch-1 forms (q4_matmul_q4, q4_qkv_matvec,
+ * q4_ffn_matvec_silu) take scales and zero points, as x, only when the kernel in front has ended. */
 typedef struct {
     const uint32_t* weight;
     const uint32_t* zeros;

@@ -402,18 +402,15 @@ __global__ void __launch_bounds__(ring::kThreads, 2) gemv_ring_kernel(const __gr
         }
         __syncwarp();
     };
-    ahead(0, min(per_pass, my_groups), 0);
-    file_meta(0, min(per_pass, my_groups), 0);   // as the weights, before the predecessor's results are waited for
-    if (nchunks > 1)                             // the later chunks' on their way into L2
-        for (int i = tid; i < my_groups * T * kRows; i += 32 * ring::kMathWarps) {
-            int row;
-            const int tile = (cta + i / (T * kRows) * grid) * T + (i / kRows) % T;
-            if (tile < p.total_tiles) {
-                const GemvMat& m = row_of<SILU>(p, tile, i & 7, row);
-                for (int g = 2 * Pc; g < p.G; g += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(m.s + (size_t)row * p.G + g));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(m.z + (size_t)row * p.PZ));
-            }
+    for (int i = tid; i < my_groups * T * kRows; i += 32 * ring::kMathWarps) {   // scales and zero points on their way into L2
+        int row;
+        const int tile = (cta + i / (T * kRows) * grid) * T + (i / kRows) % T;
+        if (tile < p.total_tiles) {
+            const GemvMat& m = row_of<SILU>(p, tile, i & 7, row);
+            for (int g = 0; g < p.G; g += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(m.s + (size_t)row * p.G + g));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(m.z + (size_t)row * p.PZ));
         }
+    }
     griddep_wait();
     griddep_launch_dependents();
     uint4 hv[2];                 // a chunk's activations, requested a chunk ahead (zero beyond K: padded weight words contribute nothing)
@@ -426,6 +423,8 @@ __global__ void __launch_bounds__(ring::kThreads, 2) gemv_ring_kernel(const __gr
         }
     };
     load_x(0);
+    ahead(0, min(per_pass, my_groups), 0);
+    file_meta(0, min(per_pass, my_groups), 0);
     for (int b0 = 0; b0 < my_groups; b0 += per_pass) {
         const int bn = min(per_pass, my_groups - b0);
         for (int c = 0; c < nchunks; c++) {

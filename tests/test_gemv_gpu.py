@@ -282,3 +282,24 @@ def test_matvec_opposite_infinities():
     with np.errstate(invalid="ignore"):
         want = (O.dequant(q, K, N)[:, [130, 201, 3, 400]] * x[[130, 201, 3, 400]].astype(np.float32)).sum(axis=1)
     assert np.array_equal(y.float().cpu().numpy(), want, equal_nan=True) and np.isnan(want).any() and np.isinf(want).any()
+
+
+@pytest.mark.parametrize("K,N", [(1024, 1024), (4352, 10400)])
+def test_scales_changed_by_the_kernel_in_front(K, N):
+    """Both forms of the kernel: scales rewritten in place on the stream directly before the call, with no wait in between."""
+    q, x, _ = mk(K, N, seed=4)
+    W, xd = ops.QWeight.from_numpy(q), dev(x)
+    base = W.scales.clone()
+    want = []
+    for f in (0.5, 1.0):
+        W.scales.copy_(base * f)
+        torch.cuda.synchronize()
+        y = torch.empty(N, dtype=torch.float16, device="cuda")
+        ops.matmul(y, xd, W, K, N)
+        torch.cuda.synchronize()
+        want.append(y)
+    out = torch.empty((200, N), dtype=torch.float16, device="cuda")
+    for i in range(200):
+        torch.mul(base, (0.5, 1.0)[i & 1], out=W.scales)
+        ops.matmul(out[i], xd, W, K, N)
+    assert all(torch.equal(out[i], want[i & 1]) for i in range(200))
