@@ -140,12 +140,13 @@ struct FParams {
 // ------------------------------------------------------------------------------------------------------------
 // device helpers
 // ------------------------------------------------------------------------------------------------------------
-// Bounded wait of a whole warp. Returns false (and records the error) when the limit is hit.
+// Bounded wait of a whole warp. Returns false (and records the error) when the limit is hit, or at once when another wait has run out.
 __device__ __noinline__ bool mbar_wait_slow(uint64_t* b, uint32_t parity, int* status, unsigned long long limit_ns) {
     unsigned long long t0 = 0;
     for (unsigned i = 0; i < kPollLimit; i++) {
         if (mbar_try(b, parity)) return true;
         if ((i & 63u) == 63u) {
+            if (*(volatile int*)status != 0) return false;
             const unsigned long long now = global_ns();
             if (t0 == 0) t0 = now;
             else if (now - t0 > limit_ns) break;

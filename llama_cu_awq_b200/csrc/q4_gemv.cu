@@ -309,6 +309,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_direct_kernel(const __grid_c
     }
 }
 
+// Q4_ERR_TIMEOUT once a wait of the ring form has run out (q4_ops_status)
+__device__ int g_status;
+
 // MULTI: more than one chunk or pass, whose activations and scales are requested while the one before is worked on (the registers that
 // takes cost a single pass 10 %).
 template <bool SILU, bool MULTI>
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(ring::kThreads, 2) gemv_ring_kernel(const __gr
                     __syncwarp();
                     if (++stage == ring::kStages) { stage = 0; parity ^= 1u; }
                 }
-        // the CTA's shared memory stays until every copy has landed (bounded; the math warps have waited for all of them unless a wait ran out)
+        // the CTA's shared memory stays until every copy has landed (bounded; the math warps have waited for all of them unless a wait ran out).
         for (int i = max(0, issued - ring::kStages); i < issued; i++) mbar_wait_warp(&full[i % ring::kStages], (i / ring::kStages) & 1);
         return;
     }
@@ -444,7 +447,10 @@ __global__ void __launch_bounds__(ring::kThreads, 2) gemv_ring_kernel(const __gr
                 ahead(last ? b0 + per_pass : b0, last ? min(per_pass, my_groups - b0 - per_pass) : bn, last ? 0 : c + 1);
             }
             for (int lg = 0; lg < bn; lg++) {
-                if (ok) ok = mbar_wait_warp(&full[stage], parity);
+                if (ok) {
+                    ok = mbar_wait_warp(&full[stage], parity);
+                    if (!ok) atomicExch(&g_status, Q4_ERR_TIMEOUT);
+                }
                 // words 4t..4t + 3 of column r in groups A and B. (Units that are not there multiply whatever lies in the stage; their sums are
                 // not kept.)
                 uint32_t me[2];
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(ring::kThreads, 2) gemv_ring_kernel(const __gr
                     pair_mma_exact(c4[j], a, b, px[j]);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[stage]);
+                if (lane == 0 && ok) mbar_arrive(&empty[stage]);   // (a stage whose copy has not come is not filled again: the producer gives up too)
                 if (++stage == ring::kStages) { stage = 0; parity ^= 1u; }
                 float y = quad_sum2(pair_share(c4[0], me[0], px[0], lane), pair_share(c4[1], me[1], px[1], lane), lane);
                 if (!ok) y = CUDART_NAN_F;   // a copy that never came must not pass for a result
@@ -564,6 +570,15 @@ GemvMat mat(const q4_qweight* w, uint16_t* out, int n, int tile0, int kv) {
 }
 
 }  // namespace
+
+extern "C" int q4_ops_status(void) {
+    int st = 0;
+    const int none = 0;
+    Q4_CUDA_TRY(cudaDeviceSynchronize());
+    Q4_CUDA_TRY(cudaMemcpyFromSymbol(&st, g_status, sizeof(st)));
+    if (st) Q4_CUDA_TRY(cudaMemcpyToSymbol(g_status, &none, sizeof(none)));
+    return st;
+}
 
 extern "C" int q4_matmul_q4(void* stream, uint16_t* xout, const uint16_t* x, const q4_qweight* w, int inpSize,
                             int opSize, int accum, int gpu_count, int loff, const int* pPos) {
