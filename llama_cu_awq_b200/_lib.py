@@ -140,6 +140,7 @@ TEST_SIGNATURES = {
     "q4_test_set_ring_depth": (None, [_I]),
     "q4_test_fail_fused_alloc": (None, [_I]),
     "q4_test_comm_set_peer": (_I, [_P, _I, _P]),
+    "q4_test_comm_set_sms": (_I, [_P, _I]),
     "q4_test_fused_gemv": (_I, [_P, _P, _P, _QW, _I, _I]),
     "q4_test_fail_rows_alloc": (None, [_I]),
     "q4_test_fail_set_pos": (None, []),

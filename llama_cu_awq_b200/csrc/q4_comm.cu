@@ -194,6 +194,10 @@ __global__ void __launch_bounds__(kCommThreads) comm_wide_kernel(PeerPtrs peers,
 int alloc_inbox(Inbox** out) {
     Q4_CUDA_TRY(cudaMalloc((void**)out, sizeof(Inbox)));
     Q4_CUDA_TRY(cudaMemset(*out, 0, sizeof(Inbox)));
+    int dev = 0, sms = 0;
+    Q4_CUDA_TRY(cudaGetDevice(&dev));
+    Q4_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    Q4_CUDA_TRY(cudaMemcpy(&(*out)->ll.sms, &sms, sizeof(sms), cudaMemcpyHostToDevice));
     Q4_CUDA_TRY(cudaDeviceSynchronize());
     return Q4_OK;
 }
@@ -458,6 +462,12 @@ extern "C" int q4_comm_destroy(q4_comm* comm) {
 extern "C" int q4_test_comm_set_peer(q4_comm* comm, int peer, q4_comm* other) {
     if (!comm || !other || peer < 0 || peer >= comm->gpu_count || peer == comm->rank) return Q4_ERR_INVALID;
     comm->peers.p[peer] = other->local;
+    return Q4_OK;
+}
+// The SM count this rank tells the others.
+extern "C" int q4_test_comm_set_sms(q4_comm* comm, int sms) {
+    if (!comm) return Q4_ERR_INVALID;
+    Q4_CUDA_TRY(cudaMemcpy(&comm->local->ll.sms, &sms, sizeof(sms), cudaMemcpyHostToDevice));
     return Q4_OK;
 }
 #endif

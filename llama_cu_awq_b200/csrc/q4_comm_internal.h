@@ -10,10 +10,12 @@ constexpr int kLLMaxVocab = 256 * 1024; // largest vocabulary of the gathered lo
 //                alternate buffers); a 32-bit word = fp16 value | tag << 16, so readers poll the data itself
 //   cand[b][r]   rank r's argmax candidate (two tagged 64-bit words: value bits, global index), b = token parity
 //   logits       all ranks' logits slices (plain fp16), complete once every candidate has arrived
+//   sms          SMs of the rank's device: the places of x's words follow from the number of CTAs, which must be the same on all ranks
 struct Q4LLArea {
     uint32_t x[2][Q4_MAX_GPUS][kLLMaxDim];
     unsigned long long cand[2][Q4_MAX_GPUS][2];
     uint16_t logits[kLLMaxVocab];
+    int sms;
 };
 
 int q4_comm_world(const q4_comm* c);

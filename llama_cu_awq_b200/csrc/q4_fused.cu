@@ -1361,6 +1361,13 @@ static int fused_build(q4_model* m, q4_fused* f) {
         for (int r = 0; r < g; r++) {
             Q4LLArea* a = q4_comm_ll_area(m->comm, r);
             if (!a) { f->unsupported = true; return Q4_ERR_UNSUPPORTED_SIZE; }
+            int peer_sms = 0;
+            Q4_CUDA_TRY(cudaMemcpy(&peer_sms, &a->sms, sizeof(peer_sms), cudaMemcpyDefault));
+            if (peer_sms != sms) {   // every rank finds the same difference and takes the per-op path
+                fprintf(stderr, "q4 fused path: rank %d has %d SMs, rank %d has %d\n", r, peer_sms, m->rank, sms);
+                f->unsupported = true;
+                return Q4_ERR_UNSUPPORTED_SIZE;
+            }
             p.xb[0][r] = &a->x[0][0][0];
             p.xb[1][r] = &a->x[1][0][0];
             p.cand[r] = &a->cand[0][0][0];

@@ -288,3 +288,22 @@ def test_ring_depth_does_not_change_a_bit(cfg):
     assert np.isfinite(out[0].astype(np.float32)).all()
     for o in out[1:]:
         assert (o.view(np.uint16) == out[0].view(np.uint16)).all()
+
+
+def test_ranks_with_different_sm_counts_take_the_per_op_path(tmp_path):
+    """The exchange layout follows from the number of CTAs: a rank whose peer reports another SM count does not take the fused path."""
+    L = _lib.test_lib()
+    path = str(tmp_path / "mid.bin")
+    synth.write_model_file(path, "mid", seed=2)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for peer_sms, best in ((sms, 2), (sms - 2, 1), (0, 1)):
+        a, b = C.c_void_p(), C.c_void_p()
+        assert L.q4_comm_create_local(C.byref(a), 2, 0) == 0 and L.q4_comm_create_local(C.byref(b), 2, 1) == 0
+        assert L.q4_test_comm_set_peer(a, 1, b) == 0
+        if peer_sms != sms:
+            assert L.q4_test_comm_set_sms(b, peer_sms) == 0
+        t = Transformer(path, rank=0, gpu_count=2, tp_mode=_lib.Q4_TP_HYBRID, comm=a, lib=L)
+        assert t.best_path() == best
+        t.close()
+        L.q4_comm_destroy(a)
+        L.q4_comm_destroy(b)
