@@ -74,34 +74,6 @@ __device__ __forceinline__ void permute_x8(const uint4& xv, uint32_t xp[4]) {
     xp[3] = prmt(xv.y, xv.w, 0x7632);
 }
 
-// Zero-point constants for one group: zlo = (1024+z, 1024+z), zhi = (-(64+z), -(64+z)) as half2 bits.
-__device__ __forceinline__ void zero_consts(uint32_t z, uint32_t& zlo, uint32_t& zhi) {
-    zlo = (0x6400u | z) * 0x00010001u;
-    zhi = (0xD400u | (z << 4)) * 0x00010001u;
-}
-
-// Dot product of 8 nibbles (one packed word) minus zero point with 8 activations, as a half2 pair of partial
-// sums (4 products per half). (w & 0x000F000F) | 0x6400 is the half 1024+q, so subtracting 1024+z gives q-z
-// exactly; (w & 0x00F000F0) | 0x6400 is 1024+16q, and fma(., 1/16, -(64+z)) gives q-z exactly.
-__device__ __forceinline__ __half2 dot8(uint32_t w, const uint32_t xp[4], uint32_t zlo, uint32_t zhi, __half2 acc) {
-    const __half2 sixteenth = u2h2(0x2C002C00u);
-    __half2 d0 = __hsub2(u2h2(lop3_and_or(w, 0x000F000Fu, 0x64006400u)), u2h2(zlo));
-    __half2 d1 = __hfma2(u2h2(lop3_and_or(w, 0x00F000F0u, 0x64006400u)), sixteenth, u2h2(zhi));
-    w >>= 8;
-    __half2 d2 = __hsub2(u2h2(lop3_and_or(w, 0x000F000Fu, 0x64006400u)), u2h2(zlo));
-    __half2 d3 = __hfma2(u2h2(lop3_and_or(w, 0x00F000F0u, 0x64006400u)), sixteenth, u2h2(zhi));
-    acc = __hfma2(d0, u2h2(xp[0]), acc);
-    acc = __hfma2(d1, u2h2(xp[1]), acc);
-    acc = __hfma2(d2, u2h2(xp[2]), acc);
-    acc = __hfma2(d3, u2h2(xp[3]), acc);
-    return acc;
-}
-
-__device__ __forceinline__ float h2sum(__half2 h) {
-    float2 f = __half22float2(h);
-    return f.x + f.y;
-}
-
 // Rotation of pair `pair` (elements pair and pair + head_size / 2) of a head at position `pos`: angle =
 // pos / theta^(2 pair / head_size), evaluated in fp32 with powf, cosf and sinf exactly as RoPERotation_kernel evaluates it
 // (gpu_kernels.h:346-350), so that rotated values round as the reference's do. Returns (cos, sin).

@@ -1555,7 +1555,7 @@ extern "C" int q4_test_fused_gemv(void* stream, uint16_t* y, const uint16_t* x, 
 #endif  // Q4_TEST_BUILD
 
 // Profiling hook: arms per-phase timestamps (CTA 0 and the last CTA) for the following fused launches and, when
-// `out` is given, copies the last launch's stamps out. Layout [2][nphases][4] of nanoseconds; also returns the
+// `out` is given, copies the last launch's stamps out. Layout [2][nphases][8] of nanoseconds (kTraceCols); also returns the
 // phase types so that the caller can group them.
 extern "C" int q4_model_trace(q4_model* m, unsigned long long* out, int* phase_types, int max_phases) {
     if (!m) return Q4_ERR_INVALID;

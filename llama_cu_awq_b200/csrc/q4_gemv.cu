@@ -186,7 +186,7 @@ __device__ __noinline__ void add_small(const GemvParams& p, float* part, int par
 }
 
 template <bool SILU>
-__global__ void __launch_bounds__(kThreads, 1) gemv_direct_kernel(const __grid_constant__ GemvParams p) {
+__global__ void __launch_bounds__(kThreads, 1) q4_gemv_kernel(const __grid_constant__ GemvParams p) {
     __shared__ __align__(16) uint8_t scratch[kWarps][kExactScratch];
     __shared__ float part[kBlockTiles * kTileStride];
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, cta = blockIdx.x;
@@ -315,7 +315,7 @@ __device__ int g_status;
 // MULTI: more than one chunk or pass, whose activations and scales are requested while the one before is worked on (the registers that
 // takes cost a single pass 10 %).
 template <bool SILU, bool MULTI>
-__global__ void __launch_bounds__(ring::kThreads, 2) gemv_ring_kernel(const __grid_constant__ GemvParams p) {
+__global__ void __launch_bounds__(ring::kThreads, 2) q4_gemv_ring_kernel(const __grid_constant__ GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full[ring::kStages], empty[ring::kStages];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -543,7 +543,7 @@ int launch(GemvParams& p, cudaStream_t s) {
         make_split(p);
         const int groups = q4_div_up(p.total_tiles, p.T);
         // (an opt-in of the function on the device, always to the same value)
-        auto* kernel = p.nchunks > 1 || groups > ring::kCtas * (ring::kBlockTiles / p.T) ? gemv_ring_kernel<SILU, true> : gemv_ring_kernel<SILU, false>;
+        auto* kernel = p.nchunks > 1 || groups > ring::kCtas * (ring::kBlockTiles / p.T) ? q4_gemv_ring_kernel<SILU, true> : q4_gemv_ring_kernel<SILU, false>;
         Q4_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring::kSmemBytes));
         Q4Launch L(dim3(std::min(groups, ring::kCtas)), dim3(ring::kThreads), ring::kSmemBytes, s);
         Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, kernel, p));
@@ -553,7 +553,7 @@ int launch(GemvParams& p, cudaStream_t s) {
     p.nt_div = p.total_tiles / grid;
     p.nt_mod = p.total_tiles % grid;
     Q4Launch L(dim3(grid), dim3(kThreads), 0, s);
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, gemv_direct_kernel<SILU>, p));
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemv_kernel<SILU>, p));
     return Q4_OK;
 }
 

@@ -105,8 +105,8 @@ def _hostile(kind, K, rng):
 @pytest.mark.parametrize("K,N", [(4096, 64), (11008, 32)])
 @pytest.mark.parametrize("kind", ["normal", "outlier100", "outlier1000", "zero_groups", "subnormal", "fp16_max"])
 def test_block_fixed_point_activations(kind, K, N):
-    """gemv_slot replaces the reference's fp16 x fp32 FMA (gpu_kernels.h:203-208) by an integer dot product over a
-    per-group 15-bit fixed-point copy of x. Hostile activation vectors must stay inside the fp16 tolerance."""
+    """The fused kernel's product (quant_pair, pair_mma) replaces the reference's fp16 x fp32 FMA (gpu_kernels.h:203-208) by an integer
+    dot product over a per-group 16-bit fixed-point copy of x. Hostile activation vectors must stay inside the fp16 tolerance."""
     L = _lib.test_lib()
     rng = np.random.default_rng(K + len(kind))
     q = synth.synth_qweight(rng, K, N)
