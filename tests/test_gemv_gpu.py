@@ -83,7 +83,7 @@ def test_matvec_kv_cache_offset():
     assert not c.any(), "wrote outside the cache row"
 
 
-@pytest.mark.parametrize("K,Nq,Nkv", [(256, 256, 256), (512, 512, 128), (4096, 4096, 4096), (8192, 1024, 128)])
+@pytest.mark.parametrize("K,Nq,Nkv", [(256, 256, 256), (512, 512, 128), (4096, 4096, 4096), (8192, 1024, 128), (256, 16000, 12000), (1024, 24000, 24000)])
 def test_qkv_matvec(K, Nq, Nkv):
     rng = np.random.default_rng(K + Nkv)
     qs = [synth.synth_qweight(rng, K, n) for n in (Nq, Nkv, Nkv)]
@@ -103,7 +103,7 @@ def test_qkv_matvec(K, Nq, Nkv):
     assert int((kc != 0).sum()) <= Nkv and int((vc != 0).sum()) <= Nkv
 
 
-@pytest.mark.parametrize("K,N", [(256, 8), (512, 1376), (4096, 11008), (5120, 1728)])
+@pytest.mark.parametrize("K,N", [(256, 8), (512, 1376), (4096, 11008), (5120, 1728), (256, 20000), (1024, 24000)])
 def test_ffn_matvec_silu(K, N):
     rng = np.random.default_rng(K + N)
     gate, up = synth.synth_qweight(rng, K, N), synth.synth_qweight(rng, K, N)
