@@ -887,8 +887,8 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
                         r->rope, r->row_seq, r->row_pos, seq_stride, loff);
         if (l == c.n_layers - 1 && want != WANT_ALL) {
             if (want == WANT_CACHE) break;
-            // one row: the split attention and the products of the batch-1 path (70B: o, gate / up and down 147 us with the few-rows kernels, 94 so,
-            // and half their error)
+            // one row: the split attention and the products of the batch-1 path (70B: o, gate / up and down 147 us with the few-rows kernels,
+            // about 105 so, and less error)
             const size_t last = (size_t)(n - 1);
             uint16_t* x = (uint16_t*)(r->X + last * dim);
             OP(q4_attention(s, (uint16_t*)r->ATT, (const uint16_t*)qp + last * ldq, (const uint16_t*)(kc + loff), (const uint16_t*)(vc + loff), m->attn_scratch, heads, m->head_size,

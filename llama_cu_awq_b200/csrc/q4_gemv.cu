@@ -19,7 +19,7 @@
 //
 // Under programmatic dependent launch the next product's packed words are requested while this one drains (weights never depend on
 // activations). Back to back on weights from HBM, with half2 FMA, with x as 16-bit fixed point in the ring form alone, and now, us:
-// 4096 x 4096 5.1, 4.4, 4.2; q|k|v 9.9, 9.2, 9.6; 4096 -> 2 x 11008 13.9, 11.0, 11.3; 11008 -> 4096 9.9, 9.6, 10.3; 28672 -> 8192 34.1, 31.3,
+// 4096 x 4096 5.1, 4.4, 4.2; q|k|v 9.9, 9.2, 9.2; 4096 -> 2 x 11008 13.9, 11.0, 11.4; 11008 -> 4096 9.9, 9.6, 10.4; 28672 -> 8192 34.1, 31.3,
 // 33.5; 11008 -> 512 5.3, 5.6, 4.0; 5120 -> 1280 4.4, 4.8, 3.7; 13520 -> 544 6.8, 7.0, 5.4; 512 x 512 1.8, 2.3, 1.7. Error against 64 bits 3.8e-4,
 // 2.1e-4, 2.1e-4 (an fp16 result's own rounding).
 #include <algorithm>
