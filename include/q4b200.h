@@ -341,7 +341,7 @@ int q4_model_set_sampler(q4_model* model, float temperature, float topp, unsigne
  * (cuda_comm.h:184,223). */
 int q4_model_set_wait_limit_ns(q4_model* model, unsigned long long ns);
 /* Synchronises the device and returns Q4_OK, or the error a bounded device-side wait recorded
- * (Q4_ERR_TIMEOUT) in the fused path or the communicator. */
+ * (Q4_ERR_TIMEOUT) in the fused path, the prompt's and batch's kernels, a batch-1 product or the communicator. */
 int q4_model_status(q4_model* model);
 /* generate_thread(): the token loop with the reference's timing window (llama2_q4.cu:708-745). Runs `steps`
  * positions starting from the n_prompt given ids, stops at EOS (id 2). out_tokens receives tokens[0..steps];
