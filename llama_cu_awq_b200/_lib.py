@@ -138,6 +138,7 @@ TEST_SIGNATURES = {
     "q4_test_set_fused_debug": (None, [_I]),
     "q4_test_set_split_len": (None, [_I]),
     "q4_test_set_ring_depth": (None, [_I]),
+    "q4_test_set_far_table": (None, [_I]),
     "q4_test_fail_fused_alloc": (None, [_I]),
     "q4_test_comm_set_peer": (_I, [_P, _I, _P]),
     "q4_test_comm_set_sms": (_I, [_P, _I]),

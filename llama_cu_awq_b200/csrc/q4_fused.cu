@@ -82,6 +82,7 @@ struct FParams {
     int n_layers, nphases;
     const uint8_t* const* stream[K_KINDS];  // [n_layers] stream-layout weights of each step
     const __half* const* norms[2];          // [n_layers] RMSNorm weights before QKV and before gate/up
+    const void* const* table;               // far form only: [n_layers][K_KINDS] of the first, then [n_layers][2] of the second
     const __half* rms_final;
     int dim, kv_n, q_n, kv_mul, n_heads, nsplit, v_n;
     long long layer_stride;        // halfs of one layer's K (or V) cache
@@ -562,6 +563,8 @@ __device__ __forceinline__ void rotate_head(const FParams& p, int first_tile, ui
 // ------------------------------------------------------------------------------------------------------------
 // The kernel
 // ------------------------------------------------------------------------------------------------------------
+// kFar: the table of addresses stays in global memory (so many layers that it would leave the rings too little).
+template <bool kFar>
 __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_constant__ FParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full_bar[kW * kMaxDepth];
@@ -574,15 +577,19 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     uint4* const xs = reinterpret_cast<uint4*>(smem + p.x_off);               // residual stream (fp16); the classifier's input
     float* const part_a = reinterpret_cast<float*>(smem + p.part_a_off);
     float* const part_b = reinterpret_cast<float*>(smem + p.part_b_off);
-    const uint8_t** const streams = reinterpret_cast<const uint8_t**>(smem + p.table_off);
-    const __half** const norms = reinterpret_cast<const __half**>(streams + K_KINDS * p.n_layers);
+    const void* const* const table = kFar ? p.table : reinterpret_cast<const void* const*>(smem + p.table_off);
+    const uint8_t* const* const streams = reinterpret_cast<const uint8_t* const*>(table);
+    const __half* const* const norms = reinterpret_cast<const __half* const*>(table + K_KINDS * p.n_layers);
 
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int cta = blockIdx.x, grid = gridDim.x;
 
     if (tid < kW * kMaxDepth) mbar_init(&full_bar[tid], 1);
-    for (int i = tid; i < K_KINDS * p.n_layers; i += kThreads) streams[i] = p.stream[i % K_KINDS][i / K_KINDS];
-    for (int i = tid; i < 2 * p.n_layers; i += kThreads) norms[i] = p.norms[i & 1][i >> 1];
+    if (!kFar) {
+        const void** const to = reinterpret_cast<const void**>(smem + p.table_off);
+        for (int i = tid; i < K_KINDS * p.n_layers; i += kThreads) to[i] = p.stream[i % K_KINDS][i / K_KINDS];
+        for (int i = tid; i < 2 * p.n_layers; i += kThreads) to[K_KINDS * p.n_layers + i] = p.norms[i & 1][i >> 1];
+    }
     mbar_init_fence();
     __syncthreads();
 
@@ -1184,6 +1191,8 @@ struct q4_fused {
     int barriers_per_launch = 0;
     unsigned long long launches = 0;
     bool unsupported = false;
+    bool far = false;               // the table of addresses does not fit beside the rings
+    void (*kernel)(FParams) = nullptr;
     unsigned long long* trace = nullptr;
     Q4LLArea* ll_local = nullptr;   // this rank's exchange area (inside the communicator's inbox, or own allocation at g = 1)
     size_t attn_part_bytes = 0, hb_bytes = 0, qkv_bytes = 0;
@@ -1194,11 +1203,13 @@ struct q4_fused {
 #ifdef Q4_TEST_BUILD
 // Switches of the test build (see Q4_DBG): set through exported functions, never through the environment.
 static int g_test_debug = 0, g_test_split_len = 0, g_test_depth = 0;
+static bool g_test_far_table = false;
 static int g_test_fail_alloc = -1;   // >= 0: the allocation with this running index fails once (host-side fault injection)
 static int g_test_alloc_index = 0;
 extern "C" void q4_test_set_fused_debug(int bits) { g_test_debug = bits; }
 extern "C" void q4_test_set_split_len(int positions) { g_test_split_len = positions; }
 extern "C" void q4_test_set_ring_depth(int chunks) { g_test_depth = chunks; }
+extern "C" void q4_test_set_far_table(int on) { g_test_far_table = on != 0; }
 extern "C" void q4_test_fail_fused_alloc(int index) { g_test_fail_alloc = index; g_test_alloc_index = 0; }
 #endif
 
@@ -1407,10 +1418,15 @@ static int fused_build(q4_model* m, q4_fused* f) {
     const int part_a = std::max(kTileStride * std::max(max_tiles(p.kind[K_QKV]), max_tiles(p.kind[K_GU])), kW * 128) * (int)sizeof(float);
     const int part_b = kTileStride * std::max(max_tiles(p.kind[K_O]), max_tiles(p.kind[K_DOWN])) * (int)sizeof(float);
     const int x_bytes = (int)align_up(2 * (size_t)c.dim, 128);
-    const size_t tables = align_up((size_t)(K_KINDS + 2) * c.n_layers * 8, 16);
+    size_t tables = align_up((size_t)(K_KINDS + 2) * c.n_layers * 8, 16);
     const size_t budget = 224 * 1024;   // + about 2 KB of static shared memory, of 227 KB per CTA
-    const size_t other = (size_t)kW * kPairScratch + x_bytes + align_up(part_a, 128) + align_up(part_b, 128) + tables;
-    int depth = other < budget ? (int)((budget - other) / (kW * kChunkBytes)) : 0;
+    const size_t other = (size_t)kW * kPairScratch + x_bytes + align_up(part_a, 128) + align_up(part_b, 128);
+    f->far = other + tables + (size_t)kMinDepth * kW * kChunkBytes > budget;
+#ifdef Q4_TEST_BUILD
+    f->far |= g_test_far_table;
+#endif
+    if (f->far) tables = 0;
+    int depth = other + tables < budget ? (int)((budget - other - tables) / (kW * kChunkBytes)) : 0;
     depth = std::min(depth, kMaxDepth);
     if (depth < kMinDepth) { f->unsupported = true; return Q4_ERR_UNSUPPORTED_SIZE; }
 #ifdef Q4_TEST_BUILD
@@ -1451,11 +1467,20 @@ static int fused_build(q4_model* m, q4_fused* f) {
     };
     for (int k = 0; k < K_KINDS; k++) FTRY(table((const void**)&p.stream[k], streams[k]));
     for (int k = 0; k < 2; k++) FTRY(table((const void**)&p.norms[k], norms[k]));
+    if (f->far) {
+        std::vector<const void*> all;
+        for (int l = 0; l < c.n_layers; l++)
+            for (int k = 0; k < K_KINDS; k++) all.push_back(streams[k][l]);
+        for (int l = 0; l < c.n_layers; l++)
+            for (int k = 0; k < 2; k++) all.push_back(norms[k][l]);
+        FTRY(table((const void**)&p.table, all));
+    }
+    f->kernel = f->far ? fused_token_kernel<true> : fused_token_kernel<false>;
     // (the limit belongs to the function, not to this model: always the largest any model may need, so that a smaller one prepared
     // later does not lower it)
-    Q4_CUDA_TRY(cudaFuncSetAttribute(fused_token_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+    Q4_CUDA_TRY(cudaFuncSetAttribute(f->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     int per_sm = 0;
-    Q4_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_token_kernel, kThreads, f->smem_bytes));
+    Q4_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f->kernel, kThreads, f->smem_bytes));
     if (per_sm < 1) {
         fprintf(stderr, "q4 fused path: kernel does not fit one SM (%zu B shared memory, %d threads)\n", f->smem_bytes, kThreads);
         f->unsupported = true;
@@ -1485,7 +1510,7 @@ int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff)
     p.launch_parity = (unsigned)(f->launches & 1);
     f->launches++;
     void* args[] = {&p};
-    Q4_CUDA_TRY(cudaLaunchCooperativeKernel((void*)fused_token_kernel, dim3(f->grid), dim3(kThreads), args, f->smem_bytes, s));
+    Q4_CUDA_TRY(cudaLaunchCooperativeKernel((void*)f->kernel, dim3(f->grid), dim3(kThreads), args, f->smem_bytes, s));
     return Q4_OK;
 }
 

@@ -307,3 +307,22 @@ def test_ranks_with_different_sm_counts_take_the_per_op_path(tmp_path):
         t.close()
         L.q4_comm_destroy(a)
         L.q4_comm_destroy(b)
+
+
+def test_table_of_addresses_in_global_memory():
+    """Where the table of a model's addresses lies (with very many layers it does not fit beside the rings; forced here on a small model)
+    does not change a bit."""
+    L = _lib.test_lib()
+    cfg = (1024, 2816, 3, 8, 2, 2048, 64, 10000.0)
+    tokens = np.random.default_rng(12).integers(3, 2048, size=12, dtype=np.int32)
+    out = []
+    try:
+        for far in (0, 1):
+            L.q4_test_set_far_table(far)
+            t = Transformer(None, lib=L, synthetic=(cfg, 6))
+            assert t.best_path() == 2
+            out.append(_run(t, tokens, queued=True))
+            t.close()
+    finally:
+        L.q4_test_set_far_table(0)
+    assert (out[0].view(np.uint16) == out[1].view(np.uint16)).all()
