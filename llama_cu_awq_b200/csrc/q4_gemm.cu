@@ -744,19 +744,18 @@ constexpr size_t kWsHeader = 256;
 constexpr int kWsMaxTiles = 16384;   // (two counters per tile of 256 features: 8192 tiles of 256 x 256 outputs)
 constexpr size_t kWsPartials = kWsHeader + sizeof(int) * kWsMaxTiles;
 
-constexpr double kConvClocks = 1250.0;
-
 struct GemmPlan { int MT, m_tiles, n_tiles, n_chunks, pairs, stages, np, slab; long long total; };
 
-// Batch tile and number of pairs, by an estimate of the slowest pair's clocks over all of them. What each line costs was read off
-// clock stamps inside the kernel; launch, first copies and last drain, much the same for every plan, are in no line, so the
-// estimate ranks plans and is not a time (4096 x 22016: 15.0 us of the 25 measured at 64 rows, 49 of 75 at 512):
-//   chunk    a 256-input chunk: 8.6 per batch row on the tensor pipe (MT / 2 per K = 16 step), or the conversion of its 128 x 256
-//            weights by the eight converter warps, whichever is longer
-//   tile     draining the accumulator; the last tile's output is not hidden by anything: 400 per 32 rows
-//   split    a tile cut by a share boundary: one partial tile written, and by the last CTA one read per other contributor
-// Large matrices end up with 256-row tiles on all pairs; small ones with smaller tiles (the conversion is repeated, but no K split
-// is needed) or with fewer pairs whose shares are whole halves or thirds of a tile.
+// Batch tile and number of pairs, by an estimate of the slowest pair's time over all of them, in us. The lines were fitted to 63 shapes
+// (K and N of the 7B, 13B and 70B projections, 24 to 512 rows) with all their tiles and 5 to 12 numbers of pairs each; the plan it
+// picks is within 1 % of the best of them on average. (Its predecessor, from clock stamps inside the kernel, took a partial
+// tile's reading for a fifth of what it costs and was 9 % off: 77 x 5120 x 5120 22.9 us, 16.9 so; 128 x 8192 x 8192 30.3, 24.1.)
+//   chunk    a 256-input chunk: 4.9 ns per batch row on the tensor pipe, 0.7 us at least, whatever the rows (issue of its 16 MMAs,
+//            conversion of its 128 x 256 weights)
+//   segment  each further tile that a share touches: its first copies and its turn at the accumulator
+//   drain    the last tile's output, which is not hidden by anything: 9 ns per row
+//   split    a tile cut by a share boundary: a partial tile written, counted and, by the last CTA, one read per other contributor at
+//            26 ns per row, which is why even shares of a whole fraction of a tile on 64 pairs beat 74 pairs
 // Rings: operand stages as tensor memory allows, the shared memory that their X slabs leave for packed weights (at few rows
 // the kernel is a weight stream: ten 16 KB copies in flight per SM cover HBM's latency).
 GemmPlan make_plan(int M, int K, int N, int sms) {
@@ -772,18 +771,17 @@ GemmPlan make_plan(int M, int K, int N, int sms) {
         last_mt = mt;
         const int mtl = q4_div_up(M, mt);
         const long long total = (long long)g.n_tiles * mtl * g.n_chunks;
-        const double t_chunk = 8.6 * mt > kConvClocks ? 8.6 * mt : kConvClocks;
+        const double t_chunk = 0.0049 * mt > 0.7 ? 0.0049 * mt : 0.7;
         for (int P = (int)(total < max_pairs ? total : max_pairs); P >= 1; P--) {
             const long long share = (total + P - 1) / P;
             if (share * t_chunk >= best) break;   // fewer pairs only take longer from here on
-            const bool even = total % P == 0;
-            double cost = share * t_chunk + 1000.0 * q4_div_up((int)share, g.n_chunks) + 12.5 * mt;
-            if (!(even && share % g.n_chunks == 0)) {
-                const bool aligned = even && g.n_chunks % share == 0;
-                const double readers = share >= g.n_chunks ? 1.0 : (double)(g.n_chunks + share - 1) / share - (aligned ? 1.0 : 0.0);
-                cost += 1000.0 + 6.0 * mt + readers * (1000.0 + 8.0 * mt);
+            const bool even = total % P == 0, whole = even && share % g.n_chunks == 0, aligned = even && g.n_chunks % share == 0;
+            double cost = share * t_chunk + 0.009 * mt + 0.75 * (q4_div_up((int)share, g.n_chunks) - (whole || aligned ? 1 : 0));
+            if (!whole) {   // contributors of a tile, at most
+                const long long parts = aligned ? g.n_chunks / share : share >= g.n_chunks ? 2 : (g.n_chunks - 2) / share + 2;
+                cost += 0.8 + (parts - 1) * 0.026 * mt;
             }
-            if (cost < best * 0.99) { best = cost; g.pairs = P; g.MT = mt; g.m_tiles = mtl; g.total = total; }
+            if (cost < best) { best = cost; g.pairs = P; g.MT = mt; g.m_tiles = mtl; g.total = total; }
         }
     }
     if (g.pairs == 0) return g;
