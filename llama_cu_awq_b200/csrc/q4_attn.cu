@@ -3,12 +3,15 @@
 // Replaces MultiHeadAttention (llama2_q4.cu:410-427; mat_vec_kernel_simple, softmax_kernel, vec_mat_kernel at
 // gpu_kernels.h:150-176,365-454,287-337).
 //
-// Pass 1: grid (splits, heads). A block takes positions [t0, t1) of one head. Eight lanes share a position
-// (16 head dims each, two 128-bit loads of K and of V), so a warp covers 4 positions per step and a block of 4
-// warps 16. Scores are rounded to fp16 like the reference's; the softmax runs online in fp32 (running max, sum
-// and un-normalised V accumulator per lane group), merged across the block in shared memory and written to
-// scratch as (max, sum, acc[head_size]).
-// Pass 2: one block per head merges the splits and writes fp16.
+// A block takes positions [t0, t1) of one head. Eight lanes share a position (16 head dims each at head size 128), a block of
+// eight warps has 64 positions in hand per step and the next 64 requested. Scores are rounded to fp16 like the reference's; the
+// softmax runs online in fp32 (running max, sum and un-normalised V accumulator per lane group), merged across the block in registers
+// and shared memory. Then, by the number of heads:
+//   16 or more  one launch: a head's blocks are a thread-block cluster and read one another's (max, sum, acc) from shared memory
+//   fewer       two launches: up to 32 blocks per head leave (max, sum, acc) in scratch, a block per head merges them and writes fp16.
+//               (a cluster has at most eight blocks: eight heads would keep 64 of 148 SMs)
+// What bounds it is latency: 32 heads at position 600 are 10 MB. Before (16 positions in hand per block, none requested ahead, always
+// two launches): 333 tokens behind 700 of one 70B layer (its last row) 238 -> 227 us, two 7B layers call by call at position 600 133 -> 120 us.
 // The sequence length comes from *pPos on the device; the grid does not depend on it.
 #include <math_constants.h>
 
@@ -20,9 +23,10 @@
 
 namespace {
 
-constexpr int kAttnThreads = 128;
-constexpr int kGroups = kAttnThreads / 8;  // positions in flight per block
+constexpr int kAttnThreads = 256, kAttnWarps = kAttnThreads / 32;
+constexpr int kGroups = kAttnThreads / 8;  // lane groups of a block; each has two positions in hand
 constexpr int kMaxHeadSize = 256;
+constexpr int kClusterHeads = 16;          // from so many heads on a head's blocks are a cluster
 
 int attn_splits(int num_heads) {
     int s = q4_div_up(2 * 148, num_heads);
@@ -30,35 +34,35 @@ int attn_splits(int num_heads) {
     if (s > 32) s = 32;
     return s;
 }
+// blocks of a head's cluster: about two to four per SM over all heads
+int attn_cluster(int num_heads) { return num_heads <= 64 ? 8 : num_heads <= 128 ? 4 : 2; }
 
 template <int HS>
-__global__ void __launch_bounds__(kAttnThreads) attn_partial_kernel(float* scratch, const __half* q, const __half* kc, const __half* vc,
-                                                                    int kv_mul, int kv_stride, const int* pPos) {
+struct AttnShared {
+    float m[kAttnWarps], l[kAttnWarps], acc[kAttnWarps][HS];
+    float M, L, out[HS];   // the block's: maximum, sum, un-normalised V sum
+};
+
+// This block's share of head h, into sm.M, sm.L and sm.out (behind a barrier).
+template <int HS>
+__device__ __forceinline__ void attn_share(AttnShared<HS>& sm, const __half* q, const __half* kc, const __half* vc, int kv_mul, int kv_stride, const int* pPos, int h,
+                                           int split, int nsplit) {
     constexpr int PER = HS / 8;      // head dims per lane
     constexpr int VEC = PER / 8;     // uint4 per lane per row
-    __shared__ float sm_m[kGroups], sm_l[kGroups];
-    __shared__ float sm_acc[kGroups][HS];
-
-    const int h = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x;
-    const int lane8 = threadIdx.x & 7, grp = threadIdx.x >> 3;
-    griddep_wait();
-    griddep_launch_dependents();
+    const int lane8 = threadIdx.x & 7, grp = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint4 qv[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; v++) qv[v] = *reinterpret_cast<const uint4*>(q + (size_t)h * HS + lane8 * PER + v * 8);
     const int T = *pPos + 1;
     // split boundaries in units of kGroups positions
     const int units = (T + kGroups - 1) / kGroups;
-    const int u0 = (int)((long long)units * split / nsplit), u1 = (int)((long long)units * (split + 1) / nsplit);
-    const int t0 = u0 * kGroups, t1 = min(u1 * kGroups, T);
-
+    const int t0 = (int)((long long)units * split / nsplit) * kGroups, t1 = min((int)((long long)units * (split + 1) / nsplit) * kGroups, T);
     float qf[PER];
-    {
-        const __half* qp = q + (size_t)h * HS + lane8 * PER;
 #pragma unroll
-        for (int v = 0; v < VEC; v++) {
-            uint4 u = *reinterpret_cast<const uint4*>(qp + v * 8);
-            const __half2* hh = reinterpret_cast<const __half2*>(&u);
+    for (int v = 0; v < VEC; v++) {
+        const __half2* hh = reinterpret_cast<const __half2*>(&qv[v]);
 #pragma unroll
-            for (int j = 0; j < 4; j++) { float2 f = __half22float2(hh[j]); qf[v * 8 + 2 * j] = f.x; qf[v * 8 + 2 * j + 1] = f.y; }
-        }
+        for (int j = 0; j < 4; j++) { const float2 f = __half22float2(hh[j]); qf[v * 8 + 2 * j] = f.x; qf[v * 8 + 2 * j + 1] = f.y; }
     }
     const float alpha = (float)(1.0 / sqrt((double)HS));
     const size_t head_off = (size_t)(h / kv_mul) * HS + lane8 * PER;
@@ -68,70 +72,156 @@ __global__ void __launch_bounds__(kAttnThreads) attn_partial_kernel(float* scrat
 #pragma unroll
     for (int i = 0; i < PER; i++) acc[i] = 0.f;
 
-    // the trip count is the same for every lane of the block (shuffles below use the full mask)
-    for (int tb = t0; tb < t1; tb += kGroups) {
-        const int t = tb + grp;
-        const bool valid = t < t1;
-        const __half* kr = kc + (size_t)(valid ? t : t0) * kv_stride + head_off;
-        const __half* vr = vc + (size_t)(valid ? t : t0) * kv_stride + head_off;
-        uint4 kv4[VEC], vv4[VEC];
+    constexpr int kStep = 2 * kGroups;
+    uint4 k4[2][VEC], v4[2][VEC];
+    // rows past the share's end read its first row and are not counted
+    auto fetch = [&](uint4 (&r)[2][VEC], const __half* cache, int tb) {
+        if (tb >= t1) return;
 #pragma unroll
-        for (int v = 0; v < VEC; v++) { kv4[v] = *reinterpret_cast<const uint4*>(kr + v * 8); vv4[v] = *reinterpret_cast<const uint4*>(vr + v * 8); }
-        float s = 0.f;
+        for (int u = 0; u < 2; u++) {
+            const int t = tb + grp + u * kGroups;
+            const uint4* src = reinterpret_cast<const uint4*>(cache + (size_t)(t < t1 ? t : t0) * kv_stride + head_off);
 #pragma unroll
-        for (int v = 0; v < VEC; v++) {
-            const __half2* hh = reinterpret_cast<const __half2*>(&kv4[v]);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                float2 f = __half22float2(hh[j]);
-                s = fmaf(f.x, qf[v * 8 + 2 * j], s);
-                s = fmaf(f.y, qf[v * 8 + 2 * j + 1], s);
-            }
+            for (int v = 0; v < VEC; v++) r[u][v] = src[v];
         }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if (valid) {
-            s = __half2float(__float2half(s * alpha));  // the reference stores scores as fp16 (gpu_kernels.h:171-175)
-            const float mn = fmaxf(m, s);
-            const float corr = expf(m - mn);            // 0 on the first position (m = -inf)
-            const float p = expf(s - mn);
-            l = l * corr + p;
+    };
+    fetch(k4, kc, t0);
+    fetch(v4, vc, t0);
+    // the trip count is the same for every lane of the block (shuffles below use the full mask)
+    for (int tb = t0; tb < t1; tb += kStep) {
+        float s[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            s[u] = 0.f;
 #pragma unroll
             for (int v = 0; v < VEC; v++) {
-                const __half2* hh = reinterpret_cast<const __half2*>(&vv4[v]);
+                const __half2* hh = reinterpret_cast<const __half2*>(&k4[u][v]);
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    float2 f = __half22float2(hh[j]);
-                    acc[v * 8 + 2 * j] = fmaf(p, f.x, acc[v * 8 + 2 * j] * corr);
-                    acc[v * 8 + 2 * j + 1] = fmaf(p, f.y, acc[v * 8 + 2 * j + 1] * corr);
+                    const float2 f = __half22float2(hh[j]);
+                    s[u] = fmaf(f.x, qf[v * 8 + 2 * j], s[u]);
+                    s[u] = fmaf(f.y, qf[v * 8 + 2 * j + 1], s[u]);
                 }
             }
-            m = mn;
         }
+        fetch(k4, kc, tb + kStep);   // into the registers just read
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int u = 0; u < 2; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            if (tb + grp + u * kGroups < t1) {
+                const float sc = __half2float(__float2half(s[u] * alpha));  // the reference stores scores as fp16 (gpu_kernels.h:171-175)
+                const float mn = fmaxf(m, sc);
+                const float base = mn == -CUDART_INF_F ? 0.f : mn;          // scores of -infinity only: their weights are 0, a NaN's is NaN
+                const float corr = expf(m - base), p = expf(sc - base);     // (corr is 0 on the first position)
+                l = l * corr + p;
+#pragma unroll
+                for (int v = 0; v < VEC; v++) {
+                    const __half2* hh = reinterpret_cast<const __half2*>(&v4[u][v]);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float2 f = __half22float2(hh[j]);
+                        acc[v * 8 + 2 * j] = fmaf(p, f.x, acc[v * 8 + 2 * j] * corr);
+                        acc[v * 8 + 2 * j + 1] = fmaf(p, f.y, acc[v * 8 + 2 * j + 1] * corr);
+                    }
+                }
+                m = mn;
+            }
+        }
+        fetch(v4, vc, tb + kStep);
     }
-
-    if (lane8 == 0) { sm_m[grp] = m; sm_l[grp] = l; }
+    // weight of a part whose maximum and sum are (pm, pl) in a whole with maximum M: nothing where nothing was added up
+    auto weight = [](float pm, float pl, float M) { return pl == 0.f ? 0.f : expf(pm - (M == -CUDART_INF_F ? 0.f : M)); };
+    // the four lane groups of a warp, then the warps
 #pragma unroll
-    for (int i = 0; i < PER; i++) sm_acc[grp][lane8 * PER + i] = acc[i];
+    for (int o = 8; o <= 16; o <<= 1) {
+        const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
+        const float mn = fmaxf(m, mo), ca = weight(m, l, mn), cb = weight(mo, lo, mn);
+        l = l * ca + lo * cb;
+#pragma unroll
+        for (int i = 0; i < PER; i++) acc[i] = acc[i] * ca + __shfl_xor_sync(0xffffffffu, acc[i], o) * cb;
+        m = mn;
+    }
+    if (lane == 0) { sm.m[warp] = m; sm.l[warp] = l; }
+    if (lane < 8) {
+#pragma unroll
+        for (int i = 0; i < PER; i += 4) *reinterpret_cast<float4*>(&sm.acc[warp][lane8 * PER + i]) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+    }
     __syncthreads();
-
-    float M = -CUDART_INF_F;
+    if (threadIdx.x < HS) {
+        float M = -CUDART_INF_F, L = 0.f, a = 0.f;
 #pragma unroll
-    for (int g = 0; g < kGroups; g++) M = fmaxf(M, sm_m[g]);
+        for (int w = 0; w < kAttnWarps; w++) M = fmaxf(M, sm.m[w]);
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; w++) {
+            const float e = weight(sm.m[w], sm.l[w], M);
+            L += sm.l[w] * e;
+            a += sm.acc[w][threadIdx.x] * e;
+        }
+        sm.out[threadIdx.x] = a;
+        if (threadIdx.x == 0) { sm.M = M; sm.L = L; }
+    }
+}
+
+// grid (cluster, heads), the blocks of a head one cluster: each merges its part of the head's dims.
+template <int HS>
+__global__ void __launch_bounds__(kAttnThreads) attn_cluster_kernel(__half* output, const __half* q, const __half* kc, const __half* vc, int kv_mul, int kv_stride,
+                                                                    const int* pPos) {
+    __shared__ __align__(16) AttnShared<HS> sm;
+    const int h = blockIdx.y, rank = blockIdx.x, nblocks = gridDim.x;
+    griddep_wait();
+    griddep_launch_dependents();
+    attn_share<HS>(sm, q, kc, vc, kv_mul, kv_stride, pPos, h, rank, nblocks);
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int dims = HS / nblocks;
+    if (threadIdx.x < dims) {
+        const int d = rank * dims + threadIdx.x;
+        auto remote = [](const float* p, int r) {
+            uint32_t addr;
+            float v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(r));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+            return v;
+        };
+        float pm[8], pl[8], pa[8], M = -CUDART_INF_F, L = 0.f, a = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            pm[r] = -CUDART_INF_F;
+            pl[r] = pa[r] = 0.f;
+            if (r < nblocks) { pm[r] = remote(&sm.M, r); pl[r] = remote(&sm.L, r); pa[r] = remote(&sm.out[d], r); }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r++) M = fmaxf(M, pm[r]);
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const float e = pl[r] == 0.f ? 0.f : expf(pm[r] - (M == -CUDART_INF_F ? 0.f : M));
+            L += pl[r] * e;
+            a += pa[r] * e;
+        }
+        output[(size_t)h * HS + d] = __float2half(a / L);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // no block leaves while another reads its shared memory
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int HS>
+__global__ void __launch_bounds__(kAttnThreads) attn_partial_kernel(float* scratch, const __half* q, const __half* kc, const __half* vc,
+                                                                    int kv_mul, int kv_stride, const int* pPos) {
+    __shared__ __align__(16) AttnShared<HS> sm;
+    const int h = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x;
+    griddep_wait();
+    griddep_launch_dependents();
+    attn_share<HS>(sm, q, kc, vc, kv_mul, kv_stride, pPos, h, split, nsplit);
+    __syncthreads();
     float* out = scratch + ((size_t)h * nsplit + split) * (HS + 2);
     if (threadIdx.x == 0) {
-        float L = 0.f;
-        for (int g = 0; g < kGroups; g++) L += (sm_m[g] == -CUDART_INF_F) ? 0.f : sm_l[g] * expf(sm_m[g] - M);
-        out[0] = M;
-        out[1] = L;
+        out[0] = sm.M;
+        out[1] = sm.L;
     }
-    for (int d = threadIdx.x; d < HS; d += kAttnThreads) {
-        float a = 0.f;
-#pragma unroll
-        for (int g = 0; g < kGroups; g++) a += (sm_m[g] == -CUDART_INF_F) ? 0.f : sm_acc[g][d] * expf(sm_m[g] - M);
-        out[2 + d] = a;
-    }
+    if (threadIdx.x < HS) out[2 + threadIdx.x] = sm.out[threadIdx.x];
 }
 
 __global__ void attn_merge_kernel(__half* output, const float* scratch, int nsplit, int head_size) {
@@ -141,17 +231,15 @@ __global__ void attn_merge_kernel(__half* output, const float* scratch, int nspl
     const float* base = scratch + (size_t)h * nsplit * (head_size + 2);
     float M = -CUDART_INF_F;
     for (int s = 0; s < nsplit; s++) M = fmaxf(M, base[(size_t)s * (head_size + 2)]);
+    auto weight = [&](int s) {
+        const float* p = base + (size_t)s * (head_size + 2);
+        return p[1] == 0.f ? 0.f : expf(p[0] - (M == -CUDART_INF_F ? 0.f : M));
+    };
     float L = 0.f;
-    for (int s = 0; s < nsplit; s++) {
-        const float ms = base[(size_t)s * (head_size + 2)];
-        if (ms != -CUDART_INF_F) L += base[(size_t)s * (head_size + 2) + 1] * expf(ms - M);
-    }
+    for (int s = 0; s < nsplit; s++) L += base[(size_t)s * (head_size + 2) + 1] * weight(s);
     for (int d = threadIdx.x; d < head_size; d += blockDim.x) {
         float a = 0.f;
-        for (int s = 0; s < nsplit; s++) {
-            const float ms = base[(size_t)s * (head_size + 2)];
-            if (ms != -CUDART_INF_F) a += base[(size_t)s * (head_size + 2) + 2 + d] * expf(ms - M);
-        }
+        for (int s = 0; s < nsplit; s++) a += base[(size_t)s * (head_size + 2) + 2 + d] * weight(s);
         output[(size_t)h * head_size + d] = __float2half(a / L);
     }
 }
@@ -163,24 +251,40 @@ extern "C" size_t q4_attention_scratch_bytes(int num_heads, int head_size) {
     return (size_t)num_heads * attn_splits(num_heads) * (head_size + 2) * sizeof(float);
 }
 
-// Launches the two passes with caller-owned scratch.
+template <int HS>
+static int attention_launch(cudaStream_t s, __half* output, const __half* q, const __half* kc, const __half* vc, float* scratch, int num_heads, int kv_mul, const int* pPos) {
+    const int kv_stride = num_heads * HS / kv_mul;
+    if (num_heads >= kClusterHeads) {
+        const int blocks = attn_cluster(num_heads);
+        Q4Launch L(dim3(blocks, num_heads), dim3(kAttnThreads), 0, s);
+        cudaLaunchAttribute attr[2] = {L.attr[0], {}};
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = blocks;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        L.cfg.attrs = attr;
+        L.cfg.numAttrs = 2;
+        Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_cluster_kernel<HS>, output, q, kc, vc, kv_mul, kv_stride, pPos));
+        return Q4_OK;
+    }
+    const int nsplit = attn_splits(num_heads);
+    Q4Launch L(dim3(nsplit, num_heads), dim3(kAttnThreads), 0, s);
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_partial_kernel<HS>, scratch, q, kc, vc, kv_mul, kv_stride, pPos));
+    Q4Launch L2(dim3(num_heads), dim3(HS < 128 ? 64 : 128), 0, s);
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L2.cfg, attn_merge_kernel, output, (const float*)scratch, nsplit, HS));
+    return Q4_OK;
+}
+
+// One or two launches (see the top); scratch is the caller's.
 static int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache,
                         float* scratch, int num_heads, int head_size, int kv_mul, const int* pPos) {
-    const int nsplit = attn_splits(num_heads);
-    const int kv_stride = num_heads * head_size / kv_mul;
-    Q4Launch L(dim3(nsplit, num_heads), dim3(kAttnThreads), 0, s);
-    const __half* qh = (const __half*)q;
-    const __half* kc = (const __half*)key_cache;
-    const __half* vc = (const __half*)value_cache;
+    __half* out = (__half*)output;
+    const __half *qh = (const __half*)q, *kc = (const __half*)key_cache, *vc = (const __half*)value_cache;
     switch (head_size) {
-        case 64: Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_partial_kernel<64>, scratch, qh, kc, vc, kv_mul, kv_stride, pPos)); break;
-        case 128: Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_partial_kernel<128>, scratch, qh, kc, vc, kv_mul, kv_stride, pPos)); break;
-        case 256: Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_partial_kernel<256>, scratch, qh, kc, vc, kv_mul, kv_stride, pPos)); break;
+        case 64: return attention_launch<64>(s, out, qh, kc, vc, scratch, num_heads, kv_mul, pPos);
+        case 128: return attention_launch<128>(s, out, qh, kc, vc, scratch, num_heads, kv_mul, pPos);
+        case 256: return attention_launch<256>(s, out, qh, kc, vc, scratch, num_heads, kv_mul, pPos);
         default: return Q4_ERR_UNSUPPORTED_SIZE;
     }
-    Q4Launch L2(dim3(num_heads), dim3(head_size < 128 ? 64 : 128), 0, s);
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L2.cfg, attn_merge_kernel, (__half*)output, (const float*)scratch, nsplit, head_size));
-    return Q4_OK;
 }
 
 extern "C" int q4_attention(void* stream, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache,

@@ -74,6 +74,44 @@ def test_attention(heads, kv_mul, hs, pos):
     assert_close(out.cpu().numpy(), ref, f"attention pos={pos}", max_rel=5e-3)
 
 
+def _attention(heads, kv_mul, hs, pos, q, kc, vc):
+    out = torch.full((heads * hs,), float("nan"), dtype=torch.float16, device="cuda")
+    ops.MultiHeadAttention(out, dev(q), dev(kc), dev(vc), ops.attention_scratch(heads, hs), heads, hs, kv_mul, pos + 1,
+                           torch.tensor([pos], dtype=torch.int32, device="cuda"))
+    return out.cpu().numpy()
+
+
+# both sides of every line between the forms (16, 64 and 128 heads), shares that are empty, end on a step of 64 positions or one past it
+@pytest.mark.parametrize("heads,kv_mul,hs", [(15, 1, 128), (16, 2, 64), (16, 1, 256), (64, 8, 128), (65, 5, 64), (129, 3, 64)])
+@pytest.mark.parametrize("pos", [0, 31, 32, 255, 256, 511, 512, 600])
+def test_attention_forms_and_share_edges(heads, kv_mul, hs, pos):
+    rng = np.random.default_rng(pos * 7 + heads)
+    stride = heads * hs // kv_mul
+    q = rng.standard_normal(heads * hs).astype(np.float16)
+    kc, vc = ((rng.standard_normal((pos + 1, stride)) * s).astype(np.float16) for s in (0.5, 1.0))
+    assert_close(_attention(heads, kv_mul, hs, pos, q, kc, vc), O.attention(q, kc, vc, heads, hs, kv_mul, pos), f"{heads} heads, pos {pos}", max_rel=5e-3)
+
+
+@pytest.mark.parametrize("heads", [4, 32])     # two launches, one cluster
+def test_attention_with_scores_that_are_not_finite(heads):
+    """A score of -infinity (rounded to fp16) has weight 0, also where it is the first or the only one a lane group sees; a NaN reaches
+    its own head's outputs and no other's."""
+    hs, pos = 128, 40
+    rng = np.random.default_rng(heads)
+    q = np.abs(rng.standard_normal(heads * hs)).astype(np.float16) + np.float16(0.5)
+    kc = (rng.standard_normal((pos + 1, heads * hs)) * 0.5).astype(np.float16)
+    vc = rng.standard_normal((pos + 1, heads * hs)).astype(np.float16)
+    low = [0, 1, 2, 33]
+    kc[low] = np.float16(-60000.0)             # scores far below -65504
+    want = O.attention(q, np.delete(kc, low, 0), np.delete(vc, low, 0), heads, hs, 1, pos - len(low))
+    assert_close(_attention(heads, 1, hs, pos, q, kc, vc), want, "scores of -infinity", max_rel=5e-3)
+    kc[35, hs] = np.nan                        # head 1
+    got = _attention(heads, 1, hs, pos, q, kc, vc)
+    assert np.isnan(got[hs:2 * hs]).all()
+    rest = np.r_[0:hs, 2 * hs:heads * hs]
+    assert_close(got[rest], want[rest], "other heads", max_rel=5e-3)
+
+
 @pytest.mark.parametrize("n,d", [(8, 8), (256, 40), (4096, 1000), (5120, 4000), (4096, 32000)])
 def test_classifier_matvec_f16(n, d):
     rng = np.random.default_rng(n + d)
