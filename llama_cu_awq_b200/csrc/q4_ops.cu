@@ -49,6 +49,53 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(__half* o, const __half* 
     griddep_wait();
     griddep_launch_dependents();
     float ss = 0.f;
+    // One block, so all of it is latency: the weights are requested with the row, both stay in registers and one 16-byte store
+    // per thread writes the result. (Read again two bytes at a time, weights only behind the sum: with the rotation below, two 7B layers call by call 120 -> 107 us.)
+    constexpr int kKeep = 2;
+    const int step = blockDim.x * 8;
+    if (size % 8 == 0 && size <= kKeep * step && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(o)) & 15) == 0) {
+        uint4 xv[kKeep], wv[kKeep];
+#pragma unroll
+        for (int c = 0; c < kKeep; c++) {
+            const int i = threadIdx.x * 8 + c * step;
+            if (i < size) {
+                xv[c] = *reinterpret_cast<const uint4*>(x + i);
+                wv[c] = *reinterpret_cast<const uint4*>(w + i);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < kKeep; c++) {
+            if (threadIdx.x * 8 + c * step < size) {
+                const __half2* h = reinterpret_cast<const __half2*>(&xv[c]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float2 f = __half22float2(h[j]);
+                    ss = fmaf(f.x, f.x, ss);
+                    ss = fmaf(f.y, f.y, ss);
+                }
+            }
+        }
+        ss = block_sum(ss, red);
+        ss /= size;
+        ss += 1e-5f;
+        ss = 1.0f / sqrtf(ss);
+#pragma unroll
+        for (int c = 0; c < kKeep; c++) {
+            const int i = threadIdx.x * 8 + c * step;
+            if (i < size) {
+                const __half2 *h = reinterpret_cast<const __half2*>(&xv[c]), *g = reinterpret_cast<const __half2*>(&wv[c]);
+                uint4 ov;
+                __half2* oh = reinterpret_cast<__half2*>(&ov);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float2 f = __half22float2(h[j]), e = __half22float2(g[j]);
+                    oh[j] = __floats2half2_rn(f.x * (ss * e.x), f.y * (ss * e.y));
+                }
+                *reinterpret_cast<uint4*>(o + i) = ov;
+            }
+        }
+        return;
+    }
     for (int i = threadIdx.x * 8; i < size; i += blockDim.x * 8) {
         if (i + 8 <= size) {
             uint4 v = *reinterpret_cast<const uint4*>(x + i);
@@ -83,12 +130,22 @@ __global__ void __launch_bounds__(256) rope_kernel(__half* q, __half* key_cache,
     griddep_wait();
     griddep_launch_dependents();
     __shared__ float2 table[256];
-    const int pos = *pPos, pairs = head_size / 2;
+    const int pairs = head_size / 2, first = blockIdx.x * kRopeHeadsPerBlock, last = min(first + kRopeHeadsPerBlock, num_heads);
+    // this thread's first pair is requested before the position's angles are evaluated: a memory latency under powf, cosf and sinf
+    const int e0 = threadIdx.x, head0 = first + e0 / pairs, i0 = e0 % pairs;
+    const bool any = e0 < (last - first) * pairs, any_key = any && head0 < num_kv_heads;
+    __half* q0 = q + (size_t)head0 * head_size + i0;
+    __half lo = __half(), hi = __half(), klo = __half(), khi = __half();
+    if (any) { lo = q0[0]; hi = q0[pairs]; }
+    const int pos = *pPos;
+    __half* key_row = key_cache + loff + (long long)pos * num_kv_heads * head_size;
+    __half* k0 = key_row + (size_t)head0 * head_size + i0;
+    if (any_key) { klo = k0[0]; khi = k0[pairs]; }
     for (int i = threadIdx.x; i < pairs; i += blockDim.x) table[i] = rope_cos_sin(pos, i, head_size, theta);
     __syncthreads();
-    __half* key_row = key_cache + loff + (long long)pos * num_kv_heads * head_size;
-    const int first = blockIdx.x * kRopeHeadsPerBlock, last = min(first + kRopeHeadsPerBlock, num_heads);
-    for (int e = threadIdx.x; e < (last - first) * pairs; e += blockDim.x) {
+    if (any) rope_rotate(&lo, &hi, q0, q0 + pairs, table[i0]);
+    if (any_key) rope_rotate(&klo, &khi, k0, k0 + pairs, table[i0]);
+    for (int e = threadIdx.x + blockDim.x; e < (last - first) * pairs; e += blockDim.x) {
         const int head = first + e / pairs, i = e % pairs;
         __half* qh = q + (size_t)head * head_size;
         rope_rotate(qh + i, qh + i + pairs, qh + i, qh + i + pairs, table[i]);

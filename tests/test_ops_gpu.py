@@ -35,6 +35,30 @@ def test_rmsnorm(n):
     assert (xd.cpu().numpy().view(np.uint16) == got.view(np.uint16)).all()
 
 
+# one and two pieces per thread, the largest row that stays in registers (8192 at 512 threads, 16384 at 1024), one past it
+@pytest.mark.parametrize("n", [8, 4088, 4104, 8184, 8192, 16384, 16392])
+def test_rmsnorm_in_registers_and_not(n):
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal(n) * 3).astype(np.float16)
+    w = rng.uniform(0.5, 1.5, n).astype(np.float16)
+    o = torch.empty(n + 8, dtype=torch.float16, device="cuda")
+    wd = dev(np.r_[w[:1], w])          # w again, two bytes further
+    xd = dev(x)
+    got = []
+    for ov, wv in ((o[:n], dev(w)), (o[1:n + 1], dev(w)), (o[:n], wd[1:])):     # the last two do not start on 16 bytes
+        ops.rmsnorm(ov, xd, wv, n)
+        got.append(ov.cpu().numpy().copy())
+    assert_close(got[0], O.rmsnorm(x, w), "rmsnorm", max_rel=2e-3)
+    for g in got[1:]:
+        assert (g.view(np.uint16) == got[0].view(np.uint16)).all()      # same sums in the same order, one rounding
+
+
+# several pairs per thread (head size 512), heads and key heads that end inside a block, a head size that is no power of two
+@pytest.mark.parametrize("heads,kv_heads,hs,pos", [(6, 6, 512, 11), (5, 2, 256, 70), (7, 3, 96, 9), (1, 1, 2, 3)])
+def test_rope_pairs_per_thread(heads, kv_heads, hs, pos):
+    test_rope(heads, kv_heads, hs, pos)
+
+
 @pytest.mark.parametrize("heads,kv_heads,hs,pos", [(2, 2, 64, 0), (32, 32, 128, 17), (8, 1, 128, 4095), (4, 2, 128, 300)])
 def test_rope(heads, kv_heads, hs, pos):
     rng = np.random.default_rng(pos + heads)
