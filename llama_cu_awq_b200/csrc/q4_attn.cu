@@ -3,7 +3,7 @@
 // Replaces MultiHeadAttention (llama2_q4.cu:410-427; mat_vec_kernel_simple, softmax_kernel, vec_mat_kernel at
 // gpu_kernels.h:150-176,365-454,287-337).
 //
-// A block takes positions [t0, t1) of one head. Eight lanes share a position (16 head dims each at head size 128), a block of
+// A block takes positions [t0, t1) of one head. Eight lanes share a position (8 dims of every 64: a load of theirs is 128 bytes in a row), a block of
 // eight warps has 64 positions in hand per step and the next 64 requested. Scores are rounded to fp16 like the reference's; the
 // softmax runs online in fp32 (running max, sum and un-normalised V accumulator per lane group), merged across the block in registers
 // and shared memory. Then, by the number of heads:
@@ -52,7 +52,7 @@ __device__ __forceinline__ void attn_share(AttnShared<HS>& sm, const __half* q, 
     const int lane8 = threadIdx.x & 7, grp = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint4 qv[VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; v++) qv[v] = *reinterpret_cast<const uint4*>(q + (size_t)h * HS + lane8 * PER + v * 8);
+    for (int v = 0; v < VEC; v++) qv[v] = *reinterpret_cast<const uint4*>(q + (size_t)h * HS + v * 64 + lane8 * 8);
     const int T = *pPos + 1;
     // split boundaries in units of kGroups positions
     const int units = (T + kGroups - 1) / kGroups;
@@ -65,7 +65,7 @@ __device__ __forceinline__ void attn_share(AttnShared<HS>& sm, const __half* q, 
         for (int j = 0; j < 4; j++) { const float2 f = __half22float2(hh[j]); qf[v * 8 + 2 * j] = f.x; qf[v * 8 + 2 * j + 1] = f.y; }
     }
     const float alpha = (float)(1.0 / sqrt((double)HS));
-    const size_t head_off = (size_t)(h / kv_mul) * HS + lane8 * PER;
+    const size_t head_off = (size_t)(h / kv_mul) * HS + lane8 * 8;
 
     float m = -CUDART_INF_F, l = 0.f;
     float acc[PER];
@@ -82,7 +82,7 @@ __device__ __forceinline__ void attn_share(AttnShared<HS>& sm, const __half* q, 
             const int t = tb + grp + u * kGroups;
             const uint4* src = reinterpret_cast<const uint4*>(cache + (size_t)(t < t1 ? t : t0) * kv_stride + head_off);
 #pragma unroll
-            for (int v = 0; v < VEC; v++) r[u][v] = src[v];
+            for (int v = 0; v < VEC; v++) r[u][v] = src[8 * v];
         }
     };
     fetch(k4, kc, t0);
@@ -147,7 +147,7 @@ __device__ __forceinline__ void attn_share(AttnShared<HS>& sm, const __half* q, 
     if (lane == 0) { sm.m[warp] = m; sm.l[warp] = l; }
     if (lane < 8) {
 #pragma unroll
-        for (int i = 0; i < PER; i += 4) *reinterpret_cast<float4*>(&sm.acc[warp][lane8 * PER + i]) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+        for (int i = 0; i < PER; i += 4) *reinterpret_cast<float4*>(&sm.acc[warp][(i >> 3) * 64 + lane8 * 8 + (i & 7)]) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
     }
     __syncthreads();
     if (threadIdx.x < HS) {

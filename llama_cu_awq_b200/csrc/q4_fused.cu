@@ -640,12 +640,14 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
 
         if (f == K_O && !(Q4_DBG(p) & 1)) {
             // ---- attention of one query per head over positions 0..pos, split over CTAs (llama2_q4.cu:410-427) ----
-            // 8 lanes per position, 16 dims each; two positions per lane group and step, the next step's keys and values each requested
-            // as soon as this step's have been used.
+            // 8 lanes per position, 16 dims each, eight of either half of the head: a load of the lane group is 128 bytes in a row (16
+            // consecutive dims per lane are every second 16 bytes twice, twice the sectors from L2: 9.3 us of a layer at position 1800,
+            // 6.4 so); two positions per lane group and step, the next step's keys and values each requested as soon as this step's
+            // have been used.
             const int pi = pi0 + LP_ATTN;
             TRACE(pi, 0);
             float* sm_acc = part_a;                              // [kW][128]; the QKV sums in it are done with after the barrier below
-            const int d0 = (tid & 7) * 16, grp = tid >> 3;
+            const int d0 = (tid & 7) * 8, d1 = d0 + 64, grp = tid >> 3;
             const int T = pos + 1;
             const float alpha = (float)(1.0 / sqrt(128.0));
             const int ns = attn_splits_for(p, T);
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                         const int t = row_of(tb + grp + u * (kThreads / 8));
                         if (t != pos) {
                             const uint4* src = reinterpret_cast<const uint4*>(cache + (size_t)t * p.kv_n + col);
-                            r[u][0] = __ldcg(src); r[u][1] = __ldcg(src + 1);
+                            r[u][0] = __ldcg(src); r[u][1] = __ldcg(src + 8);
                         }
                     }
                 };
@@ -698,7 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                 TRACE(pi, 1);
                 uint4 qh[2];
                 qh[0] = *reinterpret_cast<const uint4*>(&new_row[0][d0]);
-                qh[1] = *reinterpret_cast<const uint4*>(&new_row[0][d0 + 8]);
+                qh[1] = *reinterpret_cast<const uint4*>(&new_row[0][d1]);
                 float m = -CUDART_INF_F, l = 0.f, acc[16];
 #pragma unroll
                 for (int j = 0; j < 16; j++) acc[j] = 0.f;
@@ -707,8 +709,8 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         if (row_of(u ? tz : ta) == pos) {
-                            k[u][0] = *reinterpret_cast<const uint4*>(&new_row[1][d0]); k[u][1] = *reinterpret_cast<const uint4*>(&new_row[1][d0 + 8]);
-                            v[u][0] = *reinterpret_cast<const uint4*>(&new_row[2][d0]); v[u][1] = *reinterpret_cast<const uint4*>(&new_row[2][d0 + 8]);
+                            k[u][0] = *reinterpret_cast<const uint4*>(&new_row[1][d0]); k[u][1] = *reinterpret_cast<const uint4*>(&new_row[1][d1]);
+                            v[u][0] = *reinterpret_cast<const uint4*>(&new_row[2][d0]); v[u][1] = *reinterpret_cast<const uint4*>(&new_row[2][d1]);
                         }
                     }
                     float s0 = dot16(k[0], qh), s1 = dot16(k[1], qh);
@@ -760,7 +762,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                 if (lane == 0) { sm_m[w] = m; sm_l[w] = l; }
                 if (lane < 8) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) *reinterpret_cast<float4*>(sm_acc + w * 128 + d0 + 4 * j) = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+                    for (int j = 0; j < 4; j++) *reinterpret_cast<float4*>(sm_acc + w * 128 + (j < 2 ? d0 : d1) + 4 * (j & 1)) = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
                 }
                 __syncthreads();
                 // Slot (h, split) of a fixed [heads][nsplit] layout. The CTA that writes a head's last split in use also stamps
