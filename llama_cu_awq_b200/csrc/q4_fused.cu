@@ -1263,9 +1263,10 @@ void q4_fused_free(q4_model* m) {
 // ranks' tags must stay in step and a rank's exchange area is written by its peers, so after an error (as after
 // q4_model_prepare) every rank has to finish its reset before any rank launches again: the callers put a host
 // barrier there.
-void q4_fused_reset(q4_model* m) {
+void q4_fused_reset(q4_model* m, bool clean) {
     if (!m->fused || m->fused->unsupported) return;
     q4_fused* f = m->fused;
+    if (f->armed && clean) return;
     int st = 0;
     cudaDeviceSynchronize();
     if (f->armed && cudaMemcpy(&st, f->params.status, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && st == 0) return;
@@ -1282,6 +1283,8 @@ void q4_fused_reset(q4_model* m) {
     f->launches = 0;
     f->armed = ok;
 }
+
+const int* q4_fused_status_word(const q4_model* m) { return m->fused && !m->fused->unsupported ? m->fused->params.status : nullptr; }
 
 // Limit of every device-side wait of the fused kernel (default two seconds); takes effect with the next launch.
 void q4_fused_set_wait_limit(q4_model* m, unsigned long long ns) {

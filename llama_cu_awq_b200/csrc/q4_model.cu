@@ -175,6 +175,7 @@ extern "C" int q4_model_free(q4_model* m) {
     cudaFree(m->x); cudaFree(m->xb); cudaFree(m->hb); cudaFree(m->q); cudaFree(m->logits);
     cudaFree(m->kc); cudaFree(m->vc); cudaFree(m->attn_scratch); cudaFree(m->pos);
     if (m->shared) cudaFreeHost(m->shared);
+    if (m->gen_stream) cudaStreamDestroy(m->gen_stream);
     delete m;
     return Q4_OK;
 }
@@ -244,6 +245,8 @@ static int model_build(q4_model** out, const q4_config& c, int rank, int gpu_cou
     m->attn_scratch = nullptr;
     m->pos = nullptr;
     m->shared = nullptr;
+    m->status_word = nullptr;
+    m->gen_stream = nullptr;
 
     // device arena for this rank's weights
     size_t need = 0;
@@ -345,7 +348,8 @@ static int model_build(q4_model** out, const q4_config& c, int rank, int gpu_cou
     LOAD_CUDA(cudaMalloc((void**)&m->vc, kv_bytes));
     LOAD_CUDA(cudaMalloc((void**)&m->attn_scratch, q4_attention_scratch_bytes(c.n_heads / g, hs)));
     LOAD_CUDA(cudaMalloc((void**)&m->pos, sizeof(int)));
-    LOAD_CUDA(cudaMallocHost((void**)&m->shared, sizeof(q4_shared_data)));
+    LOAD_CUDA(cudaMallocHost((void**)&m->shared, sizeof(q4_shared_data) + sizeof(int)));
+    m->status_word = reinterpret_cast<volatile int*>(m->shared + 1);
     LOAD_CUDA(cudaMemset(m->kc, 0, kv_bytes));
     LOAD_CUDA(cudaMemset(m->vc, 0, kv_bytes));
     LOAD_CUDA(cudaMemset(m->pos, 0, sizeof(int)));
@@ -415,6 +419,12 @@ extern "C" int q4_model_read(const q4_model* m, int what, uint16_t* host_out) {
     return Q4_OK;
 }
 
+// The position into device memory and the fused kernel's status out to the host: one launch, where a copy back took twice as long.
+static __global__ void reset_kernel(int* pos_dev, int pos, const int* status, volatile int* status_word) {
+    *pos_dev = pos;
+    *status_word = *status;
+}
+
 extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int pos) {
     if (!m || n < 0 || n > Q4_MAX_SEQ_LEN || pos < 0 || pos >= m->cfg.seq_len) return Q4_ERR_INVALID;
     // the embedding gather indexes the table with these ids on the device: refuse anything outside the vocabulary here
@@ -423,10 +433,20 @@ extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int 
             if (prompt_tokens[i] < 0 || prompt_tokens[i] >= m->cfg.vocab_size) return Q4_ERR_INVALID;
     Q4_CUDA_TRY(cudaDeviceSynchronize());
     m->host_pos = pos;
-    Q4_CUDA_TRY(cudaMemcpy(m->pos, &pos, sizeof(int), cudaMemcpyHostToDevice));
+    const int* status = q4_fused_status_word(m);
+    *m->status_word = -1;
+    if (status) {
+        reset_kernel<<<1, 1>>>(m->pos, pos, status, m->status_word);
+        Q4_CUDA_TRY(cudaGetLastError());
+    } else {
+        Q4_CUDA_TRY(cudaMemcpy(m->pos, &pos, sizeof(int), cudaMemcpyHostToDevice));   // (nothing to wait for: a few microseconds less)
+    }
     m->shared->pos = pos;
     if (n > 0 && prompt_tokens) memcpy((void*)m->shared->tokens, prompt_tokens, sizeof(int) * (size_t)n);
-    q4_fused_reset(m);
+    if (status) {
+        Q4_CUDA_TRY(cudaDeviceSynchronize());
+        q4_fused_reset(m, *m->status_word == 0);
+    }
     return Q4_OK;
 }
 
@@ -548,10 +568,10 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
                            double* seconds) {
     if (!m || !prompt_tokens || n_prompt < 1) return Q4_ERR_INVALID;
     if (steps <= 0 || steps > m->cfg.seq_len) steps = m->cfg.seq_len;  // llama2_q4.cu:917
-    cudaStream_t s;
-    Q4_CUDA_TRY(cudaStreamCreate(&s));
+    if (!m->gen_stream) Q4_CUDA_TRY(cudaStreamCreate(&m->gen_stream));
+    const cudaStream_t s = m->gen_stream;
     int e = q4_model_reset(m, prompt_tokens, n_prompt, 0);
-    if (e != Q4_OK) { cudaStreamDestroy(s); return e; }
+    if (e != Q4_OK) return e;
     int pos = 0;
     const bool one_pass = (path & Q4_PATH_PROMPT_ONE_PASS) != 0;
     path &= ~Q4_PATH_PROMPT_ONE_PASS;
@@ -561,7 +581,7 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
         // first generated id (greedy or sampled). A model the many-row kernels do not serve falls back to the loop.
         e = q4_prefill_cache(m, s, n_prompt - 1);
         if (e == Q4_OK) pos = n_prompt - 1;
-        else if (e != Q4_ERR_UNSUPPORTED_SIZE) { cudaStreamDestroy(s); return e; }
+        else if (e != Q4_ERR_UNSUPPORTED_SIZE) return e;
     }
     while (pos < steps) {
         // A generated id is in the mailbox when its token is done; a prompt's ids are there already, and its positions are queued without
@@ -578,7 +598,6 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
     }
     cudaError_t ce = cudaStreamSynchronize(s);
     const auto end = std::chrono::steady_clock::now();
-    cudaStreamDestroy(s);
     if (e != Q4_OK) return e;
     Q4_CUDA_TRY(ce);
     if (seconds) *seconds = std::chrono::duration<double>(end - start).count();

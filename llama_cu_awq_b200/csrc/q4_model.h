@@ -41,6 +41,8 @@ struct q4_model {
     float* attn_scratch;
     int* pos;
     q4_shared_data* shared;
+    volatile int* status_word;  // pinned, behind the shared data: the fused kernel's status as the last reset found it
+    cudaStream_t gen_stream;    // q4_generate's, made by its first call
     cudaGraphExec_t graph[3];   // prompt phase, generating (argmax), generating without the hand-off (a sampler follows)
     bool graph_ready[3];
     // sampler state (sampler.h:10-19): temperature 0 = greedy
@@ -54,7 +56,8 @@ struct q4_model {
 // q4_fused.cu
 int q4_fused_prepare(q4_model* m);                              // builds the stream-layout weights and the phase table (lazy)
 int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff);
-void q4_fused_reset(q4_model* m);                               // re-arms barrier counters (after q4_model_reset)
+void q4_fused_reset(q4_model* m, bool clean = false);           // re-arms barrier counters (after q4_model_reset); clean: the status is known to be zero
+const int* q4_fused_status_word(const q4_model* m);             // on the device; null where nothing can have been recorded
 void q4_fused_free(q4_model* m);
 int q4_fused_status(q4_model* m);
 void q4_rows_free(q4_model* m);   // q4_batch.cu
