@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __
     const uint4* wv = reinterpret_cast<const uint4*>(w);
     const int nvec = size / 8;
     constexpr int kKeep = 4;
-    uint4 v[kKeep];
+    uint4 v[kKeep], wk[kKeep];   // (the weights are requested with the row: behind the sum they were a memory latency of their own)
     float ss = 0.f;
     auto row = [&](int i) {
         uint4 r = xr[i];
@@ -104,8 +104,11 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __
 #pragma unroll
     for (int c = 0; c < kKeep; c++) {
         const int i = threadIdx.x + c * kRowThreads;
-        if (i < nvec) { v[c] = row(i); ss += sumsq8(v[c]); }
+        if (i < nvec) { v[c] = row(i); wk[c] = __ldg(wv + i); }
     }
+#pragma unroll
+    for (int c = 0; c < kKeep; c++)
+        if (threadIdx.x + c * kRowThreads < nvec) ss += sumsq8(v[c]);
     for (int i = threadIdx.x + kKeep * kRowThreads; i < nvec; i += kRowThreads) ss += sumsq8(row(i));
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
@@ -119,7 +122,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __
 #pragma unroll
     for (int c = 0; c < kKeep; c++) {
         const int i = threadIdx.x + c * kRowThreads;
-        if (i < nvec) orow[i] = scale8(v[c], wv[i], tot);
+        if (i < nvec) orow[i] = scale8(v[c], wk[c], tot);
     }
     for (int i = threadIdx.x + kKeep * kRowThreads; i < nvec; i += kRowThreads) orow[i] = scale8(xr[i], wv[i], tot);
 }
@@ -505,13 +508,14 @@ __global__ void set_pos_kernel(int* pos_dev, volatile int* pos_pinned, int pos) 
     *pos_pinned = pos;
 }
 
-__global__ void iota_rows_kernel(int* row_seq, int* row_pos, int n, int seq, int pos0, int step_seq) {
+// rows = positions pos0, pos0 + 1, ... of sequence 0
+__global__ void iota_rows_kernel(int* row_seq, int* row_pos, int n, int pos0) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        row_seq[i] = seq + i * step_seq;
-        if (row_pos) row_pos[i] = pos0 + i;
+        row_seq[i] = 0;
+        row_pos[i] = pos0 + i;
     }
 }
 
@@ -842,7 +846,8 @@ enum RowsWanted { WANT_ALL, WANT_LAST, WANT_CACHE };
 // All layers for `n` rows whose embeddings are in r->X; K/V rows go to (kc, vc) with `seq_stride` halfs between sequences.
 // pos0 >= 0: the rows are positions pos0 .. pos0 + n - 1 of one sequence (prompt); -1: one row per sequence (batched decode).
 // In the last layer the rows that nobody asks for end at their K/V row: no later layer reads them.
-static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* vc, long long seq_stride, int pos0, RowsWanted want) {
+// row_seq, row_pos: the rows' sequences and positions, on the device.
+static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, const int* row_pos, __half* kc, __half* vc, long long seq_stride, int pos0, RowsWanted want) {
     q4_rows* r = m->rows;
     const q4_config& c = m->cfg;
     const int g = m->g, dim = c.dim;
@@ -884,7 +889,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
         const int ldq = skinny ? m->q_n : nqkv, ldkv = skinny ? m->kv_n : nqkv;
         if (pos0 >= 0)   // (batched decode: the attention kernel rotates and files)
             launch_rows(rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
-                        r->rope, r->row_seq, r->row_pos, seq_stride, loff);
+                        r->rope, row_seq, row_pos, seq_stride, loff);
         if (l == c.n_layers - 1 && want != WANT_ALL) {
             if (want == WANT_CACHE) break;
             // one row: the split attention and the products of the batch-1 path (70B: o, gate / up and down 147 us with the few-rows kernels,
@@ -892,7 +897,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
             const size_t last = (size_t)(n - 1);
             uint16_t* x = (uint16_t*)(r->X + last * dim);
             OP(q4_attention(s, (uint16_t*)r->ATT, (const uint16_t*)qp + last * ldq, (const uint16_t*)(kc + loff), (const uint16_t*)(vc + loff), m->attn_scratch, heads, m->head_size,
-                            m->kv_mul, c.seq_len, r->row_pos + last));
+                            m->kv_mul, c.seq_len, row_pos + last));
             OP(q4_matmul_q4(s, x, (const uint16_t*)r->ATT, &L.o.w, m->o_kc, dim, 1, g, -1, nullptr));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
             launch_rows(rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);
@@ -905,11 +910,11 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, __half* kc, __half* v
             launch_rows(attention_prefill_kernel, dim3(heads, q4_div_up(n, kAtRows)), dim3(128), kAtSmem, s, r->ATT, (const __half*)qp, ldq, kc + loff, vc + loff, heads,
                         m->kv_mul, n, pos0, m->kv_n);
         else if (pos0 >= 0)
-            launch_rows(attention_rows_kernel<false>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
-                        r->row_pos, seq_stride, loff, m->kv_n, (const __half*)nullptr, (const __half*)nullptr, (const float2*)nullptr);
+            launch_rows(attention_rows_kernel<false>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, row_seq,
+                        row_pos, seq_stride, loff, m->kv_n, (const __half*)nullptr, (const __half*)nullptr, (const float2*)nullptr);
         else
-            launch_rows(attention_rows_kernel<true>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, r->row_seq,
-                        r->row_pos, seq_stride, loff, m->kv_n, kp, vp, r->rope);
+            launch_rows(attention_rows_kernel<true>, dim3(heads, n), dim3(kAttWarps * 32), 0, s, r->ATT, (const __half*)qp, ldq, kc, vc, heads, m->kv_mul, row_seq,
+                        row_pos, seq_stride, loff, m->kv_n, kp, vp, r->rope);
         // x = o_proj(att) + x / g, summed over the ranks (gpu_kernels.h:237-238, llama2_q4.cu:472-476)
         if (skinny) OP(q4_matmul_q4_rows(s, (uint16_t*)r->X, (const uint16_t*)r->ATT, &L.o.w, n, m->o_kc, dim, (const uint16_t*)r->X, 1.0f / g));
         else OP(gemm(fused_add ? r->Y : r->X, r->ATT, l, 1, !fused_add));
@@ -950,9 +955,9 @@ static int prefill(q4_model* m, cudaStream_t s, int n, int gen_token, bool logit
     int e;
     if ((e = rows_prepare(m, n)) != Q4_OK) return e;
     q4_rows* r = m->rows;
-    launch_rows(iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, 0, pos0, 0);
+    launch_rows(iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, pos0);
     launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size);
-    if ((e = rows_layers(m, s, n, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) != Q4_OK) return e;
+    if ((e = rows_layers(m, s, n, r->row_seq, r->row_pos, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) != Q4_OK) return e;
     if ((e = move_pos(m, s, logits ? pos0 + n - 1 : pos0 + n)) != Q4_OK) return e;
     if (logits) {
         // the last row goes on through the batch-1 tail (llama2_q4.cu:528-537, sampler.h:77-84): final norm, classifier,
@@ -979,7 +984,7 @@ struct q4_batch {
     q4_model* m;
     int n_seq, n_prompt, max_len;
     __half *kc = nullptr, *vc = nullptr, *logits = nullptr, *xf = nullptr, *part = nullptr;
-    int *tokens = nullptr, *pos = nullptr;
+    int *tokens = nullptr, *pos = nullptr, *seq = nullptr;   // seq: 0, 1, 2, ...
     long long seq_stride;
     int steps = 0;
     // A step is the same work every time (positions and ids live in device memory), so it is captured once as a CUDA
@@ -991,7 +996,7 @@ struct q4_batch {
 extern "C" int q4_batch_free(q4_batch* b) {
     if (!b) return Q4_OK;
     if (b->step_graph) cudaGraphExecDestroy(b->step_graph);
-    cudaFree(b->kc); cudaFree(b->vc); cudaFree(b->logits); cudaFree(b->xf); cudaFree(b->part); cudaFree(b->tokens); cudaFree(b->pos);
+    cudaFree(b->kc); cudaFree(b->vc); cudaFree(b->logits); cudaFree(b->xf); cudaFree(b->part); cudaFree(b->tokens); cudaFree(b->pos); cudaFree(b->seq);
     delete b;
     return Q4_OK;
 }
@@ -1017,6 +1022,10 @@ extern "C" int q4_batch_create(q4_batch** out, q4_model* m, int n_seq) {
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->part, 2 * (size_t)n_seq * m->v_n);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->tokens, sizeof(int) * (size_t)n_seq * (c.seq_len + 1));
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->pos, sizeof(int) * n_seq);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b->seq, sizeof(int) * n_seq);
+    int order[16];
+    for (int i = 0; i < n_seq; i++) order[i] = i;
+    if (e == cudaSuccess) e = cudaMemcpy(b->seq, order, sizeof(int) * n_seq, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(b->kc, 0, kv_bytes);
     if (e == cudaSuccess) e = cudaMemset(b->vc, 0, kv_bytes);
     if (e != cudaSuccess) { q4_note_cuda_error(e, __FILE__, __LINE__); q4_batch_free(b); return Q4_ERR_CUDA; }
@@ -1073,10 +1082,9 @@ static int batch_step(q4_batch* b, cudaStream_t s) {
     q4_rows* r = m->rows;
     const q4_config& c = m->cfg;
     const int n = b->n_seq;
-    launch_rows(iota_rows_kernel, dim3(1), dim3(32), 0, s, r->row_seq, nullptr, n, 0, 0, 1);
-    Q4_CUDA_TRY(cudaMemcpyAsync(r->row_pos, b->pos, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
-    launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, b->tokens, b->max_len + 1, r->row_seq, r->row_pos, c.vocab_size);
-    if (int e = rows_layers(m, s, n, b->kc, b->vc, b->seq_stride, -1, WANT_ALL)) return e;
+    // row i is sequence i, and the hand-off moves the positions only when every kernel of the step has read them: no copies of either
+    launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, b->tokens, b->max_len + 1, b->seq, b->pos, c.vocab_size);
+    if (int e = rows_layers(m, s, n, b->seq, b->pos, b->kc, b->vc, b->seq_stride, -1, WANT_ALL)) return e;
     launch_rows(rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)nullptr, (const __half*)m->rms_final, c.dim);
     const size_t smem = 2 * (size_t)n * c.dim;
     __half* cls_out = m->g == 1 ? b->logits : b->part;   // TP: every rank computes its vocabulary slice of every row; the slices are gathered row by row
