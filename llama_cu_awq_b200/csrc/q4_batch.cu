@@ -1042,6 +1042,9 @@ extern "C" int q4_batch_reset(q4_batch* b, const int* prompts, int n_prompt) {
     Q4_CUDA_TRY(cudaMemset(b->tokens, 0, sizeof(int) * (size_t)b->n_seq * (b->max_len + 1)));
     Q4_CUDA_TRY(cudaMemcpy2D(b->tokens, sizeof(int) * (b->max_len + 1), prompts, sizeof(int) * n_prompt, sizeof(int) * n_prompt, b->n_seq, cudaMemcpyHostToDevice));
     Q4_CUDA_TRY(cudaMemset(b->pos, 0, sizeof(int) * b->n_seq));
+    // The copies and fills run on the default stream, which a caller's non-blocking stream does not wait for: a step queued right away
+    // read the positions of the run before.
+    Q4_CUDA_TRY(cudaDeviceSynchronize());
     if (b->step_graph && n_prompt != b->n_prompt) {   // the prompt length is an argument of the captured hand-off kernel
         cudaGraphExecDestroy(b->step_graph);
         b->step_graph = nullptr;
