@@ -6,8 +6,8 @@
 // kernel is built for; the tcgen05 GEMM (q4_gemm.cu) takes over from M > 16, where the contraction starts to matter.
 //
 // Work split: a unit is 16 * MT output features of one launch over the whole K axis; one persistent CTA (12 warps; 8 for
-// 9-16 rows) per SM walks the units; warp w takes the w-th share of a unit's 128-input groups, and the warps' partial
-// tiles are summed in warp order through shared memory (fixed order: results are bit-reproducible). Inside a warp the product runs on mma.sync m16n8k16 (fp16 in, fp32 out) with
+// 9-16 rows) per SM walks the units; in unit u warp w takes share (w + u) % warps of the 128-input groups, and the shares' partial
+// tiles are summed in the order of the shares through shared memory (fixed order: results are bit-reproducible). Inside a warp the product runs on mma.sync m16n8k16 (fp16 in, fp32 out) with
 // the weights as the 16-row operand and the batch as the 8-column one. The k index of an MMA is only a summation
 // label, so the packed words are used as they lie in the file: thread (g, t) of the warp loads 16 bytes = 32 inputs of
 // feature rows g and g + 8 at input offset 32 t of the group, unpacks a word into the half2 pairs (q0,q4) (q1,q5)
@@ -73,6 +73,8 @@ __device__ __forceinline__ void unpack8(uint32_t w, uint32_t zlo, uint32_t zhi, 
 #endif
 // warps of a CTA = K slices of a unit
 __host__ __device__ constexpr int warps_of(int MT, int NT) { return NT == 2 ? 8 : SK_WARPS; }   // (16 batch rows need the registers of 8-warp CTAs)
+// Units whose partial tiles wait in shared memory for one sum: all of a CTA's for the 7B shapes, and what L1 keeps is still enough for x.
+__host__ __device__ constexpr int units_at_once(int MT, int NT) { return NT == 2 ? 4 : 6; }
 
 // MT: 16-feature tiles per unit (1 or 2); NT: 8-row batch tiles (1: M <= 8, 2: M <= 16); SILU: tile 0 = gate, tile 1 = up.
 // Persistent: one CTA per SM walks units blockIdx.x, blockIdx.x + gridDim.x, ...; a warp's weight loads run D groups ahead
@@ -84,14 +86,34 @@ template <int MT, int NT, bool SILU>
 __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(const SkParams p) {
     constexpr int kWarps = warps_of(MT, NT);
     extern __shared__ float red_raw[];
-    float (*red)[kWarps][MT][NT][4][32] = reinterpret_cast<float (*)[kWarps][MT][NT][4][32]>(red_raw);   // [2]: double buffered by unit parity
+    constexpr int kUnits = units_at_once(MT, NT);
+    float (*red)[kWarps][MT][NT][4][32] = reinterpret_cast<float (*)[kWarps][MT][NT][4][32]>(red_raw);   // [unit % kUnits][share]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int units = SILU ? p.total_tiles : p.total_tiles / MT;
     const int my_units = blockIdx.x < units ? (units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    // this warp's groups of every unit
-    const int g_begin = (int)((long long)p.G * warp / kWarps), g_end = (int)((long long)p.G * (warp + 1) / kWarps);
-    const int gpw = g_end - g_begin;
-    const int total = my_units * gpw;   // (unit, group) steps of this warp, unit-major
+    // This warp's steps (unit, group), unit by unit. The shares of a unit differ by one group (32 groups over 12 warps are 2 or 3) and go
+    // round the warps from unit to unit; with a fixed share per warp and a barrier per unit all waited for those with three.
+    struct Cursor {
+        int u, share, g, g_end;
+        __device__ __forceinline__ void settle(int G, int n) {   // to the first unit from u on in which the share has a group
+            g = G * share / kWarps;
+            g_end = G * (share + 1) / kWarps;
+            while (g == g_end && u < n) {
+                u++;
+                share = share + 1 == kWarps ? 0 : share + 1;
+                g = G * share / kWarps;
+                g_end = G * (share + 1) / kWarps;
+            }
+        }
+        __device__ __forceinline__ void next(int G, int n) {
+            if (++g < g_end) return;
+            u++;
+            share = share + 1 == kWarps ? 0 : share + 1;
+            settle(G, n);
+        }
+    };
+    Cursor cur = {0, warp, 0, 0};
+    cur.settle(p.G, my_units);
 
     // rows of unit u: tile mt holds features f0 .. f0 + 15 of matrix mi
     auto unit_tile = [&](int u, int mt, int& mi, int& f0) {
@@ -118,9 +140,8 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
         __half sc[MT][2];
     };
     Stage st[D];
-    // prefetch cursor: step index, its unit, its group within the warp's slice, and the unit's row pointers (row g of each
-    // tile; row g + 8 lies 8 rows further)
-    int pf = 0, pf_u = 0, pf_gi = 0;
+    // prefetch cursor, and its unit's row pointers (row g of each tile; row g + 8 lies 8 rows further)
+    Cursor pf = cur;
     const uint4* pw[MT];
     const uint32_t* pz[MT];
     const __half* ps[MT];
@@ -136,8 +157,8 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
         }
     };
     auto prefetch = [&](Stage& d) {
-        if (pf < total) {
-            const int grp = g_begin + pf_gi;
+        if (pf.u < my_units) {
+            const int grp = pf.g, u = pf.u;
 #pragma unroll
             for (int mt = 0; mt < MT; mt++)
 #pragma unroll
@@ -146,15 +167,11 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
                     d.zw[mt][hh] = __ldg(pz[mt] + hh * 8 * p.PZ + (grp >> 3));
                     d.sc[mt][hh] = __ldg(ps[mt] + hh * 8 * p.G + grp);
                 }
-            pf++;
-            if (++pf_gi == gpw) {
-                pf_gi = 0;
-                pf_u++;
-                if (pf < total) set_rows(pf_u);
-            }
+            pf.next(p.G, my_units);
+            if (pf.u != u && pf.u < my_units) set_rows(pf.u);
         }
     };
-    if (total > 0) set_rows(0);
+    if (pf.u < my_units) set_rows(pf.u);
 #pragma unroll
     for (int d = 0; d < D; d++) prefetch(st[d]);
     griddep_wait();
@@ -188,21 +205,22 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
     };
     clear_acc();
 
-    // End of unit u for this warp: its K slice goes to shared memory; after the CTA barrier the first NT * 4 warps add the
-    // kWarps slices in warp order (fixed order: bit-reproducible), apply the epilogue and store, while the others move on.
+    // End of unit u for this warp: its share's partial tile goes to shared memory. The sums of up to kUnits units are taken together:
+    // no barrier on the way (with one per unit, eight rows of 70B gate/up 84.1 us, 77.5 so; 13B 25.6, 23.4).
     auto unit_end = [&](int u) {
-        const int par = u & 1;
+        const int share = (warp + u) % kWarps, last = u % kUnits;
 #pragma unroll
         for (int mt = 0; mt < MT; mt++)
 #pragma unroll
             for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) red[par][warp][mt][nt][e][lane] = acc[mt][nt][e];
+                for (int e = 0; e < 4; e++) red[last][share][mt][nt][e][lane] = acc[mt][nt][e];
         clear_acc();
+        if (last + 1 < kUnits && u + 1 < my_units) return;
         __syncthreads();
         // thread = (nt, e, lane): element (feature f0 + g + 8 (e >> 1), batch row 8 nt + 2 t + (e & 1)) of every tile
-        for (int i = threadIdx.x; i < NT * 4 * 32; i += kWarps * 32) {
-            const int l = i & 31, e = (i >> 5) & 3, nt = i >> 7;
+        for (int i = threadIdx.x; i < (last + 1) * NT * 4 * 32; i += kWarps * 32) {
+            const int l = i & 31, e = (i >> 5) & 3, nt = (i >> 7) % NT, par = (i >> 7) / NT, u0 = u - last + par;
             const int row = 8 * nt + 2 * (l & 3) + (e & 1);
             float v[MT];
 #pragma unroll
@@ -215,7 +233,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
             if (row >= p.M) continue;
             if (SILU) {
                 int mi, f0;
-                unit_tile(u, 0, mi, f0);
+                unit_tile(u0, 0, mi, f0);
                 float val = v[0];
                 val *= 1.0f / (1.0f + expf(-val));
                 val *= v[MT - 1];
@@ -224,7 +242,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
 #pragma unroll
                 for (int mt = 0; mt < MT; mt++) {
                     int mi, f0;
-                    unit_tile(u, mt, mi, f0);
+                    unit_tile(u0, mt, mi, f0);
                     const SkMat& mm = p.m[mi];
                     const size_t at = (size_t)row * mm.ldy + f0 + (l >> 2) + 8 * (e >> 1);
                     float val = v[mt];
@@ -233,46 +251,41 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
                 }
             }
         }
-        // the buffer of parity `par` is written again at unit u + 2, after every thread has passed the barrier of unit u + 1,
-        // which the threads that read it here reach only when they are done
+        if (u + 1 < my_units) __syncthreads();   // the buffers are written again
     };
 
-    if (gpw == 0) {   // fewer groups than warps: this warp only takes part in the reductions
-        for (int u = 0; u < my_units; u++) unit_end(u);
-        return;
-    }
-    int u = 0, gi = 0;
-    load_x(g_begin);
-    for (int base = 0; base < total; base += D) {
+    for (int u = 0; u < cur.u; u++) unit_end(u);   // (fewer groups than warps: units in which this one has none)
+    if (cur.u < my_units) load_x(cur.g);
+    while (cur.u < my_units) {
 #pragma unroll
         for (int d = 0; d < D; d++) {
-            if (base + d >= total) break;
-            const int grp = g_begin + gi;
+            if (cur.u >= my_units) break;
+            const int grp = cur.g, u = cur.u;
+            cur.next(p.G, my_units);
             // this step's x pairs in the unpack's order; the next step's x leaves now
             uint32_t xp[NT][4][4];
 #pragma unroll
             for (int nt = 0; nt < NT; nt++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) permute_x8(xn[nt][j], xp[nt][j]);
-            const int gi_next = gi + 1 == gpw ? 0 : gi + 1;
-            if (base + d + 1 < total) load_x(g_begin + gi_next);
-            const Stage& cur = st[d];
+            if (cur.u < my_units) load_x(cur.g);
+            const Stage& now = st[d];
 #pragma unroll
             for (int mt = 0; mt < MT; mt++) {
                 uint32_t zlo[2], zhi[2];
                 float sc[2];
 #pragma unroll
                 for (int hh = 0; hh < 2; hh++) {
-                    const uint32_t z = (cur.zw[mt][hh] >> (4 * (grp & 7))) & 0xFu;
+                    const uint32_t z = (now.zw[mt][hh] >> (4 * (grp & 7))) & 0xFu;
                     zlo[hh] = (0x6400u | z) * 0x00010001u;          // 1024 + z
                     zhi[hh] = (0x5400u | (z << 4)) * 0x00010001u;   // 64 + z
-                    sc[hh] = __half2float(cur.sc[mt][hh]);
+                    sc[hh] = __half2float(now.sc[mt][hh]);
                 }
                 float c[NT][4];
 #pragma unroll
                 for (int nt = 0; nt < NT; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
-                const uint32_t wa[4] = {cur.w[mt][0].x, cur.w[mt][0].y, cur.w[mt][0].z, cur.w[mt][0].w};
-                const uint32_t wb[4] = {cur.w[mt][1].x, cur.w[mt][1].y, cur.w[mt][1].z, cur.w[mt][1].w};
+                const uint32_t wa[4] = {now.w[mt][0].x, now.w[mt][0].y, now.w[mt][0].z, now.w[mt][0].w};
+                const uint32_t wb[4] = {now.w[mt][1].x, now.w[mt][1].y, now.w[mt][1].z, now.w[mt][1].w};
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     uint32_t da[4], db[4];
@@ -293,18 +306,14 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
                 }
             }
             prefetch(st[d]);   // the stage is spent: its next occupant, D steps ahead, leaves now
-            if (++gi == gpw) {
-                unit_end(u);
-                gi = 0;
-                u++;
-            }
+            for (int e = u; e < cur.u; e++) unit_end(e);
         }
     }
     if (p.late) griddep_launch_dependents();
 }
 
 constexpr int kSms = 148;   // B200: one persistent CTA per SM (a smaller part would only leave CTAs queued behind the first wave)
-constexpr size_t red_bytes(int MT, int NT) { return 2 * (size_t)warps_of(MT, NT) * MT * NT * 4 * 32 * sizeof(float); }
+constexpr size_t unit_bytes(int MT, int NT) { return (size_t)warps_of(MT, NT) * MT * NT * 4 * 32 * sizeof(float); }
 
 int fill(SkParams& p, const uint16_t* x, int M, int K) {
     if (!x || M < 1 || M > 16) return Q4_ERR_INVALID;
@@ -331,9 +340,12 @@ SkMat sk_mat(const q4_qweight* w, uint16_t* y, int ldy, int tile0) {
 
 template <int MT, int NT, bool SILU>
 int launch_variant(const SkParams& p, cudaStream_t s) {
-    constexpr size_t smem = red_bytes(MT, NT);
-    static_assert(smem <= 48 * 1024, "the reduction buffers fit the default dynamic shared memory limit: no per-device opt-in is needed");
-    const int units = SILU ? p.total_tiles : p.total_tiles / MT;
+    const int units = SILU ? p.total_tiles : p.total_tiles / MT, per_cta = q4_div_up(units, kSms);
+    constexpr int kUnits = units_at_once(MT, NT);
+    // (the limit belongs to the function: always the largest any launch needs)
+    if (kUnits * unit_bytes(MT, NT) > 48 * 1024)
+        Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kUnits * unit_bytes(MT, NT))));
+    const size_t smem = (per_cta < kUnits ? per_cta : kUnits) * unit_bytes(MT, NT);
     Q4Launch L(dim3(units < kSms ? units : kSms), dim3(warps_of(MT, NT) * 32), smem, s);
     Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_skinny_kernel<MT, NT, SILU>, p));
     return Q4_OK;
