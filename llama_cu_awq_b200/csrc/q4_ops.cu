@@ -173,6 +173,8 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const __half* __restrict__
     __shared__ int sidx[32];
     griddep_wait();
     griddep_launch_dependents();
+    int token_pos = 0;
+    if (threadIdx.x == 0) token_pos = *pPos;   // (host memory: read at the hand-off the kernel ended two microseconds later)
     float best = -CUDART_INF_F;
     int bi = 0x7fffffff;
     for (int i = threadIdx.x; i < size; i += blockDim.x) {
@@ -200,7 +202,6 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const __half* __restrict__
             if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
         }
         if (lane == 0) {
-            int token_pos = *pPos;
             token_pos++;
             if (write_token) result[token_pos] = (bi == 0x7fffffff) ? 0 : bi;
             *pPos = token_pos;

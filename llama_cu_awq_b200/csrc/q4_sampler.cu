@@ -74,16 +74,29 @@ sample_topp_kernel(__half* __restrict__ logits, int n, float temperature, float 
     griddep_wait();
     griddep_launch_dependents();
 
+    int token_pos = 0;
+    if (rank == 0 && t == 0) token_pos = *pPos;   // (host memory: read at the hand-off the kernel ended two microseconds later)
+
     // ---- softmax with temperature (softmax_logits_kernel) ----
     float mx = -CUDART_INF_F;
-    for (int j = row0; j < rows; j += kRowsAtOnce) {
-        const int i = j * kT + i_col;
-        if (i < n) {
-            float val = __half2float(logits[i]);
-            val /= temperature;
-            const __half hv = __float2half(val);
-            s_key[j * kCols + col] = __half_as_ushort(hv);
-            mx = fmaxf(mx, __half2float(hv));
+    constexpr int U = 4;   // elements of a thread in flight
+    for (int j0 = row0; j0 < rows; j0 += U * kRowsAtOnce) {
+        __half in[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = (j0 + u * kRowsAtOnce) * kT + i_col;
+            in[u] = i < n ? logits[i] : __half();
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int j = j0 + u * kRowsAtOnce;
+            if (j * kT + i_col < n) {
+                float val = __half2float(in[u]);
+                val /= temperature;
+                const __half hv = __float2half(val);
+                s_key[j * kCols + col] = __half_as_ushort(hv);
+                mx = fmaxf(mx, __half2float(hv));
+            }
         }
     }
     for (int i = t; i < 256; i += kT) s_hist2[i] = 0;
@@ -269,7 +282,6 @@ sample_topp_kernel(__half* __restrict__ logits, int n, float temperature, float 
         cluster.sync();   // CTA 0 reads the others' shared memory until here
     }
     if (rank == 0 && t == 0) {   // hand-off as in sample_top_p_kernel (gpu_kernels.h:583-591)
-        int token_pos = *pPos;
         token_pos++;
         result[token_pos] = token;
         *pPos = token_pos;

@@ -88,6 +88,25 @@ def test_ffn_silu_rows(M, K, N):
         assert_close(got[m], O.ffn_silu(x[m], gate, up, K, N, order=1), f"row {m}", max_rel=2e-3)
 
 
+# fewer groups than warps, one unit per CTA and several, more units than are summed at once (seven and thirteen)
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("kind,K,N", [(0, 1408, 4112), (0, 256, 31104), (1, 256, 28672), (1, 1664, 14336)])
+def test_units_that_are_summed_together(M, kind, K, N):
+    rng = np.random.default_rng(M + K + N + kind)
+    qs = [synth.synth_qweight(rng, K, N) for _ in range(1 + kind)]
+    W = [ops.QWeight.from_numpy(q) for q in qs]
+    x = _x(rng, M, K)
+    y = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    g, *u = (x.astype(np.float64) @ O.dequant(q, K, N).astype(np.float64).T for q in qs)
+    if kind == 0:
+        ops.matmul_rows(y, torch.from_numpy(x).cuda(), W[0], M, K, N)
+    else:
+        ops.ffn_silu_rows(y, torch.from_numpy(x).cuda(), *W, M, K, N)
+        g = g / (1 + np.exp(-g)) * u[0]
+    torch.cuda.synchronize()
+    assert_close(y.cpu().numpy(), g, "vs f64", max_rel=2e-3)
+
+
 def test_rejects_unsupported_arguments():
     rng = np.random.default_rng(0)
     q = synth.synth_qweight(rng, 128, 16)
