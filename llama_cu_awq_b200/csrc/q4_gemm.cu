@@ -625,49 +625,54 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
             if (finish) {
                 __threadfence();
-                // the first two stored partials of the next 32 columns are requested before the current ones are staged: a
-                // round trip to L2 per 32 columns and partial, one after the other, took 30 us for a 256-row tile in four parts
-                const int m0 = own_in_tmem && pair == first ? first + 1 : first;
-                const int m1 = own_in_tmem && pair == m0 + 1 ? m0 + 2 : m0 + 1;
-                float4 n0[8], n1[8];
-                auto fetch = [&](float4 (&v)[8], int pr, int c0) {
-                    const float4* part = partial_of(pr, pr == first) + (size_t)(c0 / 4) * kBN;
+                // Pieces (32 columns of one stored part) in the order they are added, two requested ahead of the sum whichever part they belong
+                // to. With the next columns of the first two parts ahead the third and fourth were a latency of L2 each: 64 x 11008 x
+                // 4096 in four parts 20.2 us, 18.2 so; 77 x 13824 x 5120 in three 25.5, 24.3. (Three or four ahead spill: no gain.)
+                const int others = last - first + (own_in_tmem ? 0 : 1);
+                constexpr int kAhead = 2;
+                float4 ring[kAhead][8];
+                float acc[32];
+                uint32_t rs[16], out[16];
+                int fetch_c = 0, fetch_j = 0, c0 = 0, j = 0;
+                auto fetch_next = [&](float4 (&v)[8]) {
+                    if (fetch_c >= MT) return;
+                    const int pr = first + fetch_j + (own_in_tmem && first + fetch_j >= pair ? 1 : 0);
+                    const float4* part = partial_of(pr, pr == first) + (size_t)(fetch_c / 4) * kBN;
 #pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = __ldcg(part + (size_t)j * kBN);
+                    for (int i = 0; i < 8; i++) v[i] = __ldcg(part + (size_t)i * kBN);
+                    if (++fetch_j == others) { fetch_j = 0; fetch_c += 32; }
                 };
-                fetch(n0, m0, 0);
-                if (m1 <= last) fetch(n1, m1, 0);
+                auto add_own = [&]() {
+                    uint32_t v[32];
+                    tc_ld32(t_lane + c0, v);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) acc[i] += __uint_as_float(v[i]);
+                };
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) fetch_next(ring[u]);
 #pragma unroll 1
-                for (int c0 = 0; c0 < MT; c0 += 32) {
-                    float acc[32];
-                    uint32_t rs[16], out[16];
-                    if (EPI == EPI_RESIDUAL) epi_load_residual(rs, res, c0, my_rows, ld);
+                while (c0 < MT) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) acc[j] = 0.f;
-                    auto add = [&](const float4 (&v)[8]) {
+                    for (int u = 0; u < kAhead; u++) {
+                        if (c0 >= MT) break;
+                        if (j == 0) {
+                            if (EPI == EPI_RESIDUAL) epi_load_residual(rs, res, c0, my_rows, ld);
 #pragma unroll
-                        for (int j = 0; j < 8; j++) { acc[4 * j] += v[j].x; acc[4 * j + 1] += v[j].y; acc[4 * j + 2] += v[j].z; acc[4 * j + 3] += v[j].w; }
-                    };
-                    for (int pr = first; pr <= last; pr++) {
-                        if (pr == m0) add(n0);
-                        else if (pr == m1) add(n1);
-                        else if (pr == pair && own_in_tmem) {
-                            uint32_t v[32];
-                            tc_ld32(t_lane + c0, v);
+                            for (int i = 0; i < 32; i++) acc[i] = 0.f;
+                            if (own_in_tmem && pair == first) add_own();
+                        }
 #pragma unroll
-                            for (int j = 0; j < 32; j++) acc[j] += __uint_as_float(v[j]);
-                        } else {
-                            float4 v[8];
-                            fetch(v, pr, c0);
-                            add(v);
+                        for (int i = 0; i < 8; i++) { acc[4 * i] += ring[u][i].x; acc[4 * i + 1] += ring[u][i].y; acc[4 * i + 2] += ring[u][i].z; acc[4 * i + 3] += ring[u][i].w; }
+                        fetch_next(ring[u]);
+                        j++;
+                        if (own_in_tmem && first + j == pair) add_own();   // its place in K order
+                        if (j == others) {
+                            epi_pack<EPI>(acc, rs, p.residual_scale, out);
+                            put(out, nt, mt * MT + c0, rows - c0);
+                            c0 += 32;
+                            j = 0;
                         }
                     }
-                    if (c0 + 32 < MT) {
-                        fetch(n0, m0, c0 + 32);
-                        if (m1 <= last) fetch(n1, m1, c0 + 32);
-                    }
-                    epi_pack<EPI>(acc, rs, p.residual_scale, out);
-                    put(out, nt, mt * MT + c0, rows - c0);
                 }
                 if (own_in_tmem) release();
                 if (etid == 0) *counter = 0;   // ready for the next launch
@@ -750,12 +755,13 @@ struct GemmPlan { int MT, m_tiles, n_tiles, n_chunks, pairs, stages, np, slab; l
 // (K and N of the 7B, 13B and 70B projections, 24 to 512 rows) with all their tiles and 5 to 12 numbers of pairs each; the plan it
 // picks is within 1 % of the best of them on average. (Its predecessor, from clock stamps inside the kernel, took a partial
 // tile's reading for a fifth of what it costs and was 9 % off: 77 x 5120 x 5120 22.9 us, 16.9 so; 128 x 8192 x 8192 30.3, 24.1.)
-//   chunk    a 256-input chunk: 4.9 ns per batch row on the tensor pipe, 0.7 us at least, whatever the rows (issue of its 16 MMAs,
+//   chunk    a 256-input chunk: 5 ns per batch row on the tensor pipe, 0.72 us at least, whatever the rows (issue of its 16 MMAs,
 //            conversion of its 128 x 256 weights)
-//   segment  each further tile that a share touches: its first copies and its turn at the accumulator
+//   segment  each further tile that a share touches: its turn at the accumulator
 //   drain    the last tile's output, which is not hidden by anything: 9 ns per row
 //   split    a tile cut by a share boundary: a partial tile written, counted and, by the last CTA, one read per other contributor at
-//            26 ns per row, which is why even shares of a whole fraction of a tile on 64 pairs beat 74 pairs
+//            9 ns per row and 0.25 us, which is why even shares of a whole fraction of a tile on 64 pairs often beat 74 pairs;
+//            shares that are no such fraction meet at other times
 // Rings: operand stages as tensor memory allows, the shared memory that their X slabs leave for packed weights (at few rows
 // the kernel is a weight stream: ten 16 KB copies in flight per SM cover HBM's latency).
 GemmPlan make_plan(int M, int K, int N, int sms) {
@@ -771,15 +777,15 @@ GemmPlan make_plan(int M, int K, int N, int sms) {
         last_mt = mt;
         const int mtl = q4_div_up(M, mt);
         const long long total = (long long)g.n_tiles * mtl * g.n_chunks;
-        const double t_chunk = 0.0049 * mt > 0.7 ? 0.0049 * mt : 0.7;
+        const double t_chunk = 0.005 * mt > 0.72 ? 0.005 * mt : 0.72;
         for (int P = (int)(total < max_pairs ? total : max_pairs); P >= 1; P--) {
             const long long share = (total + P - 1) / P;
             if (share * t_chunk >= best) break;   // fewer pairs only take longer from here on
             const bool even = total % P == 0, whole = even && share % g.n_chunks == 0, aligned = even && g.n_chunks % share == 0;
-            double cost = share * t_chunk + 0.009 * mt + 0.75 * (q4_div_up((int)share, g.n_chunks) - (whole || aligned ? 1 : 0));
+            double cost = share * t_chunk + 0.009 * mt + 0.4 * (q4_div_up((int)share, g.n_chunks) - (whole || aligned ? 1 : 0));
             if (!whole) {   // contributors of a tile, at most
                 const long long parts = aligned ? g.n_chunks / share : share >= g.n_chunks ? 2 : (g.n_chunks - 2) / share + 2;
-                cost += 0.8 + (parts - 1) * 0.026 * mt;
+                cost += 1.2 + 0.015 * mt + (parts - 1) * (0.25 + 0.009 * mt) + (aligned ? 0.0 : 0.8);
             }
             if (cost < best) { best = cost; g.pairs = P; g.MT = mt; g.m_tiles = mtl; g.total = total; }
         }
