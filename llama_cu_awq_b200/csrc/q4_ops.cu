@@ -177,7 +177,27 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const __half* __restrict__
     if (threadIdx.x == 0) token_pos = *pPos;   // (host memory: read at the hand-off the kernel ended two microseconds later)
     float best = -CUDART_INF_F;
     int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < size; i += blockDim.x) {
+    // eight words per load, four loads in flight (32000 words two bytes at a time: 7.9 us back to back, 2.7 so)
+    constexpr int U = 4;
+    const int nvec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? size / 8 : 0;
+    for (int i0 = threadIdx.x; i0 < nvec; i0 += U * blockDim.x) {
+        uint4 in[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i0 + u * (int)blockDim.x < nvec) in[u] = reinterpret_cast<const uint4*>(x)[i0 + u * blockDim.x];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = i0 + u * blockDim.x;
+            if (i >= nvec) break;
+            const __half* h = reinterpret_cast<const __half*>(&in[u]);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float v = __half2float(h[j]);
+                if (v > best) { best = v; bi = 8 * i + j; }
+            }
+        }
+    }
+    for (int i = nvec * 8 + threadIdx.x; i < size; i += blockDim.x) {
         const float v = __half2float(x[i]);
         if (v > best) { best = v; bi = i; }
     }

@@ -202,3 +202,26 @@ def test_argmax_matches_oracle(size):
         ops.sample_greedy(dev(logits), size, mb.data_ptr() + 16, mb.data_ptr(), pos_dev, True)
         torch.cuda.synchronize()
         assert int(mb[4 + 1]) == O.argmax(logits)
+
+
+# one load per thread and several, remainders behind the last eight, logits that do not start on 16 bytes
+@pytest.mark.parametrize("size", [1, 7, 8, 9, 8191, 8200, 32771, 70003])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_argmax_ties_and_remainders(size, shift):
+    rng = np.random.default_rng(size)
+    base = rng.standard_normal(size).astype(np.float16)
+    cases = [(base, None), (np.full(size, -np.inf, np.float16), 0), (np.full(size, np.nan, np.float16), 0)]
+    for a, b in ((0, size - 1), (size // 2, size - 1), (size // 3, size // 3)):     # the lowest of two equal maxima
+        v = base.copy()
+        v[[a, b]] = 9.0
+        v[max(a - 1, 0):a] = np.nan                                                 # a NaN in front does not win
+        cases.append((v, a))
+    for v, want in cases:
+        buf = torch.empty(size + 8, dtype=torch.float16, device="cuda")
+        x = buf[shift:shift + size]
+        x.copy_(torch.from_numpy(v))
+        mb = _pinned_mailbox()
+        pos_dev = torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.sample_greedy(x, size, mb.data_ptr() + 16, mb.data_ptr(), pos_dev, True)
+        torch.cuda.synchronize()
+        assert int(mb[4 + 1]) == (int(np.argmax(v)) if want is None else want)
