@@ -108,7 +108,8 @@ int q4_rope(void* stream, uint16_t* q, uint16_t* k, int num_heads, int num_kv_he
 /* MultiHeadAttention(): llama2_q4.cu:410-427, kernels gpu_kernels.h:150-176,365-454,287-337.
  * One query per head over cache rows 0..*pPos; key_cache/value_cache already point at the layer; the row
  * stride is num_heads*head_size/kv_mul halfs. `scratch` replaces the reference's `att` buffer and must hold
- * q4_attention_scratch_bytes(num_heads, head_size) bytes; it carries the per-split partial results. */
+ * q4_attention_scratch_bytes(num_heads, head_size) bytes; a call does not read or write it (the blocks of a head exchange
+ * their parts through shared memory). */
 size_t q4_attention_scratch_bytes(int num_heads, int head_size);
 int q4_attention(void* stream, uint16_t* output, const uint16_t* q, const uint16_t* key_cache,
                  const uint16_t* value_cache, void* scratch, int num_heads, int head_size, int kv_mul, int max_seq_len,
@@ -117,15 +118,8 @@ int q4_attention(void* stream, uint16_t* output, const uint16_t* q, const uint16
 /* Same computation as q4_attention for callers that cannot provide the scratch buffer because they may not
  * allocate device memory: hosts whose device memory is completely handed out at start-up, or plugins that only
  * receive the owning runtime's pointers. No counterpart in the reference (its `att` buffer is allocated by
- * malloc_run_state). The partial results go to an array of Q4_ATTENTION_STATIC_MAX_BYTES that is part of the
- * library's device image (every GPU that loads the library holds it until the process exits); shapes that need
- * more (q4_attention_scratch_bytes) are refused with Q4_ERR_LIMIT. The call allocates and frees nothing.
- * The first call on each device looks the array's device address up (cudaGetSymbolAddress); make that first call
- * outside of any stream capture. All calls share the one array: two calls that overlap on the GPU (different
- * streams) race; calls on one stream are safe. Nothing has to be cleared between calls: each call overwrites
- * every word it later reads. The array's address is remembered per CUDA device ordinal of the calling thread's
- * current device, which must be the device `stream` belongs to; the remembered address does not survive
- * cudaDeviceReset() (do not call this entry point again in a process that has reset the device). */
+ * malloc_run_state). Shapes whose q4_attention_scratch_bytes exceed Q4_ATTENTION_STATIC_MAX_BYTES are refused with
+ * Q4_ERR_LIMIT. The call allocates and frees nothing and keeps nothing between calls: calls on different streams may overlap. */
 #define Q4_ATTENTION_STATIC_MAX_BYTES (256 * 1024)
 int q4_attention_static(void* stream, uint16_t* output, const uint16_t* q, const uint16_t* key_cache,
                         const uint16_t* value_cache, int num_heads, int head_size, int kv_mul, int max_seq_len,

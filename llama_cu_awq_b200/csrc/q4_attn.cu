@@ -6,18 +6,15 @@
 // A block takes positions [t0, t1) of one head. Eight lanes share a position (8 dims of every 64: a load of theirs is 128 bytes in a row), a block of
 // eight warps has 64 positions in hand per step and the next 64 requested. Scores are rounded to fp16 like the reference's; the
 // softmax runs online in fp32 (running max, sum and un-normalised V accumulator per lane group), merged across the block in registers
-// and shared memory. Then, by the number of heads:
-//   16 or more  one launch: a head's blocks are a thread-block cluster and read one another's (max, sum, acc) from shared memory
-//   fewer       two launches: up to 32 blocks per head leave (max, sum, acc) in scratch, a block per head merges them and writes fp16.
-//               (a cluster has at most eight blocks: eight heads would keep 64 of 148 SMs)
-// What bounds it is latency: 32 heads at position 600 are 10 MB. Before (16 positions in hand per block, none requested ahead, always
-// two launches): 333 tokens behind 700 of one 70B layer (its last row) 238 -> 227 us, two 7B layers call by call at position 600 133 -> 120 us.
+// and shared memory. A head's blocks are a thread-block cluster and read one another's (max, sum, acc) from shared memory: one launch, no
+// scratch. What bounds it is latency: 32 heads at position 600 are 10 MB. Before (16 positions in hand per block, none requested
+// ahead, up to 32 blocks per head and a second launch that merged them through global memory), back to back at positions 60, 600, 1900
+// and 3800: 4 heads 8.2, 12.2, 13.6, 15.5 us, now 3.5, 4.2, 5.5, 7.7; 32 heads 8.0, 10.1, 24.3, 40.5, now 4.2, 5.3, 9.9, 15.2; 64 heads in
+// groups of 8 6.8, 11.0, 19.6, 61.6, now 4.2, 6.1, 10.4, 18.7. Two 7B layers call by call at position 600 133 -> 120 us.
 // The sequence length comes from *pPos on the device; the grid does not depend on it.
 #include <math_constants.h>
 
 #include <stdio.h>
-
-#include <mutex>
 
 #include "q4_common.cuh"
 
@@ -26,16 +23,22 @@ namespace {
 constexpr int kAttnThreads = 256, kAttnWarps = kAttnThreads / 32;
 constexpr int kGroups = kAttnThreads / 8;  // lane groups of a block; each has two positions in hand
 constexpr int kMaxHeadSize = 256;
-constexpr int kClusterHeads = 16;          // from so many heads on a head's blocks are a cluster
 
+// Blocks of a head's cluster: the most that leaves two blocks per SM over all heads, which is what fits at once (positions 60, 600, 1900
+// and 3800: 32 heads 4.2, 5.3, 9.9, 15.2 us with eight and 3.7, 5.2, 12.2, 19.9 with four; 40 heads 7.2, 9.4, 16.7, 26.1 with eight and
+// 4.1, 6.4, 13.5, 21.8 with four; 96 heads 7.1, 14.1, 26.4, 44.3 with four and 4.3, 10.1, 22.3, 40.2 with two).
+int attn_cluster(int num_heads) {
+    int blocks = 8;
+    while (blocks > 1 && blocks * num_heads > 2 * 148) blocks /= 2;
+    return blocks;
+}
+// what a host's scratch was sized by when the blocks of a head exchanged their parts through it
 int attn_splits(int num_heads) {
     int s = q4_div_up(2 * 148, num_heads);
     if (s < 1) s = 1;
     if (s > 32) s = 32;
     return s;
 }
-// blocks of a head's cluster: about two to four per SM over all heads
-int attn_cluster(int num_heads) { return num_heads <= 64 ? 8 : num_heads <= 128 ? 4 : 2; }
 
 template <int HS>
 struct AttnShared {
@@ -207,43 +210,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_cluster_kernel(__half* outp
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int HS>
-__global__ void __launch_bounds__(kAttnThreads) attn_partial_kernel(float* scratch, const __half* q, const __half* kc, const __half* vc,
-                                                                    int kv_mul, int kv_stride, const int* pPos) {
-    __shared__ __align__(16) AttnShared<HS> sm;
-    const int h = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x;
-    griddep_wait();
-    griddep_launch_dependents();
-    attn_share<HS>(sm, q, kc, vc, kv_mul, kv_stride, pPos, h, split, nsplit);
-    __syncthreads();
-    float* out = scratch + ((size_t)h * nsplit + split) * (HS + 2);
-    if (threadIdx.x == 0) {
-        out[0] = sm.M;
-        out[1] = sm.L;
-    }
-    if (threadIdx.x < HS) out[2 + threadIdx.x] = sm.out[threadIdx.x];
-}
-
-__global__ void attn_merge_kernel(__half* output, const float* scratch, int nsplit, int head_size) {
-    griddep_wait();
-    griddep_launch_dependents();
-    const int h = blockIdx.x;
-    const float* base = scratch + (size_t)h * nsplit * (head_size + 2);
-    float M = -CUDART_INF_F;
-    for (int s = 0; s < nsplit; s++) M = fmaxf(M, base[(size_t)s * (head_size + 2)]);
-    auto weight = [&](int s) {
-        const float* p = base + (size_t)s * (head_size + 2);
-        return p[1] == 0.f ? 0.f : expf(p[0] - (M == -CUDART_INF_F ? 0.f : M));
-    };
-    float L = 0.f;
-    for (int s = 0; s < nsplit; s++) L += base[(size_t)s * (head_size + 2) + 1] * weight(s);
-    for (int d = threadIdx.x; d < head_size; d += blockDim.x) {
-        float a = 0.f;
-        for (int s = 0; s < nsplit; s++) a += base[(size_t)s * (head_size + 2) + 2 + d] * weight(s);
-        output[(size_t)h * head_size + d] = __float2half(a / L);
-    }
-}
-
 }  // namespace
 
 extern "C" size_t q4_attention_scratch_bytes(int num_heads, int head_size) {
@@ -252,37 +218,27 @@ extern "C" size_t q4_attention_scratch_bytes(int num_heads, int head_size) {
 }
 
 template <int HS>
-static int attention_launch(cudaStream_t s, __half* output, const __half* q, const __half* kc, const __half* vc, float* scratch, int num_heads, int kv_mul, const int* pPos) {
-    const int kv_stride = num_heads * HS / kv_mul;
-    if (num_heads >= kClusterHeads) {
-        const int blocks = attn_cluster(num_heads);
-        Q4Launch L(dim3(blocks, num_heads), dim3(kAttnThreads), 0, s);
-        cudaLaunchAttribute attr[2] = {L.attr[0], {}};
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = blocks;
-        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-        L.cfg.attrs = attr;
-        L.cfg.numAttrs = 2;
-        Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_cluster_kernel<HS>, output, q, kc, vc, kv_mul, kv_stride, pPos));
-        return Q4_OK;
-    }
-    const int nsplit = attn_splits(num_heads);
-    Q4Launch L(dim3(nsplit, num_heads), dim3(kAttnThreads), 0, s);
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_partial_kernel<HS>, scratch, q, kc, vc, kv_mul, kv_stride, pPos));
-    Q4Launch L2(dim3(num_heads), dim3(HS < 128 ? 64 : 128), 0, s);
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L2.cfg, attn_merge_kernel, output, (const float*)scratch, nsplit, HS));
+static int attention_launch(cudaStream_t s, __half* output, const __half* q, const __half* kc, const __half* vc, int num_heads, int kv_mul, const int* pPos) {
+    const int blocks = attn_cluster(num_heads);
+    Q4Launch L(dim3(blocks, num_heads), dim3(kAttnThreads), 0, s);
+    cudaLaunchAttribute attr[2] = {L.attr[0], {}};
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = blocks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    L.cfg.attrs = attr;
+    L.cfg.numAttrs = 2;
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, attn_cluster_kernel<HS>, output, q, kc, vc, kv_mul, num_heads * HS / kv_mul, pPos));
     return Q4_OK;
 }
 
-// One or two launches (see the top); scratch is the caller's.
-static int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache,
-                        float* scratch, int num_heads, int head_size, int kv_mul, const int* pPos) {
+static int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache, int num_heads,
+                               int head_size, int kv_mul, const int* pPos) {
     __half* out = (__half*)output;
     const __half *qh = (const __half*)q, *kc = (const __half*)key_cache, *vc = (const __half*)value_cache;
     switch (head_size) {
-        case 64: return attention_launch<64>(s, out, qh, kc, vc, scratch, num_heads, kv_mul, pPos);
-        case 128: return attention_launch<128>(s, out, qh, kc, vc, scratch, num_heads, kv_mul, pPos);
-        case 256: return attention_launch<256>(s, out, qh, kc, vc, scratch, num_heads, kv_mul, pPos);
+        case 64: return attention_launch<64>(s, out, qh, kc, vc, num_heads, kv_mul, pPos);
+        case 128: return attention_launch<128>(s, out, qh, kc, vc, num_heads, kv_mul, pPos);
+        case 256: return attention_launch<256>(s, out, qh, kc, vc, num_heads, kv_mul, pPos);
         default: return Q4_ERR_UNSUPPORTED_SIZE;
     }
 }
@@ -293,40 +249,12 @@ extern "C" int q4_attention(void* stream, uint16_t* output, const uint16_t* q, c
     if (!output || !q || !key_cache || !value_cache || !scratch || !pPos || num_heads <= 0 || kv_mul <= 0 || num_heads % kv_mul)
         return Q4_ERR_INVALID;
     if (head_size > kMaxHeadSize) return Q4_ERR_UNSUPPORTED_SIZE;
-    return q4_attention_launch((cudaStream_t)stream, output, q, key_cache, value_cache, (float*)scratch, num_heads, head_size, kv_mul, pPos);
+    return q4_attention_launch((cudaStream_t)stream, output, q, key_cache, value_cache, num_heads, head_size, kv_mul, pPos);
 }
 
-// ------------------------------------------------------------------------------------------------------------
-// Attention without a caller-provided scratch buffer.
-//
-// Some hosts of this library hand it nothing but the reference's own buffers and may not allocate device memory
-// themselves: a serving process whose device memory is fully committed to weights and KV cache at start-up (the
-// reference allocates everything once, in malloc_run_state), or a plugin that only receives raw pointers from
-// the runtime that owns the memory. For them the split partial results live in a fixed array inside the
-// library's own device image instead. Every GPU that loads the library carries the array until the process ends.
-// ------------------------------------------------------------------------------------------------------------
-static __device__ __align__(256) unsigned char g_attention_static_scratch[Q4_ATTENTION_STATIC_MAX_BYTES];
-
-namespace {
-constexpr int kMaxDevices = 64;
-std::mutex g_static_mu;
-float* g_static_ptr[kMaxDevices];  // device address of the array, per device (the symbol itself is not an address on the host)
-
-int static_scratch(float** out) {
-    int dev = 0;
-    Q4_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices) return Q4_ERR_LIMIT;
-    std::lock_guard<std::mutex> lk(g_static_mu);
-    if (!g_static_ptr[dev]) {
-        void* p = nullptr;
-        Q4_CUDA_TRY(cudaGetSymbolAddress(&p, g_attention_static_scratch));
-        g_static_ptr[dev] = reinterpret_cast<float*>(p);
-    }
-    *out = g_static_ptr[dev];
-    return Q4_OK;
-}
-}  // namespace
-
+// The same for hosts that hand this library nothing but the reference's own buffers and may not allocate device memory themselves (a
+// serving process whose device memory is fully committed at start-up, a plugin that only receives raw pointers). The limit is that of
+// the array inside the library that held the partial results.
 extern "C" int q4_attention_static(void* stream, uint16_t* output, const uint16_t* q, const uint16_t* key_cache,
                                    const uint16_t* value_cache, int num_heads, int head_size, int kv_mul, int max_seq_len, const int* pPos) {
     (void)max_seq_len;
@@ -337,7 +265,5 @@ extern "C" int q4_attention_static(void* stream, uint16_t* output, const uint16_
                 q4_attention_scratch_bytes(num_heads, head_size), Q4_ATTENTION_STATIC_MAX_BYTES);
         return Q4_ERR_LIMIT;
     }
-    float* scratch = nullptr;
-    if (int e = static_scratch(&scratch)) return e;
-    return q4_attention_launch((cudaStream_t)stream, output, q, key_cache, value_cache, scratch, num_heads, head_size, kv_mul, pPos);
+    return q4_attention_launch((cudaStream_t)stream, output, q, key_cache, value_cache, num_heads, head_size, kv_mul, pPos);
 }

@@ -247,6 +247,8 @@ static int model_build(q4_model** out, const q4_config& c, int rank, int gpu_cou
     m->shared = nullptr;
     m->status_word = nullptr;
     m->gen_stream = nullptr;
+    m->device = -1;
+    (void)cudaGetDevice(&m->device);
 
     // device arena for this rank's weights
     size_t need = 0;
@@ -433,7 +435,9 @@ extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int 
             if (prompt_tokens[i] < 0 || prompt_tokens[i] >= m->cfg.vocab_size) return Q4_ERR_INVALID;
     Q4_CUDA_TRY(cudaDeviceSynchronize());
     m->host_pos = pos;
-    const int* status = q4_fused_status_word(m);
+    int device = -1;
+    Q4_CUDA_TRY(cudaGetDevice(&device));
+    const int* status = device == m->device ? q4_fused_status_word(m) : nullptr;   // (copies reach the model from any device, a launch does not)
     *m->status_word = -1;
     if (status) {
         reset_kernel<<<1, 1>>>(m->pos, pos, status, m->status_word);
@@ -443,10 +447,8 @@ extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int 
     }
     m->shared->pos = pos;
     if (n > 0 && prompt_tokens) memcpy((void*)m->shared->tokens, prompt_tokens, sizeof(int) * (size_t)n);
-    if (status) {
-        Q4_CUDA_TRY(cudaDeviceSynchronize());
-        q4_fused_reset(m, *m->status_word == 0);
-    }
+    if (status) Q4_CUDA_TRY(cudaDeviceSynchronize());
+    q4_fused_reset(m, status && *m->status_word == 0);
     return Q4_OK;
 }
 

@@ -43,6 +43,7 @@ struct q4_model {
     q4_shared_data* shared;
     volatile int* status_word;  // pinned, behind the shared data: the fused kernel's status as the last reset found it
     cudaStream_t gen_stream;    // q4_generate's, made by its first call
+    int device;                 // where the model lies
     cudaGraphExec_t graph[3];   // prompt phase, generating (argmax), generating without the hand-off (a sampler follows)
     bool graph_ready[3];
     // sampler state (sampler.h:10-19): temperature 0 = greedy

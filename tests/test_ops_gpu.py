@@ -105,10 +105,11 @@ def _attention(heads, kv_mul, hs, pos, q, kc, vc):
     return out.cpu().numpy()
 
 
-# both sides of every line between the forms (16, 64 and 128 heads), shares that are empty, end on a step of 64 positions or one past it
-@pytest.mark.parametrize("heads,kv_mul,hs", [(15, 1, 128), (16, 2, 64), (16, 1, 256), (64, 8, 128), (65, 5, 64), (129, 3, 64)])
+# both sides of every line between clusters of eight, four, two and one (37, 74 and 148 heads), shares that are empty, end on a step of
+# 64 positions or one past it
+@pytest.mark.parametrize("heads,kv_mul,hs", [(1, 1, 128), (15, 1, 128), (16, 1, 256), (37, 1, 64), (38, 2, 64), (64, 8, 128), (74, 2, 64), (75, 5, 64), (148, 4, 64), (149, 1, 64), (150, 3, 256)])
 @pytest.mark.parametrize("pos", [0, 31, 32, 255, 256, 511, 512, 600])
-def test_attention_forms_and_share_edges(heads, kv_mul, hs, pos):
+def test_attention_clusters_and_share_edges(heads, kv_mul, hs, pos):
     rng = np.random.default_rng(pos * 7 + heads)
     stride = heads * hs // kv_mul
     q = rng.standard_normal(heads * hs).astype(np.float16)
@@ -116,7 +117,7 @@ def test_attention_forms_and_share_edges(heads, kv_mul, hs, pos):
     assert_close(_attention(heads, kv_mul, hs, pos, q, kc, vc), O.attention(q, kc, vc, heads, hs, kv_mul, pos), f"{heads} heads, pos {pos}", max_rel=5e-3)
 
 
-@pytest.mark.parametrize("heads", [4, 32])     # two launches, one cluster
+@pytest.mark.parametrize("heads", [4, 149])     # eight blocks per head, one
 def test_attention_with_scores_that_are_not_finite(heads):
     """A score of -infinity (rounded to fp16) has weight 0, also where it is the first or the only one a lane group sees; a NaN reaches
     its own head's outputs and no other's."""

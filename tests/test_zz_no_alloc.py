@@ -1,7 +1,7 @@
 """q4_attention_static: the attention entry point for callers that cannot allocate device memory (hosts with all
-device memory handed out at start-up, plugins that only receive the owning runtime's pointers). Its scratch is a
-fixed array inside the library. Checked against q4_attention, which takes a caller-owned scratch buffer, on two
-calls in a row (the array keeps the previous call's contents, which must not matter)."""
+device memory handed out at start-up, plugins that only receive the owning runtime's pointers). Checked
+against q4_attention, which takes a caller-owned scratch buffer, on two
+calls in a row (nothing of the first may be left in the second)."""
 import ctypes as C
 
 import numpy as np
