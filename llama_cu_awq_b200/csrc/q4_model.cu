@@ -421,6 +421,19 @@ extern "C" int q4_model_read(const q4_model* m, int what, uint16_t* host_out) {
     return Q4_OK;
 }
 
+// The calls that launch without being handed a stream work on the model's device, whichever is current, and put that back.
+struct OnDevice {
+    int before = -1;
+    cudaError_t error;
+    explicit OnDevice(int device) {
+        error = cudaGetDevice(&before);
+        if (error == cudaSuccess && before == device) before = -1;
+        else if (error == cudaSuccess) error = cudaSetDevice(device);
+    }
+    ~OnDevice() { if (before >= 0) (void)cudaSetDevice(before); }
+    OnDevice(const OnDevice&) = delete;
+};
+
 // The position into device memory and the fused kernel's status out to the host: one launch, where a copy back took twice as long.
 static __global__ void reset_kernel(int* pos_dev, int pos, const int* status, volatile int* status_word) {
     *pos_dev = pos;
@@ -433,11 +446,11 @@ extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int 
     if (prompt_tokens)
         for (int i = 0; i < n; i++)
             if (prompt_tokens[i] < 0 || prompt_tokens[i] >= m->cfg.vocab_size) return Q4_ERR_INVALID;
+    const OnDevice on(m->device);
+    Q4_CUDA_TRY(on.error);
     Q4_CUDA_TRY(cudaDeviceSynchronize());
     m->host_pos = pos;
-    int device = -1;
-    Q4_CUDA_TRY(cudaGetDevice(&device));
-    const int* status = device == m->device ? q4_fused_status_word(m) : nullptr;   // (copies reach the model from any device, a launch does not)
+    const int* status = q4_fused_status_word(m);
     *m->status_word = -1;
     if (status) {
         reset_kernel<<<1, 1>>>(m->pos, pos, status, m->status_word);
@@ -570,10 +583,12 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
                            double* seconds) {
     if (!m || !prompt_tokens || n_prompt < 1) return Q4_ERR_INVALID;
     if (steps <= 0 || steps > m->cfg.seq_len) steps = m->cfg.seq_len;  // llama2_q4.cu:917
-    if (!m->gen_stream) Q4_CUDA_TRY(cudaStreamCreate(&m->gen_stream));
-    const cudaStream_t s = m->gen_stream;
+    const OnDevice on(m->device);   // the stream is kept: one of another device would fail every later call
+    Q4_CUDA_TRY(on.error);
     int e = q4_model_reset(m, prompt_tokens, n_prompt, 0);
     if (e != Q4_OK) return e;
+    if (!m->gen_stream) Q4_CUDA_TRY(cudaStreamCreate(&m->gen_stream));
+    const cudaStream_t s = m->gen_stream;
     int pos = 0;
     const bool one_pass = (path & Q4_PATH_PROMPT_ONE_PASS) != 0;
     path &= ~Q4_PATH_PROMPT_ONE_PASS;

@@ -193,6 +193,35 @@ def test_generation_matches_oracle_tokens(tiny_path):
     assert first_div is None or first_div[1] < 5e-2, first_div
 
 
+@pytest.mark.parametrize("prompt_one_pass", [False, True])
+def test_generate_after_a_refused_call(mid_path, prompt_one_pass):
+    """q4_generate keeps a stream with the model: a call that is refused leaves nothing behind for the calls after it."""
+    t = Transformer(mid_path)
+    prompt = np.random.default_rng(4).integers(3, t.config.vocab_size, size=9, dtype=np.int32)
+    with pytest.raises(_lib.Q4Error):
+        t.generate(np.array([3, t.config.vocab_size], np.int32), 12, path=t.best_path(), prompt_one_pass=prompt_one_pass)
+    a, b = (t.generate(prompt, 24, path=t.best_path(), prompt_one_pass=prompt_one_pass)[0] for _ in range(2))
+    fresh = Transformer(mid_path)
+    want = fresh.generate(prompt, 24, path=fresh.best_path(), prompt_one_pass=prompt_one_pass)[0]
+    assert (a == want).all() and (b == want).all()
+    t.close()
+    fresh.close()
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_reset_and_generate_while_another_device_is_current(mid_path):
+    t = Transformer(mid_path)
+    prompt = np.random.default_rng(4).integers(3, t.config.vocab_size, size=9, dtype=np.int32)
+    path = t.best_path()
+    with torch.cuda.device(1):
+        got = t.generate(prompt, 24, path=path)[0]
+        t.reset(prompt, 3)
+        assert torch.cuda.current_device() == 1
+    assert t.shared().pos == 3
+    assert (got == t.generate(prompt, 24, path=path)[0]).all()
+    t.close()
+
+
 def test_loader_rejects_bad_files(tmp_path, tiny_path):
     L = _lib.lib()
     h = C.c_void_p()
