@@ -193,6 +193,32 @@ def test_generation_matches_oracle_tokens(tiny_path):
     assert first_div is None or first_div[1] < 5e-2, first_div
 
 
+@pytest.mark.parametrize("fwd_path", [0, 1])
+def test_a_step_queued_behind_reset_reads_its_position(mid_path, fwd_path):
+    """The model's stream does not wait for the default stream: reset itself ends with the position in place. Positions far apart, so
+    that a step at the one before would leave other logits and another K/V row."""
+    t = Transformer(mid_path)
+    ids = np.random.default_rng(5).integers(3, t.config.vocab_size, size=40, dtype=np.int32)
+
+    def run(pos, wait):
+        t.reset(ids, pos)
+        if wait:
+            torch.cuda.synchronize()
+        t.forward(gen_token=False, path=fwd_path)
+        t.synchronize()
+        assert t.shared().pos == pos + 1
+        return t.logits().view(np.uint16)
+
+    t.reset(ids, 0)
+    for _ in range(40):
+        t.forward(gen_token=False, path=fwd_path)
+    want = {pos: run(pos, True) for pos in (2, 30, 39)}
+    for i in range(300):
+        pos = (2, 39, 30)[i % 3]
+        assert (run(pos, False) == want[pos]).all(), (i, pos)
+    t.close()
+
+
 @pytest.mark.parametrize("prompt_one_pass", [False, True])
 def test_generate_after_a_refused_call(mid_path, prompt_one_pass):
     """q4_generate keeps a stream with the model: a call that is refused leaves nothing behind for the calls after it."""
