@@ -801,6 +801,7 @@ static int rows_grow(q4_model* m, q4_rows* r, int rows) {
             for (int mm : {1, 16, 17, 64, 65, cap}) ws = std::max(ws, q4_matmul_q4_batched_workspace_bytes(std::min(mm, cap), s[0], s[1]));
         RTRY(rows_alloc(r, &r->ws, ws));
         Q4_CUDA_TRY(cudaMemset(r->ws, 0, ws));
+        Q4_CUDA_TRY(cudaDeviceSynchronize());   // the fill runs on the default stream; the caller's need not wait for that one, and the GEMM counts from zero
         r->ws_bytes = ws;
         r->cap = cap;
     }

@@ -225,6 +225,25 @@ def test_prefill_and_batched_decode_are_bit_reproducible(path_7b4l):
     t.close()
 
 
+def test_the_first_prompt_in_new_buffers():
+    """The GEMM's tile counters must read zero when the first prompt of a length that grows the buffers starts, on a stream that does not
+    wait for the default one: the same bits as that prompt again."""
+    dim, hid, _, H, KV, _, S, theta = synth.CONFIGS["llama2-7b"]
+    for seed in range(3):
+        t = Transformer(None, synthetic=((dim, hid, 1, H, KV, 512, S, theta), seed))
+        ids = np.random.default_rng(seed).integers(3, 512, size=333, dtype=np.int32)
+        for n in (17, 64, 77, 200, 333):
+            got = []
+            for _ in range(2):
+                t.reset(ids, 0)
+                t.prefill(n, gen_token=False)
+                t.synchronize()
+                got.append(t.logits().view(np.uint16))
+            assert (got[0] == got[1]).all(), n
+        assert t.status() == 0
+        t.close()
+
+
 @pytest.mark.parametrize("n_seq", [1, 8])
 def test_batched_decode_matches_single_sequence_decode(mid_path, n_seq):
     """n_seq sequences with different prompts advance together; each one's logits equal (to tolerance) what the single-
