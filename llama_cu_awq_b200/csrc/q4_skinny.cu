@@ -6,8 +6,9 @@
 // kernel is built for; the tcgen05 GEMM (q4_gemm.cu) takes over from M > 16, where the contraction starts to matter.
 //
 // Work split: a unit is 16 * MT output features of one launch over the whole K axis; one persistent CTA (12 warps; 8 for
-// 9-16 rows) per SM walks the units; in unit u warp w takes share (w + u) % warps of the 128-input groups, and the shares' partial
-// tiles are summed in the order of the shares through shared memory (fixed order: results are bit-reproducible). Inside a warp the product runs on mma.sync m16n8k16 (fp16 in, fp32 out) with
+// 9-16 rows) per SM walks the units; a warp takes one share of a unit's 128-input groups, its own or, going round, share
+// (w + u) % warps of unit u, and the shares' partial tiles are summed in the order of the shares through shared memory (fixed order:
+// results are bit-reproducible, and the same either way). Inside a warp the product runs on mma.sync m16n8k16 (fp16 in, fp32 out) with
 // the weights as the 16-row operand and the batch as the 8-column one. The k index of an MMA is only a summation
 // label, so the packed words are used as they lie in the file: thread (g, t) of the warp loads 16 bytes = 32 inputs of
 // feature rows g and g + 8 at input offset 32 t of the group, unpacks a word into the half2 pairs (q0,q4) (q1,q5)
@@ -73,8 +74,16 @@ __device__ __forceinline__ void unpack8(uint32_t w, uint32_t zlo, uint32_t zhi, 
 #endif
 // warps of a CTA = K slices of a unit
 __host__ __device__ constexpr int warps_of(int MT, int NT) { return NT == 2 ? 8 : SK_WARPS; }   // (16 batch rows need the registers of 8-warp CTAs)
-// Units whose partial tiles wait in shared memory for one sum: all of a CTA's for the 7B shapes, and what L1 keeps is still enough for x.
-__host__ __device__ constexpr int units_at_once(int MT, int NT) { return NT == 2 ? 4 : 6; }
+// How the groups of a CTA's units are dealt to the warps, and when the partial tiles are summed:
+//   ONE_UNIT   there is one unit (7B o with 8 rows 4.6 -> 4.5 us, 16 rows 5.8 -> 5.6 against the general forms)
+//   FIXED      a warp keeps its share; every unit is summed behind a barrier of its own, while the other warps go on
+//   ROTATING   shares go round; units are summed several at a time
+// fixed_shares() tells which. Units that wait in shared memory for one sum: as many as 72 KB hold, so that L1 keeps enough for x.
+enum Deal { ONE_UNIT, FIXED, ROTATING };
+// units whose partial tiles have a place in shared memory
+__host__ __device__ constexpr int slots_of(int NT, Deal deal) { return deal == ONE_UNIT ? 1 : deal == FIXED ? 2 : NT == 2 ? 4 : 6; }
+// units that are summed together
+__host__ __device__ constexpr int units_at_once(int NT, Deal deal) { return deal == ROTATING ? slots_of(NT, deal) : 1; }
 
 // MT: 16-feature tiles per unit (1 or 2); NT: 8-row batch tiles (1: M <= 8, 2: M <= 16); SILU: tile 0 = gate, tile 1 = up.
 // Persistent: one CTA per SM walks units blockIdx.x, blockIdx.x + gridDim.x, ...; a warp's weight loads run D groups ahead
@@ -82,17 +91,17 @@ __host__ __device__ constexpr int units_at_once(int MT, int NT) { return NT == 2
 // at K = 4096 - so a pipeline that restarted per unit would spend its time on load latency, and one-unit CTAs would
 // quantise the work badly over the SMs). Measured on the four 7B ops with 8 rows (us): 8 warps with 4 groups ahead
 // 4.4 / 10.4 / 11.9 / 19.9; 12 warps with 2-3 ahead 4.5 / 9.4 / 10.6 / 16.6; 16 warps with 2 ahead 4.8 / 9.6 / 11.6 / 19.2.
-template <int MT, int NT, bool SILU>
+template <int MT, int NT, bool SILU, Deal DEAL>
 __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(const SkParams p) {
     constexpr int kWarps = warps_of(MT, NT);
     extern __shared__ float red_raw[];
-    constexpr int kUnits = units_at_once(MT, NT);
-    float (*red)[kWarps][MT][NT][4][32] = reinterpret_cast<float (*)[kWarps][MT][NT][4][32]>(red_raw);   // [unit % kUnits][share]
+    constexpr int kSlots = slots_of(NT, DEAL), kSum = units_at_once(NT, DEAL);
+    float (*red)[kWarps][MT][NT][4][32] = reinterpret_cast<float (*)[kWarps][MT][NT][4][32]>(red_raw);   // [unit % kSlots][share]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int units = SILU ? p.total_tiles : p.total_tiles / MT;
     const int my_units = blockIdx.x < units ? (units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    // This warp's steps (unit, group), unit by unit. The shares of a unit differ by one group (32 groups over 12 warps are 2 or 3) and go
-    // round the warps from unit to unit; with a fixed share per warp and a barrier per unit all waited for those with three.
+    // This warp's steps (unit, group), unit by unit. The shares of a unit differ by one group (32 groups over 12 warps are 2 or 3): with a
+    // fixed share per warp and a barrier per unit all wait for those with three, so there they go round.
     struct Cursor {
         int u, share, g, g_end;
         __device__ __forceinline__ void settle(int G, int n) {   // to the first unit from u on in which the share has a group
@@ -100,6 +109,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
             g_end = G * (share + 1) / kWarps;
             while (g == g_end && u < n) {
                 u++;
+                if (DEAL != ROTATING) continue;
                 share = share + 1 == kWarps ? 0 : share + 1;
                 g = G * share / kWarps;
                 g_end = G * (share + 1) / kWarps;
@@ -108,6 +118,10 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
         __device__ __forceinline__ void next(int G, int n) {
             if (++g < g_end) return;
             u++;
+            if (DEAL != ROTATING) {
+                g = G * share / kWarps;
+                return;
+            }
             share = share + 1 == kWarps ? 0 : share + 1;
             settle(G, n);
         }
@@ -205,18 +219,18 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
     };
     clear_acc();
 
-    // End of unit u for this warp: its share's partial tile goes to shared memory. The sums of up to kUnits units are taken together:
-    // no barrier on the way (with one per unit, eight rows of 70B gate/up 84.1 us, 77.5 so; 13B 25.6, 23.4).
+    // End of unit u for this warp: its share's partial tile goes to shared memory. ROTATING sums up to kSum units together, without a
+    // barrier on the way (with one per unit, eight rows of 70B gate/up 84.1 us, 77.5 so; 13B 25.6, 23.4).
     auto unit_end = [&](int u) {
-        const int share = (warp + u) % kWarps, last = u % kUnits;
+        const int share = DEAL == ROTATING ? (warp + u) % kWarps : warp, slot = u % kSlots, last = u % kSum;
 #pragma unroll
         for (int mt = 0; mt < MT; mt++)
 #pragma unroll
             for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) red[last][share][mt][nt][e][lane] = acc[mt][nt][e];
+                for (int e = 0; e < 4; e++) red[slot][share][mt][nt][e][lane] = acc[mt][nt][e];
         clear_acc();
-        if (last + 1 < kUnits && u + 1 < my_units) return;
+        if (last + 1 < kSum && u + 1 < my_units) return;
         __syncthreads();
         // thread = (nt, e, lane): element (feature f0 + g + 8 (e >> 1), batch row 8 nt + 2 t + (e & 1)) of every tile
         for (int i = threadIdx.x; i < (last + 1) * NT * 4 * 32; i += kWarps * 32) {
@@ -227,7 +241,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
             for (int mt = 0; mt < MT; mt++) {
                 float sum = 0.f;
 #pragma unroll
-                for (int w = 0; w < kWarps; w++) sum += red[par][w][mt][nt][e][l];
+                for (int w = 0; w < kWarps; w++) sum += red[slot - last + par][w][mt][nt][e][l];
                 v[mt] = sum;
             }
             if (row >= p.M) continue;
@@ -251,7 +265,7 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
                 }
             }
         }
-        if (u + 1 < my_units) __syncthreads();   // the buffers are written again
+        if (DEAL == ROTATING && u + 1 < my_units) __syncthreads();   // the buffers are written again (FIXED: behind the next unit's barrier only)
     };
 
     for (int u = 0; u < cur.u; u++) unit_end(u);   // (fewer groups than warps: units in which this one has none)
@@ -338,17 +352,44 @@ SkMat sk_mat(const q4_qweight* w, uint16_t* y, int ldy, int tile0) {
     return m;
 }
 
+template <int MT, int NT, bool SILU, Deal DEAL>
+int launch_deal(const SkParams& p, int units, cudaStream_t s) {
+    constexpr int kSlots = slots_of(NT, DEAL);
+    const int per_cta = q4_div_up(units, kSms);
+    // (the limit belongs to the function: always the largest any launch needs)
+    if (kSlots * unit_bytes(MT, NT) > 48 * 1024)
+        Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU, DEAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSlots * unit_bytes(MT, NT))));
+    const size_t smem = (per_cta < kSlots ? per_cta : kSlots) * unit_bytes(MT, NT);
+    Q4Launch L(dim3(units < kSms ? units : kSms), dim3(warps_of(MT, NT) * 32), smem, s);
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_skinny_kernel<MT, NT, SILU, DEAL>, p));
+    return Q4_OK;
+}
+
+// Whether a warp keeps its share of every unit: where shares that go round make no warp's load lighter, a barrier per unit and one unit's
+// sum at a time are cheaper than cursors that move and a sum of several units at the end (us, fixed against going round).
+//   9 to 16 rows, equal shares of one group or an even number: 7B q|k|v 14.9, 15.3; gate/up 24.4, 24.9; 1024 -> 2 x 20000 13.3, 14.3;
+//   6144 -> 2 x 11008 34.2, 36.0; 8192 -> 2 x 28672 the same. With shares of three or five groups going round is the
+//   faster one all the same (13B q|k|v 35.6, 34.3; o 15.1, 14.8).
+//   Two units per CTA whose heaviest pair of neighbouring shares is two heaviest ones: 8 rows, 4096 -> 2 x 4096 7.3, 7.6; 16 rows, 11008 ->
+//   8192 24.4, 24.8; with very long shares the barrier costs more (8 rows, 28672 -> 8192 42.0, 41.6).
+bool fixed_shares(int G, int warps, int NT, int per_cta) {
+    if (NT == 2 && G % warps == 0) return G == warps || G / warps % 2 == 0;
+    if (per_cta != 2 || G > 12 * warps) return false;
+    auto share = [&](int i) { return G * (i % warps + 1) / warps - G * (i % warps) / warps; };
+    int most = 0, pair = 0;
+    for (int i = 0; i < warps; i++) {
+        most = share(i) > most ? share(i) : most;
+        pair = share(i) + share(i + 1) > pair ? share(i) + share(i + 1) : pair;
+    }
+    return pair == 2 * most;
+}
+
 template <int MT, int NT, bool SILU>
 int launch_variant(const SkParams& p, cudaStream_t s) {
-    const int units = SILU ? p.total_tiles : p.total_tiles / MT, per_cta = q4_div_up(units, kSms);
-    constexpr int kUnits = units_at_once(MT, NT);
-    // (the limit belongs to the function: always the largest any launch needs)
-    if (kUnits * unit_bytes(MT, NT) > 48 * 1024)
-        Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kUnits * unit_bytes(MT, NT))));
-    const size_t smem = (per_cta < kUnits ? per_cta : kUnits) * unit_bytes(MT, NT);
-    Q4Launch L(dim3(units < kSms ? units : kSms), dim3(warps_of(MT, NT) * 32), smem, s);
-    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_skinny_kernel<MT, NT, SILU>, p));
-    return Q4_OK;
+    const int units = SILU ? p.total_tiles : p.total_tiles / MT;
+    if (units <= kSms) return launch_deal<MT, NT, SILU, ONE_UNIT>(p, units, s);
+    if (fixed_shares(p.G, warps_of(MT, NT), NT, q4_div_up(units, kSms))) return launch_deal<MT, NT, SILU, FIXED>(p, units, s);
+    return launch_deal<MT, NT, SILU, ROTATING>(p, units, s);
 }
 
 template <bool SILU>
