@@ -626,8 +626,8 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (finish) {
                 __threadfence();
                 // Pieces (32 columns of one stored part) in the order they are added, two requested ahead of the sum whichever part they belong
-                // to. With the next columns of the first two parts ahead the third and fourth were a latency of L2 each: 64 x 11008 x
-                // 4096 in four parts 20.2 us, 18.2 so; 77 x 13824 x 5120 in three 25.5, 24.3. (Three or four ahead spill: no gain.)
+                // to. With the next columns of the first two parts ahead the third and fourth were a latency of L2 each: 77 x 13824 x
+                // 5120 in three parts 25.5 us, 24.3 so. (Three or four ahead spill: no gain.)
                 const int others = last - first + (own_in_tmem ? 0 : 1);
                 constexpr int kAhead = 2;
                 float4 ring[kAhead][8];
@@ -751,17 +751,17 @@ constexpr size_t kWsPartials = kWsHeader + sizeof(int) * kWsMaxTiles;
 
 struct GemmPlan { int MT, m_tiles, n_tiles, n_chunks, pairs, stages, np, slab; long long total; };
 
-// Batch tile and number of pairs, by an estimate of the slowest pair's time over all of them, in us. The lines were fitted to 63 shapes
+// Batch tile and number of pairs, by an estimate of the slowest pair's time over all of them, in us. The lines were fitted to 70 shapes
 // (K and N of the 7B, 13B and 70B projections, 24 to 512 rows) with all their tiles and 5 to 12 numbers of pairs each; the plan it
-// picks is within 1 % of the best of them on average. (Its predecessor, from clock stamps inside the kernel, took a partial
-// tile's reading for a fifth of what it costs and was 9 % off: 77 x 5120 x 5120 22.9 us, 16.9 so; 128 x 8192 x 8192 30.3, 24.1.)
+// picks is 0.4 % off the best of them on average, 5 % at most. (Where only shares of equal length counted as aligned it was 1.4 and
+// 14 %: 64 x 11008 x 4096 on 68 pairs, five parts to a tile, 19.5 us, on 64 pairs with four 18.0; 77 x 5120 x 5120 16.7, 16.0.)
 //   chunk    a 256-input chunk: 5 ns per batch row on the tensor pipe, 0.72 us at least, whatever the rows (issue of its 16 MMAs,
 //            conversion of its 128 x 256 weights)
 //   segment  each further tile that a share touches: its turn at the accumulator
 //   drain    the last tile's output, which is not hidden by anything: 9 ns per row
 //   split    a tile cut by a share boundary: a partial tile written, counted and, by the last CTA, one read per other contributor at
-//            9 ns per row and 0.25 us, which is why even shares of a whole fraction of a tile on 64 pairs often beat 74 pairs;
-//            shares that are no such fraction meet at other times
+//            9 ns per row and 0.25 us, which is why 64 pairs with every tile in two or four parts often beat 74 (a multiple of the
+//            number of tiles does that whatever the chunks: shares are dealt out balanced, pair_of); other shares meet at other times
 // Rings: operand stages as tensor memory allows, the shared memory that their X slabs leave for packed weights (at few rows
 // the kernel is a weight stream: ten 16 KB copies in flight per SM cover HBM's latency).
 GemmPlan make_plan(int M, int K, int N, int sms) {
@@ -776,15 +776,16 @@ GemmPlan make_plan(int M, int K, int N, int sms) {
         if (mt == last_mt || (long long)g.n_tiles * q4_div_up(M, mt) * 2 > kWsMaxTiles) continue;
         last_mt = mt;
         const int mtl = q4_div_up(M, mt);
-        const long long total = (long long)g.n_tiles * mtl * g.n_chunks;
+        const int tiles = g.n_tiles * mtl;
+        const long long total = (long long)tiles * g.n_chunks;
         const double t_chunk = 0.005 * mt > 0.72 ? 0.005 * mt : 0.72;
         for (int P = (int)(total < max_pairs ? total : max_pairs); P >= 1; P--) {
             const long long share = (total + P - 1) / P;
             if (share * t_chunk >= best) break;   // fewer pairs only take longer from here on
-            const bool even = total % P == 0, whole = even && share % g.n_chunks == 0, aligned = even && g.n_chunks % share == 0;
+            const bool whole = tiles % P == 0, aligned = P % tiles == 0;   // no share, or every tile, starts where a tile does
             double cost = share * t_chunk + 0.009 * mt + 0.4 * (q4_div_up((int)share, g.n_chunks) - (whole || aligned ? 1 : 0));
             if (!whole) {   // contributors of a tile, at most
-                const long long parts = aligned ? g.n_chunks / share : share >= g.n_chunks ? 2 : (g.n_chunks - 2) / share + 2;
+                const long long parts = aligned ? P / tiles : share >= g.n_chunks ? 2 : (g.n_chunks - 2) / share + 2;
                 cost += 1.2 + 0.015 * mt + (parts - 1) * (0.25 + 0.009 * mt) + (aligned ? 0.0 : 0.8);
             }
             if (cost < best) { best = cost; g.pairs = P; g.MT = mt; g.m_tiles = mtl; g.total = total; }
@@ -937,5 +938,12 @@ extern "C" int q4_time_matmul_q4_batched(void* stream, uint16_t* y, const uint16
 extern "C" int q4_test_gemm_silu(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* interleaved, int M, int K, int N,
                                  void* workspace, size_t workspace_bytes) {
     return q4_gemm_launch(stream, y, x, w, interleaved, M, K, N, nullptr, 0.f, true, workspace, workspace_bytes);
+}
+// What make_plan picks on a GPU with `sms` SMs (host only): batch tile and number of pairs.
+extern "C" int q4_test_gemm_plan(int M, int K, int N, int sms, int* mt, int* pairs) {
+    const GemmPlan g = make_plan(M, K, N, sms);
+    *mt = g.MT;
+    *pairs = g.pairs;
+    return g.pairs ? Q4_OK : Q4_ERR_UNSUPPORTED_SIZE;
 }
 #endif  // Q4_TEST_BUILD
