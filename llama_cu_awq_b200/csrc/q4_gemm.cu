@@ -755,8 +755,9 @@ struct GemmPlan { int MT, m_tiles, n_tiles, n_chunks, pairs, stages, np, slab; l
 // (K and N of the 7B, 13B and 70B projections, 24 to 512 rows) with all their tiles and 5 to 12 numbers of pairs each; the plan it
 // picks is 0.4 % off the best of them on average, 5 % at most. (Where only shares of equal length counted as aligned it was 1.4 and
 // 14 %: 64 x 11008 x 4096 on 68 pairs, five parts to a tile, 19.5 us, on 64 pairs with four 18.0; 77 x 5120 x 5120 16.7, 16.0.)
-//   chunk    a 256-input chunk: 5 ns per batch row on the tensor pipe, 0.72 us at least, whatever the rows (issue of its 16 MMAs,
-//            conversion of its 128 x 256 weights)
+//   chunk    a 256-input chunk: 4.6 ns per batch row on the tensor pipe and 0.08 us whatever the rows, 0.72 us at least (issue of its 16
+//            MMAs, conversion of its 128 x 256 weights). With 5 ns per row and nothing else, eight tiles of 160 rows were as good as five of
+//            256: 1200 x 28672 x 8192 470 us, 443 so; 1200 x 8192 x 57344 851, 793; 900 x 28672 x 8192 353, 331
 //   segment  each further tile that a share touches: its turn at the accumulator
 //   drain    the last tile's output, which is not hidden by anything: 9 ns per row
 //   split    a tile cut by a share boundary: a partial tile written, counted and, by the last CTA, one read per other contributor at
@@ -778,7 +779,7 @@ GemmPlan make_plan(int M, int K, int N, int sms) {
         const int mtl = q4_div_up(M, mt);
         const int tiles = g.n_tiles * mtl;
         const long long total = (long long)tiles * g.n_chunks;
-        const double t_chunk = 0.005 * mt > 0.72 ? 0.005 * mt : 0.72;
+        const double t_rows = 0.08 + 0.0046 * mt, t_chunk = t_rows > 0.72 ? t_rows : 0.72;
         for (int P = (int)(total < max_pairs ? total : max_pairs); P >= 1; P--) {
             const long long share = (total + P - 1) / P;
             if (share * t_chunk >= best) break;   // fewer pairs only take longer from here on
