@@ -17,6 +17,7 @@
 #include <stdio.h>
 
 #include "q4_common.cuh"
+#include "q4_model.h"
 
 namespace {
 
@@ -231,7 +232,8 @@ static int attention_launch(cudaStream_t s, __half* output, const __half* q, con
     return Q4_OK;
 }
 
-static int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache, int num_heads,
+// What both entry points and the model launch.
+int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache, int num_heads,
                                int head_size, int kv_mul, const int* pPos) {
     __half* out = (__half*)output;
     const __half *qh = (const __half*)q, *kc = (const __half*)key_cache, *vc = (const __half*)value_cache;
@@ -253,16 +255,16 @@ extern "C" int q4_attention(void* stream, uint16_t* output, const uint16_t* q, c
 }
 
 // The same for hosts that hand this library nothing but the reference's own buffers and may not allocate device memory themselves (a
-// serving process whose device memory is fully committed at start-up, a plugin that only receives raw pointers). The limit is that of
-// the array inside the library that held the partial results.
+// serving process whose device memory is fully committed at start-up, a plugin that only receives raw pointers). The kernel has no such
+// limit: it is what this call has always refused, by the size of a scratch nobody writes any more, and stays part of its contract.
 extern "C" int q4_attention_static(void* stream, uint16_t* output, const uint16_t* q, const uint16_t* key_cache,
                                    const uint16_t* value_cache, int num_heads, int head_size, int kv_mul, int max_seq_len, const int* pPos) {
     (void)max_seq_len;
     if (!output || !q || !key_cache || !value_cache || !pPos || num_heads <= 0 || kv_mul <= 0 || num_heads % kv_mul) return Q4_ERR_INVALID;
     if (head_size > kMaxHeadSize) return Q4_ERR_UNSUPPORTED_SIZE;
     if (q4_attention_scratch_bytes(num_heads, head_size) > (size_t)Q4_ATTENTION_STATIC_MAX_BYTES) {
-        fprintf(stderr, "q4_attention_static: %d heads of size %d need %zu bytes of scratch, the built-in array holds %d\n", num_heads, head_size,
-                q4_attention_scratch_bytes(num_heads, head_size), Q4_ATTENTION_STATIC_MAX_BYTES);
+        fprintf(stderr, "q4_attention_static: %d heads of size %d are beyond this call's limit (q4_attention_scratch_bytes %zu, at most %d); q4_attention takes them\n", num_heads,
+                head_size, q4_attention_scratch_bytes(num_heads, head_size), Q4_ATTENTION_STATIC_MAX_BYTES);
         return Q4_ERR_LIMIT;
     }
     return q4_attention_launch((cudaStream_t)stream, output, q, key_cache, value_cache, num_heads, head_size, kv_mul, pPos);

@@ -897,8 +897,8 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, c
             // about 105 so, and less error)
             const size_t last = (size_t)(n - 1);
             uint16_t* x = (uint16_t*)(r->X + last * dim);
-            OP(q4_attention(s, (uint16_t*)r->ATT, (const uint16_t*)qp + last * ldq, (const uint16_t*)(kc + loff), (const uint16_t*)(vc + loff), m->attn_scratch, heads, m->head_size,
-                            m->kv_mul, c.seq_len, row_pos + last));
+            OP(q4_attention_launch(s, (uint16_t*)r->ATT, (const uint16_t*)qp + last * ldq, (const uint16_t*)(kc + loff), (const uint16_t*)(vc + loff), heads, m->head_size, m->kv_mul,
+                                   row_pos + last));
             OP(q4_matmul_q4(s, x, (const uint16_t*)r->ATT, &L.o.w, m->o_kc, dim, 1, g, -1, nullptr));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
             launch_rows(rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);

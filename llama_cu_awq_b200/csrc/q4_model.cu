@@ -173,7 +173,7 @@ extern "C" int q4_model_free(q4_model* m) {
         if (m->graph_ready[i]) cudaGraphExecDestroy(m->graph[i]);
     cudaFree(m->arena);
     cudaFree(m->x); cudaFree(m->xb); cudaFree(m->hb); cudaFree(m->q); cudaFree(m->logits);
-    cudaFree(m->kc); cudaFree(m->vc); cudaFree(m->attn_scratch); cudaFree(m->pos);
+    cudaFree(m->kc); cudaFree(m->vc); cudaFree(m->pos);
     if (m->shared) cudaFreeHost(m->shared);
     if (m->gen_stream) cudaStreamDestroy(m->gen_stream);
     delete m;
@@ -242,7 +242,6 @@ static int model_build(q4_model** out, const q4_config& c, int rank, int gpu_cou
     m->host_pos = 0;
     m->arena = nullptr;
     m->x = m->xb = m->hb = m->q = m->logits = m->kc = m->vc = nullptr;
-    m->attn_scratch = nullptr;
     m->pos = nullptr;
     m->shared = nullptr;
     m->status_word = nullptr;
@@ -348,7 +347,6 @@ static int model_build(q4_model** out, const q4_config& c, int rank, int gpu_cou
     LOAD_CUDA(cudaMalloc((void**)&m->logits, 2 * (size_t)c.vocab_size));
     LOAD_CUDA(cudaMalloc((void**)&m->kc, kv_bytes));
     LOAD_CUDA(cudaMalloc((void**)&m->vc, kv_bytes));
-    LOAD_CUDA(cudaMalloc((void**)&m->attn_scratch, q4_attention_scratch_bytes(c.n_heads / g, hs)));
     LOAD_CUDA(cudaMalloc((void**)&m->pos, sizeof(int)));
     LOAD_CUDA(cudaMallocHost((void**)&m->shared, sizeof(q4_shared_data) + sizeof(int)));
     m->status_word = reinterpret_cast<volatile int*>(m->shared + 1);
@@ -479,8 +477,7 @@ static int launch_token(q4_model* m, cudaStream_t s, int gen_token, bool handoff
         OP(q4_rmsnorm(s, m->xb, m->x, L.rms_att, dim));
         OP(q4_qkv_matvec(s, m->q, m->kc, m->vc, m->xb, &L.q.w, &L.k.w, &L.v.w, dim, m->q_n, m->kv_n, loff, m->pos));
         OP(q4_rope(s, m->q, m->kc, c.n_heads / g, c.n_kv_heads / g, hs, m->pos, loff, c.rope_theta));
-        OP(q4_attention(s, m->xb + m->o_kb, m->q, m->kc + loff, m->vc + loff, m->attn_scratch, c.n_heads / g, hs, m->kv_mul,
-                        c.seq_len, m->pos));
+        OP(q4_attention_launch(s, m->xb + m->o_kb, m->q, m->kc + loff, m->vc + loff, c.n_heads / g, hs, m->kv_mul, m->pos));
         const int xs = rank * (dim / g), xn = dim / g;   // this rank's slice of x in column mode
         if (m->column) {   // llama2_q4.cu:479-493: gather the attention output, o projection on a column slice, gather x
             OP(q4_all_gather(m->comm, s, m->xb + m->o_kb, m->xb, m->o_kc));

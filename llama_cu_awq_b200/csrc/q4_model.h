@@ -38,7 +38,6 @@ struct q4_model {
     uint16_t *emb, *wcls, *rms_final;
     std::vector<DevLayer> layers;
     uint16_t *x, *xb, *hb, *q, *logits, *kc, *vc;
-    float* attn_scratch;
     int* pos;
     q4_shared_data* shared;
     volatile int* status_word;  // pinned, behind the shared data: the fused kernel's status as the last reset found it
@@ -54,6 +53,9 @@ struct q4_model {
     int host_pos;               // forward calls since the last reset + the reset's position (bounds the K/V row written)
 };
 
+// q4_attn.cu: q4_attention without the scratch it takes and does not use
+int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, const uint16_t* key_cache, const uint16_t* value_cache, int num_heads, int head_size, int kv_mul,
+                        const int* pPos);
 // q4_fused.cu
 int q4_fused_prepare(q4_model* m);                              // builds the stream-layout weights and the phase table (lazy)
 int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff);
