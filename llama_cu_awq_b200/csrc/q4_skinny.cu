@@ -75,13 +75,12 @@ __device__ __forceinline__ void unpack8(uint32_t w, uint32_t zlo, uint32_t zhi, 
 // warps of a CTA = K slices of a unit
 __host__ __device__ constexpr int warps_of(int MT, int NT) { return NT == 2 ? 8 : SK_WARPS; }   // (16 batch rows need the registers of 8-warp CTAs)
 // How the groups of a CTA's units are dealt to the warps, and when the partial tiles are summed:
-//   ONE_UNIT   there is one unit (7B o with 8 rows 4.6 -> 4.5 us, 16 rows 5.8 -> 5.6 against the general forms)
 //   FIXED      a warp keeps its share; every unit is summed behind a barrier of its own, while the other warps go on
 //   ROTATING   shares go round; units are summed several at a time
 // fixed_shares() tells which. Units that wait in shared memory for one sum: as many as 72 KB hold, so that L1 keeps enough for x.
-enum Deal { ONE_UNIT, FIXED, ROTATING };
+enum Deal { FIXED, ROTATING };
 // units whose partial tiles have a place in shared memory
-__host__ __device__ constexpr int slots_of(int NT, Deal deal) { return deal == ONE_UNIT ? 1 : deal == FIXED ? 2 : NT == 2 ? 4 : 6; }
+__host__ __device__ constexpr int slots_of(int NT, Deal deal) { return deal == FIXED ? 2 : NT == 2 ? 4 : 6; }
 // units that are summed together
 __host__ __device__ constexpr int units_at_once(int NT, Deal deal) { return deal == ROTATING ? slots_of(NT, deal) : 1; }
 
@@ -370,11 +369,14 @@ int launch_deal(const SkParams& p, int units, cudaStream_t s) {
 //   9 to 16 rows, equal shares of one group or an even number: 7B q|k|v 14.9, 15.3; gate/up 24.4, 24.9; 1024 -> 2 x 20000 13.3, 14.3;
 //   6144 -> 2 x 11008 34.2, 36.0; 8192 -> 2 x 28672 the same. With shares of three or five groups going round is the
 //   faster one all the same (13B q|k|v 35.6, 34.3; o 15.1, 14.8).
-//   Two units per CTA whose heaviest pair of neighbouring shares is two heaviest ones: 8 rows, 4096 -> 2 x 4096 7.3, 7.6; 16 rows, 11008 ->
-//   8192 24.4, 24.8; with very long shares the barrier costs more (8 rows, 28672 -> 8192 42.0, 41.6).
-bool fixed_shares(int G, int warps, int NT, int per_cta) {
+//   9 to 16 rows, one unit per CTA: 7B o 5.6, 5.8. (With up to 8 rows 4.5, 4.6 too, but there q|k|v goes round, and launches that take turns
+//   with those of another kernel start more slowly than they gain: eight sequences, 32 steps of four 7B layers 7350 us, 7190 with one.)
+//   Gate/up with two units per CTA whose heaviest pair of neighbouring shares is two heaviest ones: 8 rows, 4096 -> 2 x 4096 7.3, 7.6; with
+//   very long shares the barrier costs more (8 rows, 28672 -> 8192 in two units 42.0, 41.6).
+bool fixed_shares(int G, int warps, int NT, bool silu, int per_cta) {
+    if (NT == 2 && per_cta == 1) return true;
     if (NT == 2 && G % warps == 0) return G == warps || G / warps % 2 == 0;
-    if (per_cta != 2 || G > 12 * warps) return false;
+    if (!silu || per_cta != 2 || G > 12 * warps) return false;
     auto share = [&](int i) { return G * (i % warps + 1) / warps - G * (i % warps) / warps; };
     int most = 0, pair = 0;
     for (int i = 0; i < warps; i++) {
@@ -387,8 +389,7 @@ bool fixed_shares(int G, int warps, int NT, int per_cta) {
 template <int MT, int NT, bool SILU>
 int launch_variant(const SkParams& p, cudaStream_t s) {
     const int units = SILU ? p.total_tiles : p.total_tiles / MT;
-    if (units <= kSms) return launch_deal<MT, NT, SILU, ONE_UNIT>(p, units, s);
-    if (fixed_shares(p.G, warps_of(MT, NT), NT, q4_div_up(units, kSms))) return launch_deal<MT, NT, SILU, FIXED>(p, units, s);
+    if (fixed_shares(p.G, warps_of(MT, NT), NT, SILU, q4_div_up(units, kSms))) return launch_deal<MT, NT, SILU, FIXED>(p, units, s);
     return launch_deal<MT, NT, SILU, ROTATING>(p, units, s);
 }
 

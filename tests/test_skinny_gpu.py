@@ -107,9 +107,9 @@ def test_units_that_are_summed_together(M, kind, K, N):
     assert_close(y.cpu().numpy(), g, "vs f64", max_rel=2e-3)
 
 
-# both sides of the rule that says which warps keep their share: two units per CTA (8 groups on 12 warps, some without one; 86 on 8),
-# equal shares of one, two, three and four groups on 8 warps, and several units of each, an odd number among them
-@pytest.mark.parametrize("M,kind,K,N", [(8, 1, 1024, 4096), (8, 1, 4096, 2384), (16, 0, 11008, 2384), (16, 0, 1024, 7136), (16, 1, 1024, 4752), (9, 1, 2048, 9504),
+# both sides of the rule that says which warps keep their share: two units per CTA (8 groups on 12 warps, some without one; 12 and 86 on
+# 8), one unit, equal shares of one, two, three and four groups on 8 warps, and several units of each, an odd number among them
+@pytest.mark.parametrize("M,kind,K,N", [(8, 1, 1024, 4096), (8, 1, 4096, 2384), (16, 0, 11008, 2384), (16, 0, 11008, 2368), (16, 1, 1536, 2384), (9, 1, 11008, 2384), (16, 0, 1024, 7136), (16, 1, 1024, 4752), (9, 1, 2048, 9504),
                                         (16, 1, 3072, 4752), (16, 0, 4096, 14240), (12, 1, 1024, 16592)])
 def test_warps_that_keep_their_share(M, kind, K, N):
     test_units_that_are_summed_together(M, kind, K, N)
