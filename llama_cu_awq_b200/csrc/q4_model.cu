@@ -432,11 +432,10 @@ struct OnDevice {
     OnDevice(const OnDevice&) = delete;
 };
 
-// The position into device memory and, where the fused kernel is in use, its status out to the host: one launch, where a copy back took
-// twice as long.
+// The position into device memory and the fused kernel's status out to the host: one launch, where a copy back took twice as long.
 static __global__ void reset_kernel(int* pos_dev, int pos, const int* status, volatile int* status_word) {
     *pos_dev = pos;
-    if (status) *status_word = *status;
+    *status_word = *status;
 }
 
 extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int pos) {
@@ -450,15 +449,19 @@ extern "C" int q4_model_reset(q4_model* m, const int* prompt_tokens, int n, int 
     Q4_CUDA_TRY(cudaDeviceSynchronize());
     m->host_pos = pos;
     const int* status = q4_fused_status_word(m);
-    *m->status_word = -1;
-    reset_kernel<<<1, 1>>>(m->pos, pos, status, m->status_word);
-    Q4_CUDA_TRY(cudaGetLastError());
     m->shared->pos = pos;
     if (n > 0 && prompt_tokens) memcpy((void*)m->shared->tokens, prompt_tokens, sizeof(int) * (size_t)n);
-    // The launch is on the default stream, which a caller's non-blocking stream does not wait for: without this wait a step queued right
-    // away could read the position of the run before. (A pageable copy of the position instead of the launch needs it as well: it may
-    // return before its transfer has ended. 14 us with it, the launch or the copy; 9 without.)
-    Q4_CUDA_TRY(cudaDeviceSynchronize());
+    // Both ways the position is there when the call returns: they run on the default stream, which a caller's non-blocking stream does not
+    // wait for, and a step queued right away could read the position of the run before. A copy from pinned memory returns when it is done;
+    // one from pageable memory may return earlier (5 us less, and not safe); the launch and a wait take 1 us longer than the copy.
+    *m->status_word = -1;
+    if (status) {
+        reset_kernel<<<1, 1>>>(m->pos, pos, status, m->status_word);
+        Q4_CUDA_TRY(cudaGetLastError());
+        Q4_CUDA_TRY(cudaDeviceSynchronize());
+    } else {
+        Q4_CUDA_TRY(cudaMemcpy(m->pos, (const void*)&m->shared->pos, sizeof(int), cudaMemcpyHostToDevice));
+    }
     q4_fused_reset(m, status && *m->status_word == 0);
     return Q4_OK;
 }
