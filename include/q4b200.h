@@ -281,7 +281,8 @@ const uint16_t* q4_model_logits(const q4_model* model); /* device, vocab_size ha
 const uint16_t* q4_model_x(const q4_model* model);      /* device, dim halfs */
 /* Synchronous device-to-host copy of a run-state vector: what = 0 logits (vocab_size halfs), 1 x (dim halfs). */
 int q4_model_read(const q4_model* model, int what, uint16_t* host_out);
-/* Resets position counters (device and pinned) to `pos` and copies `n` prompt ids into the mailbox.
+/* Resets position counters (device and pinned) to `pos` and copies `n` prompt ids into the mailbox. Waits for the device first;
+ * position and ids are in place when the call returns, for steps on any stream. Any device may be current (q4_generate too).
  * Q4_ERR_INVALID when an id lies outside [0, vocab_size): the embedding gather would read outside the table. */
 int q4_model_reset(q4_model* model, const int* prompt_tokens, int n, int pos);
 /* run_transformer(): one token at the current position on `stream`: embedding .. logits, then the greedy
