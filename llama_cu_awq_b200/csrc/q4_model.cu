@@ -411,15 +411,7 @@ extern "C" q4_shared_data* q4_model_shared(q4_model* m) { return m ? m->shared :
 extern "C" const uint16_t* q4_model_logits(const q4_model* m) { return m ? m->logits : nullptr; }
 extern "C" const uint16_t* q4_model_x(const q4_model* m) { return m ? m->x : nullptr; }
 
-extern "C" int q4_model_read(const q4_model* m, int what, uint16_t* host_out) {
-    if (!m || !host_out || what < 0 || what > 1) return Q4_ERR_INVALID;
-    Q4_CUDA_TRY(cudaDeviceSynchronize());
-    if (what == 0) Q4_CUDA_TRY(cudaMemcpy(host_out, m->logits, 2 * (size_t)m->cfg.vocab_size, cudaMemcpyDeviceToHost));
-    else Q4_CUDA_TRY(cudaMemcpy(host_out, m->x, 2 * (size_t)m->cfg.dim, cudaMemcpyDeviceToHost));
-    return Q4_OK;
-}
-
-// The calls that launch without being handed a stream work on the model's device, whichever is current, and put that back.
+// The calls that launch or wait without being handed a stream do so on the model's device, whichever is current, and put that back.
 struct OnDevice {
     int before = -1;
     cudaError_t error;
@@ -431,6 +423,16 @@ struct OnDevice {
     ~OnDevice() { if (before >= 0) (void)cudaSetDevice(before); }
     OnDevice(const OnDevice&) = delete;
 };
+
+extern "C" int q4_model_read(const q4_model* m, int what, uint16_t* host_out) {
+    if (!m || !host_out || what < 0 || what > 1) return Q4_ERR_INVALID;
+    const OnDevice on(m->device);
+    Q4_CUDA_TRY(on.error);
+    Q4_CUDA_TRY(cudaDeviceSynchronize());
+    if (what == 0) Q4_CUDA_TRY(cudaMemcpy(host_out, m->logits, 2 * (size_t)m->cfg.vocab_size, cudaMemcpyDeviceToHost));
+    else Q4_CUDA_TRY(cudaMemcpy(host_out, m->x, 2 * (size_t)m->cfg.dim, cudaMemcpyDeviceToHost));
+    return Q4_OK;
+}
 
 // The position into device memory and the fused kernel's status out to the host: one launch, where a copy back took twice as long.
 static __global__ void reset_kernel(int* pos_dev, int pos, const int* status, volatile int* status_word) {
@@ -571,6 +573,8 @@ extern "C" int q4_model_set_wait_limit_ns(q4_model* m, unsigned long long ns) {
 
 extern "C" int q4_model_status(q4_model* m) {
     if (!m) return Q4_ERR_INVALID;
+    const OnDevice on(m->device);
+    Q4_CUDA_TRY(on.error);
     Q4_CUDA_TRY(cudaDeviceSynchronize());
     int st = q4_fused_status(m);
     if (st == Q4_OK) st = q4_rows_status(m);

@@ -241,10 +241,13 @@ def test_reset_and_generate_while_another_device_is_current(mid_path):
     path = t.best_path()
     with torch.cuda.device(1):
         got = t.generate(prompt, 24, path=path)[0]
+        logits = t.logits()
+        assert t.status() == 0
         t.reset(prompt, 3)
         assert torch.cuda.current_device() == 1
     assert t.shared().pos == 3
     assert (got == t.generate(prompt, 24, path=path)[0]).all()
+    assert (logits.view(np.uint16) == t.logits().view(np.uint16)).all()
     t.close()
 
 
