@@ -131,10 +131,10 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __
 // the key heads are rotated on their way into cache row `pos` of the row's sequence, the value heads are copied there.
 // head_size 128. A thread takes eight rotation pairs of one head (16 bytes of each half of the head); the angles come from a
 // table [position][pair] built once with the reference's arithmetic (evaluating powf, cosf and sinf per block of four heads,
-// two bytes per access, took 21.6 us for 512 rows of 32 + 32 heads). grid (rows, parts), block 256.
+// two bytes per access, took 21.6 us for 512 rows of 32 + 32 heads). grid (rows, parts), block 256. Rows below q_row0 have no query.
 __global__ void __launch_bounds__(256) rope_store_rows_kernel(__half* q, const __half* k, const __half* v, int ldq, int ldkv, __half* kc, __half* vc, int n_heads,
                                                               int n_kv_heads, const float2* table, const int* row_seq, const int* row_pos, long long seq_stride,
-                                                              long long loff) {
+                                                              long long loff, int q_row0) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
     constexpr int HS = 128, kPer = 8;   // threads per head
@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(256) rope_store_rows_kernel(__half* q, const _
             continue;
         }
         const bool is_q = hh < n_heads;
+        if (is_q && m < q_row0) continue;
         const __half* src = is_q ? q + (size_t)m * ldq + (size_t)hh * HS : k + (size_t)m * ldkv + (size_t)(hh - n_heads) * HS;
         __half* dst = is_q ? q + (size_t)m * ldq + (size_t)hh * HS : kc + dst0 + (size_t)(hh - n_heads) * HS;
         uint4 lo = *reinterpret_cast<const uint4*>(src + i), hi = *reinterpret_cast<const uint4*>(src + i + HS / 2);
@@ -861,7 +862,16 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, c
         return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &gmat.w, gmat.wi, n, gmat.K, gmat.N, residual ? (const uint16_t*)y : nullptr, 1.0f / g, mat == 2, r->ws,
                               r->ws_bytes);
     };
-    // q, k, v of the rows: three buffers (few-rows kernels) or three slices of the fused GEMM's output
+    // k and v alone: the rows of q|k|v behind q's
+    auto gemm_kv = [&](__half* y, const __half* x, int l) {
+        q4_rows::GemmMat part = r->gm[(size_t)l * 4];
+        part.wi += (size_t)m->q_n * q4_pw(part.K);
+        part.w.weight = part.wi;
+        part.w.zeros += (size_t)m->q_n * q4_pz(part.K);
+        part.w.scales += (size_t)m->q_n * q4_groups(part.K);
+        return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &part.w, part.wi, n, part.K, 2 * m->kv_n, nullptr, 1.0f / g, false, r->ws, r->ws_bytes);
+    };
+    // q, k, v of the rows: three buffers (few-rows kernels) or three slices of the fused GEMM's output (two in a prompt's last layer)
     const int nqkv = m->q_n + 2 * m->kv_n;
     const bool skinny = n <= kSkinnyRows;
     // (the attention of batched decode takes k and v as the few-rows kernels leave them, and behind the GEMMs the last layer's down
@@ -879,18 +889,27 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, c
         const DevLayer& L = m->layers[l];
         const long long loff = (long long)l * c.seq_len * m->kv_n;
         norm((const __half*)L.rms_att, fused_add && l > 0 ? r->Y : nullptr);
-        if (skinny) {
+        // The last layer of a prompt: nobody reads the other rows' queries (of 70B's q|k|v four fifths; 333 rows behind 700 of one 70B layer
+        // 222 us, 203 so; 2000 rows of two 7B layers 1113, 1064), so k and v alone go through the GEMM and the last row's query, if asked
+        // for, through the batch-1 product.
+        const bool kv_only = !skinny && l == c.n_layers - 1 && want != WANT_ALL;
+        if (kv_only) {
+            if (want == WANT_LAST) OP(q4_matmul_q4(s, (uint16_t*)r->Q, (const uint16_t*)(r->XB + (size_t)(n - 1) * dim), &L.q.w, dim, m->q_n, 0, 1, -1, nullptr));
+            OP(gemm_kv(r->QKV, r->XB, l));
+        } else if (skinny) {
             OP(q4_qkv_rows_launch(s, (uint16_t*)r->Q, (uint16_t*)r->K, (uint16_t*)r->V, (const uint16_t*)r->XB, &L.q.w, &L.k.w, &L.v.w, n, dim, m->q_n, m->kv_n, pos0 < 0));
         } else {
             OP(gemm(r->QKV, r->XB, l, 0, false));
         }
-        __half* qp = skinny ? r->Q : r->QKV;
-        const __half* kp = skinny ? r->K : r->QKV + m->q_n;
-        const __half* vp = skinny ? r->V : r->QKV + m->q_n + m->kv_n;
-        const int ldq = skinny ? m->q_n : nqkv, ldkv = skinny ? m->kv_n : nqkv;
-        if (pos0 >= 0)   // (batched decode: the attention kernel rotates and files)
-            launch_rows(rope_store_rows_kernel, dim3(n, q4_div_up((heads + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, heads, kv_heads,
-                        r->rope, row_seq, row_pos, seq_stride, loff);
+        __half* qp = skinny || kv_only ? r->Q : r->QKV;
+        const __half* kp = skinny ? r->K : kv_only ? r->QKV : r->QKV + m->q_n;
+        const __half* vp = skinny ? r->V : kp + m->kv_n;
+        const int ldq = kv_only ? 0 : skinny ? m->q_n : nqkv, ldkv = kv_only ? 2 * m->kv_n : skinny ? m->kv_n : nqkv;   // (kv_only: one query, the last row's)
+        if (pos0 >= 0) {   // (batched decode: the attention kernel rotates and files)
+            const int queries = kv_only && want == WANT_CACHE ? 0 : heads;
+            launch_rows(rope_store_rows_kernel, dim3(n, q4_div_up((queries + 2 * kv_heads) * 8, 256)), dim3(256), 0, s, qp, kp, vp, ldq, ldkv, kc, vc, queries, kv_heads,
+                        r->rope, row_seq, row_pos, seq_stride, loff, kv_only ? n - 1 : 0);
+        }
         if (l == c.n_layers - 1 && want != WANT_ALL) {
             if (want == WANT_CACHE) break;
             // one row: the split attention and the products of the batch-1 path (70B: o, gate / up and down 147 us with the few-rows kernels,

@@ -66,6 +66,33 @@ def test_prefill_matches_token_by_token_and_the_oracle(mid_path, n_prompt):
     m.close()
 
 
+@pytest.mark.parametrize("cfg,history,n", [("mid-gqa", 0, 17), ("mid-gqa", 3, 18), ("mid", 0, 17), ("mid", 40, 65)])
+def test_a_prompts_last_layer_keeps_keys_and_values_of_all_rows(tmp_path, cfg, history, n):
+    """In a prompt's last layer k and v alone are computed for all rows and q for the last one: its logits, and those of the next token, which
+    reads the last layer's rows of all positions, against the oracle."""
+    path = str(tmp_path / "m.bin")
+    synth.write_model_file(path, cfg, seed=6)
+    tokens = np.random.default_rng(n).integers(3, synth.CONFIGS[cfg][5], size=history + n + 1, dtype=np.int32)
+    t = Transformer(path)
+    t.reset(tokens, 0)
+    if history:
+        t.prefill(history, gen_token=False)
+    t.prefill(n, gen_token=False)
+    t.synchronize()
+    got = [t.logits()]
+    t.forward(gen_token=False, path=1)
+    t.synchronize()
+    got.append(t.logits())
+    assert t.status() == 0
+    t.close()
+    m = O.Model(open(path, "rb").read())
+    for pos, tok in enumerate(tokens):
+        m.forward(int(tok), pos, order=0)
+        if pos >= history + n - 1:
+            assert_close(got[pos - (history + n - 1)], m.logits(), f"{cfg}, {n} rows behind {history}, logits at {pos} vs oracle")
+    m.close()
+
+
 def test_prefill_hand_off_and_pieces(mid_path):
     """gen_token writes the greedy id after the prompt; a prompt fed in two pieces gives the same cache (to tolerance)."""
     vocab = synth.CONFIGS["mid-gqa"][5]
