@@ -89,7 +89,9 @@ def test_a_prompts_last_layer_keeps_keys_and_values_of_all_rows(tmp_path, cfg, h
     for pos, tok in enumerate(tokens):
         m.forward(int(tok), pos, order=0)
         if pos >= history + n - 1:
-            assert_close(got[pos - (history + n - 1)], m.logits(), f"{cfg}, {n} rows behind {history}, logits at {pos} vs oracle")
+            # (the next token's own path is up to 1.1e-2 off the oracle on these models; another token at one position of the prompt moves
+            # its logits by 6e-2 at least)
+            assert_close(got[pos - (history + n - 1)], m.logits(), f"{cfg}, {n} rows behind {history}, logits at {pos} vs oracle", max_rel=2 * MAX_REL)
     m.close()
 
 
