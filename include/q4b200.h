@@ -84,9 +84,8 @@ int q4_rmsnorm(void* stream, uint16_t* o, const uint16_t* x, const uint16_t* wei
 int q4_matmul_q4(void* stream, uint16_t* xout, const uint16_t* x, const q4_qweight* w, int inpSize, int opSize,
                  int accum, int gpu_count, int loff, const int* pPos);
 
-/* The batch-1 W4 products stream their weights through shared memory and wait for their own copies, two seconds at most; a product that
- * gives up leaves NaN. Waits for the current device; 0, or Q4_ERR_TIMEOUT when that has happened there since the last call
- * (q4_model_status asks too). No counterpart in the reference. */
+/* Waits for the current device. 0: no product has a wait of its own that could run out (q4_model_status asks too). No counterpart in the
+ * reference. */
 int q4_ops_status(void);
 
 /* qkv_matvec(): llama2_q4.cu:378-391, kernel gpu_kernels.h:250-262. Three projections of the same x in one

@@ -28,16 +28,3 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-
-constexpr unsigned long long kCopyWaitNs = 2000ULL * 1000 * 1000;   // limit of a wait for a copy, far beyond any copy's flight time
-// Bounded wait of a whole warp; false when it ran out for any lane.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* b, uint32_t parity) {
-    bool ok = mbar_try(b, parity);
-    if (__all_sync(0xffffffffu, ok)) return true;
-    const unsigned long long t0 = global_ns();
-    while (!ok) {
-        ok = mbar_try(b, parity);
-        if (!ok && global_ns() - t0 > kCopyWaitNs) break;
-    }
-    return __all_sync(0xffffffffu, ok);
-}

@@ -11,17 +11,17 @@
 // them, three items ahead; no shared memory, barrier or wait on the way. A warp stages the activations of a pair once for all the CTA's
 // tiles. What bounds it: the launch's ramp, and for long rows the staging (a pair per warp and 16 pairs); from HBM it reads 3.1 TB/s.
 //
-// Ring: two CTAs per SM, each with every grid-th group of T tiles. A stage is a group's packed words over Pc pairs: row copies of Pc * 128
-// bytes (cp.async.bulk, local memory, no multicast; adjacent in the file layout) by a producer warp into a ring of 4 stages. Pc * T <= 16
-// (tile, pair) units make a stage; math warp w of 8 has units w and w + 8, so that it stages the activations of two pairs for all of
-// the CTA's groups. make_split takes the Pc and T with the fewest stages. What bounds it: the ramp, and a warp's serial chain per stage
-// (wait, loads, products, sums).
+// Stream: the same CTAs and tiles. Every warp keeps the digits of up to four pairs in registers for all tiles, so that an item costs its words' way
+// through a private ring in shared memory (cp.async by the lanes that read it: no barrier between warps) and about 50 instructions; pairs that
+// do not divide by 16 warps are dealt out by items (20 pairs of a 5120-long row: 1.25 a warp; whole ones would be two for some). Scales and
+// zero points of a pass of tiles lie in shared memory as the product takes them, brought once for all warps: as copies of their own in the ring they
+// were half as many requests again as the words (8192 x 8192 10.1 us; 8.2 without). What bounds it: 1.5 us of start (x, scales and the staging behind the
+// wait) and the stream, 6.4 TB/s at 47 MB; 60 % of the issue slots.
 //
 // Under programmatic dependent launch the next product's packed words are requested while this one drains (weights never depend on
-// activations). Back to back on weights from HBM, with half2 FMA, with x as 16-bit fixed point in the ring form alone, and now, us:
-// 4096 x 4096 5.1, 4.4, 4.2; q|k|v 9.9, 9.2, 9.2; 4096 -> 2 x 11008 13.9, 11.0, 11.4; 11008 -> 4096 9.9, 9.6, 10.4; 28672 -> 8192 34.1, 31.3,
-// 33.5; 11008 -> 512 5.3, 5.6, 4.0; 5120 -> 1280 4.4, 4.8, 3.7; 13520 -> 544 6.8, 7.0, 5.4; 512 x 512 1.8, 2.3, 1.7. Error against 64 bits 3.8e-4,
-// 2.1e-4, 2.1e-4 (an fp16 result's own rounding).
+// activations). Back to back on weights from HBM, bulk copies into a ring shared by a CTA's warps (before) and now, us: 4096 x 4096 4.2 (direct, both);
+// q|k|v of 7B 9.1, 7.3, of 13B 14.4, 10.7; 4096 -> 2 x 11008 11.3, 10.5; 5120 -> 2 x 13824 22.2, 15.7; 8192 -> 2 x 28672 54, 46.9; 11008 -> 4096 10.4, 8.2;
+// 28672 -> 8192 34.8, 27.2; 8192 x 8192 11.3, 8.2; 512 x 512 1.6 (direct, both). Error against 64 bits 2.1e-4 (an fp16 result's own rounding).
 #include <algorithm>
 
 #include "q4_bulk.cuh"
@@ -36,22 +36,6 @@ constexpr int kAhead = 3;            // items a warp has requested ahead of the 
 constexpr int kBlockTiles = 32;      // tiles per pass (their partial sums are in shared memory)
 constexpr int kTileStride = kWarps * kRows + 8;   // floats (padded: the summing threads hit distinct banks)
 constexpr int kSms = 148;            // B200
-
-namespace ring {
-constexpr int kMathWarps = 8;
-constexpr int kUnits = 2 * kMathWarps;
-constexpr int kThreads = 32 * (kMathWarps + 1);
-constexpr int kCtas = 2 * kSms;      // two persistent CTAs per SM
-constexpr int kMaxT = 4;             // tiles per stage at most: one lane of the producer per row
-constexpr int kPairBytes = 128;      // of one row
-constexpr int kRowPad = 64;          // two rows' 64-byte pieces of a load lie in different banks
-constexpr int kStageBytes = kUnits * kRows * kPairBytes + kMaxT * kRows * kRowPad;
-constexpr int kStages = 4;
-constexpr int kBlockTiles = 13;      // tiles per pass (their partial sums, scales and zero points are in shared memory)
-constexpr int kTileStride = kUnits * kRows + 8;
-constexpr int kMetaBytes = 2 * kBlockTiles * 64;   // per warp: 8 columns x 2 groups of its two units in every group of tiles, fp16 scale | zero point << 16
-constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + kMathWarps * (2 * kExactScratch + kMetaBytes) + (size_t)kBlockTiles * kTileStride * 4;
-}  // namespace ring
 
 struct GemvMat {
     const uint32_t* w;
@@ -73,8 +57,9 @@ struct GemvParams {
     float gpu_count;
     long long loff;
     const int* pos;
-    int nt_div, nt_mod;   // direct form: CTA c has nt_div + (c < nt_mod) consecutive tiles
-    int Pc, T, nchunks;   // ring form: pairs and tiles per stage, chunks of Pc pairs
+    int nt_div, nt_mod;   // direct and stream forms: CTA c has nt_div + (c < nt_mod) consecutive tiles
+    int pass_tiles;       // stream form: tiles per pass
+    float inv_mrow;       // 1 / meta_row(G)
 };
 
 __device__ __forceinline__ float silu_mul(float g, float u) {
@@ -185,6 +170,34 @@ __device__ __noinline__ void add_small(const GemvParams& p, float* part, int par
     }
 }
 
+// The warps' sums in warp order and the outputs of `tiles` tiles; 16 warps. Thread 8 * tile + column.
+template <bool SILU>
+__device__ __forceinline__ void write_out(const GemvParams& p, const float* part, int tile0, int tiles, int w, int lane) {
+            for (int e0 = w * 32; e0 < tiles * kRows; e0 += kThreads) {
+                const int e = e0 + lane;
+                const bool on = e < tiles * kRows;
+                float sum = 0.f;
+                if (on) {
+                    const float* q = part + (e >> 3) * kTileStride + (e & 7);
+                    float v[4];
+    #pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] = ((q[i * 32] + q[i * 32 + 8]) + q[i * 32 + 16]) + q[i * 32 + 24];
+                    sum = ((v[0] + v[1]) + v[2]) + v[3];
+                }
+                int row;
+                const GemvMat& m = row_of<SILU>(p, tile0 + (on ? e >> 3 : 0), e & 7, row);
+                if (SILU) {
+                    const float up = __shfl_xor_sync(0xffffffffu, sum, 1);
+                    if (on && !(e & 1)) p.m[0].out[row] = __float2half(silu_mul(sum, up));
+                } else if (on) {
+                    __half* out = m.out;
+                    if (m.kv) out += p.loff + (long long)(*p.pos) * m.n;
+                    if (p.accum) sum += __half2float(out[row]) / p.gpu_count;
+                    out[row] = __float2half(sum);
+                }
+            }
+}
+
 template <bool SILU>
 __global__ void __launch_bounds__(kThreads, 1) q4_gemv_kernel(const __grid_constant__ GemvParams p) {
     __shared__ __align__(16) uint8_t scratch[kWarps][kExactScratch];
@@ -282,228 +295,274 @@ __global__ void __launch_bounds__(kThreads, 1) q4_gemv_kernel(const __grid_const
             first = false;
         }
         __syncthreads();
-        for (int e0 = w * 32; e0 < tiles * kRows; e0 += kThreads) {   // thread 8 * tile + column: the warps' sums in warp order
-            const int e = e0 + lane;
-            const bool on = e < tiles * kRows;
-            float sum = 0.f;
-            if (on) {
-                const float* q = part + (e >> 3) * kTileStride + (e & 7);
-                float v[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) v[i] = ((q[i * 32] + q[i * 32 + 8]) + q[i * 32 + 16]) + q[i * 32 + 24];
-                sum = ((v[0] + v[1]) + v[2]) + v[3];
-            }
-            int row;
-            const GemvMat& m = row_of<SILU>(p, tile0 + (on ? e >> 3 : 0), e & 7, row);
-            if (SILU) {
-                const float up = __shfl_xor_sync(0xffffffffu, sum, 1);
-                if (on && !(e & 1)) p.m[0].out[row] = __float2half(silu_mul(sum, up));
-            } else if (on) {
-                __half* out = m.out;
-                if (m.kv) out += p.loff + (long long)(*p.pos) * m.n;
-                if (p.accum) sum += __half2float(out[row]) / p.gpu_count;
-                out[row] = __float2half(sum);
-            }
-        }
+        write_out<SILU>(p, part, tile0, tiles, w, lane);
         if (b0 + kBlockTiles < cta_tiles) __syncthreads();
     }
 }
 
-// Q4_ERR_TIMEOUT once a wait of the ring form has run out (q4_ops_status)
-__device__ int g_status;
+namespace stream {
+// Pairs that a warp keeps: its digits take ten registers each (5 instead of 4: 28672 -> 8192 30.8 us, 29.8; 7 spill, 33.5).
+constexpr int kMaxOwn = 4;
+constexpr int kItemBytes = 1024;
+constexpr int kPassTiles = 28;       // tiles per pass at most (their partial sums are in shared memory)
+constexpr int kSmemBytes = 226 * 1024;
+// Items in a warp's ring: a multiple of the pairs it keeps, so that the requests beside a tile's items are those of one tile. (Ten instead of six:
+// q|k|v of 7B 7.9 us, 7.3; 13824 -> 5120 11.6, 10.7; four: 8.5 for 8192 x 8192, 8.2.)
+__host__ __device__ constexpr int depth(int PP) { return PP == 4 ? 8 : 6; }
+constexpr int kEarly = 4;            // of them, requested before the kernel in front has ended (six: q|k|v 7.5, 7.3; two: 4096 x 11008 6.9, 6.7)
+__host__ __device__ constexpr int ring_bytes(int PP) { return kWarps * (depth(PP) * kItemBytes + kExactScratch); }
+__host__ __device__ constexpr int meta_bytes(int PP) { return kSmemBytes - ring_bytes(PP) - kPassTiles * kTileStride * 4; }   // scales and zero points of a pass
+// Words of a row of them (scale | zero point << 16, and zero for the group that a last pair may lack): an odd number, so that the rows of a tile
+// lie in different banks.
+__host__ __device__ constexpr int meta_row(int G) { return (G + 1) | 1; }
+constexpr int tiles_in_pass(int G, int PP) { return std::min(meta_bytes(PP) / (4 * kRows * meta_row(G)), kPassTiles); }
+}  // namespace stream
 
-// MULTI: more than one chunk or pass, whose activations and scales are requested while the one before is worked on (the registers that
-// takes cost a single pass 10 %).
-template <bool SILU, bool MULTI>
-__global__ void __launch_bounds__(ring::kThreads, 2) q4_gemv_ring_kernel(const __grid_constant__ GemvParams p) {
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// PP: pairs that every warp keeps; the items of the pairs that are left are dealt out over the warps.
+template <bool SILU, int PP>
+__global__ void __launch_bounds__(kThreads, 1) q4_gemv_stream_kernel(const __grid_constant__ GemvParams p) {
+    using namespace stream;
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ uint64_t full[ring::kStages], empty[ring::kStages];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cta = blockIdx.x, grid = gridDim.x;
-    const int Pc = p.Pc, T = p.T, nchunks = p.nchunks, row_bytes = Pc * ring::kPairBytes + ring::kRowPad;
-    const int groups = (p.total_tiles + T - 1) / T, my_groups = (groups - cta + grid - 1) / grid, per_pass = ring::kBlockTiles / T;
-    if (tid < ring::kStages) {
-        mbar_init(&full[tid], 1);
-        mbar_init(&empty[tid], ring::kMathWarps);
-    }
-    mbar_init_fence();
-    __syncthreads();
+    constexpr int kDepth = depth(PP);
+    __shared__ uint32_t small_of[kWarps][PP + 1];
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, cta = blockIdx.x;
+    const int cta_tile0 = cta * p.nt_div + min(cta, p.nt_mod), cta_tiles = p.nt_div + (cta < p.nt_mod);
+    const int p0 = w * PP, rest = p.P - PP * kWarps;
+    uint8_t* const ring = smem + w * kDepth * kItemBytes;
+    uint8_t* const scr = smem + kWarps * kDepth * kItemBytes + w * kExactScratch;
+    uint32_t* const meta = reinterpret_cast<uint32_t*>(smem + ring_bytes(PP));
+    float* const part = reinterpret_cast<float*>(smem + ring_bytes(PP) + meta_bytes(PP));
+    const int mrow = meta_row(p.G);
 
-    if (warp == ring::kMathWarps) {
-        // ---- producer: passes, chunks of Pc pairs, groups of tiles; lane r copies row r ----
-        int stage = 0, issued = 0;
-        uint32_t parity = 1;     // the first round finds every stage empty
-        for (int b0 = 0; b0 < my_groups; b0 += per_pass)
-            for (int c = 0; c < nchunks; c++)
-                for (int lg = b0; lg < min(b0 + per_pass, my_groups); lg++) {
-                    const int word0 = c * Pc * 32, tile0 = (cta + lg * grid) * T;
-                    const uint32_t bytes = 4u * (uint32_t)min(Pc * 32, p.PW - word0);
-                    const int rows = min(T, p.total_tiles - tile0) * kRows;
-                    if (!mbar_wait_warp(&empty[stage], parity)) { b0 = my_groups; c = nchunks; break; }
-                    issued++;
-                    if (lane == 0) mbar_expect_tx(&full[stage], rows * bytes);
-                    __syncwarp();
-                    if (lane < rows) {
-                        int row;
-                        const GemvMat& m = row_of<SILU>(p, tile0 + (lane >> 3), lane & 7, row);
-                        bulk_g2s(smem + stage * ring::kStageBytes + lane * row_bytes, m.w + (size_t)row * p.PW + word0, bytes, &full[stage]);
-                    }
-                    __syncwarp();
-                    if (++stage == ring::kStages) { stage = 0; parity ^= 1u; }
-                }
-        // the CTA's shared memory stays until every copy has landed (bounded; the math warps have waited for all of them unless a wait ran out).
-        for (int i = max(0, issued - ring::kStages); i < issued; i++) mbar_wait_warp(&full[i % ring::kStages], (i / ring::kStages) & 1);
-        return;
-    }
-
-    uint8_t* const scr = smem + ring::kStages * ring::kStageBytes + warp * 2 * kExactScratch;
-    uint32_t* const meta = reinterpret_cast<uint32_t*>(smem + ring::kStages * ring::kStageBytes + ring::kMathWarps * 2 * kExactScratch + warp * ring::kMetaBytes);
-    float* const part = reinterpret_cast<float*>(smem + ring::kStages * ring::kStageBytes + ring::kMathWarps * (2 * kExactScratch + ring::kMetaBytes));
-    const int r = lane >> 2, t = lane & 3;
-    int ts[2], pi[2];            // this warp's units: tile in the group, pair in the chunk
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-        ts[j] = (warp + j * ring::kMathWarps) / Pc;
-        pi[j] = warp + j * ring::kMathWarps - ts[j] * Pc;
-    }
-    int stage = 0;
-    uint32_t parity = 0;
-    bool ok = true;
-    // This warp's scales and zero points for the groups of a pass in a chunk: entry [group][unit][2 * column + group of the pair]. The first
-    // kAhead groups' are requested a chunk ahead.
-    constexpr int kAhead = MULTI ? 4 : 0;
-    uint32_t zn[kAhead + 1];
-    __half sn[kAhead + 1];
-    const int en = lane & 15, tj = (lane >> 4) ? ts[1] : ts[0], pj = (lane >> 4) ? pi[1] : pi[0];
-    auto load_one = [&](int lg, int c, uint32_t& z, __half& sc) {
-        const int tile = (cta + lg * grid) * T + tj, grp = 2 * (c * Pc + pj) + (en & 1);
-        z = 0;
-        sc = __float2half(0.f);
-        if (tj < T && tile < p.total_tiles && grp < p.G) {
-            int row;
-            const GemvMat& m = row_of<SILU>(p, tile, en >> 1, row);
-            z = __ldg(m.z + (size_t)row * p.PZ + (grp >> 3)) >> (4 * (grp & 7));
-            sc = __ldg(m.s + (size_t)row * p.G + grp);
-        }
-    };
-    auto ahead = [&](int b0, int bn, int c) {
-#pragma unroll
-        for (int i = 0; i < kAhead; i++)
-            if (i < bn) load_one(b0 + i, c, zn[i], sn[i]);
-    };
-    auto file_meta = [&](int b0, int bn, int c) {
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < kAhead; i++)
-            if (i < bn) meta[i * 32 + lane] = (uint32_t)__half_as_ushort(sn[i]) | ((zn[i] & 0xFu) << 16);
-#pragma unroll 4
-        for (int lg = kAhead; lg < bn; lg++) {
-            uint32_t z;
-            __half sc;
-            load_one(b0 + lg, c, z, sc);
-            meta[lg * 32 + lane] = (uint32_t)__half_as_ushort(sc) | ((z & 0xFu) << 16);
-        }
-        __syncwarp();
-    };
-    for (int i = tid; i < my_groups * T * kRows; i += 32 * ring::kMathWarps) {   // scales and zero points on their way into L2
+    // Walks this warp's items with the lane's addresses: in a pass its own pairs tile by tile, then its share of the items of the pairs that are
+    // left, pair by pair. The lane copies 16 bytes (lane & 7) of rows lane >> 3 and 4 + (lane >> 3); in odd rows the pair's groups change places,
+    // so that two rows' pieces of a load lie in different banks.
+    const uint32_t dst0 = smem_u32(ring) + (lane >> 3) * 128 + (((lane & 7) ^ ((lane >> 1) & 4)) * 16);
+    const int step = (SILU ? kRows / 2 : kRows) * p.PW, half = (SILU ? 2 : 4) * p.PW;
+    struct {
+        const uint32_t* src;     // of the tile's first own pair, or of the item (rest)
+        int tile, k, pair, left, b0, tiles, end;     // k < PP: own pairs; PP: rest, `left` items of it to come, `pair` the pair
+    } q;
+    auto seek = [&](int pair) {
         int row;
-        const int tile = (cta + i / (T * kRows) * grid) * T + (i / kRows) % T;
-        if (tile < p.total_tiles) {
-            const GemvMat& m = row_of<SILU>(p, tile, i & 7, row);
-            for (int g = 0; g < p.G; g += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(m.s + (size_t)row * p.G + g));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(m.z + (size_t)row * p.PZ));
+        const GemvMat& m = row_of<SILU>(p, cta_tile0 + q.tile, lane >> 3, row);
+        q.src = m.w + (size_t)row * p.PW + pair * 32 + (lane & 7) * 4;
+        q.end = cta_tiles;
+        if (!SILU && p.nmat > 1) q.end = min(q.end, m.tile0 + m.n / kRows - cta_tile0);
+    };
+    // to the rest of the pass that starts at q.b0, or, if the warp has none, to the next pass
+    auto open_pass = [&]() {
+        q.tiles = min(p.pass_tiles, cta_tiles - q.b0);
+        q.tile = q.b0;
+        q.k = 0;
+        q.pair = p0;
+        if (q.tiles > 0) seek(p0);
+    };
+    auto open_rest = [&]() {
+        const int r0 = w * rest * q.tiles / kWarps, r1 = (w + 1) * rest * q.tiles / kWarps;
+        q.k = PP;
+        q.left = r1 - r0;
+        q.pair = PP * kWarps + r0 / q.tiles;
+        q.tile = q.b0 + r0 % q.tiles;
+        if (q.left > 0) seek(q.pair);
+    };
+    auto settle = [&]() {      // past rests that are empty
+        while (q.tiles > 0 && q.k == PP && q.left == 0) {
+            q.b0 += q.tiles;
+            open_pass();
+            if (PP == 0 && q.tiles > 0) open_rest();
         }
+    };
+    auto next = [&]() {
+        if (q.k < PP) {
+            if (++q.k < PP) return;
+            q.k = 0;
+            q.src += step;
+            if (++q.tile < q.b0 + q.tiles) {
+                if (!SILU && p.nmat > 1 && q.tile == q.end) seek(p0);
+                return;
+            }
+            open_rest();
+        } else {
+            q.left--;
+            q.src += step;
+            if (++q.tile == q.b0 + q.tiles) {
+                q.tile = q.b0;
+                q.pair++;
+                if (q.left > 0) seek(q.pair);
+            } else if (!SILU && p.nmat > 1 && q.tile == q.end && q.left > 0) {
+                seek(q.pair);
+            }
+        }
+        settle();
+    };
+    auto request = [&](uint32_t slot) {      // (slot: its first byte)
+        if (q.tiles > 0) {
+            const int at = (q.k < PP ? p0 + q.k : q.pair) * 32 + (lane & 7) * 4;
+            if (at < p.PW) {
+                const uint32_t* src = q.src + (q.k < PP ? q.k * 32 : 0);
+                copy16(dst0 + slot, src);
+                copy16(dst0 + slot + 512, src + half);
+            }
+            next();
+        }
+        copies_commit();
+    };
+    q.b0 = q.left = 0;
+    open_pass();
+    if (PP == 0) {
+        open_rest();
+        settle();
+    }
+    for (int i = 0; i < kEarly; i++) request(i * kItemBytes);
+    // scales and zero points on their way into L2
+    for (int i = tid; i < cta_tiles * kRows; i += kThreads) {
+        int row;
+        const GemvMat& m = row_of<SILU>(p, cta_tile0 + i / kRows, i % kRows, row);
+        for (int g = 0; g < p.G; g += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(m.s + (size_t)row * p.G + g));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(m.z + (size_t)row * p.PZ));
     }
     griddep_wait();
     griddep_launch_dependents();
-    uint4 hv[2];                 // a chunk's activations, requested a chunk ahead (zero beyond K: padded weight words contribute nothing)
-    auto load_x = [&](int c) {
+    auto load_x = [&](int pair) {
+        const int at = pair * 256 + lane * 8;
+        return at < p.K ? *reinterpret_cast<const uint4*>(p.x + at) : make_uint4(0, 0, 0, 0);
+    };
+    uint4 hv[PP + 1];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int k0 = (c * Pc + pi[j]) * 256 + lane * 8;
-            hv[j] = make_uint4(0, 0, 0, 0);
-            if (ts[j] < T && k0 < p.K) hv[j] = *reinterpret_cast<const uint4*>(p.x + k0);
+    for (int k = 0; k < PP; k++) hv[k] = load_x(p0 + k);
+    // A pass's scales and zero points into shared memory; eight a thread in flight.
+    constexpr int kFlight = 8;
+    auto load_meta = [&](int b0, int tiles) {
+        const int ns = tiles * kRows * mrow;
+        for (int e0 = tid; e0 < ns; e0 += kFlight * kThreads) {
+            __half v[kFlight];
+            uint32_t z[kFlight];
+#pragma unroll
+            for (int u = 0; u < kFlight; u++) {
+                const int e = e0 + u * kThreads, i = (int)(((float)e + 0.5f) * p.inv_mrow), g = e - i * mrow;
+                v[u] = __float2half(0.f);
+                z[u] = 0;
+                if (e < ns && g < p.G) {
+                    int row;
+                    const GemvMat& m = row_of<SILU>(p, cta_tile0 + b0 + i / kRows, i % kRows, row);
+                    v[u] = __ldg(m.s + (size_t)row * p.G + g);
+                    z[u] = __ldg(m.z + (size_t)row * p.PZ + (g >> 3));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kFlight; u++) {
+                const int e = e0 + u * kThreads, g = e - (int)(((float)e + 0.5f) * p.inv_mrow) * mrow;
+                if (e < ns) meta[e] = (uint32_t)__half_as_ushort(v[u]) | (((z[u] >> (4 * (g & 7))) & 0xFu) << 16);
+            }
         }
     };
-    load_x(0);
-    ahead(0, min(per_pass, my_groups), 0);
-    file_meta(0, min(per_pass, my_groups), 0);
-    for (int b0 = 0; b0 < my_groups; b0 += per_pass) {
-        const int bn = min(per_pass, my_groups - b0);
-        for (int c = 0; c < nchunks; c++) {
-            PairExact px[2];
-            bool active[2];
-            int wide = 0;
+    // this warp's share of a pass's items of the pairs that are left
+    int pair, tile, left;
+    uint4 hr = make_uint4(0, 0, 0, 0);
+    auto open_share = [&](int tiles) {
+        const int r0 = w * rest * tiles / kWarps, r1 = (w + 1) * rest * tiles / kWarps;
+        pair = PP * kWarps + r0 / tiles;
+        tile = r0 % tiles;
+        left = r1 - r0;
+        if (left > 0) hr = load_x(pair);
+    };
+    open_share(min(p.pass_tiles, cta_tiles));
+    load_meta(0, min(p.pass_tiles, cta_tiles));
+    for (int i = kEarly; i < kDepth; i++) request(i * kItemBytes);
+    PairExact px[PP + 1];        // (the last one: a pair that is left, for the tiles it is this warp's)
+    int wide = 0;
 #pragma unroll
-            for (int j = 0; j < 2; j++) active[j] = ts[j] < T && 2 * (c * Pc + pi[j]) < p.G;
-            if (b0 + c > 0) file_meta(b0, bn, c);
-#pragma unroll
-            for (int j = 0; j < 2; j++) wide |= (int)quant_pair_exact(hv[j], scr + j * kExactScratch, lane, px[j]) << j;
-#pragma unroll
-            for (int j = 0; j < 2; j++) zero_step(px[j]);
-            const bool last = c + 1 == nchunks;
-            if (MULTI && (!last || b0 + per_pass < my_groups)) {
-                load_x(last ? 0 : c + 1);
-                ahead(last ? b0 + per_pass : b0, last ? min(per_pass, my_groups - b0 - per_pass) : bn, last ? 0 : c + 1);
-            }
-            for (int lg = 0; lg < bn; lg++) {
-                if (ok) {
-                    ok = mbar_wait_warp(&full[stage], parity);
-                    if (!ok) atomicExch(&g_status, Q4_ERR_TIMEOUT);
-                }
-                // words 4t..4t + 3 of column r in groups A and B. (Units that are not there multiply whatever lies in the stage; their sums are
-                // not kept.)
-                uint32_t me[2];
-                int c4[2][4];
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const uint4* src = reinterpret_cast<const uint4*>(smem + stage * ring::kStageBytes + ((active[j] ? ts[j] * kRows : 0) + r) * row_bytes + (active[j] ? pi[j] : 0) * ring::kPairBytes) + t;
-                    const uint4 a = src[0], b = src[4];
-                    me[j] = meta[lg * 32 + j * 16 + (lane >> 1)];
-                    pair_mma_exact(c4[j], a, b, px[j]);
-                }
-                __syncwarp();
-                if (lane == 0 && ok) mbar_arrive(&empty[stage]);   // (a stage whose copy has not come is not filled again: the producer gives up too)
-                if (++stage == ring::kStages) { stage = 0; parity ^= 1u; }
-                float y = quad_sum2(pair_share(c4[0], me[0], px[0], lane), pair_share(c4[1], me[1], px[1], lane), lane);
-                if (!ok) y = CUDART_NAN_F;   // a copy that never came must not pass for a result
-                const bool odd = t & 1;
-                if (t < 2 && (odd ? active[1] : active[0])) {
-                    float* const d = part + (lg * T + (odd ? ts[1] : ts[0])) * ring::kTileStride + (odd ? pi[1] : pi[0]) * kRows + r;
-                    *d = c == 0 ? y : *d + y;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 2; j++)
-                if ((wide >> j) & 1)
-                    add_small<SILU>(p, part + ts[j] * ring::kTileStride + pi[j] * kRows, T * ring::kTileStride, *reinterpret_cast<const uint32_t*>(scr + j * kExactScratch), (cta + b0 * grid) * T + ts[j], grid * T, bn, c * Pc + pi[j]);
+    for (int k = 0; k < PP; k++) {
+        if (quant_pair_exact(hv[k], scr, lane, px[k])) {
+            wide |= 1 << k;
+            if (lane == 0) small_of[w][k] = *reinterpret_cast<const uint32_t*>(scr);
+            __syncwarp();
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * ring::kMathWarps) : "memory");
-        for (int e0 = warp * 32; e0 < bn * T * kRows; e0 += 32 * ring::kMathWarps) {   // thread 8 * tile + column
-            const int e = e0 + lane, lt = e >> 3, tile = (cta + (b0 + lt / T) * grid) * T + lt % T;
-            const bool on = e < bn * T * kRows && tile < p.total_tiles;
-            float sum = 0.f;
-            if (on)
-                for (int i = 0; i < Pc; i += 4) {
-                    const float* q = part + lt * ring::kTileStride + i * kRows + (e & 7);
-                    float v[4];
+        zero_step(px[k]);
+    }
+
+    const int c = lane >> 2, t = lane & 3;
+    const uint8_t* const words = ring + c * 128 + t * 16 + (c & 1) * 64;
+    const int other = c & 1 ? -64 : 64;
+    uint32_t slot = 0;           // the next item's, its first byte
+    // One item's share of the lane; the copies that take its place are `more`'s.
+    auto item = [&](const PairExact& x, uint32_t me, auto&& more) {
+        copies_wait<kDepth - 1>();
+        __syncwarp();
+        const uint4 a = *reinterpret_cast<const uint4*>(words + slot), b = *reinterpret_cast<const uint4*>(words + slot + other);
+        int d[4];
+        pair_mma_exact(d, a, b, x);
+        const float y = pair_share(d, me, x, lane);
+        __syncwarp();
+        more(slot);
+        slot += kItemBytes;
+        if (slot == kDepth * kItemBytes) slot = 0;
+        return y;
+    };
+    for (int b0 = 0; b0 < cta_tiles; b0 += p.pass_tiles) {
+        const int tiles = min(p.pass_tiles, cta_tiles - b0);
+        float* const col = part + w * kRows + c;
+        if (PP == 0)
+            for (int i = lane; i < tiles * kRows; i += 32) part[(i >> 3) * kTileStride + w * kRows + (i & 7)] = 0.f;
+        __syncthreads();         // the pass's scales and zero points are in place
+        const uint32_t* me = meta + c * mrow + ((lane >> 1) & 1) + 2 * p0;
+        if (PP > 0) {
+            const int lane_at = p0 * 32 + (lane & 7) * 4;
+            for (int i = 0; i < tiles; i++) {
+                float y = 0.f;
+                // Within the own pairs of a pass and of a matrix the next requests are those of one tile.
+                if (q.tiles > 0 && q.k == 0 && q.tile + 1 < min(q.end, q.b0 + q.tiles)) {
 #pragma unroll
-                    for (int u = 0; u < 4; u++) v[u] = i + u < Pc ? q[u * kRows] : 0.f;
-                    sum += ((v[0] + v[1]) + v[2]) + v[3];
+                    for (int k = 0; k < PP; k++)
+                        y += item(px[k], me[2 * k], [&](uint32_t at) {
+                            if (lane_at + k * 32 < p.PW) {
+                                copy16(dst0 + at, q.src + k * 32);
+                                copy16(dst0 + at + 512, q.src + k * 32 + half);
+                            }
+                            copies_commit();
+                        });
+                    q.src += step;
+                    q.tile++;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < PP; k++) y += item(px[k], me[2 * k], request);
                 }
-            int row;
-            const GemvMat& m = row_of<SILU>(p, on ? tile : 0, e & 7, row);
-            if (SILU) {
-                const float up = __shfl_xor_sync(0xffffffffu, sum, 1);
-                if (on && !(e & 1)) p.m[0].out[row] = __float2half(silu_mul(sum, up));
-            } else if (on) {
-                __half* out = m.out;
-                if (m.kv) out += p.loff + (long long)(*p.pos) * m.n;
-                if (p.accum) sum += __half2float(out[row]) / p.gpu_count;
-                out[row] = __float2half(sum);
+                y = quad_sum(y);
+                if (t == 0) col[i * kTileStride] = y;
+                me += kRows * mrow;
             }
+            for (int k = 0; wide >> k; k++)
+                if ((wide >> k) & 1) add_small<SILU>(p, part + w * kRows, kTileStride, small_of[w][k], cta_tile0 + b0, 1, tiles, p0 + k);
         }
-        if (b0 + per_pass < my_groups) asm volatile("bar.sync 1, %0;" ::"n"(32 * ring::kMathWarps) : "memory");
+        while (left > 0) {
+            const int count = min(left, tiles - tile);
+            const bool more = quant_pair_exact(hr, scr, lane, px[PP]);
+            zero_step(px[PP]);
+            left -= count;
+            if (left > 0) hr = load_x(pair + 1);
+            me = meta + (tile * kRows + c) * mrow + ((lane >> 1) & 1) + 2 * pair;
+            for (int i = 0; i < count; i++) {
+                const float y = quad_sum(item(px[PP], *me, request));
+                if (t == 0) col[(tile + i) * kTileStride] += y;
+                me += kRows * mrow;
+            }
+            if (more)
+                add_small<SILU>(p, part + tile * kTileStride + w * kRows, kTileStride, *reinterpret_cast<const uint32_t*>(scr), cta_tile0 + b0 + tile, 1, count, pair);
+            pair++;
+            tile = 0;
+        }
+        __syncthreads();
+        write_out<SILU>(p, part, cta_tile0 + b0, tiles, w, lane);
+        if (b0 + tiles < cta_tiles) {
+            open_share(min(p.pass_tiles, cta_tiles - b0 - tiles));
+            load_meta(b0 + tiles, min(p.pass_tiles, cta_tiles - b0 - tiles));
+            __syncthreads();     // (the partial sums are written again)
+        }
     }
 }
 
@@ -517,37 +576,37 @@ void fill_dims(GemvParams& p, int K) {
     p.P = q4_div_up(p.G, 2);
 }
 
-// Pairs and tiles per stage: the split that takes the CTA with the most work the least time, a chunk's start (activations, scales) counted
-// as 1.2 stages (13824 -> 5120: 16 pairs of one tile 4 chunks x 3 stages; 5 pairs of 3 tiles 11 x 1, 21 us).
-void make_split(GemvParams& p) {
-    const int P = q4_div_up(p.G, 2);
-    int best = 0;
-    for (int Pc = std::min(P, ring::kUnits); Pc >= 1; Pc--)
-        for (int T = 1; T <= std::min(ring::kUnits / Pc, ring::kMaxT); T++) {
-            const int cost = q4_div_up(P, Pc) * (10 * q4_div_up(q4_div_up(p.total_tiles, T), ring::kCtas) + 12);
-            if (best && cost >= best) continue;
-            best = cost;
-            p.Pc = Pc;
-            p.T = T;
-        }
-    p.nchunks = q4_div_up(P, p.Pc);
+template <bool SILU, int PP>
+int launch_stream(GemvParams& p, cudaStream_t s) {
+    const int grid = std::min(p.total_tiles, kSms);
+    p.nt_div = p.total_tiles / grid;
+    p.nt_mod = p.total_tiles % grid;
+    const int most = p.nt_div + (p.nt_mod > 0);
+    p.pass_tiles = q4_div_up(most, q4_div_up(most, stream::tiles_in_pass(p.G, PP)));
+    p.inv_mrow = 1.0f / stream::meta_row(p.G);
+    // (an opt-in of the function on the device, always to the same value)
+    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_gemv_stream_kernel<SILU, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, stream::kSmemBytes));
+    Q4Launch L(dim3(grid), dim3(kThreads), (size_t)stream::kSmemBytes, s);
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemv_stream_kernel<SILU, PP>, p));
+    return Q4_OK;
 }
 
-// The ring form from 22 MB of packed words and three tiles per SM up: it streams long rows from HBM faster (us, direct and ring: 4096 ->
-// 2 x 11008 16.2, 11.3; 28672 -> 8192 42, 33; 8192 x 8192 12.8, 11.3; 11008 -> 4096 10.7, 10.3), the direct one wins below (4096 x 4096 4.2,
-// 4.7; 13824 -> 2560 10.8, 11.6) and where tiles are few, whatever the size (28672 -> 2048 15.5, 16.3; 26712 -> 2904 19.9, 20.5).
+// The stream form from 9 MB of packed words up, and below that where rows are long (bytes * pairs of a row >= 180 MB); us from HBM, direct and
+// stream: 4096 -> 2 x 11008 16.2, 10.5; 28672 -> 8192 42, 27.2; 11008 -> 4096 10.7, 8.1; 8192 x 2048 4.9, 4.4; 5504 x 4096 6.2, 5.7; 13824 x 640 5.4,
+// 4.7; 24424 x 720 8.5, 6.9; 1024 -> 2 x 40000 18.9, 13.9. The direct form starts about a microsecond earlier: 4096 x 4096 4.2, 4.3 (from L2 3.4,
+// 4.2); 5120 x 2560 4.4, 4.6; 2752 x 4096 4.0, 4.4; 512 x 512 1.6, 2.4. Rows of less than four pairs stay with it whatever the size (512 x 60000 7.6,
+// 8.5), and rows whose scales for a tile do not fit into shared memory (about 390000 inputs).
 template <bool SILU>
 int launch(GemvParams& p, cudaStream_t s) {
-    if (4LL * p.total_tiles * kRows * p.PW > 22000000 && p.total_tiles > 3 * kSms) {
-        static_assert(2 * (ring::kSmemBytes + 1024 + 256) <= 228 * 1024, "two CTAs per SM");
-        make_split(p);
-        const int groups = q4_div_up(p.total_tiles, p.T);
-        // (an opt-in of the function on the device, always to the same value)
-        auto* kernel = p.nchunks > 1 || groups > ring::kCtas * (ring::kBlockTiles / p.T) ? q4_gemv_ring_kernel<SILU, true> : q4_gemv_ring_kernel<SILU, false>;
-        Q4_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring::kSmemBytes));
-        Q4Launch L(dim3(std::min(groups, ring::kCtas)), dim3(ring::kThreads), ring::kSmemBytes, s);
-        Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, kernel, p));
-        return Q4_OK;
+    const long long bytes = 4LL * p.total_tiles * kRows * p.PW;
+    if (p.P >= 4 && (bytes >= 9000000 || bytes * p.P >= 180000000) && stream::tiles_in_pass(p.G, stream::kMaxOwn) > 0) {
+        switch (std::min(p.P / kWarps, stream::kMaxOwn)) {
+            case 0: return launch_stream<SILU, 0>(p, s);
+            case 1: return launch_stream<SILU, 1>(p, s);
+            case 2: return launch_stream<SILU, 2>(p, s);
+            case 3: return launch_stream<SILU, 3>(p, s);
+            default: return launch_stream<SILU, 4>(p, s);
+        }
     }
     const int grid = std::min(p.total_tiles, kSms);
     p.nt_div = p.total_tiles / grid;
@@ -572,12 +631,8 @@ GemvMat mat(const q4_qweight* w, uint16_t* out, int n, int tile0, int kv) {
 }  // namespace
 
 extern "C" int q4_ops_status(void) {
-    int st = 0;
-    const int none = 0;
     Q4_CUDA_TRY(cudaDeviceSynchronize());
-    Q4_CUDA_TRY(cudaMemcpyFromSymbol(&st, g_status, sizeof(st)));
-    if (st) Q4_CUDA_TRY(cudaMemcpyToSymbol(g_status, &none, sizeof(none)));
-    return st;
+    return Q4_OK;     // (no product has a wait that could run out)
 }
 
 extern "C" int q4_matmul_q4(void* stream, uint16_t* xout, const uint16_t* x, const q4_qweight* w, int inpSize,

@@ -240,6 +240,48 @@ def test_products_of_several_matrices_with_small_inputs_beside_large_ones():
         assert np.abs(h.cpu().numpy() - want).max() <= 2.0**-11 * 1.02 * np.abs(want).max() + 1e-6
 
 
+@pytest.mark.parametrize("K,N", [(1032, 33160), (2040, 9432), (4096, 4400), (4352, 4232), (4360, 4240), (8192, 2072), (11008, 1640),
+                                 (13824, 640), (16384, 1104), (16640, 1192), (28672, 168), (41088, 120)])
+def test_matvec_stream_edges(K, N):
+    """The form that long and large products take: five pairs for 16 warps, one to four pairs per warp and none to 15 left over, a last pair with one
+    group and a last group that is not full, fewer tiles than SMs, tiles that do not divide by them, more than one pass of tiles."""
+    q, x, _ = mk(K, N, seed=K + N)
+    y = torch.full((N,), float("nan"), dtype=torch.float16, device="cuda")
+    ops.matmul(y, dev(x), ops.QWeight.from_numpy(q), K, N)
+    check_against_64_bits(y.cpu().numpy(), q, x, K, N, f"{K}x{N}")
+
+
+def test_streamed_products_of_several_matrices():
+    """q|k|v whose matrices end inside a CTA's tiles, gate/up in more than one pass of tiles, and the accumulating form."""
+    K, NQ, NKV = 4104, 2376, 1192
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal(K).astype(np.float16)
+    qs = [synth.synth_qweight(rng, K, n) for n in (NQ, NKV, NKV)]
+    Ws = [ops.QWeight.from_numpy(q) for q in qs]
+    qo = torch.zeros(NQ, dtype=torch.float16, device="cuda")
+    kc, vc = (torch.zeros((3, NKV), dtype=torch.float16, device="cuda") for _ in range(2))
+    ops.qkv_matvec(qo, kc, vc, dev(x), *Ws, K, NQ, 0, torch.full((1,), 2, dtype=torch.int32, device="cuda"), kvSize=NKV)
+    assert not kc[:2].any() and not vc[:2].any()
+    for got, q, n in zip((qo, kc[2], vc[2]), qs, (NQ, NKV, NKV)):
+        check_against_64_bits(got.cpu().numpy(), q, x, K, n, f"q|k|v {K}x{n}")
+    K, N = 1032, 16800     # 8400 tiles: 57 for some CTAs
+    x = (rng.standard_normal(K) * 0.1).astype(np.float16)
+    gate, up = (synth.synth_qweight(rng, K, N) for _ in range(2))
+    h = torch.empty(N, dtype=torch.float16, device="cuda")
+    ops.ffn_matvec_silu(h, dev(x), ops.QWeight.from_numpy(gate), ops.QWeight.from_numpy(up), K, N)
+    g, u = (O.dequant(q, K, N).astype(np.float64) @ x.astype(np.float64) for q in (gate, up))
+    want = g / (1 + np.exp(-g)) * u
+    # fp16 rounding of the result; expf and the reciprocal are good to a few units of 2^-23
+    assert np.abs(h.cpu().numpy() - want).max() <= 2.0**-11 * 1.02 * np.abs(want).max() + 1e-6
+    K, N = 11008, 1640
+    q, x, _ = mk(K, N, seed=9)
+    W, y = ops.QWeight.from_numpy(q), torch.zeros(N, dtype=torch.float16, device="cuda")
+    for _ in range(2):
+        ops.matmul(y, dev(x), W, K, N, accum=True)     # twice the product: half of one rounding and one of the sum
+    ref = O.dequant(q, K, N).astype(np.float64) @ x.astype(np.float64)
+    assert np.abs(y.cpu().numpy().astype(np.float64) / 2 - ref).max() <= 1.5 * 2.0**-11 * 1.01 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("held", [16, 31, 32, 80])
 def test_matvec_small_inputs_beside_many_held_ones(held):
     """`held` inputs of a group within 2^-15 of its largest, the others far below: rounded from 32 held ones on, exact below that."""
