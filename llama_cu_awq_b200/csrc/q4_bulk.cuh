@@ -1,4 +1,4 @@
-// Bulk copies (cp.async.bulk, 1-D, local memory) and the mbarriers they complete on.
+// Copies into shared memory: bulk ones (cp.async.bulk, 1-D, local memory) and the mbarriers they complete on, and cp.async.
 #pragma once
 #include "q4_common.cuh"
 
@@ -28,3 +28,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+
+// Copies of 16 bytes by the lanes (cp.async), in groups that a lane waits for in order
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }

@@ -318,10 +318,6 @@ __host__ __device__ constexpr int meta_row(int G) { return (G + 1) | 1; }
 constexpr int tiles_in_pass(int G, int PP) { return std::min(meta_bytes(PP) / (4 * kRows * meta_row(G)), kPassTiles); }
 }  // namespace stream
 
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // PP: pairs that every warp keeps; the items of the pairs that are left are dealt out over the warps.
 template <bool SILU, int PP>
 __global__ void __launch_bounds__(kThreads, 1) q4_gemv_stream_kernel(const __grid_constant__ GemvParams p) {

@@ -5,7 +5,9 @@
 // still read once per STEP, so the op stays bound by HBM as long as the per-weight work is small. That is what this
 // kernel is built for; the tcgen05 GEMM (q4_gemm.cu) takes over from M > 16, where the contraction starts to matter.
 //
-// Work split: a unit is 16 * MT output features of one launch over the whole K axis; one persistent CTA (12 warps; 8 for
+// Two forms of the kernel; streamed() has the line between them and both sides' figures.
+//
+// Sliced: a unit is 16 * MT output features of one launch over the whole K axis; one persistent CTA (12 warps; 8 for
 // 9-16 rows) per SM walks the units; a warp takes one share of a unit's 128-input groups, its own or, going round, share
 // (w + u) % warps of unit u, and the shares' partial tiles are summed in the order of the shares through shared memory (fixed order:
 // results are bit-reproducible, and the same either way). Inside a warp the product runs on mma.sync m16n8k16 (fp16 in, fp32 out) with
@@ -17,9 +19,19 @@
 // fp32 tile is scaled by the group's fp16 scale in fp32, as the reference does (gpu_kernels.h:222-228), so weights
 // are never rounded to fp16 after scaling.
 //
+//
+// Stream: a CTA of 16 warps per SM has consecutive tiles of 16 features. Each warp keeps the x fragments of its own groups (two with up to
+// eight rows, one with more) in registers for all of them, and the items of the groups that are left are dealt out over the warps tile by
+// tile; an item (16 features over a group, 1 KB) comes through the warp's private ring of four (cp.async; a lane reads what it has copied
+// itself, so that no barrier is needed), the first ones ahead of griddepcontrol.wait. Scales and zero points of a pass of tiles lie in shared
+// memory, one word for both. The warps' partial tiles wait there for one sum at the end of the pass. What bounds it: the unpack and the products (150 clocks of a scheduler per item where nothing else runs, about 220 here; HBM's
+// rate is 200) and, with few tiles, the start: x of all rows goes to every SM, 64 KB with 8 rows of 4096. gate/up of 7B, 8 rows 13.6 us = 3.5 TB/s
+// (17.0 sliced), 8192 -> 10240 15.3 = 2.9 (22.5), 70B gate/up 64.5 = 3.9 (77.4).
+//
 // Epilogues: plain, residual (y = product + residual * scale: matmul(QWeight)'s accum form, gpu_kernels.h:237-238),
 // and SiLU (ffn_matvec_silu_kernel, gpu_kernels.h:251-283: the CTA holds 16 gate and the same 16 up features and writes
 // silu(gate) * up without rounding gate or up to fp16 first).
+#include "q4_bulk.cuh"
 #include "q4_model.h"
 
 namespace {
@@ -325,6 +337,338 @@ __global__ void __launch_bounds__(warps_of(MT, NT) * 32, 1) q4_skinny_kernel(con
     if (p.late) griddep_launch_dependents();
 }
 
+// ------------------------------------------------------------------------------------------------------------
+// Stream form
+// ------------------------------------------------------------------------------------------------------------
+namespace stream {
+constexpr int kWarps = 16;
+constexpr int kThreads = 32 * kWarps;
+constexpr int kItemBytes = 1024;     // a tile's 16 rows over a group
+constexpr int kDepth = 4;            // items in a warp's ring, a multiple of those that are kept (12: 70B gate/up 83 us, 64: fewer tiles fit into a pass)
+constexpr int kSmemBytes = 226 * 1024;
+constexpr int kRingBytes = kWarps * kDepth * kItemBytes;
+__host__ __device__ constexpr int part_bytes(int NT) { return NT * kWarps * 512; }      // partial sums of a tile
+// Words of a row of scales and zero points (scale | zero point << 16): an odd number, so that the rows of a tile lie in different banks.
+__host__ __device__ constexpr int meta_row(int G) { return G | 1; }
+constexpr int tiles_in_pass(int G, int NT) { return (kSmemBytes - kRingBytes) / (part_bytes(NT) + 64 * meta_row(G)); }
+}  // namespace stream
+
+struct StreamParams {
+    SkParams s;
+    int tiles, nt_div, nt_mod;       // of 16 rows (SILU: eight gate and the same eight up features); CTA c has nt_div + (c < nt_mod) consecutive ones
+    int pass_tiles;
+    float inv_mrow;                  // 1 / meta_row(G)
+};
+
+// NT: batch columns of eight; GP: groups that every warp keeps; the items of the groups that are left are dealt out over the warps.
+template <int NT, int GP, bool SILU>
+__global__ void __launch_bounds__(stream::kThreads, 1) q4_rows_stream_kernel(const __grid_constant__ StreamParams r) {
+    using namespace stream;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const SkParams& p = r.s;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, cta = blockIdx.x;
+    const int cta_tile0 = cta * r.nt_div + min(cta, r.nt_mod), cta_tiles = r.nt_div + (cta < r.nt_mod);
+    const int g0 = w * GP, rest = p.G - GP * kWarps, mrow = meta_row(p.G);
+    uint8_t* const mine = smem + w * kDepth * kItemBytes + lane * 16;
+    float* const part = reinterpret_cast<float*>(smem + kRingBytes);
+    uint32_t* const meta = reinterpret_cast<uint32_t*>(smem + kRingBytes + r.pass_tiles * part_bytes(NT));
+    // matrix and row of row i (0-15) of a tile; the rows 0-7 and 8-15 are the product's
+    auto row_of = [&](int tile, int i, int& row) -> const SkMat& {
+        if (SILU) {
+            row = tile * 8 + (i & 7);
+            return p.m[i >> 3];
+        }
+        const int mi = p.nmat > 2 && tile >= p.m[2].tile0 ? 2 : p.nmat > 1 && tile >= p.m[1].tile0 ? 1 : 0;
+        row = (tile - p.m[mi].tile0) * 16 + i;
+        return p.m[mi];
+    };
+
+    // Walks this warp's items: in a pass its own groups tile by tile, then its share of the items of the groups that are left, group by group. A lane
+    // copies the 16 bytes of rows g and 8 + g that it reads.
+    const uint32_t dst0 = smem_u32(mine);
+    const int step = (SILU ? 8 : 16) * p.PW;
+    struct {
+        const uint32_t *src, *src8;  // rows g and 8 + g of the tile: its first own group, or the item (rest)
+        int tile, k, grp, left, b0, tiles;     // k < GP: own groups; GP: rest, `left` items of it to come, `grp` the group
+        int end;                     // the tiles of this pass and matrix end here
+    } q;
+    auto seek = [&](int grp) {
+        int row;
+        const SkMat& m = row_of(cta_tile0 + q.tile, g, row);
+        q.src = m.w + (size_t)row * p.PW + grp * 16 + t * 4;
+        q.src8 = SILU ? p.m[1].w + (size_t)row * p.PW + grp * 16 + t * 4 : q.src + 8 * p.PW;
+        q.end = q.b0 + q.tiles;
+        if (!SILU && p.nmat > 1) {
+            const int last = cta_tile0 + q.tile >= p.m[2].tile0 ? r.tiles : cta_tile0 + q.tile >= p.m[1].tile0 ? p.m[2].tile0 : p.m[1].tile0;
+            q.end = min(q.end, last - cta_tile0);
+        }
+    };
+    auto open_pass = [&]() {
+        q.tiles = min(r.pass_tiles, cta_tiles - q.b0);
+        q.tile = q.b0;
+        q.k = 0;
+        if (q.tiles > 0) seek(g0);
+    };
+    auto open_rest = [&]() {
+        const int r0 = w * rest * q.tiles / kWarps, r1 = (w + 1) * rest * q.tiles / kWarps;
+        q.k = GP;
+        q.left = r1 - r0;
+        q.grp = GP * kWarps + r0 / q.tiles;
+        q.tile = q.b0 + r0 % q.tiles;
+        if (q.left > 0) seek(q.grp);
+    };
+    auto settle = [&]() {      // past rests that are empty
+        while (q.tiles > 0 && q.k == GP && q.left == 0) {
+            q.b0 += q.tiles;
+            open_pass();
+        }
+    };
+    auto next = [&]() {
+        if (q.k < GP) {
+            if (++q.k < GP) return;
+            q.k = 0;
+            q.src += step;
+            q.src8 += step;
+            if (++q.tile < q.end) return;
+            if (q.tile < q.b0 + q.tiles) {
+                seek(g0);
+                return;
+            }
+            open_rest();
+        } else {
+            q.left--;
+            q.src += step;
+            q.src8 += step;
+            if (++q.tile == q.b0 + q.tiles) {
+                q.tile = q.b0;
+                q.grp++;
+                if (q.left > 0) seek(q.grp);
+            } else if (q.tile == q.end && q.left > 0) {
+                seek(q.grp);
+            }
+        }
+        settle();
+    };
+    auto request = [&](uint32_t slot) {      // (slot: its first byte)
+        if (q.k == GP && q.left > 1 && q.tile + 1 < q.end) {     // (the next item is the next tile's)
+            copy16(dst0 + slot, q.src);
+            copy16(dst0 + slot + 512, q.src8);
+            q.src += step;
+            q.src8 += step;
+            q.tile++;
+            q.left--;
+        } else if (q.tiles > 0) {
+            const int k = q.k < GP ? q.k * 16 : 0;
+            copy16(dst0 + slot, q.src + k);
+            copy16(dst0 + slot + 512, q.src8 + k);
+            next();
+        }
+        copies_commit();
+    };
+    q.b0 = q.left = q.end = q.tile = 0;
+    open_pass();
+    for (int i = 0; i < kDepth; i++) request(i * kItemBytes);
+    // A pass's scales and zero points into shared memory, several of a thread in flight.
+    constexpr int kFlight = NT == 2 ? 4 : 8;     // (registers)
+    struct Meta {
+        __half s[kFlight];
+        uint32_t z[kFlight];
+    };
+    auto fetch_meta = [&](Meta& v, int e0, int b0, int n) {
+#pragma unroll
+        for (int u = 0; u < kFlight; u++) {
+            const int e = e0 + u * kThreads, i = (int)(((float)e + 0.5f) * r.inv_mrow), grp = e - i * mrow;
+            v.s[u] = __float2half(0.f);
+            v.z[u] = 0;
+            if (e < n && grp < p.G) {
+                int row;
+                const SkMat& m = row_of(cta_tile0 + b0 + (i >> 4), i & 15, row);
+                v.s[u] = __ldg(m.s + (size_t)row * p.G + grp);
+                v.z[u] = __ldg(m.z + (size_t)row * p.PZ + (grp >> 3));
+            }
+        }
+    };
+    auto file_meta = [&](const Meta& v, int e0, int n) {
+#pragma unroll
+        for (int u = 0; u < kFlight; u++) {
+            const int e = e0 + u * kThreads, grp = e - (int)(((float)e + 0.5f) * r.inv_mrow) * mrow;
+            if (e < n) meta[e] = (uint32_t)__half_as_ushort(v.s[u]) | (((v.z[u] >> (4 * (grp & 7))) & 0xFu) << 16);
+        }
+    };
+    auto load_meta = [&](int e0, int b0, int n) {
+        for (; e0 < n; e0 += kFlight * kThreads) {
+            Meta v;
+            fetch_meta(v, e0, b0, n);
+            file_meta(v, e0, n);
+        }
+    };
+    Meta first;
+    const int first_n = min(r.pass_tiles, cta_tiles) * 16 * mrow;
+    fetch_meta(first, tid, 0, first_n);
+    griddep_wait();
+    if (!p.late) griddep_launch_dependents();
+
+    // The rows' inputs of a group, in the order of the unpacked pairs. 32 bytes in one access: with 16 every sector would come from L2 twice (next to
+    // this much shared memory there is little L1).
+    const bool whole = ((uintptr_t)p.x & 31) == 0;
+    auto load_x = [&](int grp, uint4 (&v)[NT][4]) {
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                uint4 &a = v[nt][j], &b = v[nt][j + 1];
+                a = b = make_uint4(0, 0, 0, 0);
+                if (g + 8 * nt >= p.M) continue;
+                const __half* src = p.x + (size_t)(g + 8 * nt) * p.K + 128 * grp + 32 * t + 8 * j;
+                if (whole) {
+                    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "l"(src));
+                } else {
+                    a = reinterpret_cast<const uint4*>(src)[0];
+                    b = reinterpret_cast<const uint4*>(src)[1];
+                }
+            }
+    };
+    struct X { uint32_t v[NT][4][4]; };
+    X xp[GP + 1];        // (the last one: a group that is left, for the tiles it is this warp's)
+    auto permute = [&](const uint4 (&v)[NT][4], X& x) {
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) permute_x8(v[nt][j], x.v[nt][j]);
+    };
+    {
+        uint4 xv[GP][NT][4];
+#pragma unroll
+        for (int k = 0; k < GP; k++) load_x(g0 + k, xv[k]);
+        file_meta(first, tid, first_n);
+        load_meta(tid + kFlight * kThreads, 0, first_n);
+#pragma unroll
+        for (int k = 0; k < GP; k++) permute(xv[k], xp[k]);
+    }
+
+    uint32_t slot = 0;           // the next item's, its first byte
+    // acc += one item's product; the copies that take its place are `more`'s
+    auto item = [&](float (&acc)[NT][4], const X& x, const uint32_t* me, auto&& more) {
+        copies_wait<kDepth - 1>();
+        const uint4 va = *reinterpret_cast<const uint4*>(mine + slot), vb = *reinterpret_cast<const uint4*>(mine + slot + 512);
+        const uint32_t ma = me[0], mb = me[8 * mrow];
+        const uint32_t wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
+        const uint32_t zla = 0x64006400u + (ma >> 16) * 0x00010001u, zha = 0x54005400u + (ma >> 16) * 0x00100010u;      // 1024 + z, 64 + z
+        const uint32_t zlb = 0x64006400u + (mb >> 16) * 0x00010001u, zhb = 0x54005400u + (mb >> 16) * 0x00100010u;
+        float c[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            uint32_t da[4], db[4];
+            unpack8(wa[j], zla, zha, da);
+            unpack8(wb[j], zlb, zhb, db);
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                mma_f16(c[nt], da[0], db[0], da[1], db[1], x.v[nt][j][0], x.v[nt][j][1]);
+                mma_f16(c[nt], da[2], db[2], da[3], db[3], x.v[nt][j][2], x.v[nt][j][3]);
+            }
+        }
+        more(slot);
+        slot += kItemBytes;
+        if (slot == kDepth * kItemBytes) slot = 0;
+        const float sa = __half2float(__ushort_as_half((unsigned short)(ma & 0xFFFFu))), sb = __half2float(__ushort_as_half((unsigned short)(mb & 0xFFFFu)));
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) {
+            acc[nt][0] = fmaf(sa, c[nt][0], acc[nt][0]);
+            acc[nt][1] = fmaf(sa, c[nt][1], acc[nt][1]);
+            acc[nt][2] = fmaf(sb, c[nt][2], acc[nt][2]);
+            acc[nt][3] = fmaf(sb, c[nt][3], acc[nt][3]);
+        }
+    };
+    for (int b0 = 0; b0 < cta_tiles; b0 += r.pass_tiles) {
+        const int tiles = min(r.pass_tiles, cta_tiles - b0);
+        float4* const col = reinterpret_cast<float4*>(part + w * 128) + lane;      // this lane's sums: [tile][NT][warp][lane]
+        __syncthreads();         // the pass's scales and zero points are in place, and the sums of the one before are done with
+        const uint32_t* me = meta + g * mrow + g0;
+        for (int i = 0; i < tiles; i++) {
+            float acc[NT][4];
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+            // Within the own groups of a pass and of a matrix the next requests are those of one tile.
+            if (q.tiles > 0 && q.k == 0 && q.tile + 1 < q.end) {
+#pragma unroll
+                for (int k = 0; k < GP; k++)
+                    item(acc, xp[k], me + k, [&](uint32_t at) {
+                        copy16(dst0 + at, q.src + k * 16);
+                        copy16(dst0 + at + 512, q.src8 + k * 16);
+                        copies_commit();
+                    });
+                q.src += step;
+                q.src8 += step;
+                q.tile++;
+            } else {
+#pragma unroll
+                for (int k = 0; k < GP; k++) item(acc, xp[k], me + k, request);
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) col[(i * NT + nt) * kWarps * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+            me += 16 * mrow;
+        }
+        // this warp's share of the items of the groups that are left
+        const int r0 = w * rest * tiles / kWarps, r1 = (w + 1) * rest * tiles / kWarps;
+        int grp = GP * kWarps + r0 / tiles, tile = r0 % tiles, left = r1 - r0;
+        while (left > 0) {
+            const int count = min(left, tiles - tile);
+            uint4 xv[NT][4];
+            load_x(grp, xv);
+            permute(xv, xp[GP]);
+            left -= count;
+            me = meta + (tile * 16 + g) * mrow + grp;
+            for (int i = tile; i < tile + count; i++) {
+                float acc[NT][4];
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++) {
+                    const float4 v = col[(i * NT + nt) * kWarps * 32];
+                    acc[nt][0] = v.x; acc[nt][1] = v.y; acc[nt][2] = v.z; acc[nt][3] = v.w;
+                }
+                item(acc, xp[GP], me, request);
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++) col[(i * NT + nt) * kWarps * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+                me += 16 * mrow;
+            }
+            grp++;
+            tile = 0;
+        }
+        __syncthreads();
+        // the warps' sums in warp order; lane 4g + t has rows g and 8 + g of the tile for batch rows 2t and 2t + 1
+        for (int i = w; i < tiles * NT; i += kWarps) {
+            const float4* src = reinterpret_cast<const float4*>(part) + (size_t)i * kWarps * 32 + lane;
+            float4 v = src[0];
+#pragma unroll
+            for (int u = 1; u < kWarps; u++) {
+                const float4 a = src[u * 32];
+                v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+            }
+            int f;
+            const SkMat& m = row_of(cta_tile0 + b0 + i / NT, g, f);
+            const int row = 8 * (i % NT) + 2 * t;
+            const float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < (SILU ? 2 : 4); e++) {
+                if (row + (e & 1) >= p.M) continue;
+                const size_t to = (size_t)(row + (e & 1)) * m.ldy + f + (e >> 1) * 8;
+                float y = o[e];
+                if (SILU) {
+                    y *= 1.0f / (1.0f + expf(-y));
+                    y *= o[e + 2];
+                } else if (p.residual) {
+                    y += __half2float(p.residual[to]) * p.rscale;
+                }
+                m.y[to] = __float2half(y);
+            }
+        }
+        if (b0 + tiles < cta_tiles) load_meta(tid, b0 + tiles, min(r.pass_tiles, cta_tiles - b0 - tiles) * 16 * mrow);
+    }
+    if (p.late) griddep_launch_dependents();
+}
+
+
 constexpr int kSms = 148;   // B200: one persistent CTA per SM (a smaller part would only leave CTAs queued behind the first wave)
 constexpr size_t unit_bytes(int MT, int NT) { return (size_t)warps_of(MT, NT) * MT * NT * 4 * 32 * sizeof(float); }
 
@@ -358,6 +702,9 @@ int launch_deal(const SkParams& p, int units, cudaStream_t s) {
     // (the limit belongs to the function: always the largest any launch needs)
     if (kSlots * unit_bytes(MT, NT) > 48 * 1024)
         Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU, DEAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSlots * unit_bytes(MT, NT))));
+    // x comes out of L1 again and again: behind a kernel that takes all of the SM's memory as shared (the stream form) the split would stay as it is
+    // (eight sequences, 32 steps of four 7B layers 7600 us, 6860 so).
+    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU, DEAL>, cudaFuncAttributePreferredSharedMemoryCarveout, 50));
     const size_t smem = (per_cta < kSlots ? per_cta : kSlots) * unit_bytes(MT, NT);
     Q4Launch L(dim3(units < kSms ? units : kSms), dim3(warps_of(MT, NT) * 32), smem, s);
     Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_skinny_kernel<MT, NT, SILU, DEAL>, p));
@@ -393,8 +740,43 @@ int launch_variant(const SkParams& p, cudaStream_t s) {
     return launch_deal<MT, NT, SILU, ROTATING>(p, units, s);
 }
 
+template <int NT, int GP, bool SILU>
+int launch_stream(const SkParams& p, cudaStream_t s) {
+    StreamParams r;
+    r.s = p;
+    r.tiles = SILU ? 2 * p.total_tiles : p.total_tiles;
+    const int grid = r.tiles < kSms ? r.tiles : kSms;
+    r.nt_div = r.tiles / grid;
+    r.nt_mod = r.tiles % grid;
+    const int most = r.nt_div + (r.nt_mod > 0);
+    r.pass_tiles = q4_div_up(most, q4_div_up(most, stream::tiles_in_pass(p.G, NT)));
+    r.inv_mrow = 1.0f / stream::meta_row(p.G);
+    // (the limit belongs to the function: always the largest any launch needs)
+    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_rows_stream_kernel<NT, GP, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, stream::kSmemBytes));
+    Q4Launch L(dim3(grid), dim3(stream::kThreads), (size_t)stream::kSmemBytes, s);
+    Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_rows_stream_kernel<NT, GP, SILU>, r));
+    return Q4_OK;
+}
+
+// The stream form where an SM has three or more of the tiles of 16 rows (gate/up: eight of each) and rows are 4096 inputs or longer; from
+// seven tiles also from 2048 inputs. us, sliced and stream, 8 rows and 16: 7B gate/up 17.0, 13.6 and 24.6, 21.8; q|k|v 10.3, 9.4 and 15.0, 13.3;
+// 13B q|k|v 20.1, 13.3 and 34.2, 18.6; gate/up 23.4, 19.2 and 36.1, 29.7; 13824 -> 5120 21.5, 17.1 and 34.7, 23.3; 70B gate/up 77.4, 64.5 and 120,
+// 89; 8192 -> 10240 22.5, 15.3 and 36.1, 20.8; 2048 -> 16384 9.9, 7.8 and 14.7, 9.8. Below, the sliced form's shorter start wins: two tiles 7B o 4.7,
+// 5.5 and 5.7, 8.0; 11008 -> 4096 9.5, 11.4 and 12.8, 16.7; 2048 -> 3 x 4096 6.0, 6.8 and 8.2, 8.6. Four tiles (445 to 592 in all) are two even rounds of
+// the sliced form's pairs, which keeps up then: 4096 -> 3 x 3072 8.1, 8.2 and 10.6, 11.5; 8192 x 8192 13.4, 13.5 and 19.6, 18.1.
+bool streamed(int G, int tiles) {
+    const int most = q4_div_up(tiles, kSms);
+    if (stream::tiles_in_pass(G, 2) == 0) return false;
+    if (G < 32) return G >= 16 && most >= 7;
+    return most >= 3 && (most != 4 || G >= 64);
+}
+
 template <bool SILU>
 int launch(const SkParams& p, cudaStream_t s) {
+    if (streamed(p.G, SILU ? 2 * p.total_tiles : p.total_tiles)) {
+        if (p.M > 8) return launch_stream<2, 1, SILU>(p, s);
+        return p.G >= 2 * stream::kWarps ? launch_stream<1, 2, SILU>(p, s) : launch_stream<1, 1, SILU>(p, s);
+    }
     const bool two = p.M > 8;
     if (SILU) return two ? launch_variant<2, 2, true>(p, s) : launch_variant<2, 1, true>(p, s);
     // Two tiles per unit halve the reads of x but double the grain the work is dealt in: take pairs when the most loaded

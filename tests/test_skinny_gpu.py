@@ -127,3 +127,56 @@ def test_rejects_unsupported_arguments():
     assert L.q4_matmul_q4_rows(s, ops._p(y), ops._p(x), W.ref, 4, 96, 16, None, 0.0) == _lib.Q4_ERR_UNSUPPORTED_SIZE     # K % 128
     assert L.q4_matmul_q4_rows(s, ops._p(y), ops._p(x), W.ref, 4, 128, 8, None, 0.0) == _lib.Q4_ERR_UNSUPPORTED_SIZE     # N % 16
     assert L.q4_qkv_matmul_rows(s, ops._p(y), ops._p(y), ops._p(y), ops._p(x), W.ref, W.ref, W.ref, 4, 128, 16, 16) == _lib.Q4_ERR_UNSUPPORTED_SIZE
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("K,N", [(2048, 16640), (2176, 16592), (4096, 4752), (4224, 4768), (5120, 28672), (8064, 7120)])
+def test_streamed_rows(M, K, N):
+    """The form with x in registers: no groups left over, one, and more than warps; an odd number of groups; a number of tiles that does not divide by the
+    SMs; more than one pass of tiles; x on 16 bytes instead of 32. fp16 rounding of the result and fp32 sums."""
+    rng = np.random.default_rng(M + K + N)
+    q = synth.synth_qweight(rng, K, N)
+    x = _x(rng, M, K)
+    W = ops.QWeight.from_numpy(q)
+    w = O.dequant(q, K, N)
+    want = torch.from_numpy(x).cuda().double() @ torch.from_numpy(w).cuda().double().T
+    buf = torch.zeros(M * K + 8, dtype=torch.float16, device="cuda")
+    outs = []
+    for skip in (0, 8):
+        xd = buf[skip:skip + M * K]
+        xd.copy_(torch.from_numpy(x).cuda().flatten())
+        y = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        ops.matmul_rows(y, xd, W, M, K, N)
+        torch.cuda.synchronize()
+        outs.append(y)
+    assert torch.equal(outs[0], outs[1])
+    # 2^-11 of each value, and sums of K / 128 group sums of 128 products each
+    bound = 2.0**-11 * want.abs() + 2.0**-23 * (K / 128 + 128) * (torch.from_numpy(x).cuda().double().abs() @ torch.from_numpy(w).cuda().double().abs().T) + 2.0**-25
+    assert ((outs[0].double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M", [3, 12])
+def test_streamed_rows_of_several_matrices(M):
+    """q|k|v whose matrices end inside a CTA's tiles, gate/up, and the residual form in place."""
+    K, NQ, NKV = 4224, 3232, 992
+    rng = np.random.default_rng(M)
+    x = _x(rng, M, K)
+    xd = torch.from_numpy(x).cuda()
+    qs = [synth.synth_qweight(rng, K, n) for n in (NQ, NKV, NKV)]
+    Ws = [ops.QWeight.from_numpy(q) for q in qs]
+    outs = [torch.full((M, n), float("nan"), dtype=torch.float16, device="cuda") for n in (NQ, NKV, NKV)]
+    ops.qkv_matmul_rows(*outs, xd, *Ws, M, K, NQ, NKV)
+    for y, q, n in zip(outs, qs, (NQ, NKV, NKV)):
+        assert_close(y.cpu().numpy(), x.astype(np.float64) @ O.dequant(q, K, n).astype(np.float64).T, f"{M} rows, {n} of q|k|v", max_rel=1e-3)
+    N = 2608      # 326 tiles of eight gate and eight up rows
+    gate, up = (synth.synth_qweight(rng, K, N) for _ in range(2))
+    h = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    ops.ffn_silu_rows(h, xd, ops.QWeight.from_numpy(gate), ops.QWeight.from_numpy(up), M, K, N)
+    g, u = (x.astype(np.float64) @ O.dequant(q, K, N).astype(np.float64).T for q in (gate, up))
+    assert_close(h.cpu().numpy(), g / (1 + np.exp(-g)) * u, f"{M} rows, silu(gate) * up", max_rel=1e-3)
+    N = 4800
+    q = synth.synth_qweight(rng, K, N)
+    res = rng.standard_normal((M, N)).astype(np.float16)
+    y = torch.from_numpy(res.copy()).cuda()
+    ops.matmul_rows(y, xd, ops.QWeight.from_numpy(q), M, K, N, residual=y, residual_scale=0.5)
+    assert_close(y.cpu().numpy(), x.astype(np.float64) @ O.dequant(q, K, N).astype(np.float64).T + 0.5 * res, f"{M} rows, residual", max_rel=1e-3)
