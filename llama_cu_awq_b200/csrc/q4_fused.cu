@@ -1,4 +1,4 @@
-// Fused decode path: ONE persistent cooperative kernel per token (one CTA per SM) instead of ~9 launches per layer.
+// Fused decode path: ONE persistent cooperative kernel per token (one CTA per SM; a prompt fed token by token: per 32 positions) instead of ~9 launches per layer.
 // Replaces the launch sequence of run_llama_network (llama2_q4.cu:430-538), on one GPU or on every rank of a
 // tensor-parallel group (hybrid split, llama2_q4.cu:45-50).
 //
@@ -113,7 +113,8 @@ struct FParams {
     int g, rank, vocab_off, vocab_size;
     unsigned launch_parity;
     uint32_t *hb, *qkv;      // tagged, in exchange layout: SiLU output; q | k | v
-    unsigned tag_base;
+    unsigned tag_base;       // of the first position
+    int n_tokens;            // positions of this launch, one after the other; the hand-off is the last one's
     __half *logits, *kc, *vc;
     const __half *emb, *wcls;
     const float* rope;       // [seq_len][64] (cos, sin)
@@ -127,7 +128,7 @@ struct FParams {
     unsigned long long bar_base;  // barriers completed by earlier launches
     int* status;
     int write_token;
-    int no_handoff;              // 1: leave the token mailbox and the position alone (a sampling kernel follows on the stream)
+    int no_handoff;              // 1: leave the token mailbox and the last position's step alone (a sampling kernel follows on the stream)
     int debug;                   // test build only (Q4_TEST_BUILD; always 0 and compiled out of the product library):
                                  // 1 = consumers skip the waits and the math (pure streaming), 16 = tensor-parallel exchange kept local (no NVLink dependency)
     unsigned long long wait_ns;  // limit of every device-side wait on the global timer; on expiry the kernel records Q4_ERR_TIMEOUT
@@ -204,7 +205,7 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 }
 
 // ---- tagged activations -----------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t tag_of(const FParams& p, int phase) { return ((p.tag_base + (unsigned)phase + 1u) & 0xFFFFu) << 16; }
+__device__ __forceinline__ uint32_t tag_of(unsigned base, int phase) { return ((base + (unsigned)phase + 1u) & 0xFFFFu) << 16; }   // base: the position's first
 __device__ __forceinline__ uint32_t tagged(__half v, uint32_t tag_hi) { return tag_hi | (uint32_t)__half_as_ushort(v); }
 // Tagged words are exchanged between CTAs without a barrier, so both sides use strong (volatile) accesses: a weak load
 // may be served from a stale copy for as long as it likes (observed: polling with ld.global.cg never saw the update),
@@ -353,6 +354,7 @@ struct Requests {           // the segment being requested: this warp's chunks o
     uint32_t left, chunk;   // bytes left in it, bytes per chunk
     uint32_t step;          // distance between chunks
     int seg, rot, row;
+    int more;               // positions behind the one it belongs to
 };
 struct Ring {
     uint8_t* base;
@@ -366,7 +368,13 @@ __device__ __forceinline__ void next_segment(Requests& r, const FParams& p, cons
     const int cta = blockIdx.x, grid = gridDim.x, w = threadIdx.x >> 5;
     int seg = r.seg, rot = r.rot;
     r.left = 0;
-    while (seg < K_KINDS * p.n_layers) {
+    for (;;) {
+        if (seg == K_KINDS * p.n_layers) {
+            if (r.row < p.v_n || r.more == 0) break;
+            r.more--;
+            r.row = cta * kW + w;
+            seg = rot = 0;
+        }
         const FKind& k = p.kind[seg & (K_KINDS - 1)];
         const Share s = share_of(k, rot, cta, grid, w);
         rot = next_rot(k, rot, grid);
@@ -564,7 +572,8 @@ __device__ __forceinline__ void rotate_head(const FParams& p, int first_tile, ui
 // The kernel
 // ------------------------------------------------------------------------------------------------------------
 // kFar: the table of addresses stays in global memory (so many layers that it would leave the rings too little).
-template <bool kFar>
+// kMany: several positions in one launch (a form of its own: with the loop around it a single position took 1 us longer).
+template <bool kFar, bool kMany>
 __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_constant__ FParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full_bar[kW * kMaxDepth];
@@ -572,6 +581,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     __shared__ float ssq[(kMaxDim + 255) / 256];
     __shared__ __align__(16) __half new_row[3][128];   // this position's rotated query, rotated key and value of the head at hand
     __shared__ float sm_m[kW], sm_l[kW];
+    __shared__ int next_id;            // kMany: token of the position behind this one (CTAs that embed)
     __shared__ int sm_i[kW];
 
     uint4* const xs = reinterpret_cast<uint4*>(smem + p.x_off);               // residual stream (fp16); the classifier's input
@@ -604,32 +614,35 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         Requests& r = requests[w];
         r.seg = r.rot = 0;
         r.row = cta * kW + w;
+        r.more = kMany ? p.n_tokens - 1 : 0;
         next_segment(r, p, streams);
         for (int i = 0; i < p.depth; i++) ring_request(ring, i, p, streams);
     }
     __syncwarp();
 
     uint8_t* const scr = smem + p.scr_off + w * kPairScratch;
-    const int pos = *p.pos_dev;
-    unsigned nbar = 0;
-    int rot = 0;
+    int pos = *p.pos_dev;
+    unsigned nbar = 0, tag0 = p.tag_base;
+    int token_pos = 0;
+    const bool embeds = cta * kThreads < p.dim / 8;      // (the grid has more threads than the longest x has words)
 
+    const int n_tokens = kMany ? p.n_tokens : 1;
+    for (int more = n_tokens - 1;; more--) {
     // ---- embedding: copy_embedding_kernel (gpu_kernels.h:61-69); the token id comes from the pinned host mailbox ----
     TRACE(0, 0);
-    if (cta * kThreads + tid < p.dim / 8) {
-        const int token = p.tokens_pinned[pos];
-        const uint4* src = reinterpret_cast<const uint4*>(p.emb + (size_t)token * p.dim);
-        const uint32_t tg = tag_of(p, 0);
+    int rot = 0;
+    const int word = cta * kThreads + tid;
+    if (word < p.dim / 8) {
+        const int token = more == n_tokens - 1 ? p.tokens_pinned[pos] : next_id;
+        const uint4 v = reinterpret_cast<const uint4*>(p.emb + (size_t)token * p.dim)[word];
+        const uint32_t tg = tag_of(tag0, 0);
         // every rank files the row as slot 0 of its own buffer 1 and zeros as the other ranks' partials
-        for (int i = cta * kThreads + tid; i < p.dim / 8; i += grid * kThreads) {
-            const uint4 v = src[i];
-            uint32_t* dst = p.xb[1][p.rank] + exchange_at(p.kind[K_DOWN], i);
-            st_tagged4(dst, make_uint4(tg | (v.x & 0xFFFFu), tg | (v.x >> 16), tg | (v.y & 0xFFFFu), tg | (v.y >> 16)));
-            st_tagged4(dst + 4, make_uint4(tg | (v.z & 0xFFFFu), tg | (v.z >> 16), tg | (v.w & 0xFFFFu), tg | (v.w >> 16)));
-            for (int r = 1; r < p.g; r++) {
-                st_tagged4(dst + (size_t)r * kLLMaxDim, make_uint4(tg, tg, tg, tg));
-                st_tagged4(dst + (size_t)r * kLLMaxDim + 4, make_uint4(tg, tg, tg, tg));
-            }
+        uint32_t* dst = p.xb[1][p.rank] + exchange_at(p.kind[K_DOWN], word);
+        st_tagged4(dst, make_uint4(tg | (v.x & 0xFFFFu), tg | (v.x >> 16), tg | (v.y & 0xFFFFu), tg | (v.y >> 16)));
+        st_tagged4(dst + 4, make_uint4(tg | (v.z & 0xFFFFu), tg | (v.z >> 16), tg | (v.w & 0xFFFFu), tg | (v.w >> 16)));
+        for (int r = 1; r < p.g; r++) {
+            st_tagged4(dst + (size_t)r * kLLMaxDim, make_uint4(tg, tg, tg, tg));
+            st_tagged4(dst + (size_t)r * kLLMaxDim + 4, make_uint4(tg, tg, tg, tg));
         }
     }
 
@@ -637,6 +650,9 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         const int layer = seg / K_KINDS, f = seg % K_KINDS;
         const int pi0 = 1 + layer * kLayerPhases;
         const long long loff = layer * p.layer_stride;
+        // The next position's token, from host memory, while nobody waits for it
+        if (kMany && more > 0 && seg == K_KINDS * (p.n_layers - 1) && embeds && tid == 0)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&next_id)), "l"(p.tokens_pinned + pos + 1) : "memory");
 
         if (f == K_O && !(Q4_DBG(p) & 1)) {
             // ---- attention of one query per head over positions 0..pos, split over CTAs (llama2_q4.cu:410-427) ----
@@ -652,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
             const float alpha = (float)(1.0 / sqrt(128.0));
             const int ns = attn_splits_for(p, T);
             const int nitems = p.n_heads * ns;
-            const uint32_t want = tag_of(p, pi0 + LP_QKV), out_tag = tag_of(p, pi);
+            const uint32_t want = tag_of(tag0, pi0 + LP_QKV), out_tag = tag_of(tag0, pi);
             const __half* kc = p.kc + loff;
             const __half* vc = p.vc + loff;
             for (int id = cta; id < nitems; id += grid) {
@@ -817,7 +833,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         if (norm) {
             nw = norms[2 * layer + (f == K_GU)];
             if (left > 0 && (pair * 32 + lane) * 8 < kd.K) nwv = __ldg(reinterpret_cast<const uint4*>(nw) + pair * 32 + lane);
-            if (!(Q4_DBG(p) & 1)) inv_rms = stage_residual(p, f == K_QKV ? 1 : 0, tag_of(p, f == K_QKV ? pi - 1 : pi0 + LP_O), xs, ssq, w, lane, 0x60000 + pi);
+            if (!(Q4_DBG(p) & 1)) inv_rms = stage_residual(p, f == K_QKV ? 1 : 0, tag_of(tag0, f == K_QKV ? pi - 1 : pi0 + LP_O), xs, ssq, w, lane, 0x60000 + pi);
         }
         TRACE(pi, 4);
         Tagged8 ahead;           // down: the next pair's words, requested while this one is worked on
@@ -843,12 +859,12 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                     AttnWord aw;
                     for (;;) {   // this poll is the op boundary between the attention phase and the o projection
                         uint32_t bad = 0;
-                        attn_word_load(aw, p, ns, wd, valid, tag_of(p, pi - 1), bad);
+                        attn_word_load(aw, p, ns, wd, valid, tag_of(tag0, pi - 1), bad);
                         if (bad == 0 || !keep_polling(polls, t0, p.status, p.wait_ns, 0x80000 + pi)) break;
                     }
                     if (valid) hv = attn_word_merge(aw);
                 } else {
-                    const uint32_t want = tag_of(p, pi - 1);
+                    const uint32_t want = tag_of(tag0, pi - 1);
                     auto load = [&](int word) {   // 8 elements: two tiles of the gate/up step
                         ahead.a = ld_poll(reinterpret_cast<const uint4*>(p.hb + exchange_at(p.kind[K_GU], 2 * word)));
                         ahead.b = ld_poll(reinterpret_cast<const uint4*>(p.hb + exchange_at(p.kind[K_GU], 2 * word + 1)));
@@ -914,7 +930,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         __syncthreads();
         TRACE(pi, 2);
         // ---- sums over the warps (in warp order) and outputs: thread 8 * tile + row ----
-        const uint32_t out_tag = tag_of(p, pi);
+        const uint32_t out_tag = tag_of(tag0, pi);
         const int out_at = s.run * kd.xstride;     // this CTA's lines of the output vector
         for (int e0 = w * 32; e0 < s.tiles * 8; e0 += kThreads) {
             const int e = e0 + lane, r = e & 7, t = s.t0 + (e >> 3);
@@ -958,7 +974,6 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     }
 
     // ---- classifier: fp16 rows streamed through the same rings, one warp per row; per-CTA argmax candidate ----
-    int token_pos = 0;
     {
         const int pi = p.nphases - 2;
         TRACE(pi, 0);
@@ -966,10 +981,12 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         // Host memory: read at the hand-off it was two to three microseconds of every token (four 7B layers 149 -> 146 us per position).
         if (cta == 0 && tid == 0) token_pos = *p.pos_pinned;
         if (!(Q4_DBG(p) & 1)) {
-            const float inv_rms = stage_residual(p, 1, tag_of(p, pi - 1), xs, ssq, w, lane, 0x60000 + pi);
+            const float inv_rms = stage_residual(p, 1, tag_of(tag0, pi - 1), xs, ssq, w, lane, 0x60000 + pi);
             for (int i = tid; i < nwords; i += kThreads) xs[i] = norm_word(xs[i], __ldg(reinterpret_cast<const uint4*>(p.rms_final) + i), inv_rms);
         }
+        if (kMany) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
+        if (kMany && more > 0 && word < p.dim / 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(p.emb + (size_t)next_id * p.dim) + word));
         TRACE(pi, 1);
         float best = -CUDART_INF_F;
         int bi = 0x7fffffff;
@@ -1014,8 +1031,13 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
             p.cand_idx[cta] = bi;
         }
         TRACE(pi, 2);
+        // (A further position's embedding and its attention's reads of the cache are behind this barrier, as they are behind the launch else.)
         grid_barrier(p, nbar);
         TRACE(pi, 3);
+    }
+    if (!kMany || more == 0) break;
+    pos++;
+    tag0 += (unsigned)p.nphases;
     }
     if (ring.dead) {   // before the CTA's shared memory goes: every requested copy must have landed (bounded; the last slots may hold none)
         for (int n = p.depth; n > 0; n--) {
@@ -1049,7 +1071,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                 // mailbox. The system-scope fence orders this rank's logits slice (stored by all its CTAs before
                 // the grid barrier above) before the candidate, so a rank that holds all candidates also holds all
                 // logits. Every rank picks the same winner (highest value, lowest index).
-                const unsigned long long tg = (unsigned long long)(tag_of(p, pi) >> 16) << 32;
+                const unsigned long long tg = (unsigned long long)(tag_of(tag0, pi) >> 16) << 32;
                 const size_t slot = ((size_t)p.launch_parity * Q4_MAX_GPUS + p.rank) * 2;
                 if (lane == 0) {
                     __threadfence_system();
@@ -1082,9 +1104,9 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                     if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
                 }
             }
-            if (lane == 0 && !p.no_handoff) {
-                token_pos++;
-                if (p.write_token) p.tokens_pinned[token_pos] = (bi == 0x7fffffff) ? 0 : bi;
+            if (lane == 0 && (!p.no_handoff || kMany)) {
+                token_pos += n_tokens - (p.no_handoff ? 1 : 0);     // (a sampling kernel steps past the last position itself)
+                if (p.write_token && !p.no_handoff) p.tokens_pinned[token_pos] = (bi == 0x7fffffff) ? 0 : bi;
                 *p.pos_pinned = token_pos;
                 *p.pos_dev = token_pos;
             }
@@ -1193,10 +1215,10 @@ struct q4_fused {
     size_t smem_bytes = 0;
     int grid = 0;
     int barriers_per_launch = 0;
-    unsigned long long launches = 0;
+    unsigned long long launches = 0;   // positions, whatever the number of launches
     bool unsupported = false;
     bool far = false;               // the table of addresses does not fit beside the rings
-    void (*kernel)(FParams) = nullptr;
+    void (*kernel)(FParams) = nullptr, (*kernel_many)(FParams) = nullptr;   // one position, several
     unsigned long long* trace = nullptr;
     Q4LLArea* ll_local = nullptr;   // this rank's exchange area (inside the communicator's inbox, or own allocation at g = 1)
     size_t attn_part_bytes = 0, hb_bytes = 0, qkv_bytes = 0;
@@ -1482,13 +1504,16 @@ static int fused_build(q4_model* m, q4_fused* f) {
             for (int k = 0; k < 2; k++) all.push_back(norms[k][l]);
         FTRY(table((const void**)&p.table, all));
     }
-    f->kernel = f->far ? fused_token_kernel<true> : fused_token_kernel<false>;
+    f->kernel = f->far ? fused_token_kernel<true, false> : fused_token_kernel<false, false>;
+    f->kernel_many = f->far ? fused_token_kernel<true, true> : fused_token_kernel<false, true>;
     // (the limit belongs to the function, not to this model: always the largest any model may need, so that a smaller one prepared
     // later does not lower it)
     Q4_CUDA_TRY(cudaFuncSetAttribute(f->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
-    int per_sm = 0;
+    Q4_CUDA_TRY(cudaFuncSetAttribute(f->kernel_many, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+    int per_sm = 0, many_per_sm = 0;
     Q4_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f->kernel, kThreads, f->smem_bytes));
-    if (per_sm < 1) {
+    Q4_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&many_per_sm, f->kernel_many, kThreads, f->smem_bytes));
+    if (per_sm < 1 || many_per_sm < 1) {
         fprintf(stderr, "q4 fused path: kernel does not fit one SM (%zu B shared memory, %d threads)\n", f->smem_bytes, kThreads);
         f->unsupported = true;
         return Q4_ERR_UNSUPPORTED_SIZE;
@@ -1497,7 +1522,7 @@ static int fused_build(q4_model* m, q4_fused* f) {
     return Q4_OK;
 }
 
-int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff) {
+int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff, int n_tokens) {
     q4_fused* f = m->fused;
     if (!f || f->unsupported) return Q4_ERR_UNSUPPORTED_SIZE;
     if (!f->armed) return Q4_ERR_CUDA;   // the last re-arm did not complete
@@ -1512,12 +1537,14 @@ int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff)
     p.debug = g_test_debug & 31;
     if (g_test_split_len > 0) p.split_len = g_test_split_len;
 #endif
+    if (n_tokens < 1 || (n_tokens > 1 && m->g > 1)) return Q4_ERR_INVALID;
+    p.n_tokens = n_tokens;
     p.bar_base = f->launches * (unsigned long long)f->barriers_per_launch;
     p.tag_base = (unsigned)((f->launches * (unsigned long long)f->nphases) & 0xFFFFu);
     p.launch_parity = (unsigned)(f->launches & 1);
-    f->launches++;
+    f->launches += n_tokens;
     void* args[] = {&p};
-    Q4_CUDA_TRY(cudaLaunchCooperativeKernel((void*)f->kernel, dim3(f->grid), dim3(kThreads), args, f->smem_bytes, s));
+    Q4_CUDA_TRY(cudaLaunchCooperativeKernel((void*)(n_tokens > 1 ? f->kernel_many : f->kernel), dim3(f->grid), dim3(kThreads), args, f->smem_bytes, s));
     return Q4_OK;
 }
 

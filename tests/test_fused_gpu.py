@@ -326,3 +326,28 @@ def test_table_of_addresses_in_global_memory():
     finally:
         L.q4_test_set_far_table(0)
     assert (out[0].view(np.uint16) == out[1].view(np.uint16)).all()
+
+
+def test_many_positions_in_one_launch_with_the_far_table():
+    """Both forms of the table of addresses run a prompt's positions in one launch, three layers, 70 positions in three launches."""
+    L = _lib.test_lib()
+    cfg = (512, 768, 3, 4, 2, 512, 96, 10000.0)
+    tokens = np.random.default_rng(12).integers(3, 512, size=70, dtype=np.int32)
+    out = []
+    try:
+        for far in (0, 1):
+            L.q4_test_set_far_table(far)
+            t = Transformer(None, lib=L, synthetic=(cfg, 6))
+            assert t.best_path() == 2
+            t.generate(tokens, 70, path=2)
+            out.append(t.logits().view(np.uint16))
+            t.reset(tokens, 0)
+            for _ in range(70):
+                t.forward(gen_token=False, path=2)
+            t.synchronize()
+            out.append(t.logits().view(np.uint16))
+            assert t.status() == 0
+            t.close()
+    finally:
+        L.q4_test_set_far_table(0)
+    assert all((o == out[0]).all() for o in out[1:])

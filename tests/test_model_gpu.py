@@ -234,6 +234,42 @@ def test_generate_after_a_refused_call(mid_path, prompt_one_pass):
     fresh.close()
 
 
+@pytest.mark.parametrize("which", ["mid", "gqa"])
+@pytest.mark.parametrize("n_prompt,steps,temperature", [(2, 5, 0.0), (32, 32, 0.0), (33, 36, 0.0), (50, 50, 0.0), (50, 41, 0.0), (50, 55, 0.8), (50, 50, 0.8)])
+def test_generate_takes_a_prompts_positions_in_one_launch(which, n_prompt, steps, temperature, mid_path, mid_gqa_path):
+    """The fused kernel runs up to 32 prompt positions per launch: the same bits, ids and positions as one launch each."""
+    t = Transformer(mid_path if which == "mid" else mid_gqa_path)
+    if t.best_path() != 2:
+        pytest.skip("the fused kernel does not serve this model")
+    ids = np.random.default_rng(n_prompt).integers(3, t.config.vocab_size, size=n_prompt, dtype=np.int32)
+    t.set_sampler(temperature, 0.9, 11)
+    t.reset(ids, 0)
+    for pos in range(steps):
+        t.forward(gen_token=pos >= n_prompt - 1, path=2)
+        t.synchronize()
+        if t.shared().tokens[pos] == 2 and pos > 0:
+            break
+    want, want_pos, want_ids = t.logits().view(np.uint16), t.shared().pos, list(t.shared().tokens[:steps + 1])
+    for _ in range(2):
+        t.set_sampler(temperature, 0.9, 11)
+        out, timed, _ = t.generate(ids, steps, path=2)
+        assert (t.logits().view(np.uint16) == want).all()
+        assert t.shared().pos == want_pos and list(out[:want_pos]) == want_ids[:want_pos]
+    assert t.status() == 0
+    t.close()
+
+
+@pytest.mark.parametrize("end,ran", [(0, 45), (1, 2), (31, 32), (32, 33), (44, 45)])
+def test_generate_ends_behind_an_end_token_in_the_prompt(mid_path, end, ran):
+    """An end token that is not the first ends the generation behind its own position, in whichever launch it lies."""
+    t = Transformer(mid_path)
+    ids = np.random.default_rng(3).integers(3, t.config.vocab_size, size=45, dtype=np.int32)
+    ids[end] = 2
+    _, timed, _ = t.generate(ids, 45, path=2)
+    assert t.shared().pos == ran and timed == (ran - 2 if end else ran - 1)
+    t.close()
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_reset_and_generate_while_another_device_is_current(mid_path):
     t = Transformer(mid_path)
