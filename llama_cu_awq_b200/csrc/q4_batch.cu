@@ -28,18 +28,15 @@ cudaError_t launch_rows(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
     return cudaLaunchKernelEx(&L.cfg, kernel, KArgs(args)...);
 }
 
-// ids of the rows' tokens: tok_base[seq * tok_stride + pos]
-__global__ void embed_rows_kernel(__half* x, const __half* table, int dim, const int* tok_base, long long tok_stride, const int* row_seq, const int* row_pos,
-                                  int vocab) {
-    griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
-    griddep_launch_dependents();
-    const int m = blockIdx.x;
-    int token = tok_base[(long long)row_seq[m] * tok_stride + row_pos[m]];
-    if (token < 0 || token >= vocab) token = 0;   // (ids are validated on the host; a generated id is always in range)
-    const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)token * dim);
-    uint4* dst = reinterpret_cast<uint4*>(x + (size_t)m * dim);
-    for (int i = threadIdx.x; i < dim / 8; i += blockDim.x) dst[i] = src[i];
-}
+// Where the rows come from: row m is the token at tok_base[seq * tok_stride + pos] of sequence row_seq[m] and position row_pos[m]; pos0 >= 0: of sequence 0 and
+// position pos0 + m, and the two are written.
+struct Embed {
+    const __half* table;
+    const int* tok_base;
+    long long tok_stride;
+    int *row_seq, *row_pos;
+    int vocab, pos0;
+};
 
 // rmsnorm_kernel (gpu_kernels.h:72-105) per row: o = x * (rsqrt(mean(x^2) + 1e-5) * w), fp32 inside, fp16 out.
 // size % 8 == 0; a thread keeps up to four 8-element pieces of the row in registers between the two passes.
@@ -78,13 +75,27 @@ __device__ __forceinline__ uint4 add8(const uint4& x, const uint4& y) {
     }
     return o;
 }
-// ADD: the row is x + y first, and goes back to x (a prompt's projections on one GPU: the GEMM's own residual epilogue reads two
-// bytes per lane and row, 20 us per 512 x 4096 tile row, where this pass has the row in registers anyway).
-template <bool ADD>
-__global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __half* x, const __half* y, const __half* w, int size) {
+// ROW_ADD: the row is x + y first, and goes back to x (a prompt's projections on one GPU: the GEMM's own residual epilogue reads two
+// bytes per lane and row, 20 us per 512 x 4096 tile row, where this pass has the row in registers anyway). ROW_EMBED: it is its token's row of the
+// table, and goes to x (as kernels of their own the rows' positions and embedding were two launches in front of the first product: 78 tokens of two 13B
+// layers 316.5 us, 308.8 so; 333 behind 700 of a 70B layer 180.4, 176).
+enum RowSource { ROW_X, ROW_ADD, ROW_EMBED };
+template <RowSource SRC>
+__global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __half* x, const __half* y, const __half* w, int size, Embed em) {
     griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
     griddep_launch_dependents();
     __shared__ float red[kRowThreads / 32];
+    const uint4* token_row = nullptr;
+    if (SRC == ROW_EMBED) {
+        const int m = blockIdx.x, seq = em.pos0 >= 0 ? 0 : em.row_seq[m], pos = em.pos0 >= 0 ? em.pos0 + m : em.row_pos[m];
+        int token = em.tok_base[(long long)seq * em.tok_stride + pos];
+        if (token < 0 || token >= em.vocab) token = 0;   // (ids are validated on the host; a generated id is always in range)
+        token_row = reinterpret_cast<const uint4*>(em.table + (size_t)token * size);
+        if (em.pos0 >= 0 && threadIdx.x == 0) {
+            em.row_seq[m] = 0;
+            em.row_pos[m] = pos;
+        }
+    }
     uint4* xr = reinterpret_cast<uint4*>(x + (size_t)blockIdx.x * size);
     const uint4* yr = reinterpret_cast<const uint4*>(y + (size_t)blockIdx.x * size);
     uint4* orow = reinterpret_cast<uint4*>(o + (size_t)blockIdx.x * size);
@@ -94,11 +105,9 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(__half* o, __
     uint4 v[kKeep], wk[kKeep];   // (the weights are requested with the row: behind the sum they were a memory latency of their own)
     float ss = 0.f;
     auto row = [&](int i) {
-        uint4 r = xr[i];
-        if (ADD) {
-            r = add8(r, yr[i]);
-            xr[i] = r;
-        }
+        uint4 r = SRC == ROW_EMBED ? token_row[i] : xr[i];
+        if (SRC == ROW_ADD) r = add8(r, yr[i]);
+        if (SRC != ROW_X) xr[i] = r;
         return r;
     };
 #pragma unroll
@@ -509,17 +518,6 @@ __global__ void set_pos_kernel(int* pos_dev, volatile int* pos_pinned, int pos) 
     *pos_pinned = pos;
 }
 
-// rows = positions pos0, pos0 + 1, ... of sequence 0
-__global__ void iota_rows_kernel(int* row_seq, int* row_pos, int n, int pos0) {
-    griddep_wait();   // launched with programmatic stream serialisation: wait for the producer, then let the consumer's prologue start
-    griddep_launch_dependents();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        row_seq[i] = 0;
-        row_pos[i] = pos0 + i;
-    }
-}
-
 // mat_vec_kernel (gpu_kernels.h:117-147) for B rows of x at once: a warp takes one classifier row and B dot products, so the
 // classifier is read once per step, not once per sequence. x rows sit in shared memory. B <= 16.
 __global__ void __launch_bounds__(256) matvec_f16_rows_kernel(__half* y, const __half* x, const __half* w, int n, int d, int B, int y_stride) {
@@ -845,12 +843,13 @@ static int rows_all_reduce(q4_model* m, cudaStream_t s, __half* buf, size_t coun
 // or nothing but the K/V rows (a prompt whose last position follows through another path).
 enum RowsWanted { WANT_ALL, WANT_LAST, WANT_CACHE };
 
-// All layers for `n` rows whose embeddings are in r->X; K/V rows go to (kc, vc) with `seq_stride` halfs between sequences.
-// pos0 >= 0: the rows are positions pos0 .. pos0 + n - 1 of one sequence (prompt); -1: one row per sequence (batched decode).
+// All layers for `n` rows, from their tokens' embeddings on; K/V rows go to (kc, vc) with `seq_stride` halfs between sequences.
+// embed.pos0 >= 0: the rows are positions pos0 .. pos0 + n - 1 of one sequence (prompt); -1: one row per sequence (batched decode).
 // In the last layer the rows that nobody asks for end at their K/V row: no later layer reads them.
-// row_seq, row_pos: the rows' sequences and positions, on the device.
-static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, const int* row_pos, __half* kc, __half* vc, long long seq_stride, int pos0, RowsWanted want) {
+// embed.row_seq, embed.row_pos: the rows' sequences and positions, on the device.
+static int rows_layers(q4_model* m, cudaStream_t s, int n, const Embed& embed, __half* kc, __half* vc, long long seq_stride, RowsWanted want) {
     q4_rows* r = m->rows;
+    const int *row_seq = embed.row_seq, *row_pos = embed.row_pos, pos0 = embed.pos0;
     const q4_config& c = m->cfg;
     const int g = m->g, dim = c.dim;
     const int heads = c.n_heads / g, kv_heads = c.n_kv_heads / g;
@@ -882,13 +881,14 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, c
     const bool fused_add = !skinny && g == 1;
     if (pos0 >= 0 && !skinny) Q4_CUDA_TRY(cudaFuncSetAttribute(attention_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAtSmem));
     auto norm = [&](const __half* w, const __half* y) {
-        if (y) launch_rows(rmsnorm_rows_kernel<true>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, y, w, dim);
-        else launch_rows(rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, w, dim);
+        if (y) launch_rows(rmsnorm_rows_kernel<ROW_ADD>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, y, w, dim, Embed{});
+        else launch_rows(rmsnorm_rows_kernel<ROW_X>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, w, dim, Embed{});
     };
     for (int l = 0; l < c.n_layers; l++) {
         const DevLayer& L = m->layers[l];
         const long long loff = (long long)l * c.seq_len * m->kv_n;
-        norm((const __half*)L.rms_att, fused_add && l > 0 ? r->Y : nullptr);
+        if (l == 0) launch_rows(rmsnorm_rows_kernel<ROW_EMBED>, dim3(n), dim3(kRowThreads), 0, s, r->XB, r->X, (const __half*)nullptr, (const __half*)L.rms_att, dim, embed);
+        else norm((const __half*)L.rms_att, fused_add ? r->Y : nullptr);
         // The last layer of a prompt: nobody reads the other rows' queries (of 70B's q|k|v four fifths; 333 rows behind 700 of one 70B layer
         // 222 us, 203 so; 2000 rows of two 7B layers 1113, 1064), so k and v alone go through the GEMM and the last row's query, if asked
         // for, through the batch-1 product.
@@ -920,7 +920,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const int* row_seq, c
                                    row_pos + last));
             OP(q4_matmul_q4(s, x, (const uint16_t*)r->ATT, &L.o.w, m->o_kc, dim, 1, g, -1, nullptr));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
-            launch_rows(rmsnorm_rows_kernel<false>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim);
+            launch_rows(rmsnorm_rows_kernel<ROW_X>, dim3(1), dim3(kRowThreads), 0, s, r->XB, (__half*)x, (const __half*)nullptr, (const __half*)L.rms_ffn, dim, Embed{});
             OP(q4_ffn_matvec_silu(s, (uint16_t*)r->G, (const uint16_t*)r->XB, &L.gate.w, &L.up.w, dim, m->h_kc));
             OP(q4_matmul_q4(s, x, (const uint16_t*)r->G, &L.down.w, m->h_kc, dim, 1, g, -1, nullptr));
             OP(rows_all_reduce(m, s, (__half*)x, dim, true));
@@ -975,9 +975,8 @@ static int prefill(q4_model* m, cudaStream_t s, int n, int gen_token, bool logit
     int e;
     if ((e = rows_prepare(m, n)) != Q4_OK) return e;
     q4_rows* r = m->rows;
-    launch_rows(iota_rows_kernel, dim3(q4_div_up(n, 256)), dim3(256), 0, s, r->row_seq, r->row_pos, n, pos0);
-    launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size);
-    if ((e = rows_layers(m, s, n, r->row_seq, r->row_pos, (__half*)m->kc, (__half*)m->vc, 0, pos0, logits ? WANT_LAST : WANT_CACHE)) != Q4_OK) return e;
+    const Embed embed = {(const __half*)m->emb, (const int*)m->shared->tokens, 0, r->row_seq, r->row_pos, c.vocab_size, pos0};
+    if ((e = rows_layers(m, s, n, embed, (__half*)m->kc, (__half*)m->vc, 0, logits ? WANT_LAST : WANT_CACHE)) != Q4_OK) return e;
     if ((e = move_pos(m, s, logits ? pos0 + n - 1 : pos0 + n)) != Q4_OK) return e;
     if (logits) {
         // the last row goes on through the batch-1 tail (llama2_q4.cu:528-537, sampler.h:77-84): final norm, classifier,
@@ -1106,9 +1105,9 @@ static int batch_step(q4_batch* b, cudaStream_t s) {
     const q4_config& c = m->cfg;
     const int n = b->n_seq;
     // row i is sequence i, and the hand-off moves the positions only when every kernel of the step has read them: no copies of either
-    launch_rows(embed_rows_kernel, dim3(n), dim3(kRowThreads), 0, s, r->X, (const __half*)m->emb, c.dim, b->tokens, b->max_len + 1, b->seq, b->pos, c.vocab_size);
-    if (int e = rows_layers(m, s, n, b->seq, b->pos, b->kc, b->vc, b->seq_stride, -1, WANT_ALL)) return e;
-    launch_rows(rmsnorm_rows_kernel<false>, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)nullptr, (const __half*)m->rms_final, c.dim);
+    const Embed embed = {(const __half*)m->emb, b->tokens, b->max_len + 1, b->seq, b->pos, c.vocab_size, -1};
+    if (int e = rows_layers(m, s, n, embed, b->kc, b->vc, b->seq_stride, WANT_ALL)) return e;
+    launch_rows(rmsnorm_rows_kernel<ROW_X>, dim3(n), dim3(kRowThreads), 0, s, b->xf, r->X, (const __half*)nullptr, (const __half*)m->rms_final, c.dim, Embed{});
     const size_t smem = 2 * (size_t)n * c.dim;
     __half* cls_out = m->g == 1 ? b->logits : b->part;   // TP: every rank computes its vocabulary slice of every row; the slices are gathered row by row
     const int cls_stride = m->g == 1 ? c.vocab_size : m->v_n;
