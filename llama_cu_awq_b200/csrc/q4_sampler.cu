@@ -16,9 +16,11 @@
 // 121 us (32 elements per thread and pass, 64-bit shared-memory atomics that all fall on the few exponents a softmax
 // produces, bin scans by one thread, contiguous 32-element walks per thread); eight CTAs with the elements kept in shared
 // memory and the partial results exchanged through distributed shared memory bring a sampled token's tail (classifier of
-// 32000 x 4096 and this kernel, launched together) from 197 to 73 us. Eight is the largest portable cluster.
+// 32000 x 4096 and this kernel, launched together) from 197 to 65 us. Eight is the largest portable cluster.
 #include <cooperative_groups.h>
 #include <math_constants.h>
+
+#include <type_traits>
 
 #include "q4_common.cuh"
 
@@ -60,9 +62,10 @@ sample_topp_kernel(__half* __restrict__ logits, int n, float temperature, float 
     __shared__ float s_red[32];
     __shared__ float s_max[kCtas], s_wsum[32];
     __shared__ unsigned s_part[kRowsAtOnce][64];            // high-byte histogram, one copy per group of 128 threads
-    __shared__ unsigned s_hist[64], s_hist2[256];           // this CTA's histograms, read by the whole cluster
+    __shared__ __align__(16) unsigned s_hist[64], s_hist2[256];   // this CTA's histograms, read by the whole cluster
     __shared__ unsigned s_cnt[kMaxRows];                    // per row: matches (or units) among this CTA's 128 columns
     __shared__ unsigned s_all[kMaxRows * kCtas];            // CTA 0: the same of all CTAs, in index order
+    __shared__ __align__(16) unsigned s_hists[kCtas * 256]; // all CTAs' histograms
     __shared__ unsigned s_last[kCtas];
     __shared__ int s_bin;
     __shared__ unsigned s_before, s_seg, s_seg_before;
@@ -171,27 +174,49 @@ sample_topp_kernel(__half* __restrict__ logits, int n, float temperature, float 
             s_hist[t] = h;
         }
         cluster.sync();
-        auto find_bin = [&](const unsigned* hist, int per_lane, unsigned before) {   // warp 0; lane's bins, highest first
-            unsigned v[8], tot = 0;
+        // The cluster's histograms into this CTA's memory, a warp to each, whole lines at a time (all read by warp 0, bin by bin, the second one took
+        // 5300 clocks, now 1900)
+        auto gather = [&](const unsigned* hist, auto bins) {
+            constexpr int per_lane = decltype(bins)::value, kV = per_lane < 4 ? per_lane : 4;
+            struct alignas(4 * kV) Words { unsigned w[kV]; };
+            if (warp < kCtas) {
+                const Words* from = reinterpret_cast<const Words*>(cluster.map_shared_rank(hist, warp));
+                Words* to = reinterpret_cast<Words*>(s_hists + warp * 32 * per_lane);
+#pragma unroll
+                for (int u = 0; u < per_lane / kV; u++) to[u * 32 + lane] = from[u * 32 + lane];
+            }
+            __syncthreads();
+        };
+        auto find_bin = [&](auto bins, unsigned before) {   // warp 0; lane's bins, highest first
+            constexpr int per_lane = decltype(bins)::value;
+            unsigned v[per_lane], tot = 0;
             const int top = per_lane * (32 - lane) - 1;
+#pragma unroll
             for (int b = 0; b < per_lane; b++) {
                 v[b] = 0;
 #pragma unroll
-                for (int r = 0; r < kCtas; r++) v[b] += cluster.map_shared_rank(hist, r)[top - b];
-                tot += v[b];
+                for (int r = 0; r < kCtas; r++) v[b] += s_hists[r * 32 * per_lane + top - b];
             }
+#pragma unroll
+            for (int b = 0; b < per_lane; b++) tot += v[b];
             const unsigned incl = warp_scan(tot, lane);
             unsigned c = before + incl - tot;
             const unsigned hit = __ballot_sync(0xffffffffu, before + incl >= need);
             if (hit == 0) { if (lane == 0) s_bin = -1; return; }
             if (lane == __ffs(hit) - 1) {
-                int b = 0;
-                while (c + v[b] < need) c += v[b++];
-                s_bin = top - b;
+                int at = top;
+                bool on = true;
+#pragma unroll
+                for (int b = 0; b < per_lane; b++) {
+                    on = on && c + v[b] < need;
+                    if (on) { c += v[b]; at--; }
+                }
+                s_bin = at;
                 s_before = c;
             }
         };
-        if (warp == 0) find_bin(s_hist, 2, 0u);
+        gather(s_hist, std::integral_constant<int, 2>());
+        if (warp == 0) find_bin(std::integral_constant<int, 2>(), 0u);
         __syncthreads();
         if (s_bin < 0) {
             // the threshold is never reached: the last element of the order = lowest probability, highest index among equals
@@ -222,7 +247,8 @@ sample_topp_kernel(__half* __restrict__ logits, int n, float temperature, float 
                 }
             }
             cluster.sync();
-            if (warp == 0) find_bin(s_hist2, 8, before);
+            gather(s_hist2, std::integral_constant<int, 8>());
+            if (warp == 0) find_bin(std::integral_constant<int, 8>(), before);
             __syncthreads();
             key = (key << 8) | s_bin;
             // the k-th element (index order) among those whose probability has exactly this bit pattern
@@ -267,9 +293,13 @@ sample_topp_kernel(__half* __restrict__ logits, int n, float temperature, float 
                     const int j = (int)(s_seg / kCtas), r = (int)(s_seg % kCtas);
                     const unsigned short* keys = cluster.map_shared_rank(s_key, r) + j * kCols;
                     unsigned c = s_seg_before;
-                    for (int c0 = 0; c0 < kCols; c0 += 32) {
-                        const int i = j * kT + r * kCols + c0 + lane;
-                        const unsigned short k = i < n ? keys[c0 + lane] : (unsigned short)0;
+                    unsigned short mine[kCols / 32];       // (all requested at once)
+#pragma unroll
+                    for (int u = 0; u < kCols / 32; u++) mine[u] = j * kT + r * kCols + 32 * u + lane < n ? keys[32 * u + lane] : (unsigned short)0;
+#pragma unroll
+                    for (int u = 0; u < kCols / 32; u++) {
+                        const int c0 = 32 * u, i = j * kT + r * kCols + c0 + lane;
+                        const unsigned short k = mine[u];
                         const unsigned v = i >= n ? 0u : sorted ? (unsigned)(k == (unsigned short)key) : prob_units(k);
                         const unsigned here = c + warp_scan(v, lane);
                         const unsigned hit = __ballot_sync(0xffffffffu, here >= target);
@@ -304,9 +334,9 @@ extern "C" int q4_sample_topp(void* stream, uint16_t* logits, int n, float tempe
                               volatile int* pos_pinned, int* pos_dev) {
     if (!logits || !tokens_pinned || !pos_pinned || !pos_dev || n <= 0 || n > (1 << 18) || !(temperature > 0.f)) return Q4_ERR_INVALID;
     const size_t smem = kRowBytes * q4_div_up(n, kT);
-    // The static arrays take 13 KB of the 48 KB that need no opt-in. The limit belongs to the function on the device and not to this
+    // The static arrays take 21 KB of the 48 KB that need no opt-in. The limit belongs to the function on the device and not to this
     // call: it is always set to the largest size, so that calls of other threads between here and the launch cannot lower it.
-    if (smem > 32 * 1024) Q4_CUDA_TRY(cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRowBytes * kMaxRows)));
+    if (smem > 24 * 1024) Q4_CUDA_TRY(cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRowBytes * kMaxRows)));
     Q4Launch L(dim3(kCtas), dim3(kT), smem, (cudaStream_t)stream);
     Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, sample_topp_kernel, (__half*)logits, n, temperature, topp, coin, tokens_pinned, pos_pinned, pos_dev));
     return Q4_OK;
