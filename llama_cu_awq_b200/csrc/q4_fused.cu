@@ -354,24 +354,25 @@ struct Requests {           // the segment being requested: this warp's chunks o
     uint32_t left, chunk;   // bytes left in it, bytes per chunk
     uint32_t step;          // distance between chunks
     int seg, rot, row;
-    int more;               // positions behind the one it belongs to
 };
 struct Ring {
     uint8_t* base;
     uint64_t* bar;
     Requests* rq;
+    int* more;              // kMany: positions behind the one whose segment is being requested
     int slot;
     uint32_t parity;        // of the round the next wait is for
     bool dead;              // a wait ran out: nothing more is requested or read
 };
-__device__ __forceinline__ void next_segment(Requests& r, const FParams& p, const uint8_t* const* streams) {
+template <bool kMany>
+__device__ __forceinline__ void next_segment(Requests& r, int* more, const FParams& p, const uint8_t* const* streams) {
     const int cta = blockIdx.x, grid = gridDim.x, w = threadIdx.x >> 5;
     int seg = r.seg, rot = r.rot;
     r.left = 0;
     for (;;) {
         if (seg == K_KINDS * p.n_layers) {
-            if (r.row < p.v_n || r.more == 0) break;
-            r.more--;
+            if (!kMany || r.row < p.v_n || *more == 0) break;
+            --*more;
             r.row = cta * kW + w;
             seg = rot = 0;
         }
@@ -397,6 +398,7 @@ __device__ __forceinline__ void next_segment(Requests& r, const FParams& p, cons
     r.row += grid * kW;
 }
 // Requests the next chunk into `slot` (free: released just now, or never used). Lane 0.
+template <bool kMany>
 __device__ __forceinline__ void ring_request(const Ring& ring, int slot, const FParams& p, const uint8_t* const* streams) {
     Requests& r = *ring.rq;
     const uint32_t left = r.left, bytes = min(left, r.chunk);
@@ -406,7 +408,7 @@ __device__ __forceinline__ void ring_request(const Ring& ring, int slot, const F
     bulk_g2s(ring.base + slot * kChunkBytes, src, bytes, &ring.bar[slot]);
     r.left = left - bytes;
     r.src = src + r.step;
-    if (left == bytes) next_segment(r, p, streams);
+    if (left == bytes) next_segment<kMany>(r, ring.more, p, streams);
 }
 __device__ __forceinline__ const uint8_t* ring_wait(Ring& r, const FParams& p) {
     if (!r.dead && !__all_sync(0xffffffffu, mbar_try(&r.bar[r.slot], r.parity))) {
@@ -417,10 +419,11 @@ __device__ __forceinline__ const uint8_t* ring_wait(Ring& r, const FParams& p) {
 }
 // The warp has read the chunk: a shuffle or vote of values made from all that each lane read of it is behind the caller (a barrier alone
 // does not wait for loads in flight).
+template <bool kMany>
 __device__ __forceinline__ void ring_release(Ring& r, const FParams& p, const uint8_t* const* streams) {
     __syncwarp();
     if (r.dead) return;
-    if ((threadIdx.x & 31) == 0) ring_request(r, r.slot, p, streams);
+    if ((threadIdx.x & 31) == 0) ring_request<kMany>(r, r.slot, p, streams);
     if (++r.slot == p.depth) { r.slot = 0; r.parity ^= 1u; }
 }
 
@@ -578,6 +581,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full_bar[kW * kMaxDepth];
     __shared__ Requests requests[kW];
+    __shared__ int behind[kMany ? kW : 1];
     __shared__ float ssq[(kMaxDim + 255) / 256];
     __shared__ __align__(16) __half new_row[3][128];   // this position's rotated query, rotated key and value of the head at hand
     __shared__ float sm_m[kW], sm_l[kW];
@@ -607,6 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     ring.base = smem + (size_t)w * p.depth * kChunkBytes;
     ring.bar = full_bar + w * kMaxDepth;
     ring.rq = requests + w;
+    ring.more = behind + (kMany ? w : 0);
     ring.slot = 0;
     ring.parity = 0;
     ring.dead = false;
@@ -614,9 +619,9 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         Requests& r = requests[w];
         r.seg = r.rot = 0;
         r.row = cta * kW + w;
-        r.more = kMany ? p.n_tokens - 1 : 0;
-        next_segment(r, p, streams);
-        for (int i = 0; i < p.depth; i++) ring_request(ring, i, p, streams);
+        if (kMany) *ring.more = p.n_tokens - 1;
+        next_segment<kMany>(r, ring.more, p, streams);
+        for (int i = 0; i < p.depth; i++) ring_request<kMany>(ring, i, p, streams);
     }
     __syncwarp();
 
@@ -897,7 +902,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                 if ((lane & 3) == 0) *dst = first ? y : *dst + y;
                 dst += kTileStride;
                 sub ^= 1;
-                if (sub == 0 || left + n == 1) ring_release(ring, p, streams);
+                if (sub == 0 || left + n == 1) ring_release<kMany>(ring, p, streams);
                 n--;
             };
             if (sub) one();
@@ -917,7 +922,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                         if ((lane & 2) == 0) *dst2 = first ? y : *dst2 + y;
                         dst2 += 2 * kTileStride;
                     }
-                    ring_release(ring, p, streams);
+                    ring_release<kMany>(ring, p, streams);
                 }
                 dst += 2 * chunks * kTileStride;
                 n -= 2 * chunks;
@@ -1009,7 +1014,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
                 }
                 // The vote needs every lane's a[0], and that every one of its loads of the chunk; no product leaves this NaN's bits.
                 if (!__all_sync(0xffffffffu, __float_as_uint(a[0]) != 0x7F800001u)) break;
-                ring_release(ring, p, streams);
+                ring_release<kMany>(ring, p, streams);
             }
             const float sum = warp_sum(((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])));
             const int n = p.vocab_off + row;   // global vocabulary index
