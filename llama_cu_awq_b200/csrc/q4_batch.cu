@@ -858,7 +858,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const Embed& embed, _
     // mat: 0 q|k|v, 1 o, 2 gate / up with silu(gate) * up, 3 down; residual: y = product + y / g
     auto gemm = [&](__half* y, const __half* x, int l, int mat, bool residual) {
         const q4_rows::GemmMat& gmat = r->gm[(size_t)l * 4 + mat];
-        return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &gmat.w, gmat.wi, n, gmat.K, gmat.N, residual ? (const uint16_t*)y : nullptr, 1.0f / g, mat == 2, r->ws,
+        return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &gmat.w, gmat.wi, n, gmat.K, gmat.N, residual ? (const uint16_t*)y : nullptr, 1.0f / g, mat == 2, true, r->ws,
                               r->ws_bytes);
     };
     // k and v alone: the rows of q|k|v behind q's
@@ -868,7 +868,7 @@ static int rows_layers(q4_model* m, cudaStream_t s, int n, const Embed& embed, _
         part.w.weight = part.wi;
         part.w.zeros += (size_t)m->q_n * q4_pz(part.K);
         part.w.scales += (size_t)m->q_n * q4_groups(part.K);
-        return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &part.w, part.wi, n, part.K, 2 * m->kv_n, nullptr, 1.0f / g, false, r->ws, r->ws_bytes);
+        return q4_gemm_launch(s, (uint16_t*)y, (const uint16_t*)x, &part.w, part.wi, n, part.K, 2 * m->kv_n, nullptr, 1.0f / g, false, true, r->ws, r->ws_bytes);
     };
     // q, k, v of the rows: three buffers (few-rows kernels) or three slices of the fused GEMM's output (two in a prompt's last layer)
     const int nqkv = m->q_n + 2 * m->kv_n;

@@ -70,6 +70,7 @@ struct GemmParams {
     int M, K, N, G, PZ;
     int MT, m_tiles, n_chunks;
     long long total_chunks;   // tiles * n_chunks
+    int settled;         // 1: no kernel in flight writes the packed words
     int stages, np, slab_bytes;   // operand stages (A in tensor memory, X in shared memory), weight copies in flight, bytes of an X slab
 };
 
@@ -137,6 +138,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_addr(dst)),
                  "l"(map), "r"(smem_addr(bar)), "r"(x), "r"(y)
                  : "memory");
+}
+// the same box into L2 only
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 // into this CTA's shared memory, reporting to a barrier of either CTA of the pair (no multicast)
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -323,8 +328,10 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t*)&s_tmem_base;
     // everything above overlaps the tail of the previous kernel on the stream (programmatic dependent launch) where both fit an SM,
-    // that is, not behind another of these, whose shared memory fills it; from here on this kernel reads what that kernel wrote, but for the
-    // packed words, which are nobody's result (64 x 4096 x 22016 back to back 25.5 us, 24.7 so)
+    // that is, not behind another of these, whose shared memory fills it; from here on this kernel reads what that kernel wrote. The warp of the
+    // packed words starts before: a model's words are nobody's result by then, a caller's may be that kernel's (q4_gemm_interleave_weights)
+    // and come as far as L2 only. us, both behind the wait, the caller's and the model's form: 64 x 4096 x 22016 back to back 25.6, 24.7, 24.9;
+    // 78 tokens of two 13B layers 309.5, 308.9, 307.2
     if (warp != 0) griddep_wait();
     griddep_launch_dependents();
     Segments seg(p, pair, pairs);
@@ -336,8 +343,12 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             int ps = 0;
             uint32_t ph = 1;
             unsigned issued = 0;
-            bool ok = true;
-            while (ok && seg.next()) {
+            bool ok = true, more = seg.next();
+            if (!p.settled) {
+                for (int c = seg.c0; more && c < seg.c1 && c < seg.c0 + p.np; c++) tma_prefetch_2d(&map_w, c * (kChunkK / 8), (seg.tile / p.m_tiles) * kPairN + rank * kBN);
+                griddep_wait();
+            }
+            for (; ok && more; more = seg.next()) {
                 const int row = (seg.tile / p.m_tiles) * kPairN + rank * kBN;
                 for (int c = seg.c0; c < seg.c1; c++) {
                     if (!mb_wait(&empty_p[ps], ph, p.status, 0x100)) { ok = false; break; }
@@ -842,11 +853,11 @@ extern "C" int q4_matmul_q4_batched(void* stream, uint16_t* y, const uint16_t* x
 
 extern "C" int q4_matmul_q4_batched_residual(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M,
                                              int K, int N, const uint16_t* residual, float residual_scale, void* workspace, size_t workspace_bytes) {
-    return q4_gemm_launch(stream, y, x, w, weight_interleaved, M, K, N, residual, residual_scale, false, workspace, workspace_bytes);
+    return q4_gemm_launch(stream, y, x, w, weight_interleaved, M, K, N, residual, residual_scale, false, false, workspace, workspace_bytes);
 }
 
 int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M, int K, int N,
-                   const uint16_t* residual, float residual_scale, bool silu, void* workspace, size_t workspace_bytes) {
+                   const uint16_t* residual, float residual_scale, bool silu, bool settled, void* workspace, size_t workspace_bytes) {
     if (!y || !x || !w || !w->zeros || !w->scales || !workspace || M <= 0 || K <= 0 || N <= 0) return Q4_ERR_INVALID;
     if (!w->weight && !weight_interleaved) return Q4_ERR_INVALID;
     if ((K % 128) || (N % 8)) return Q4_ERR_UNSUPPORTED_SIZE;
@@ -870,6 +881,7 @@ int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweigh
     p.G = q4_groups(K);
     p.PZ = q4_pz(K);
     p.MT = g.MT; p.m_tiles = g.m_tiles; p.n_chunks = g.n_chunks; p.total_chunks = g.total;
+    p.settled = settled;
     p.stages = g.stages; p.np = g.np; p.slab_bytes = g.slab;
     // (status word and tile counters start at zero: the caller zeroes the workspace once, the kernel leaves the counters at
     // zero; after a recorded time-out the caller zeroes it again)
@@ -939,7 +951,7 @@ extern "C" int q4_time_matmul_q4_batched(void* stream, uint16_t* y, const uint16
 // up j; `interleaved` as from q4_gemm_interleave_weights; y is [M][N / 2].
 extern "C" int q4_test_gemm_silu(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* interleaved, int M, int K, int N,
                                  void* workspace, size_t workspace_bytes) {
-    return q4_gemm_launch(stream, y, x, w, interleaved, M, K, N, nullptr, 0.f, true, workspace, workspace_bytes);
+    return q4_gemm_launch(stream, y, x, w, interleaved, M, K, N, nullptr, 0.f, true, false, workspace, workspace_bytes);
 }
 // What make_plan picks on a GPU with `sms` SMs (host only): batch tile and number of pairs.
 extern "C" int q4_test_gemm_plan(int M, int K, int N, int sms, int* mt, int* pairs) {

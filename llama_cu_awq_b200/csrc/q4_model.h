@@ -78,6 +78,7 @@ int q4_qkv_rows_launch(void* stream, uint16_t* q, uint16_t* k, uint16_t* v, cons
                        int M, int inpSize, int opSize, int kvSize, bool late);
 
 // q4_gemm.cu: q4_matmul_q4_batched_residual, and with silu = true (interleaved weights only) the fused gate / up form: rows 2j and
-// 2j + 1 of the weights are gate j and up j, y is [M][N / 2] = silu(gate) * up.
+// 2j + 1 of the weights are gate j and up j, y is [M][N / 2] = silu(gate) * up. settled: the packed words were complete on the device
+// before this call was made (they are read ahead of the kernels before it on the stream).
 int q4_gemm_launch(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* weight_interleaved, int M, int K, int N,
-                   const uint16_t* residual, float residual_scale, bool silu, void* workspace, size_t workspace_bytes);
+                   const uint16_t* residual, float residual_scale, bool silu, bool settled, void* workspace, size_t workspace_bytes);

@@ -11,6 +11,10 @@ from oracle import q4_oracle as O
 pytestmark = pytest.mark.gpu
 
 
+def interleave(dst, src, K, N):
+    ops.check(ops._lib.lib().q4_gemm_interleave_weights(ops._stream(), ops._p(dst), ops._p(src), K, N), "interleave_weights")
+
+
 def _case(M, K, N, seed, interleave):
     rng = np.random.default_rng(seed)
     q = synth.synth_qweight(rng, K, N)
@@ -96,6 +100,30 @@ def test_back_to_back_launches_are_bit_reproducible():
         for o in outs:
             assert torch.equal(o, first)
     assert mm.status() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(64, 4096, 22016), (33, 512, 264)])
+def test_weights_written_by_the_kernel_before(M, K, N):
+    """A call behind the kernel that wrote its packed words, without a wait between them: two matrices in turn in one buffer, the bits of
+    the calls on settled words each time."""
+    rng = np.random.default_rng(K)
+    xd = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float16)).cuda()
+    W = [ops.QWeight.from_numpy(synth.synth_qweight(rng, K, N)) for _ in range(2)]
+    mm = ops.BatchedMatmul(W[0], K, N, M)
+    other = ops.BatchedMatmul(W[1], K, N, M)
+    want = torch.empty((2, M, N), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    mm(want[0], xd, M)
+    mm.wi, other.wi = other.wi, mm.wi
+    mm(want[1], xd, M)
+    y = torch.empty((20, M, N), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(20):
+        interleave(mm.wi, W[i % 2].weight, K, N)
+        mm(y[i], xd, M)
+    assert mm.status() == 0
+    for i in range(20):
+        assert (y[i].view(torch.int16) == want[i % 2].view(torch.int16)).all(), i
 
 
 @pytest.mark.parametrize("M,K,N", [(40, 1024, 520), (300, 4096, 256), (512, 11008, 512)])
