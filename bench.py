@@ -683,7 +683,7 @@ def main():
     else:
         launches_per_token = 4 + 9 * cfg[2] + (2 * cfg[2] + 1 if world > 1 else 0)
         k = (extra.get("kernels") or {}).get("ffn_gate_up_silu") or {}
-        roof = {"bound": "hbm", "kernel": "q4_gemv_ring_kernel (fused gate/up + SiLU)", "achieved": k.get("gbs"), "peak": pk["hbm_gbs"], "unit": "GB/s",
+        roof = {"bound": "hbm", "kernel": "q4_gemv_stream_kernel (fused gate/up + SiLU)", "achieved": k.get("gbs"), "peak": pk["hbm_gbs"], "unit": "GB/s",
                 "frac": k.get("frac_of_hbm_peak"), "peak_kind": pk_kind, "traffic": None, "bytes_per_launch": k.get("bytes"), "us_per_launch": k.get("us")}
     if not args.no_extras:
         try:

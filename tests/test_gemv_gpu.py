@@ -160,8 +160,8 @@ def test_unsupported_sizes_return_status():
                                  (4352, 10400), (520, 90000), (4096, 11008), (4096, 3 * 148 * 8)])
 def test_matvec_splits(K, N):
     """Both forms of the kernel as the launch chooses them. Direct: fewer items than warps, pairs beyond a multiple of 16, more tiles than
-    one pass holds. Ring: several tiles of short rows in a stage, a last group of tiles that is not full, more tiles than one pass holds,
-    many chunks, a last chunk with one pair. Bound: the rounding of the result to fp16 (2^-11 of
+    one pass holds. Stream: short rows of many tiles, more tiles than one pass holds, several pairs per warp, pairs beyond a multiple of 16.
+    Bound: the rounding of the result to fp16 (2^-11 of
     each value, relative to the largest at most 4.9e-4) and the fixed-point step of x (2^-16 of a group's largest, averaged over K)."""
     q, x, _ = mk(K, N, seed=K + N)
     W = ops.QWeight.from_numpy(q)
