@@ -616,6 +616,7 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
         e = q4_prefill_cache(m, s, n_prompt - 1);
         if (e == Q4_OK) pos = n_prompt - 1;
         else if (e != Q4_ERR_UNSUPPORTED_SIZE) return e;
+        e = Q4_OK;
     }
     // A prompt's ids are all known, so the fused kernel takes many positions in one launch (48 positions of four 7B layers 6880 us one by one,
     // 6470 so); 32 at most, so that other streams get their turn. As the loop below does, it ends behind an end token that is not the first.
@@ -632,10 +633,11 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
             ended = false;
             break;
         }
-        if ((e = forward_many(m, s, n, pos + n == n_prompt)) != Q4_OK) return e;
+        e = forward_many(m, s, n, pos + n == n_prompt);
+        if (e != Q4_OK) break;
         pos += ended ? n - 1 : n;
     }
-    while (pos < steps && !ended) {
+    while (e == Q4_OK && pos < steps && !ended) {
         // A generated id is in the mailbox when its token is done; a prompt's ids are there already, and its positions are queued without
         // a wait (48 positions of four 7B layers: 7.55 ms with one each).
         if (pos >= n_prompt) cudaStreamSynchronize(s);
