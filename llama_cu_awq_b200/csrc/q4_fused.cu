@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     __shared__ float ssq[(kMaxDim + 255) / 256];
     __shared__ __align__(16) __half new_row[3][128];   // this position's rotated query, rotated key and value of the head at hand
     __shared__ float sm_m[kW], sm_l[kW];
-    __shared__ int next_id;            // kMany: token of the position behind this one (CTAs that embed)
+    __shared__ int next_id[2];         // kMany: tokens of the positions with an even and an odd number behind them (CTAs that embed)
     __shared__ int sm_i[kW];
 
     uint4* const xs = reinterpret_cast<uint4*>(smem + p.x_off);               // residual stream (fp16); the classifier's input
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     int rot = 0;
     const int word = cta * kThreads + tid;
     if (word < p.dim / 8) {
-        const int token = more == n_tokens - 1 ? p.tokens_pinned[pos] : next_id;
+        const int token = more == n_tokens - 1 ? p.tokens_pinned[pos] : next_id[more & 1];
         const uint4 v = reinterpret_cast<const uint4*>(p.emb + (size_t)token * p.dim)[word];
         const uint32_t tg = tag_of(tag0, 0);
         // every rank files the row as slot 0 of its own buffer 1 and zeros as the other ranks' partials
@@ -655,9 +655,10 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         const int layer = seg / K_KINDS, f = seg % K_KINDS;
         const int pi0 = 1 + layer * kLayerPhases;
         const long long loff = layer * p.layer_stride;
-        // The next position's token, from host memory, while nobody waits for it
+        // The next position's token, from host memory, while nobody waits for it. (The word is not the one the embedding above reads: with one
+        // layer there is no barrier between the two.)
         if (kMany && more > 0 && seg == K_KINDS * (p.n_layers - 1) && embeds && tid == 0)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&next_id)), "l"(p.tokens_pinned + pos + 1) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&next_id[~more & 1])), "l"(p.tokens_pinned + pos + 1) : "memory");
 
         if (f == K_O && !(Q4_DBG(p) & 1)) {
             // ---- attention of one query per head over positions 0..pos, split over CTAs (llama2_q4.cu:410-427) ----
@@ -991,7 +992,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
         }
         if (kMany) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        if (kMany && more > 0 && word < p.dim / 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(p.emb + (size_t)next_id * p.dim) + word));
+        if (kMany && more > 0 && word < p.dim / 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(p.emb + (size_t)next_id[~more & 1] * p.dim) + word));
         TRACE(pi, 1);
         float best = -CUDART_INF_F;
         int bi = 0x7fffffff;

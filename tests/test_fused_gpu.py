@@ -351,3 +351,19 @@ def test_many_positions_in_one_launch_with_the_far_table():
     finally:
         L.q4_test_set_far_table(0)
     assert all((o == out[0]).all() for o in out[1:])
+
+
+@pytest.mark.parametrize("cfg", [(512, 768, 1, 4, 2, 512, 96, 10000.0),            # one layer: no step between the embedding and the last layer's first
+                                 (5120, 1024, 1, 40, 8, 512, 96, 10000.0)])        # two CTAs embed
+def test_many_positions_of_one_layer_in_one_launch(cfg):
+    """The next position's id is fetched while this one's may still be read: the bits of one launch per position, ids that all differ."""
+    tokens = np.random.default_rng(13).permutation(np.arange(3, 512, dtype=np.int32))[:70]
+    t = Transformer(None, synthetic=(cfg, 7))
+    assert t.best_path() == 2
+    for n in (2, 3, 32, 70):
+        want = _run(t, tokens[:n], queued=True)[-1]
+        for _ in range(5):
+            t.generate(tokens[:n], n, path=2)
+            assert (t.logits().view(np.uint16) == want.view(np.uint16)).all(), n
+    assert t.status() == 0
+    t.close()
