@@ -49,10 +49,11 @@ typedef struct {
  *   weight u32[N][4*ceil(K/32)]  nibble i of word j holds q(n, 8j+i)
  *   zeros  u32[N][ceil(ceil(K/128)/8)]
  *   scales f16[N][ceil(K/128)]
- * A call may read the packed words before the kernel in front of it on the stream has ended (programmatic dependent
- * launch); the few-rows forms read scales and zero points as early. A host that changes a matrix in place
- * by a kernel puts an event or a copy between that kernel and the call. The batch-1 forms (q4_matmul_q4, q4_qkv_matvec,
- * q4_ffn_matvec_silu) take scales and zero points, as x, only when the kernel in front has ended. */
+ * What a call reads before the kernel directly in front of it on the stream has ended (programmatic dependent launch): the
+ * batch-1 forms (q4_matmul_q4, q4_qkv_matvec, q4_ffn_matvec_silu) the packed words, the few-rows forms (q4_matmul_q4_rows,
+ * q4_qkv_matmul_rows, q4_ffn_silu_rows) scales and zero points too, q4_matmul_f16 its w. A host that writes these by that
+ * kernel puts an event or a copy between the two. Everything else, and all that the batched form (q4_matmul_q4_batched) reads,
+ * is taken only when the kernel in front has ended; kernels further in front have ended before a call starts. */
 typedef struct {
     const uint32_t* weight;
     const uint32_t* zeros;
@@ -166,7 +167,8 @@ int q4_time_matmul_q4_batched(void* stream, uint16_t* y, const uint16_t* x, cons
                               size_t workspace_bytes, int reps, double* us_per_launch);
 
 /* matmul(half*): llama2_q4.cu:357-365, kernel gpu_kernels.h:117-147. fp16 GEMV used for the classifier:
- * xout[d] = alpha * sum_n w[d][n] * x[n]. n and d must be multiples of 8. */
+ * xout[d] = alpha * sum_n w[d][n] * x[n]. n and d must be multiples of 8. w may be read before the kernel in front has
+ * ended (see q4_qweight). */
 int q4_matmul_f16(void* stream, uint16_t* xout, const uint16_t* x, const uint16_t* w, int n, int d, float alpha);
 
 /* Embedding row gather: copy_embedding_kernel launch at llama2_q4.cu:441 (gpu_kernels.h:61-69).

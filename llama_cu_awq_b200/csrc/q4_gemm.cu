@@ -332,8 +332,12 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // packed words starts before: a model's words are nobody's result by then, a caller's may be that kernel's (q4_gemm_interleave_weights)
     // and come as far as L2 only. us, both behind the wait, the caller's and the model's form: 64 x 4096 x 22016 back to back 25.6, 24.7, 24.9;
     // 78 tokens of two 13B layers 309.5, 308.9, 307.2
-    if (warp != 0) griddep_wait();
-    griddep_launch_dependents();
+    // The kernel behind is let in by warps that have waited (the first signal of a CTA counts for all of it): its words are read ahead of its own wait,
+    // and may be the result of the kernel in front of this one.
+    if (warp != 0) {
+        griddep_wait();
+        griddep_launch_dependents();
+    }
     Segments seg(p, pair, pairs);
 
     if (warp < 4) {
@@ -952,6 +956,19 @@ extern "C" int q4_time_matmul_q4_batched(void* stream, uint16_t* y, const uint16
 extern "C" int q4_test_gemm_silu(void* stream, uint16_t* y, const uint16_t* x, const q4_qweight* w, const uint32_t* interleaved, int M, int K, int N,
                                  void* workspace, size_t workspace_bytes) {
     return q4_gemm_launch(stream, y, x, w, interleaved, M, K, N, nullptr, 0.f, true, false, workspace, workspace_bytes);
+}
+// A writer that lets the next kernel in at once and writes late: src to dst, `ns` nanoseconds after it has started (bounded by a number of turns too).
+// Few blocks, without shared memory, so that the kernel behind it finds room beside them.
+static __global__ void __launch_bounds__(256) test_write_late_kernel(uint32_t* dst, const uint32_t* src, size_t n, unsigned long long ns) {
+    griddep_launch_dependents();
+    const unsigned long long t0 = gtimer();
+    for (int i = 0; i < 1000000 && gtimer() - t0 < ns; i++) {}
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = src[i];
+}
+extern "C" int q4_test_write_late(void* stream, uint32_t* dst, const uint32_t* src, size_t n, unsigned long long ns) {
+    test_write_late_kernel<<<8, 256, 0, (cudaStream_t)stream>>>(dst, src, n, ns);
+    Q4_CUDA_TRY(cudaGetLastError());
+    return Q4_OK;
 }
 // What make_plan picks on a GPU with `sms` SMs (host only): batch tile and number of pairs.
 extern "C" int q4_test_gemm_plan(int M, int K, int N, int sms, int* mt, int* pairs) {

@@ -126,6 +126,50 @@ def test_weights_written_by_the_kernel_before(M, K, N):
         assert (y[i].view(torch.int16) == want[i % 2].view(torch.int16)).all(), i
 
 
+@pytest.mark.parametrize("M,K,N", [(64, 4096, 22016), (17, 512, 264)])
+@pytest.mark.parametrize("behind", ["gemm", "gemv", "gemv stream", "rows"])
+def test_weights_of_a_writer_that_lets_the_next_kernel_in_early(M, K, N, behind):
+    """The kernel in front signals its dependents first and writes the packed words late. A GEMM on those words reads them when it has ended; a product
+    behind a GEMM on another matrix, whose words may be read ahead of its own wait, starts only when the GEMM has waited."""
+    from llama_cu_awq_b200 import _lib
+    L = _lib.test_lib()
+    rng = np.random.default_rng(K)
+    xd = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float16)).cuda()
+    front = ops.BatchedMatmul(ops.QWeight.from_numpy(synth.synth_qweight(rng, K, N)), K, N, M)
+    K2, N2 = {"gemm": (K, N), "gemv": (1024, 1024), "gemv stream": (11008, 4096), "rows": (1024, 1024)}[behind]
+    q = synth.synth_qweight(rng, K2, N2)
+    W, src = ops.QWeight.from_numpy(q), [torch.from_numpy(synth.synth_qweight(rng, K2, N2)["weight"].view(np.int32)).cuda() for _ in range(2)]
+    x2 = torch.from_numpy(rng.standard_normal((M if behind == "gemm" else 8, K2)).astype(np.float16)).cuda()
+    mm = ops.BatchedMatmul(W, K2, N2, M, interleave=False)
+    out = torch.empty((10, M if behind == "gemm" else 8, N2), dtype=torch.float16, device="cuda")
+    yf = torch.empty((M, N), dtype=torch.float16, device="cuda")
+
+    def product(y):
+        if behind == "gemm":
+            mm(y, x2, M)
+        elif behind == "rows":
+            ops.matmul_rows(y, x2, W, 8, K2, N2)
+        else:
+            ops.matmul(y[0], x2[0], W, K2, N2)
+
+    want = torch.zeros_like(out[:2])
+    out.zero_()
+    for i in range(2):
+        W.weight.copy_(src[i])
+        torch.cuda.synchronize()
+        product(want[i])
+        torch.cuda.synchronize()
+    for i in range(10):
+        assert L.q4_test_write_late(ops._stream(), ops._p(W.weight), ops._p(src[i % 2]), W.weight.numel(), 40000) == 0
+        if behind != "gemm":
+            front(yf, xd, M)
+        product(out[i])
+    torch.cuda.synchronize()
+    assert mm.status() == 0 and front.status() == 0
+    for i in range(10):
+        assert torch.equal(out[i], want[i % 2]), i
+
+
 @pytest.mark.parametrize("M,K,N", [(40, 1024, 520), (300, 4096, 256), (512, 11008, 512)])
 def test_residual_epilogue(M, K, N):
     """y = product + y * scale in place (q4_matmul_q4_batched_residual), whole tiles and tiles in several parts."""
