@@ -587,15 +587,18 @@ int launch_stream(GemvParams& p, cudaStream_t s) {
     return Q4_OK;
 }
 
-// The stream form from 9 MB of packed words up, and below that where rows are long (bytes * pairs of a row >= 180 MB); us from HBM, direct and
-// stream: 4096 -> 2 x 11008 16.2, 10.5; 28672 -> 8192 42, 27.2; 11008 -> 4096 10.7, 8.1; 8192 x 2048 4.9, 4.4; 5504 x 4096 6.2, 5.7; 13824 x 640 5.4,
-// 4.7; 24424 x 720 8.5, 6.9; 1024 -> 2 x 40000 18.9, 13.9. The direct form starts about a microsecond earlier: 4096 x 4096 4.2, 4.3 (from L2 3.4,
-// 4.2); 5120 x 2560 4.4, 4.6; 2752 x 4096 4.0, 4.4; 512 x 512 1.6, 2.4. Rows of less than four pairs stay with it whatever the size (512 x 60000 7.6,
-// 8.5), and rows whose scales for a tile do not fit into shared memory (about 390000 inputs).
+// The stream form from 20 MB of packed words up, and from rows of 32 pairs on below that (bytes * pairs of a row >= 180 MB). The direct form starts about
+// a microsecond earlier, which a call on words that are in L2 already (one matrix again and again) shows most; a model's come from HBM. The line lies where
+// what one side loses is what the other gains. us, direct and stream, from HBM; from L2: 1024 x 24000 5.4, 5.5; 4.2, 5.3. 2048 x 9216 4.6, 4.9; 3.8, 4.8.
+// 4096 x 4608 4.5, 4.5; 3.6, 4.4. 5120 x 5120 6.6, 6.1; 4.9, 6.0. 4096 x 8192 6.9, 6.1; 4.7, 5.8. 4096 x 10240 (21 MB) 8.1, 6.6; 5.5, 6.3.
+// 8192 x 2048 4.9, 4.5; 4.3, 4.5. 8192 x 4096 7.6, 6.1; 5.6, 5.8. 12288 x 1024 4.9, 4.5; 4.7, 4.5. 13824 x 640 5.4, 4.9; 5.1, 4.9. 28672 x 512 9.6, 7.8;
+// 8.3, 8.0. Ratio over the range (3 to 28 MB), L2 and HBM: 4 to 12 pairs 1.2, 1.1 at 9 MB, 1.2, 0.9 at 18, 1.14, 0.85 at 22; 16 to 28 pairs 1.2, 0.9 at 16, 1.1,
+// 0.8 at 22; 32 to 43 pairs 1.0 to 1.1, 0.75 to 0.9 from 6 MB; 48 and 64 pairs 0.9 to 1.0, 0.65 to 0.9. Rows of less than four pairs stay with the direct form whatever the
+// size (512 x 60000 7.6, 8.5 from HBM), and rows whose scales for a tile do not fit into shared memory (more than 266496 inputs).
 template <bool SILU>
 int launch(GemvParams& p, cudaStream_t s) {
     const long long bytes = 4LL * p.total_tiles * kRows * p.PW;
-    if (p.P >= 4 && (bytes >= 9000000 || bytes * p.P >= 180000000) && stream::tiles_in_pass(p.G, stream::kMaxOwn) > 0) {
+    if (p.P >= 4 && (bytes >= 20000000 || (p.P >= 32 && bytes * p.P >= 180000000)) && stream::tiles_in_pass(p.G, stream::kMaxOwn) > 0) {
         switch (std::min(p.P / kWarps, stream::kMaxOwn)) {
             case 0: return launch_stream<SILU, 0>(p, s);
             case 1: return launch_stream<SILU, 1>(p, s);

@@ -241,9 +241,10 @@ def test_products_of_several_matrices_with_small_inputs_beside_large_ones():
 
 
 @pytest.mark.parametrize("K,N", [(1032, 33160), (2040, 9432), (4096, 4400), (4352, 4232), (4360, 4240), (8192, 2072), (11008, 1640),
-                                 (13824, 640), (16384, 1104), (16640, 1192), (28672, 168), (41088, 120)])
+                                 (13824, 640), (16384, 1104), (16640, 1192), (28672, 168), (41088, 120),
+                                 (1032, 38800), (2040, 19608), (4096, 9800), (4352, 9200), (4360, 9176), (8064, 5560)])
 def test_matvec_stream_edges(K, N):
-    """The form that long and large products take: five pairs for 16 warps, one to four pairs per warp and none to 15 left over, a last pair with one
+    """The form that long and large products take, and sizes close to the line on its other side: five pairs for 16 warps, one to four pairs per warp and none to 15 left over, a last pair with one
     group and a last group that is not full, fewer tiles than SMs, tiles that do not divide by them, more than one pass of tiles."""
     q, x, _ = mk(K, N, seed=K + N)
     y = torch.full((N,), float("nan"), dtype=torch.float16, device="cuda")
@@ -251,9 +252,10 @@ def test_matvec_stream_edges(K, N):
     check_against_64_bits(y.cpu().numpy(), q, x, K, N, f"{K}x{N}")
 
 
-def test_streamed_products_of_several_matrices():
-    """q|k|v whose matrices end inside a CTA's tiles, gate/up in more than one pass of tiles, and the accumulating form."""
-    K, NQ, NKV = 4104, 2376, 1192
+@pytest.mark.parametrize("NQ,NKV,NGU,ND", [(2376, 1192, 16800, 1640), (4952, 2456, 19408, 3640)])
+def test_streamed_products_of_several_matrices(NQ, NKV, NGU, ND):
+    """q|k|v whose matrices end inside a CTA's tiles, gate/up in more than one pass of tiles, and the accumulating form; on both sides of 20 MB."""
+    K = 4104
     rng = np.random.default_rng(5)
     x = rng.standard_normal(K).astype(np.float16)
     qs = [synth.synth_qweight(rng, K, n) for n in (NQ, NKV, NKV)]
@@ -264,7 +266,7 @@ def test_streamed_products_of_several_matrices():
     assert not kc[:2].any() and not vc[:2].any()
     for got, q, n in zip((qo, kc[2], vc[2]), qs, (NQ, NKV, NKV)):
         check_against_64_bits(got.cpu().numpy(), q, x, K, n, f"q|k|v {K}x{n}")
-    K, N = 1032, 16800     # 8400 tiles: 57 for some CTAs
+    K, N = 1032, NGU     # 8400 and 9704 tiles: 57 and 66 for some CTAs
     x = (rng.standard_normal(K) * 0.1).astype(np.float16)
     gate, up = (synth.synth_qweight(rng, K, N) for _ in range(2))
     h = torch.empty(N, dtype=torch.float16, device="cuda")
@@ -273,7 +275,7 @@ def test_streamed_products_of_several_matrices():
     want = g / (1 + np.exp(-g)) * u
     # fp16 rounding of the result; expf and the reciprocal are good to a few units of 2^-23
     assert np.abs(h.cpu().numpy() - want).max() <= 2.0**-11 * 1.02 * np.abs(want).max() + 1e-6
-    K, N = 11008, 1640
+    K, N = 11008, ND
     q, x, _ = mk(K, N, seed=9)
     W, y = ops.QWeight.from_numpy(q), torch.zeros(N, dtype=torch.float16, device="cuda")
     for _ in range(2):
