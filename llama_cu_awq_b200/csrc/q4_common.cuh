@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/q4b200.h"
 
 #define Q4_CUDA_TRY(call)                                   \
@@ -37,6 +39,20 @@ struct Q4Launch {
         cfg.numAttrs = 1;
     }
 };
+
+// A function's preferred split of the SM's memory (a hint, always the same one, without which a launch is only slower): set once per device, as the
+// driver's call takes 0.08 of the 2.4 us that a call of the smallest product takes the host. `set` has a bit per device (beyond 64 devices it is set
+// each time); two threads may both set it.
+template <typename F>
+static inline cudaError_t q4_prefer_carveout(F* kernel, int percent, std::atomic<unsigned long long>& set) {
+    int device = 0;
+    if (cudaError_t e = cudaGetDevice(&device)) return e;
+    const unsigned long long bit = device < 64 ? 1ULL << device : 0;
+    if (set.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent)) return e;
+    set.fetch_or(bit, std::memory_order_relaxed);
+    return cudaSuccess;
+}
 
 #ifdef __CUDACC__
 

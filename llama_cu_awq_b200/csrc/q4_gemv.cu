@@ -613,7 +613,8 @@ int launch(GemvParams& p, cudaStream_t s) {
     Q4Launch L(dim3(grid), dim3(kThreads), 0, s);
     // (scales and zero words are read from L1 again and again: behind a kernel that has taken the SM's memory as shared, as the stream form does, the
     // split would stay as it is. Two layers call by call 99.7 us, 97.9 so)
-    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_gemv_kernel<SILU>, cudaFuncAttributePreferredSharedMemoryCarveout, 20));
+    static std::atomic<unsigned long long> preferred{0};
+    Q4_CUDA_TRY(q4_prefer_carveout(q4_gemv_kernel<SILU>, 20, preferred));
     Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_gemv_kernel<SILU>, p));
     return Q4_OK;
 }

@@ -704,7 +704,8 @@ int launch_deal(const SkParams& p, int units, cudaStream_t s) {
         Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU, DEAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSlots * unit_bytes(MT, NT))));
     // x comes out of L1 again and again: behind a kernel that takes all of the SM's memory as shared (the stream form) the split would stay as it is
     // (eight sequences, 32 steps of four 7B layers 7600 us, 6860 so).
-    Q4_CUDA_TRY(cudaFuncSetAttribute(q4_skinny_kernel<MT, NT, SILU, DEAL>, cudaFuncAttributePreferredSharedMemoryCarveout, 50));
+    static std::atomic<unsigned long long> preferred{0};
+    Q4_CUDA_TRY(q4_prefer_carveout(q4_skinny_kernel<MT, NT, SILU, DEAL>, 50, preferred));
     const size_t smem = (per_cta < kSlots ? per_cta : kSlots) * unit_bytes(MT, NT);
     Q4Launch L(dim3(units < kSms ? units : kSms), dim3(warps_of(MT, NT) * 32), smem, s);
     Q4_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, q4_skinny_kernel<MT, NT, SILU, DEAL>, p));
