@@ -341,7 +341,9 @@ int q4_model_set_wait_limit_ns(q4_model* model, unsigned long long ns);
 int q4_model_status(q4_model* model);
 /* generate_thread(): the token loop with the reference's timing window (llama2_q4.cu:708-745). Runs `steps`
  * positions starting from the n_prompt given ids, stops at EOS (id 2). out_tokens receives tokens[0..steps];
- * *timed_tokens = pos-1 and *seconds is the wall time of the loop. */
+ * *timed_tokens = pos-1 and *seconds is the wall time of the loop. On path 2 and one GPU the given ids go through the
+ * token kernel several positions per launch (up to 32, about 4 ms at most), and a kernel of another stream runs between two
+ * launches; q4_model_forward launches one position. */
 /* OR-ed into `path`: the prompt positions but the last go through q4_model_prefill in one pass (the last prompt
  * position and everything after it through `path` as usual); models the many-row kernels do not serve fall back to the
  * token loop. Same timing window, same *timed_tokens. */

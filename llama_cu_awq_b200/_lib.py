@@ -146,6 +146,7 @@ TEST_SIGNATURES = {
     "q4_test_fail_rows_alloc": (None, [_I]),
     "q4_test_fail_set_pos": (None, []),
     "q4_test_gemm_silu": (_I, [_P, _P, _P, _QW, _P, _I, _I, _I, _P, C.c_size_t]),
+    "q4_test_positions_at_once": (_I, [C.c_double, _I]),
     "q4_test_write_late": (_I, [_P, _P, _P, C.c_size_t, C.c_ulonglong]),
     "q4_test_gemm_plan": (_I, [_I, _I, _I, _I, C.POINTER(_I), C.POINTER(_I)]),
 }

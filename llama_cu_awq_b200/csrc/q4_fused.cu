@@ -1,4 +1,4 @@
-// Fused decode path: ONE persistent cooperative kernel per token (one CTA per SM; a prompt fed token by token: per 32 positions) instead of ~9 launches per layer.
+// Fused decode path: ONE persistent cooperative kernel per token (one CTA per SM; a prompt fed token by token: per up to 32 positions) instead of ~9 launches per layer.
 // Replaces the launch sequence of run_llama_network (llama2_q4.cu:430-538), on one GPU or on every rank of a
 // tensor-parallel group (hybrid split, llama2_q4.cu:45-50).
 //
@@ -1528,6 +1528,15 @@ static int fused_build(q4_model* m, q4_fused* f) {
     return Q4_OK;
 }
 
+// Positions of one launch: 32 at most, and no more than about 4 ms of them, as a launch keeps every SM and another stream's kernels wait for its end. (A
+// position takes about 8 us per layer beside its bytes at 5 TB/s: four 7B layers 123 us, measured 130; 7B 0.98 ms, 1.05; two 70B layers 0.20, 0.20. So four
+// positions of 7B, two of 13B, one of 70B; what a launch saves, some 8 us per position, is next to nothing there.) Tags have 16 bits.
+static int positions_at_once(double bytes, int n_layers) {
+    const double us = bytes / 5e6 + 8.0 * n_layers;
+    return std::max(1, std::min(std::min(32, (int)(4000.0 / us)), 32768 / (1 + kLayerPhases * n_layers + 2)));
+}
+int q4_fused_positions_at_once(const q4_model* m, int pos) { return positions_at_once(q4_model_token_bytes(m, pos), m->cfg.n_layers); }
+
 int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff, int n_tokens) {
     q4_fused* f = m->fused;
     if (!f || f->unsupported) return Q4_ERR_UNSUPPORTED_SIZE;
@@ -1555,6 +1564,7 @@ int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff,
 }
 
 #ifdef Q4_TEST_BUILD
+extern "C" int q4_test_positions_at_once(double bytes, int n_layers) { return positions_at_once(bytes, n_layers); }
 // Test build only: the fused path's W4 dot product (staging to block fixed point, product) on a caller's activation
 // vector, outside the token kernel, so that tests can feed it vectors the model never produces on its own (outliers, empty
 // groups, subnormals, the largest fp16 values). One CTA per 8-column tile; plain loads, not tuned.

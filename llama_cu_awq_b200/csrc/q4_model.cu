@@ -619,10 +619,10 @@ extern "C" int q4_generate(q4_model* m, const int* prompt_tokens, int n_prompt, 
         e = Q4_OK;
     }
     // A prompt's ids are all known, so the fused kernel takes many positions in one launch (48 positions of four 7B layers 6880 us one by one,
-    // 6470 so); 32 at most, so that other streams get their turn. As the loop below does, it ends behind an end token that is not the first.
+    // 6470 so). As the loop below does, it ends behind an end token that is not the first.
     bool ended = false;
-    const int many = path == 2 && m->g == 1 ? std::min(32, 32768 / (5 * m->cfg.n_layers + 3)) : 1;     // (tags have 16 bits)
-    while (many > 1 && !ended) {
+    while (path == 2 && m->g == 1 && !ended) {
+        const int many = q4_fused_positions_at_once(m, pos);
         const int upto = std::min(std::min(n_prompt, steps), pos + many);
         int n = 0;
         while (pos + n < upto && !ended && m->host_pos + n < std::min(m->cfg.seq_len, Q4_MAX_SEQ_LEN - 1)) {

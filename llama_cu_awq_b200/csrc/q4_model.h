@@ -59,6 +59,7 @@ int q4_attention_launch(cudaStream_t s, uint16_t* output, const uint16_t* q, con
 // q4_fused.cu
 int q4_fused_prepare(q4_model* m);                              // builds the stream-layout weights and the phase table (lazy)
 int q4_fused_forward(q4_model* m, cudaStream_t s, int gen_token, int no_handoff, int n_tokens = 1);   // n_tokens positions in a row (more than one: one GPU only); logits and hand-off are the last one's
+int q4_fused_positions_at_once(const q4_model* m, int pos);      // how many positions from pos on a launch of several takes at most
 void q4_fused_reset(q4_model* m, bool clean = false);           // re-arms barrier counters (after q4_model_reset); clean: the status is known to be zero
 const int* q4_fused_status_word(const q4_model* m);             // on the device; null where nothing can have been recorded
 void q4_fused_free(q4_model* m);

@@ -354,8 +354,9 @@ def test_many_positions_in_one_launch_with_the_far_table():
 
 
 @pytest.mark.parametrize("cfg", [(512, 768, 1, 4, 2, 512, 96, 10000.0),            # one layer: no step between the embedding and the last layer's first
-                                 (5120, 1024, 1, 40, 8, 512, 96, 10000.0)])        # two CTAs embed
-def test_many_positions_of_one_layer_in_one_launch(cfg):
+                                 (5120, 1024, 1, 40, 8, 512, 96, 10000.0),         # two CTAs embed
+                                 (256, 512, 70, 2, 2, 512, 96, 10000.0)])          # so many layers that a launch takes seven positions
+def test_many_positions_in_one_launch_by_layers_and_width(cfg):
     """The next position's id is fetched while this one's may still be read: the bits of one launch per position, ids that all differ."""
     tokens = np.random.default_rng(13).permutation(np.arange(3, 512, dtype=np.int32))[:70]
     t = Transformer(None, synthetic=(cfg, 7))
