@@ -130,7 +130,8 @@ struct FParams {
     int write_token;
     int no_handoff;              // 1: leave the token mailbox and the last position's step alone (a sampling kernel follows on the stream)
     int debug;                   // test build only (Q4_TEST_BUILD; always 0 and compiled out of the product library):
-                                 // 1 = consumers skip the waits and the math (pure streaming), 16 = tensor-parallel exchange kept local (no NVLink dependency)
+                                 // 1 = consumers skip the waits and the math (pure streaming), 2 = the positions behind a launch's first embed
+                                 // nothing, so that their readers' waits run out, 16 = tensor-parallel exchange kept local (no NVLink dependency)
     unsigned long long wait_ns;  // limit of every device-side wait on the global timer; on expiry the kernel records Q4_ERR_TIMEOUT
     int depth;                   // ring chunks per warp
     int split_len;               // positions per attention split (a head is split in ceil(T / split_len) parts, at most nsplit)
@@ -637,7 +638,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_token_kernel(const __grid_c
     TRACE(0, 0);
     int rot = 0;
     const int word = cta * kThreads + tid;
-    if (word < p.dim / 8) {
+    if (word < p.dim / 8 && !(kMany && (Q4_DBG(p) & 2) && more < n_tokens - 1)) {
         const int token = more == n_tokens - 1 ? p.tokens_pinned[pos] : next_id[more & 1];
         const uint4 v = reinterpret_cast<const uint4*>(p.emb + (size_t)token * p.dim)[word];
         const uint32_t tg = tag_of(tag0, 0);

@@ -368,3 +368,27 @@ def test_many_positions_in_one_launch_by_layers_and_width(cfg):
             assert (t.logits().view(np.uint16) == want.view(np.uint16)).all(), n
     assert t.status() == 0
     t.close()
+
+
+def test_a_wait_of_several_positions_in_one_launch_runs_out():
+    """Positions behind a launch's first whose embedding nobody writes (test switch): the waits for it end after the shortened limit, the launch ends, the
+    time-out is reported, and the next generation, which re-arms the path, has the bits of the one before."""
+    L = _lib.test_lib()
+    cfg = (1024, 2816, 2, 8, 2, 2048, 64, 10000.0)
+    tokens = np.random.default_rng(14).integers(3, 2048, size=40, dtype=np.int32)
+    t = Transformer(None, lib=L, synthetic=(cfg, 8))
+    assert t.best_path() == 2
+    t.set_wait_limit_ns(20_000_000)   # 20 ms instead of 2 s
+    try:
+        t.generate(tokens, 40, path=2)
+        assert t.status() == 0
+        want = t.logits().view(np.uint16).copy()
+        L.q4_test_set_fused_debug(2)
+        _, _, seconds = t.generate(tokens, 32, path=2)
+        assert t.status() == _lib.Q4_ERR_TIMEOUT and seconds < 1.0
+        L.q4_test_set_fused_debug(0)
+        t.generate(tokens, 40, path=2)
+        assert t.status() == 0 and (t.logits().view(np.uint16) == want).all()
+    finally:
+        L.q4_test_set_fused_debug(0)
+        t.close()

@@ -214,9 +214,16 @@ def test_matvec_small_inputs_beside_large_ones(K, N, ratio, large):
     check_against_64_bits(y.cpu().numpy(), q, x, K, N, f"{K}x{N}, 1 : {ratio:g}")
 
 
+@pytest.mark.parametrize("large", [(64,), (1, 2, 3, 4, 5, 6, 7, 8, 9)])
+@pytest.mark.parametrize("K,N", [(2040, 19608), (8192, 2072), (13824, 640), (16640, 1192)])
+def test_streamed_small_inputs_beside_large_ones(K, N, large):
+    """The same in the stream form: no pairs of a warp's own, two, three, four and some left over."""
+    test_matvec_small_inputs_beside_large_ones(K, N, 5000.0, large)
+
+
 def test_products_of_several_matrices_with_small_inputs_beside_large_ones():
-    """q|k|v and gate/up with several tiles per stage and several chunks, the accumulating form with several chunks."""
-    for K, N, Nkv in [(384, 2368, 2368), (5000, 1024, 256)]:
+    """q|k|v, gate/up and the accumulating form: fewer pairs than warps, some left over, and the stream form with matrices that end inside a CTA's tiles."""
+    for K, N, Nkv in [(384, 2368, 2368), (5000, 1024, 256), (4104, 4952, 4952)]:
         rng = np.random.default_rng(K)
         x = (rng.standard_normal(K) * 0.01).astype(np.float16)
         ks = list(range(5, K, 128))
@@ -299,10 +306,10 @@ def test_matvec_small_inputs_beside_many_held_ones(held):
     check_against_64_bits(y.cpu().numpy(), q, x, K, N, f"{held} held")
 
 
+@pytest.mark.parametrize("K,N", [(512, 64), (4104, 9800), (16640, 1192)])      # direct; stream with a last group of eight inputs; four pairs and some left
 @pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
-def test_matvec_non_finite_inputs(value):
+def test_matvec_non_finite_inputs(value, K, N):
     """A NaN in x makes every output NaN, an infinity makes it infinite with the weight's sign, or NaN where the weight is zero."""
-    K, N = 512, 64
     q, x, _ = mk(K, N, seed=3)
     x[300] = value
     x[37] = value                       # an odd position of another group
@@ -315,9 +322,9 @@ def test_matvec_non_finite_inputs(value):
     assert np.array_equal(y.float().cpu().numpy(), want, equal_nan=True)
 
 
-def test_matvec_opposite_infinities():
+@pytest.mark.parametrize("K,N", [(512, 128), (4104, 9800)])
+def test_matvec_opposite_infinities(K, N):
     """Infinities of both signs in one group, and of one sign in two groups: what IEEE sums of the products give."""
-    K, N = 512, 128
     q, x, _ = mk(K, N, seed=8)
     x[[130, 201]] = np.inf, -np.inf
     x[[3, 400]] = np.inf
