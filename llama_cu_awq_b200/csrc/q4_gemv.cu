@@ -15,8 +15,8 @@
 // through a private ring in shared memory (cp.async by the lanes that read it: no barrier between warps) and about 50 instructions; pairs that
 // do not divide by 16 warps are dealt out by items (20 pairs of a 5120-long row: 1.25 a warp; whole ones would be two for some). Scales and
 // zero points of a pass of tiles lie in shared memory as the product takes them, brought once for all warps: as copies of their own in the ring they
-// were half as many requests again as the words (8192 x 8192 10.1 us; 8.2 without). What bounds it: 1.5 us of start (x, scales and the staging behind the
-// wait) and the stream, 6.4 TB/s at 47 MB; 60 % of the issue slots.
+// were half as many requests again as the words (8192 x 8192 10.1 us; 8.2 without). What bounds it: 2.5 us of start and end (x, scales and the staging behind
+// the wait; the sums) and the stream, 5.4 to 5.9 TB/s (2 x 23.4, 2 x 122 MB beyond 23 and 47); 60 % of the issue slots.
 //
 // Under programmatic dependent launch the next product's packed words are requested while this one drains (weights never depend on
 // activations). Back to back on weights from HBM, bulk copies into a ring shared by a CTA's warps (before) and now, us: 4096 x 4096 4.2 (direct, both);
@@ -173,29 +173,29 @@ __device__ __noinline__ void add_small(const GemvParams& p, float* part, int par
 // The warps' sums in warp order and the outputs of `tiles` tiles; 16 warps. Thread 8 * tile + column.
 template <bool SILU>
 __device__ __forceinline__ void write_out(const GemvParams& p, const float* part, int tile0, int tiles, int w, int lane) {
-            for (int e0 = w * 32; e0 < tiles * kRows; e0 += kThreads) {
-                const int e = e0 + lane;
-                const bool on = e < tiles * kRows;
-                float sum = 0.f;
-                if (on) {
-                    const float* q = part + (e >> 3) * kTileStride + (e & 7);
-                    float v[4];
-    #pragma unroll
-                    for (int i = 0; i < 4; i++) v[i] = ((q[i * 32] + q[i * 32 + 8]) + q[i * 32 + 16]) + q[i * 32 + 24];
-                    sum = ((v[0] + v[1]) + v[2]) + v[3];
-                }
-                int row;
-                const GemvMat& m = row_of<SILU>(p, tile0 + (on ? e >> 3 : 0), e & 7, row);
-                if (SILU) {
-                    const float up = __shfl_xor_sync(0xffffffffu, sum, 1);
-                    if (on && !(e & 1)) p.m[0].out[row] = __float2half(silu_mul(sum, up));
-                } else if (on) {
-                    __half* out = m.out;
-                    if (m.kv) out += p.loff + (long long)(*p.pos) * m.n;
-                    if (p.accum) sum += __half2float(out[row]) / p.gpu_count;
-                    out[row] = __float2half(sum);
-                }
-            }
+    for (int e0 = w * 32; e0 < tiles * kRows; e0 += kThreads) {
+        const int e = e0 + lane;
+        const bool on = e < tiles * kRows;
+        float sum = 0.f;
+        if (on) {
+            const float* q = part + (e >> 3) * kTileStride + (e & 7);
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = ((q[i * 32] + q[i * 32 + 8]) + q[i * 32 + 16]) + q[i * 32 + 24];
+            sum = ((v[0] + v[1]) + v[2]) + v[3];
+        }
+        int row;
+        const GemvMat& m = row_of<SILU>(p, tile0 + (on ? e >> 3 : 0), e & 7, row);
+        if (SILU) {
+            const float up = __shfl_xor_sync(0xffffffffu, sum, 1);
+            if (on && !(e & 1)) p.m[0].out[row] = __float2half(silu_mul(sum, up));
+        } else if (on) {
+            __half* out = m.out;
+            if (m.kv) out += p.loff + (long long)(*p.pos) * m.n;
+            if (p.accum) sum += __half2float(out[row]) / p.gpu_count;
+            out[row] = __float2half(sum);
+        }
+    }
 }
 
 template <bool SILU>
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4_gemv_kernel(const __grid_const
 }
 
 namespace stream {
-// Pairs that a warp keeps: its digits take ten registers each (5 instead of 4: 28672 -> 8192 30.8 us, 29.8; 7 spill, 33.5).
+// Pairs that a warp keeps: its digits take ten registers each (5 instead of 4: 28672 -> 8192 30.8 us, 29.8; 7 spill dozens, 33.5; gate/up with 4 spills one, once).
 constexpr int kMaxOwn = 4;
 constexpr int kItemBytes = 1024;
 constexpr int kPassTiles = 28;       // tiles per pass at most (their partial sums are in shared memory)

@@ -19,14 +19,14 @@
 // fp32 tile is scaled by the group's fp16 scale in fp32, as the reference does (gpu_kernels.h:222-228), so weights
 // are never rounded to fp16 after scaling.
 //
-//
 // Stream: a CTA of 16 warps per SM has consecutive tiles of 16 features. Each warp keeps the x fragments of its own groups (two with up to
 // eight rows, one with more) in registers for all of them, and the items of the groups that are left are dealt out over the warps tile by
 // tile; an item (16 features over a group, 1 KB) comes through the warp's private ring of four (cp.async; a lane reads what it has copied
 // itself, so that no barrier is needed), the first ones ahead of griddepcontrol.wait. Scales and zero points of a pass of tiles lie in shared
-// memory, one word for both. The warps' partial tiles wait there for one sum at the end of the pass. What bounds it: the unpack and the products (150 clocks of a scheduler per item where nothing else runs, about 220 here; HBM's
-// rate is 200) and, with few tiles, the start: x of all rows goes to every SM, 64 KB with 8 rows of 4096. gate/up of 7B, 8 rows 13.6 us = 3.5 TB/s
-// (17.0 sliced), 8192 -> 10240 15.3 = 2.9 (22.5), 70B gate/up 64.5 = 3.9 (77.4).
+// memory, one word for both. The warps' partial tiles wait there for one sum at the end of the pass. What bounds it: the unpack and the products
+// (150 clocks of a scheduler per item where nothing else runs, about 220 here; HBM's rate is 200) and, with few tiles, the start: x of all rows goes
+// to every SM, 64 KB with 8 rows of 4096. Back to back from HBM, 8 rows: gate/up of 7B 13.0 us = 3.6 TB/s (16.4 sliced), 8192 -> 10240 15.2 = 2.9 (22.0),
+// 70B gate/up 64.3 = 3.8 (77.9).
 //
 // Epilogues: plain, residual (y = product + residual * scale: matmul(QWeight)'s accum form, gpu_kernels.h:237-238),
 // and SiLU (ffn_matvec_silu_kernel, gpu_kernels.h:251-283: the CTA holds 16 gate and the same 16 up features and writes
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(stream::kThreads, 1) q4_rows_stream_kernel(con
     open_pass();
     for (int i = 0; i < kDepth; i++) request(i * kItemBytes);
     // A pass's scales and zero points into shared memory, several of a thread in flight.
-    constexpr int kFlight = NT == 2 ? 4 : 8;     // (registers)
+    constexpr int kFlight = NT == 2 ? 4 : 8;     // (registers: the form for more than eight rows spills three to five of them once)
     struct Meta {
         __half s[kFlight];
         uint32_t z[kFlight];
@@ -713,14 +713,17 @@ int launch_deal(const SkParams& p, int units, cudaStream_t s) {
 }
 
 // Whether a warp keeps its share of every unit: where shares that go round make no warp's load lighter, a barrier per unit and one unit's
-// sum at a time are cheaper than cursors that move and a sum of several units at the end (us, fixed against going round).
-//   9 to 16 rows, equal shares of one group or an even number: 7B q|k|v 14.9, 15.3; gate/up 24.4, 24.9; 1024 -> 2 x 20000 13.3, 14.3;
-//   6144 -> 2 x 11008 34.2, 36.0; 8192 -> 2 x 28672 the same. With shares of three or five groups going round is the
-//   faster one all the same (13B q|k|v 35.6, 34.3; o 15.1, 14.8).
-//   9 to 16 rows, one unit per CTA: 7B o 5.6, 5.8. (With up to 8 rows 4.5, 4.6 too, but there q|k|v goes round, and launches that take turns
-//   with those of another kernel start more slowly than they gain: eight sequences, 32 steps of four 7B layers 7350 us, 7190 with one.)
-//   Gate/up with two units per CTA whose heaviest pair of neighbouring shares is two heaviest ones: 8 rows, 4096 -> 2 x 4096 7.3, 7.6; with
-//   very long shares the barrier costs more (8 rows, 28672 -> 8192 in two units 42.0, 41.6).
+// sum at a time are cheaper than cursors that move and a sum of several units at the end (us from HBM, fixed against going round, on shapes that
+// streamed() leaves to this form).
+//   9 to 16 rows, equal shares of one group or an even number: 4096 -> 8192 9.5, 10.1 (9 rows), 10.0, 10.2 (16); 6144 -> 8192 13.6, 14.3 and 14.2, 14.6;
+//   4096 -> 2 x 4096 9.4, 10.1 and 10.0, 10.5; 1024 -> 2 x 20000 11.9, 13.1 and 13.0, 13.9. With shares of three or five groups the two are close, and
+//   going round wins with 16 rows of long launches (3072 -> 12288 11.4, 11.5 and 12.2, 11.7); with unequal ones it wins clearly (2560 -> 3 x 2560 7.3,
+//   6.7 and 7.9, 6.9).
+//   9 to 16 rows, one unit per CTA: 7B o 5.3, 5.6 and 5.6, 5.8; the step of nine sequences (32 steps of four 7B layers) 8985 us, 9055 going round. With up to
+//   8 rows 4.4, 4.6 alone, but there the step, whose launches take turns with the stream form's, says the opposite: eight sequences 7015 us, 6835 going
+//   round; one 6530, 6330.
+//   Gate/up with two units per CTA whose heaviest pair of neighbouring shares is two heaviest ones: 8 rows, 4096 -> 2 x 4096 7.2, 7.6; 7168 -> 2 x 4096
+//   11.3, 11.6 (and 5120 -> 2 x 4096, where it is not, 9.0, 8.6). With very long shares the barrier costs more (28672 -> 8192 in two units 42.0, 41.6).
 bool fixed_shares(int G, int warps, int NT, bool silu, int per_cta) {
     if (NT == 2 && per_cta == 1) return true;
     if (NT == 2 && G % warps == 0) return G == warps || G / warps % 2 == 0;
@@ -760,11 +763,12 @@ int launch_stream(const SkParams& p, cudaStream_t s) {
 }
 
 // The stream form where an SM has three or more of the tiles of 16 rows (gate/up: eight of each) and rows are 4096 inputs or longer; from
-// seven tiles also from 2048 inputs. us, sliced and stream, 8 rows and 16: 7B gate/up 17.0, 13.6 and 24.6, 21.8; q|k|v 10.3, 9.4 and 15.0, 13.3;
-// 13B q|k|v 20.1, 13.3 and 34.2, 18.6; gate/up 23.4, 19.2 and 36.1, 29.7; 13824 -> 5120 21.5, 17.1 and 34.7, 23.3; 70B gate/up 77.4, 64.5 and 120,
-// 89; 8192 -> 10240 22.5, 15.3 and 36.1, 20.8; 2048 -> 16384 9.9, 7.8 and 14.7, 9.8. Below, the sliced form's shorter start wins: two tiles 7B o 4.7,
-// 5.5 and 5.7, 8.0; 11008 -> 4096 9.5, 11.4 and 12.8, 16.7; 2048 -> 3 x 4096 6.0, 6.8 and 8.2, 8.6. Four tiles (445 to 592 in all) are two even rounds of
-// the sliced form's pairs, which keeps up then: 4096 -> 3 x 3072 8.1, 8.2 and 10.6, 11.5; 8192 x 8192 13.4, 13.5 and 19.6, 18.1.
+// seven tiles also from 2048 inputs. us back to back from HBM, sliced and stream, 8 rows and 16: 7B gate/up 16.4, 13.0 and 23.1, 22.3; q|k|v 10.1, 9.3 and
+// 14.3, 13.4; 13B q|k|v 20.2, 13.3 and 31.5, 18.7; gate/up 23.2, 18.9 and 36.1, 30.8; 13824 -> 5120 21.6, 17.4 and 35.3, 23.0; 70B gate/up 77.9, 64.3 and
+// 120, 94; 8192 -> 10240 22.0, 15.2 and 36.6, 20.6; 2048 -> 16384 9.8, 7.6 and 14.7, 9.3 (16640, whose pairs of tiles divide better 7.6, 7.7 and 10.4, 9.5).
+// Below, the sliced form's shorter start wins: two tiles 7B o 4.7, 5.5 and 5.6, 7.6; 11008 -> 4096 9.5, 11.5 and 12.7, 15.8; 2048 -> 3 x 4096 5.9, 6.7 and
+// 8.1, 8.1. Four tiles (445 to 592 in all) are two even rounds of the sliced form's pairs, which keeps up then: 4096 -> 3 x 3072 7.9, 8.3 and 10.3, 10.9;
+// 8192 x 8192 13.1, 13.0 and 19.4, 17.4 (8 rows on words in L2 12.0, 12.3).
 bool streamed(int G, int tiles) {
     const int most = q4_div_up(tiles, kSms);
     if (stream::tiles_in_pass(G, 2) == 0) return false;
