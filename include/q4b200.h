@@ -148,8 +148,8 @@ int q4_matmul_q4_batched_status(void* stream, const void* workspace);
 
 /* The same products for a handful of rows (1 <= M <= 16): the projections of batched decode, where every sequence adds one
  * row and the weights are still read once per step. HBM-bound like the batch-1 kernels they widen (mat_vec_kernel_int4,
- * qkv_matvec_kernel, ffn_matvec_silu_kernel: gpu_kernels.h:179-283), so no tcgen05 tiles here: packed words straight from
- * global memory into mma.sync fragments, fp32 accumulation, group scale applied in fp32, no workspace, results
+ * qkv_matvec_kernel, ffn_matvec_silu_kernel: gpu_kernels.h:179-283), so no tcgen05 tiles here: packed words into mma.sync
+ * fragments as they lie in the file (large products bring them through shared memory), fp32 accumulation, group scale applied in fp32, no workspace, results
  * bit-reproducible. x is [M][inpSize], every y [M][its opSize], row-major fp16; inpSize a multiple of 128.
  *   q4_matmul_q4_rows : y = x * deq(w) [+ residual * residual_scale when residual is not NULL; residual may be y]; opSize % 16 == 0
  *   q4_qkv_matmul_rows: q, k, v from one read of x (opSize, kvSize multiples of 32)
