@@ -589,7 +589,7 @@ int launch_stream(GemvParams& p, cudaStream_t s) {
 
 // The stream form from 20 MB of packed words up, and from rows of 32 pairs on below that (bytes * pairs of a row >= 180 MB). The direct form starts about
 // a microsecond earlier, which a call on words that are in L2 already (one matrix again and again) shows most; a model's come from HBM. The line lies where
-// what one side loses is what the other gains. us, direct and stream, from HBM; from L2: 1024 x 24000 5.4, 5.5; 4.2, 5.3. 2048 x 9216 4.6, 4.9; 3.8, 4.8.
+// what one side loses is what the other gains (two layers of 13B call by call, whose o is 13 MB: 129.4 us, 128.3 in the stream form). us, direct and stream, from HBM; from L2: 1024 x 24000 5.4, 5.5; 4.2, 5.3. 2048 x 9216 4.6, 4.9; 3.8, 4.8.
 // 4096 x 4608 4.5, 4.5; 3.6, 4.4. 5120 x 5120 6.6, 6.1; 4.9, 6.0. 4096 x 8192 6.9, 6.1; 4.7, 5.8. 4096 x 10240 (21 MB) 8.1, 6.6; 5.5, 6.3.
 // 8192 x 2048 4.9, 4.5; 4.3, 4.5. 8192 x 4096 7.6, 6.1; 5.6, 5.8. 12288 x 1024 4.9, 4.5; 4.7, 4.5. 13824 x 640 5.4, 4.9; 5.1, 4.9. 28672 x 512 9.6, 7.8;
 // 8.3, 8.0. Ratio over the range (3 to 28 MB), L2 and HBM: 4 to 12 pairs 1.2, 1.1 at 9 MB, 1.2, 0.9 at 18, 1.14, 0.85 at 22; 16 to 28 pairs 1.2, 0.9 at 16, 1.1,
